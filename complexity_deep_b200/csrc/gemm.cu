@@ -291,6 +291,11 @@ ClusterSplitPlan plan_cluster_split(int M, int N, int kb64, int unsplit_bn, int 
 
 }  // namespace
 
+// gemm_few_rows.cu
+bool few_rows_taken(int M, int num_groups, bool second, int kind, int cols, int K, int sm_count);
+cudaError_t launch_few_rows(const GemmParams& g, int kind, const GemmOperand& op0, const GemmOperand* op1, const GemmSecond* second,
+                            int block_n, int sm_count, cudaStream_t stream);
+
 bool encode_map_2d(void* map_out, const void* base, long long rows, long long cols, long long ld,
                    int box_rows) {
   return make_map(static_cast<CUtensorMap*>(map_out), base, rows, cols, ld, box_rows);
@@ -430,39 +435,6 @@ int launch_gemm(int M, int N, int num_groups, const int* seg_offsets, const Gemm
   DeviceInfo* di = device_info(&st);
   if (!di) return st;
 
-  // dense store-epilogue calls of few rows may take the cluster form of split-K (128-wide tiles)
-  int csk_splits = 1;
-  if (num_groups == 1 && !second && (epi.kind == kEpiStore || epi.kind == kEpiStoreF32) && !epi.rope_cos && !epi.selftest_stall &&
-      !epi.out_row_ptrs && block_n <= 128 && choose_cta_group(M, 128, di->sm_count) == 1) {
-    const int kb64 = (op0.K + kBoxK - 1) / kBoxK + (op1 ? (op1->K + kBoxK - 1) / kBoxK : 0);
-    csk_splits = plan_cluster_split(M, N, kb64, block_n, di->sm_count).splits;
-    if (csk_splits > 1) block_n = 128;
-  }
-  const int cg = choose_cta_group(M, block_n, di->sm_count);
-  const int b_box = block_n / cg;
-  CUtensorMap a0, b0, a1, b1;
-  if (!make_map(&a0, op0.a, M, op0.K, op0.lda, kBlockM) ||
-      !make_map(&b0, op0.b, op0.b_rows, op0.K, op0.ldb, b_box)) {
-    snprintf(g_cuda_err, sizeof(g_cuda_err), "cuTensorMapEncodeTiled failed (operand 0)");
-    return CD_ERR_CUDA;
-  }
-  if (op1) {
-    if (!make_map(&a1, op1->a, M, op1->K, op1->lda, kBlockM) ||
-        !make_map(&b1, op1->b, op1->b_rows, op1->K, op1->ldb, b_box)) {
-      snprintf(g_cuda_err, sizeof(g_cuda_err), "cuTensorMapEncodeTiled failed (operand 1)");
-      return CD_ERR_CUDA;
-    }
-  } else if (second) {
-    a1 = a0;
-    if (!make_map(&b1, second->b, second->n_rows, op0.K, second->ldb, b_box)) {
-      snprintf(g_cuda_err, sizeof(g_cuda_err), "cuTensorMapEncodeTiled failed (second problem)");
-      return CD_ERR_CUDA;
-    }
-  } else {
-    a1 = a0;
-    b1 = b0;
-  }
-
   GemmParams p;
   memset(&p, 0, sizeof(p));
   p.M = M;
@@ -521,6 +493,47 @@ int launch_gemm(int M, int N, int num_groups, const int* seg_offsets, const Gemm
   p.wait_limit_ns = epi.wait_limit_ns;
   p.status = di->status;
 
+  const int kind = epi.rope_cos ? static_cast<int>(kEpiStoreRope)
+                   : (epi.out_lo || epi.residual_lo) ? static_cast<int>(kEpiStoreSplit) : epi.kind;
+  if (kind != kEpiStoreRope && !epi.selftest_stall &&
+      few_rows_taken(M, num_groups, second != nullptr, kind, epi.out_cols, op0.K + (op1 ? op1->K : 0), di->sm_count)) {
+    cudaError_t e = launch_few_rows(p, kind, op0, op1, second, block_n, di->sm_count, stream);
+    return e == cudaSuccess ? CD_OK : cuda_fail(e, "few-row gemm launch");
+  }
+
+  // dense store-epilogue calls of few rows may take the cluster form of split-K (128-wide tiles)
+  int csk_splits = 1;
+  if (num_groups == 1 && !second && (epi.kind == kEpiStore || epi.kind == kEpiStoreF32) && !epi.rope_cos && !epi.selftest_stall &&
+      !epi.out_row_ptrs && block_n <= 128 && choose_cta_group(M, 128, di->sm_count) == 1) {
+    const int kb64 = (op0.K + kBoxK - 1) / kBoxK + (op1 ? (op1->K + kBoxK - 1) / kBoxK : 0);
+    csk_splits = plan_cluster_split(M, N, kb64, block_n, di->sm_count).splits;
+    if (csk_splits > 1) block_n = 128;
+  }
+  const int cg = choose_cta_group(M, block_n, di->sm_count);
+  const int b_box = block_n / cg;
+  CUtensorMap a0, b0, a1, b1;
+  if (!make_map(&a0, op0.a, M, op0.K, op0.lda, kBlockM) ||
+      !make_map(&b0, op0.b, op0.b_rows, op0.K, op0.ldb, b_box)) {
+    snprintf(g_cuda_err, sizeof(g_cuda_err), "cuTensorMapEncodeTiled failed (operand 0)");
+    return CD_ERR_CUDA;
+  }
+  if (op1) {
+    if (!make_map(&a1, op1->a, M, op1->K, op1->lda, kBlockM) ||
+        !make_map(&b1, op1->b, op1->b_rows, op1->K, op1->ldb, b_box)) {
+      snprintf(g_cuda_err, sizeof(g_cuda_err), "cuTensorMapEncodeTiled failed (operand 1)");
+      return CD_ERR_CUDA;
+    }
+  } else if (second) {
+    a1 = a0;
+    if (!make_map(&b1, second->b, second->n_rows, op0.K, second->ldb, b_box)) {
+      snprintf(g_cuda_err, sizeof(g_cuda_err), "cuTensorMapEncodeTiled failed (second problem)");
+      return CD_ERR_CUDA;
+    }
+  } else {
+    a1 = a0;
+    b1 = b0;
+  }
+
   // Upper bound of the tile count without reading the segment sizes (they live on the
   // device): every group adds at most one partial m-tile.
   const int tile_m = kBlockM * cg;
@@ -553,8 +566,6 @@ int launch_gemm(int M, int N, int num_groups, const int* seg_offsets, const Gemm
 
   cudaError_t e;
   std::lock_guard<std::mutex> lk(g_mu);
-  const int kind = epi.rope_cos ? static_cast<int>(kEpiStoreRope)
-                   : (epi.out_lo || epi.residual_lo) ? static_cast<int>(kEpiStoreSplit) : epi.kind;
   e = (cg == 2) ? launch_any<2>(block_n, kind, grid, a0, b0, a1, b1, p, *di, stream)
                 : launch_any<1>(block_n, kind, grid, a0, b0, a1, b1, p, *di, stream);
   if (e != cudaSuccess) return cuda_fail(e, "gemm launch");

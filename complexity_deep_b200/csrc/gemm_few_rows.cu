@@ -1,0 +1,426 @@
+// Matrix products of few rows (decode steps, short prompts): out[r, n] = epilogue(sum_k A[r, k] W[n, k]).
+//
+// Such a call is a read of the weights: 2 bytes per weight against at most 64 rows of work. The tile kernel
+// (gemm_sm100.cuh) runs it as chains of 128-row tensor-core tiles with barriers, tensor memory and an
+// issuing thread between them: 4.9 us before its first result and 0.21 us per 64 elements of K, whatever the
+// rows. Here a block takes 16 (or 32) weight rows and its eight warps a share of K each; weights and rows go
+// from global memory straight into the fragments of m16n8k16 products (weights as the 16-row operand, tokens
+// as the 8-column one), with no staging and no barrier before the one at which the warps' partial sums meet.
+//   * K is permuted inside a step of 32 so that a lane's 16-byte load is two steps' worth of one row: both
+//     operands use the same permutation, and the four lanes of a row read 64 consecutive bytes.
+//   * A block asks for its weights in L2 BEFORE it waits for the kernel ahead of it. A prefetch reads nothing into
+//     the program, so it may run ahead of whatever still writes; it takes the DRAM latency out of the step.
+//   * The partial sums are added in the order of the warps: results do not depend on timing.
+//   * Once it has started, a block asks for the weights of the block that will follow it on the SM.
+// Row groups (experts) are walked in passes of at most 32 rows of one group; empty groups end at once.
+// Bound by: L2 to SM traffic (weights once, the rows once per block: 7 to 9 TB/s) from 16 rows on, before that by
+// the launch (2.1 us at K = N = 768, one row; the tile kernel 6.8). The other figures stand at few_rows_taken.
+#include <cuda_bf16.h>
+#include "../../include/cdeep.h"
+#include "checks.cuh"
+#include "elem.cuh"
+#include "gemm_sm100.cuh"
+#include "kernels.h"
+#include "mma.cuh"
+
+namespace cdeep {
+namespace {
+
+constexpr int kStep = 32;          // elements of K per step: one 16-byte load per lane and row
+
+struct FewParams {
+  GemmParams g;                    // shapes and epilogue, as the tile kernel takes them
+  const bf16 *a0, *b0, *a1, *b1;   // a1 / b1: second K segment, or b1 the second problem's weights
+  long long lda0, ldb0, lda1, ldb1;
+  int half;                        // gated units: rows of a gate block, up rows follow (packed layout)
+  int tiles, tiles2;               // blocks per group, of the second problem
+  int prefetch;                    // ask for the block's own weights ahead of the kernel before
+  int ahead;                       // blocks on the device at a time
+};
+
+__device__ __forceinline__ uint4 load_stream(const bf16* p) {
+  uint4 v;
+  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ void prefetch_row(const void* p, uint32_t bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+}
+
+struct Weights {                   // of the block's group, one matrix per K segment
+  const bf16 *b0, *b1;
+  long long ld0, ld1;
+};
+
+template <int MT>
+constexpr int kRowFloats = 16 * MT + 4;                    // partial sums of a token: the accumulators' writes hit 32 banks
+
+// One pass: the block's weight rows against the tokens [m0, m0 + 8 NT) of a group that ends at m_end.
+template <int EPI, int MT, int NT, int WK>
+__device__ __forceinline__ void few_pass(const FewParams& p, float* red, const Weights& wt, const int (&w_row)[MT][2], int n_steps0,
+                                         int n_steps, int m0, int m_end, int col0, bool second) {
+  constexpr bool kGated = EPI == kEpiSwiGLU || EPI == kEpiGlu;
+  constexpr bool kSplit = EPI == kEpiStoreSplit;
+  constexpr bool kF32 = EPI == kEpiStoreF32;
+  constexpr int kRow = kRowFloats<MT>;
+  constexpr int kU = MT * 2 * 4 <= 8 ? 4 : 2;              // steps of weights in flight
+  constexpr int kAhead = NT >= 6 ? 1 : 2;                  // steps of tokens in flight
+  const GemmParams& g = p.g;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q8 = (lane & 3) * 8;
+
+  // what the epilogue reads, ahead of the products
+  constexpr int kQuads = 4 * (kGated ? 1 : MT);            // outputs of a token in fours
+  constexpr int kItems = (8 * NT * kQuads + (WK * 32) - 1) / (WK * 32);
+  const int out_cols = second ? g.out_cols2 : g.out_cols;
+  long long at[kItems];                                    // destination row, -1: nothing to store
+  uint2 hi[kItems], lo[kItems], r2[kItems];
+  float4 rf[kItems];
+#pragma unroll
+  for (int i = 0; i < kItems; ++i) {
+    const int item = threadIdx.x + i * (WK * 32);
+    const int r = m0 + item / kQuads, col = col0 + (item % kQuads) * 4;
+    at[i] = -1;
+    hi[i] = lo[i] = r2[i] = make_uint2(0, 0);
+    rf[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (item >= 8 * NT * kQuads || r >= m_end || col >= out_cols) continue;
+    if constexpr (kGated) {
+      at[i] = r;
+    } else {
+      if (!kF32 && !kSplit && g.out_row_ptrs) {
+        const long long addr = g.out_row_ptrs[r];
+        if (row_address_ok(addr, g.status)) at[i] = addr;
+        continue;
+      }
+      const int o = g.row_map ? g.row_map[r] : r;
+      if (kChecks && g.row_map && g.out_rows > 0 && !index_ok(o, g.out_rows, g.status)) continue;
+      at[i] = o;
+      if constexpr (kF32) {
+        if (g.residual) rf[i] = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(g.residual) + static_cast<long long>(o) * g.ldr + col);
+      } else {
+        if (g.residual) hi[i] = *reinterpret_cast<const uint2*>(g.residual + static_cast<long long>(o) * g.ldr + col);
+        if (kSplit && g.residual_lo) lo[i] = *reinterpret_cast<const uint2*>(g.residual_lo + static_cast<long long>(o) * g.ldr + col);
+        if (g.residual2) r2[i] = *reinterpret_cast<const uint2*>(g.residual2 + static_cast<long long>(r) * g.ldr2 + col);
+      }
+    }
+  }
+
+  int t_row[NT];
+#pragma unroll
+  for (int n = 0; n < NT; ++n) t_row[n] = min(m0 + n * 8 + (lane >> 2), m_end - 1);   // rows past the end are not stored
+  // this warp's steps; a lane whose 8 elements lie past K takes zeros for both operands
+  const int s_lo = warp * n_steps / WK, s_hi = (warp + 1) * n_steps / WK;
+  const uint4 zero = make_uint4(0, 0, 0, 0);
+  auto load_w = [&](int s, uint4 (&v)[MT][2]) {
+    const bool one = s >= n_steps0;
+    const int k = (one ? s - n_steps0 : s) * kStep + q8;
+    const bool in = s < s_hi && k < (one ? g.K1 : g.K0);
+    const bf16* base = (one ? wt.b1 : wt.b0) + k;
+    const long long ld = one ? wt.ld1 : wt.ld0;
+#pragma unroll
+    for (int m = 0; m < MT; ++m)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) v[m][h] = in ? load_stream(base + w_row[m][h] * ld) : zero;
+  };
+  auto load_t = [&](int s, uint4 (&v)[NT]) {
+    const bool one = s >= n_steps0;
+    const int k = (one ? s - n_steps0 : s) * kStep + q8;
+    const bool in = s < s_hi && k < (one ? g.K1 : g.K0);
+    const bf16* base = (one ? p.a1 : p.a0) + k;
+    const long long ld = one ? p.lda1 : p.lda0;
+#pragma unroll
+    for (int n = 0; n < NT; ++n) v[n] = in ? __ldg(reinterpret_cast<const uint4*>(base + t_row[n] * ld)) : zero;
+  };
+  float acc[MT][NT][4];
+#pragma unroll
+  for (int m = 0; m < MT; ++m)
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[m][n][e] = 0.f;
+  uint4 w[kU][MT][2], t[kAhead][NT];
+#pragma unroll
+  for (int u = 0; u < kU; ++u) load_w(s_lo + u, w[u]);
+#pragma unroll
+  for (int u = 0; u < kAhead; ++u) load_t(s_lo + u, t[u]);
+  for (int s = s_lo; s < s_hi; s += kU) {
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      uint4 (&tt)[NT] = t[u % kAhead];
+      uint4 (&ww)[MT][2] = w[u];
+#pragma unroll
+      for (int m = 0; m < MT; ++m) {
+        const uint32_t f0[4] = {ww[m][0].x, ww[m][1].x, ww[m][0].y, ww[m][1].y};
+        const uint32_t f1[4] = {ww[m][0].z, ww[m][1].z, ww[m][0].w, ww[m][1].w};
+#pragma unroll
+        for (int n = 0; n < NT; ++n) {
+          mma16816(acc[m][n], f0, tt[n].x, tt[n].y);
+          mma16816(acc[m][n], f1, tt[n].z, tt[n].w);
+        }
+      }
+      load_w(s + u + kU, ww);
+      load_t(s + u + kAhead, tt);
+    }
+  }
+
+  // partial sums: [warp][token][feature]
+  {
+    float* mine = red + warp * (8 * NT * kRow);
+#pragma unroll
+    for (int m = 0; m < MT; ++m)
+#pragma unroll
+      for (int n = 0; n < NT; ++n) {
+        float* row = mine + (n * 8 + (lane & 3) * 2) * kRow + m * 16 + (lane >> 2);
+        row[0] = acc[m][n][0];
+        row[kRow] = acc[m][n][1];
+        row[8] = acc[m][n][2];
+        row[kRow + 8] = acc[m][n][3];
+      }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < kItems; ++i) {
+    if (at[i] < 0) continue;
+    const int item = threadIdx.x + i * (WK * 32);
+    const int tok = item / kQuads, quad = item % kQuads, col = col0 + quad * 4;
+    float f[4] = {0.f, 0.f, 0.f, 0.f}, u[4] = {0.f, 0.f, 0.f, 0.f};
+    const float* src = red + tok * kRow + quad * 4;
+#pragma unroll
+    for (int w_ = 0; w_ < WK; ++w_) {
+      const float4 v = *reinterpret_cast<const float4*>(src + w_ * (8 * NT * kRow));
+      f[0] += v.x; f[1] += v.y; f[2] += v.z; f[3] += v.w;
+      if constexpr (kGated) {
+        const float4 x = *reinterpret_cast<const float4*>(src + 16 + w_ * (8 * NT * kRow));
+        u[0] += x.x; u[1] += x.y; u[2] += x.z; u[3] += x.w;
+      }
+    }
+    if constexpr (kF32) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) f[j] *= g.acc_scale;
+      if (g.col_scale) {
+        const uint2 c = *reinterpret_cast<const uint2*>(g.col_scale + col);
+        f[0] *= bf_lo(c.x); f[1] *= bf_hi(c.x); f[2] *= bf_lo(c.y); f[3] *= bf_hi(c.y);
+      }
+      *reinterpret_cast<float4*>(reinterpret_cast<float*>(g.out) + at[i] * g.ldo + col) =
+          make_float4(f[0] + rf[i].x, f[1] + rf[i].y, f[2] + rf[i].z, f[3] + rf[i].w);
+    } else if constexpr (kGated) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        f[j] = EPI == kEpiGlu ? clamped_glu_f(f[j], u[j], g.glu_alpha, g.glu_limit, g.glu_offset) : silu_f(f[j]) * u[j];
+      *reinterpret_cast<uint2*>((second ? g.out2 : g.out) + at[i] * (second ? g.ldo2 : g.ldo) + col) =
+          make_uint2(bf_pack(f[0], f[1]), bf_pack(f[2], f[3]));
+    } else {
+      if (!kSplit && g.act == 1) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) f[j] = fmaxf(f[j], 0.f) * fmaxf(f[j], 0.f);
+      }
+      if (g.bias) {
+        const uint2 b = *reinterpret_cast<const uint2*>(g.bias + col);
+        const float bb[4] = {bf_lo(b.x), bf_hi(b.x), bf_lo(b.y), bf_hi(b.y)};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) f[j] += fminf(fmaxf(bb[j], g.bias_lo), g.bias_hi);
+      }
+      auto add = [&](const uint2& v) { f[0] += bf_lo(v.x); f[1] += bf_hi(v.x); f[2] += bf_lo(v.y); f[3] += bf_hi(v.y); };
+      if (g.residual) add(hi[i]);
+      if (kSplit && g.residual_lo) add(lo[i]);
+      if (g.residual2) add(r2[i]);
+      if (g.do_clamp) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) f[j] = fminf(fmaxf(f[j], g.clamp_lo), g.clamp_hi);
+      }
+      const uint2 o = make_uint2(bf_pack(f[0], f[1]), bf_pack(f[2], f[3]));
+      if (!kSplit && g.out_row_ptrs) {
+        *reinterpret_cast<uint2*>(reinterpret_cast<bf16*>(at[i]) + col) = o;
+      } else {
+        if (g.out) *reinterpret_cast<uint2*>(g.out + at[i] * g.ldo + col) = o;
+        if (kSplit && g.out_lo)
+          *reinterpret_cast<uint2*>(g.out_lo + at[i] * g.ldo + col) =
+              make_uint2(bf_pack(f[0] - bf_lo(o.x), f[1] - bf_hi(o.x)), bf_pack(f[2] - bf_lo(o.y), f[3] - bf_hi(o.y)));
+      }
+    }
+  }
+}
+
+struct Block {
+  int group, col0;                 // row group, first output column
+  bool second;                     // dense block against the second problem's weights
+};
+template <int EPI, int MT>
+__device__ __forceinline__ Block locate(const FewParams& p, int block) {
+  constexpr bool kGated = EPI == kEpiSwiGLU || EPI == kEpiGlu;
+  const int grouped = p.tiles * p.g.num_groups;
+  Block b;
+  b.second = kGated && block >= grouped;
+  b.group = b.second ? 0 : block / p.tiles;
+  b.col0 = (b.second ? block - grouped : block - b.group * p.tiles) * 16 * (kGated ? 1 : MT);
+  return b;
+}
+__device__ __forceinline__ Weights weights_of(const FewParams& p, const Block& b) {
+  Weights w;
+  w.b0 = b.second ? p.b1 : p.b0 + static_cast<long long>(b.group) * p.g.b0_group_rows * p.ldb0;
+  w.b1 = p.b1 + static_cast<long long>(b.group) * p.g.b1_group_rows * p.ldb1;
+  w.ld0 = b.second ? p.ldb1 : p.ldb0;
+  w.ld1 = p.ldb1;
+  return w;
+}
+// Weight row i of the block's m-th 16 (clamped into the group's rows: what a clamped row gives is not stored).
+template <int EPI>
+__device__ __forceinline__ int weight_row(const FewParams& p, const Block& b, int m, int i) {
+  const int last = (b.second ? p.g.N2 : p.g.N) - 1;
+  if constexpr (EPI == kEpiSwiGLU || EPI == kEpiGlu) {
+    const int j = b.col0 + i, blk = j / p.half;
+    return min(blk * 2 * p.half + m * p.half + (j - blk * p.half), last);
+  } else {
+    return min(b.col0 + m * 16 + i, last);
+  }
+}
+template <int EPI, int MT>
+__device__ __forceinline__ void prefetch_block(const FewParams& p, const Block& b) {
+  if (threadIdx.x >= 16 * MT) return;
+  const Weights w = weights_of(p, b);
+  const long long row = weight_row<EPI>(p, b, threadIdx.x >> 4, threadIdx.x & 15);
+  prefetch_row(w.b0 + row * w.ld0, static_cast<uint32_t>(p.g.K0) * 2);
+  if (p.g.K1 > 0) prefetch_row(w.b1 + row * w.ld1, static_cast<uint32_t>(p.g.K1) * 2);
+}
+
+template <int EPI, int MT, int NTMAX, int WK>
+__global__ void __launch_bounds__(WK * 32, (NTMAX >= 8 ? 8 : 16) / WK) few_rows_kernel(const __grid_constant__ FewParams p) {
+  static_assert((EPI != kEpiSwiGLU && EPI != kEpiGlu) || MT == 2, "a gated unit takes its gate rows and its up rows together");
+  extern __shared__ float4 smem4[];
+  float* red = reinterpret_cast<float*>(smem4);
+  const GemmParams& g = p.g;
+  const int lane = threadIdx.x & 31;
+  const Block at = locate<EPI, MT>(p, blockIdx.x);
+  // this lane's weight rows
+  int w_row[MT][2];
+  const Weights wt = weights_of(p, at);
+#pragma unroll
+  for (int m = 0; m < MT; ++m)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) w_row[m][h] = weight_row<EPI>(p, at, m, (lane >> 2) + h * 8);
+  if (p.prefetch) prefetch_block<EPI, MT>(p, at);
+  pdl_enter();
+
+  int m_lo = 0, m_hi = g.M;
+  if (g.seg_offsets && !at.second) {
+    m_lo = g.seg_offsets[at.group];
+    m_hi = g.seg_offsets[at.group + 1];
+  }
+  // the weights of the block that takes this one's place are asked for now
+  if (p.ahead > 0 && blockIdx.x + p.ahead < gridDim.x) {
+    const Block next = locate<EPI, MT>(p, blockIdx.x + p.ahead);
+    if (next.second || !g.seg_offsets || g.seg_offsets[next.group] < g.seg_offsets[next.group + 1])
+      prefetch_block<EPI, MT>(p, next);
+  }
+  if (kChecks && g.seg_offsets) {
+    // checking build: a segment table that is not 0 <= s[0] <= s[1] <= ... <= M stores nothing
+    bool bad = false;
+    for (int i = 0; i < g.num_groups; ++i) {
+      const int lo = g.seg_offsets[i], hi = g.seg_offsets[i + 1];
+      bad = bad || lo < 0 || hi < lo || hi > g.M;
+    }
+    if (bad) {
+      if (threadIdx.x == 0 && g.status) atomicMax(g.status, kStatusBounds);
+      return;
+    }
+  }
+  const int n_steps0 = (g.K0 + kStep - 1) / kStep;
+  const int n_steps = n_steps0 + (g.K1 + kStep - 1) / kStep;
+  for (int m0 = m_lo; m0 < m_hi; m0 += 8 * NTMAX) {
+    const int left = m_hi - m0;
+    if (m0 > m_lo) __syncthreads();                        // the sums of the pass before are read
+    if constexpr (NTMAX == 1) {
+      few_pass<EPI, MT, 1, WK>(p, red, wt, w_row, n_steps0, n_steps, m0, m_hi, at.col0, at.second);
+    } else if constexpr (NTMAX == 4) {
+      if (left <= 8) few_pass<EPI, MT, 1, WK>(p, red, wt, w_row, n_steps0, n_steps, m0, m_hi, at.col0, at.second);
+      else if (left <= 16) few_pass<EPI, MT, 2, WK>(p, red, wt, w_row, n_steps0, n_steps, m0, m_hi, at.col0, at.second);
+      else few_pass<EPI, MT, 4, WK>(p, red, wt, w_row, n_steps0, n_steps, m0, m_hi, at.col0, at.second);
+    } else {
+      if (left <= 48) few_pass<EPI, MT, 6, WK>(p, red, wt, w_row, n_steps0, n_steps, m0, m_hi, at.col0, at.second);
+      else few_pass<EPI, MT, 8, WK>(p, red, wt, w_row, n_steps0, n_steps, m0, m_hi, at.col0, at.second);
+    }
+  }
+}
+
+template <int EPI, int MT, int NTMAX, int WK>
+cudaError_t launch_few(const FewParams& p, cudaStream_t stream) {
+  constexpr int smem = WK * 8 * NTMAX * kRowFloats<MT> * 4;
+  cudaError_t e = allow_smem<few_rows_kernel<EPI, MT, NTMAX, WK>>(smem);
+  if (e != cudaSuccess) return e;
+  FewParams q = p;
+  q.ahead = p.ahead * (NTMAX >= 8 ? 8 : 16) / WK;
+  const unsigned grid = static_cast<unsigned>(p.tiles * p.g.num_groups + p.tiles2);
+  return launch_kernel(few_rows_kernel<EPI, MT, NTMAX, WK>, dim3(grid), dim3(WK * 32), smem, stream, q);
+}
+
+template <int EPI, int MT, int WK>
+cudaError_t launch_warps(const FewParams& p, cudaStream_t stream) {
+  if (p.g.M <= 8) return launch_few<EPI, MT, 1, WK>(p, stream);
+  return p.g.num_groups > 1 || p.g.M <= 32 ? launch_few<EPI, MT, 4, WK>(p, stream) : launch_few<EPI, MT, 8, WK>(p, stream);
+}
+// Many blocks: four warps each, twice as many blocks on an SM, since a block is then mostly its own start and end
+// (64 experts of 704 x 2048, 8 rows: 14.5 us with eight warps, 9.4 with four); few blocks: eight warps, a shorter chain.
+template <int EPI, int MT>
+cudaError_t launch_rows(const FewParams& p, cudaStream_t stream) {
+  const long long blocks = static_cast<long long>(p.tiles) * p.g.num_groups + p.tiles2;
+  return blocks >= 3LL * p.ahead ? launch_warps<EPI, MT, 4>(p, stream) : launch_warps<EPI, MT, 8>(p, stream);
+}
+
+template <int EPI>
+cudaError_t launch_store(const FewParams& p, int mt, cudaStream_t stream) {
+  return mt == 2 ? launch_rows<EPI, 2>(p, stream) : launch_rows<EPI, 1>(p, stream);
+}
+
+}  // namespace
+
+// 32 weight rows per block once that still gives every SM two blocks: half the reads of the tokens.
+static int store_mt(long long cols, int num_groups, int sm_count) { return num_groups * ((cols + 31) / 32) >= 2LL * sm_count ? 2 : 1; }
+
+// Which calls stream (us on one B200, this kernel / the tile kernel):
+//   row groups: up to 64 rows, or 4 per group. 64 experts of 2 x 704 x 2048: 104 rows 64 / 80, 512 rows 94 / 84 (8 rows
+//     of an expert fill half of a product, and the tile kernel reads the weights at the same rate whatever the rows);
+//     8 experts and a shared one: 32 rows 14 / 26, 64 rows 15 / 26.
+//   dense: up to 64 rows, unless the tokens, which every block reads again, cost more than the tile kernel's chains.
+//     K 2048, N 2048: 32 rows 5.5 / 11.6, 64 rows 7.1 / 11.6; K 4096, N 4096: 32 rows 12.9 / 16.1, 48 rows 17.6 / 16.1;
+//     K 2048, N 32000: 8 rows 29 / 37, 32 rows 41 / 27. The estimates below put the line between these: both sides in
+//     bytes per ns at the rates that they reach, 4.9 us and 0.21 us per 64 of K for a chain.
+bool few_rows_taken(int M, int num_groups, bool second, int kind, int cols, int K, int sm_count) {
+  if (num_groups > 1 || second) return M <= 64 || (!second && M <= 4 * num_groups);
+  if (M > 64) return false;
+  const bool gated = kind == kEpiSwiGLU || kind == kEpiGlu;
+  const int per_block = gated ? 16 : 16 * store_mt(cols, 1, sm_count);
+  const long long weights = 2LL * cols * K * (gated ? 2 : 1);
+  const long long tokens = 2LL * M * K * ((cols + per_block - 1) / per_block);
+  const long long stream_ns = 2000 + (weights + tokens) / 7500;
+  const long long chain_ns = 4900 + 210LL * ((K + 63) / 64), read_ns = 4000 + weights / 5800;
+  return stream_ns <= (chain_ns > read_ns ? chain_ns : read_ns);
+}
+
+cudaError_t launch_few_rows(const GemmParams& g, int kind, const GemmOperand& op0, const GemmOperand* op1, const GemmSecond* second,
+                            int block_n, int sm_count, cudaStream_t stream) {
+  FewParams p;
+  p.g = g;
+  p.a0 = static_cast<const bf16*>(op0.a);
+  p.b0 = static_cast<const bf16*>(op0.b);
+  p.lda0 = op0.lda;
+  p.ldb0 = op0.ldb;
+  p.a1 = op1 ? static_cast<const bf16*>(op1->a) : p.a0;
+  p.b1 = op1 ? static_cast<const bf16*>(op1->b) : second ? static_cast<const bf16*>(second->b) : p.b0;
+  p.lda1 = op1 ? op1->lda : op0.lda;
+  p.ldb1 = op1 ? op1->ldb : second ? second->ldb : op0.ldb;
+  p.half = block_n / 2;
+  p.tiles2 = second ? (second->out_cols + 15) / 16 : 0;
+  // of a grouped call only as much is asked for ahead of time as its rows are sure to use
+  p.prefetch = g.num_groups == 1 || g.M >= 2 * g.num_groups;
+  p.ahead = sm_count;
+  if (kind == kEpiSwiGLU || kind == kEpiGlu) {
+    p.tiles = (g.out_cols + 15) / 16;
+    return kind == kEpiSwiGLU ? launch_rows<kEpiSwiGLU, 2>(p, stream) : launch_rows<kEpiGlu, 2>(p, stream);
+  }
+  const int mt = store_mt(g.out_cols, g.num_groups, sm_count);
+  p.tiles = (g.out_cols + 16 * mt - 1) / (16 * mt);
+  if (kind == kEpiStoreF32) return launch_store<kEpiStoreF32>(p, mt, stream);
+  if (kind == kEpiStoreSplit) return launch_store<kEpiStoreSplit>(p, mt, stream);
+  return launch_store<kEpiStore>(p, mt, stream);
+}
+
+}  // namespace cdeep

@@ -67,7 +67,9 @@ int cd_splitk_config(int flags);
 size_t cd_splitk_workspace_bytes(void);
 int cd_splitk_workspace_set(void* workspace, size_t bytes, void* stream);
 /* Number of K ranges cd_linear (or cd_mu_proj; cd_mu_qkv with K = the sum of its two K extents)
- * would use for a [T, K] x [N, K]^T call on the current device as it is set up now (1 = unsplit). */
+ * would use for a [T, K] x [N, K]^T call on the current device as it is set up now (1 = unsplit),
+ * where the tile kernel takes the call: calls of at most 64 rows mostly stream their weights through a
+ * kernel without tiles (csrc/gemm_few_rows.cu), whose blocks share K out among their own warps. */
 int cd_splitk_ranges(int T, int K, int N);
 /* 1 when this library is the checking build (libcdeep_checks.so, compiled with -DCDEEP_CHECKS),
  * else 0.  The checking build validates what its kernels read from device memory before using it
