@@ -357,12 +357,13 @@ cudaError_t launch_warps(const FewParams& p, cudaStream_t stream) {
   if (p.g.M <= 8) return launch_few<EPI, MT, 1, WK>(p, stream);
   return p.g.num_groups > 1 || p.g.M <= 32 ? launch_few<EPI, MT, 4, WK>(p, stream) : launch_few<EPI, MT, 8, WK>(p, stream);
 }
-// Many blocks: four warps each, twice as many blocks on an SM, since a block is then mostly its own start and end
-// (64 experts of 704 x 2048, 8 rows: 14.5 us with eight warps, 9.4 with four); few blocks: eight warps, a shorter chain.
+// More blocks than the two of eight warps that an SM holds: four warps each and four on an SM, since a block is then
+// mostly its own start and end (64 experts of 704 x 2048, 8 rows: 14.5 us with eight warps, 9.4 with four). Fewer
+// blocks: eight warps, a shorter chain.
 template <int EPI, int MT>
 cudaError_t launch_rows(const FewParams& p, cudaStream_t stream) {
   const long long blocks = static_cast<long long>(p.tiles) * p.g.num_groups + p.tiles2;
-  return blocks >= 3LL * p.ahead ? launch_warps<EPI, MT, 4>(p, stream) : launch_warps<EPI, MT, 8>(p, stream);
+  return blocks > 2LL * p.ahead ? launch_warps<EPI, MT, 4>(p, stream) : launch_warps<EPI, MT, 8>(p, stream);
 }
 
 template <int EPI>
