@@ -1,6 +1,6 @@
 // Kernels around a residual stream kept in fp32: embedding gather into the stream, RMSNorm or layer
-// norm of a stream row into the operand type of the next product, and the 32-bit matrix product used
-// when a model runs entirely in fp32 (no reduced-precision mode anywhere on that path).
+// norm of a stream row into the operand type of the next product, and the gated unit of models that run
+// entirely in fp32.
 #include "elem.cuh"
 #include "kernels.h"
 
@@ -112,65 +112,6 @@ rmsnorm_f32_kernel(const float* __restrict__ x, const T* __restrict__ w, float e
   });
 }
 
-// out[m, n] = residual[m, n] + scale * col_scale[n] * act(sum_k a[m, k] b[n, k]), all fp32 (FMA pipe).
-// Tile 64 x 64, 256 threads, 4 x 4 outputs per thread.  The order of the additions over k does not
-// depend on the number of rows.  With `seg` the grid's third axis is the group: its rows
-// [seg[g], seg[g + 1]) of a meet the g-th N rows of b.
-constexpr int kTM = 64, kTN = 64, kTK = 16;
-__global__ void __launch_bounds__(256)
-linear_f32_kernel(const float* __restrict__ a, long long lda, const float* __restrict__ b, const float* residual,
-                  const float* __restrict__ col_scale, float scale, int act, float* out,
-                  const int* __restrict__ seg, int M, int K, int N) {
-  __shared__ float sa[kTK][kTM + 4], sb[kTK][kTN + 4];
-  pdl_enter();
-  int m0 = blockIdx.y * kTM;
-  const int n0 = blockIdx.x * kTN;
-  if (seg) {
-    m0 += max(seg[blockIdx.z], 0);
-    M = min(M, seg[blockIdx.z + 1]);
-    b += static_cast<long long>(blockIdx.z) * N * K;
-    if (m0 >= M) return;
-  }
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  const int lr = threadIdx.x >> 2, lk = (threadIdx.x & 3) * 4;   // this thread's row and k of a tile load
-  float acc[4][4] = {};
-  for (int k0 = 0; k0 < K; k0 += kTK) {
-    float4 va = make_float4(0.f, 0.f, 0.f, 0.f), vb = va;
-    if (m0 + lr < M && k0 + lk < K) va = *reinterpret_cast<const float4*>(a + (m0 + lr) * lda + k0 + lk);
-    if (n0 + lr < N && k0 + lk < K) vb = *reinterpret_cast<const float4*>(b + static_cast<size_t>(n0 + lr) * K + k0 + lk);
-    sa[lk][lr] = va.x; sa[lk + 1][lr] = va.y; sa[lk + 2][lr] = va.z; sa[lk + 3][lr] = va.w;
-    sb[lk][lr] = vb.x; sb[lk + 1][lr] = vb.y; sb[lk + 2][lr] = vb.z; sb[lk + 3][lr] = vb.w;
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < kTK; ++k) {
-      const float4 fa = *reinterpret_cast<const float4*>(&sa[k][ty * 4]);
-      const float4 fb = *reinterpret_cast<const float4*>(&sb[k][tx * 4]);
-      const float av[4] = {fa.x, fa.y, fa.z, fa.w}, bv[4] = {fb.x, fb.y, fb.z, fb.w};
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int m = m0 + ty * 4 + i;
-    if (m >= M) continue;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int n = n0 + tx * 4 + j;
-      if (n >= N) continue;
-      float v = acc[i][j];
-      if (act == 1) v = fmaxf(v, 0.f) * fmaxf(v, 0.f);
-      v *= scale;
-      if (col_scale) v *= col_scale[n];
-      if (residual) v += residual[static_cast<size_t>(m) * N + n];
-      out[static_cast<size_t>(m) * N + n] = v;
-    }
-  }
-}
-
 // h[t, j] = g * sigmoid(alpha g) * (u + offset), g = min(gu[t, j], limit), u = clamp(gu[t, I + j], +-limit)
 __global__ void __launch_bounds__(256)
 glu_f32_kernel(const float* __restrict__ gu, float* __restrict__ h, long long n, int I, float alpha,
@@ -221,14 +162,6 @@ cudaError_t launch_rmsnorm_f32(const float* x, const void* w, float eps, float o
                 : rmsnorm_any<bf16, true>(x, w, eps, offset, out, rows, W, ldx, st);
   return fp32 ? rmsnorm_any<float, false>(x, w, eps, offset, out, rows, W, ldx, st)
               : rmsnorm_any<bf16, false>(x, w, eps, offset, out, rows, W, ldx, st);
-}
-
-cudaError_t launch_linear_f32(const float* a, long long lda, const float* b, const float* residual,
-                              const float* col_scale, float scale, int act, float* out, const int* seg, int groups,
-                              int M, int K, int N, cudaStream_t st) {
-  if (M == 0) return cudaSuccess;
-  return launch_kernel(linear_f32_kernel, dim3((N + kTN - 1) / kTN, (M + kTM - 1) / kTM, seg ? groups : 1), dim3(256),
-                       0, st, a, lda, b, residual, col_scale, scale, act, out, seg, M, K, N);
 }
 
 cudaError_t launch_glu_f32(const float* gu, float* h, int T, int I, float alpha, float limit, float offset,
