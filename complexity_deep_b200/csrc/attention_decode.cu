@@ -26,24 +26,37 @@ namespace {
 constexpr int kAttnThreads = 128;
 constexpr int kMaxGroup = 4;    // query heads per KV head handled by one block (the entry point refuses more)
 constexpr int kLanesPerRow = 8;
+constexpr int kMaxSplits = 64;
 
 __device__ __forceinline__ float lo_f(uint32_t v) { return __uint_as_float(v << 16); }
 __device__ __forceinline__ float hi_f(uint32_t v) { return __uint_as_float(v & 0xffff0000u); }
 
+// Blocks that an SM holds at a time, by the registers of G query heads of D dimensions.
+__host__ __device__ constexpr int blocks_per_sm(int G, int D) { return G * D > 384 ? 2 : G * D > 256 ? 3 : 4; }
+
 // Blocks per (batch, kv head) pair.  Also evaluated on the device when the cache length is
-// read from device memory, so both forms split (and therefore round) identically.
-// kTargetBlocks is a tuning constant (16 blocks for each of a B200's 148 SMs), not a limit: any
-// other SM count only changes how many blocks share the work.
-constexpr int kTargetBlocks = 16 * 148;
-__host__ __device__ inline int choose_splits(int B, int hkv, int L) {
-  const int pairs = B * hkv;
-  int splits = (kTargetBlocks + pairs - 1) / pairs;   // several waves of blocks: small tail
-  // at least 512 rows per block (measured against 128 and 256: 10-15 % faster for short
-  // caches and few sequences, equal elsewhere)
-  const int max_splits = (L + 511) / 512;
+// read from device memory, so both forms split (and therefore round) identically; never falls as L grows.
+// kSms is a tuning constant (a B200's 148 SMs), not a limit: any other SM count only changes how many
+// blocks share the work.
+//   Two splits of every pair fit the device at once: as many as do, down to 48 rows a block, in one wave (at most 32:
+//   the combining kernel reads them all). us, this rule / at least 512 rows a block and up to four waves, partial and
+//   combine, cold L2: 1 sequence x 4 kv heads x 302 rows 11 / 17; 1 x 8 x 2064 13 / 24; 8 x 8 x 1000 18 / 24;
+//   32 x 8 x 2064 64 / 73 (1 280 blocks are 2.2 waves).
+//   More pairs: several waves of at least 512 rows a block keep the last one short.
+constexpr int kSms = 148;
+__host__ __device__ inline int choose_splits(int B, int hkv, int L, int per_sm) {
+  const int pairs = B * hkv, one_wave = per_sm * kSms / pairs;
+  int splits, max_splits;
+  if (one_wave >= 2) {
+    splits = one_wave < 32 ? one_wave : 32;
+    max_splits = (L + 47) / 48;
+  } else {
+    splits = (16 * kSms + pairs - 1) / pairs;
+    max_splits = (L + 511) / 512;
+  }
   if (splits > max_splits) splits = max_splits;
   if (splits < 1) splits = 1;
-  if (splits > 64) splits = 64;
+  if (splits > kMaxSplits) splits = kMaxSplits;
   return splits;
 }
 
@@ -80,7 +93,7 @@ constexpr int kStages = 4;   // row steps staged in shared memory per thread (3 
 // 4 blocks per SM keep ~100 KB on the way) and reads them back with 16-byte loads, so no
 // block-level synchronisation is needed inside the loop.
 template <int DPL, int G>
-__global__ void __launch_bounds__(kAttnThreads, (G * DPL > 48) ? 2 : (G * DPL > 32) ? 3 : 4)
+__global__ void __launch_bounds__(kAttnThreads, blocks_per_sm(G, DPL * kLanesPerRow))
 decode_attn_partial_kernel(const __nv_bfloat16* __restrict__ q, long long q_stride_b,
                            const __nv_bfloat16* __restrict__ k, const __nv_bfloat16* __restrict__ v,
                            long long kv_stride_b, long long kv_stride_h, long long kv_stride_t,
@@ -101,7 +114,7 @@ decode_attn_partial_kernel(const __nv_bfloat16* __restrict__ q, long long q_stri
   const int splits = gridDim.x;
   if (len_dev) {
     L = max(0, min(L, __ldg(len_dev)));
-    const int live = choose_splits(gridDim.z, gridDim.y, L);
+    const int live = choose_splits(gridDim.z, gridDim.y, L, blocks_per_sm(G, D));
     if (split >= live) return;       // whole block; the combine kernel skips these slots
     chunk = chunk_rows(L, live);
   }
@@ -263,25 +276,46 @@ decode_attn_partial_kernel(const __nv_bfloat16* __restrict__ q, long long q_stri
   }
 }
 
-// out[b, h, :] = sum_s w_s acc_s / sum_s w_s l_s, w_s = exp(m_s - max m)
+// out[b, h, :] = sum_s w_s acc_s / sum_s w_s l_s, w_s = exp(m_s - max m). The weights of the (at most 64) splits are
+// found by one warp, a lane per split, so that what follows is one chain of independent loads per column.
 __global__ void __launch_bounds__(128)
 decode_attn_combine_kernel(const float* __restrict__ part_acc, const float* __restrict__ part_ml,
                            int splits, int D, __nv_bfloat16* __restrict__ out, int B, int hkv,
-                           int L, const int* __restrict__ len_dev) {
+                           int L, int per_sm, const int* __restrict__ len_dev) {
+  __shared__ float s_w[kMaxSplits];
+  __shared__ float s_sum;
   griddep_wait();
   griddep_launch_dependents();
   const long long row0 = static_cast<long long>(blockIdx.x) * splits;   // (b, h)
-  if (len_dev) splits = choose_splits(B, hkv, max(0, min(L, __ldg(len_dev))));
-  float m = -FLT_MAX;
-  for (int s = 0; s < splits; ++s) m = fmaxf(m, part_ml[(row0 + s) * 2]);
-  for (int d = threadIdx.x; d < D; d += blockDim.x) {
-    float l = 0.f, a = 0.f;
-    for (int s = 0; s < splits; ++s) {
-      const float ms = part_ml[(row0 + s) * 2];
-      const float w = (ms > -FLT_MAX) ? __expf(ms - m) : 0.f;
-      l += part_ml[(row0 + s) * 2 + 1] * w;
-      a += part_acc[(row0 + s) * D + d] * w;
+  if (len_dev) splits = choose_splits(B, hkv, max(0, min(L, __ldg(len_dev))), per_sm);
+  const int lane = threadIdx.x & 31;
+  if (threadIdx.x < 32) {
+    float ms[kMaxSplits / 32], ls[kMaxSplits / 32], m = -FLT_MAX, sum = 0.f;
+#pragma unroll
+    for (int i = 0; i < kMaxSplits / 32; ++i) {
+      const int s = lane + 32 * i;
+      ms[i] = s < splits ? part_ml[(row0 + s) * 2] : -FLT_MAX;
+      ls[i] = s < splits ? part_ml[(row0 + s) * 2 + 1] : 0.f;
+      m = fmaxf(m, ms[i]);
     }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+#pragma unroll
+    for (int i = 0; i < kMaxSplits / 32; ++i) {
+      const float w = ms[i] > -FLT_MAX ? __expf(ms[i] - m) : 0.f;
+      s_w[lane + 32 * i] = w;
+      sum += ls[i] * w;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if (lane == 0) s_sum = sum;
+  }
+  __syncthreads();
+  const float l = s_sum;
+  for (int d = threadIdx.x; d < D; d += blockDim.x) {
+    float a = 0.f;
+#pragma unroll 8
+    for (int s = 0; s < splits; ++s) a += part_acc[(row0 + s) * D + d] * s_w[s];
     out[static_cast<long long>(blockIdx.x) * D + d] = __float2bfloat16_rn(l > 0.f ? a / l : 0.f);
   }
 }
@@ -312,7 +346,7 @@ cudaError_t launch_partial(int G, dim3 grid, cudaStream_t st, const __nv_bfloat1
 }  // namespace
 
 size_t decode_attention_workspace_bytes(int B, int hq, int hkv, int L, int D) {
-  const size_t splits = choose_splits(B, hkv, L);
+  const size_t splits = choose_splits(B, hkv, L, blocks_per_sm(hq / hkv, D));
   return static_cast<size_t>(B) * hq * splits * (D + 2) * sizeof(float);
 }
 
@@ -323,7 +357,7 @@ cudaError_t launch_decode_attention(const void* q, long long q_stride_b, const v
                                     int L, int D, void* out, void* ws, cudaStream_t stream,
                                     const int* kv_len_dev) {
   const int G = hq / hkv;
-  const int splits = choose_splits(B, hkv, L);
+  const int splits = choose_splits(B, hkv, L, blocks_per_sm(G, D));
   const int chunk = chunk_rows(L, splits);
   float* part_acc = static_cast<float*>(ws);
   float* part_ml = part_acc + static_cast<size_t>(B) * hq * splits * D;
@@ -345,7 +379,7 @@ cudaError_t launch_decode_attention(const void* q, long long q_stride_b, const v
     return cudaErrorInvalidValue;
   if (e != cudaSuccess) return e;
   return launch_kernel(decode_attn_combine_kernel, dim3(B * hq), dim3(128), 0, stream, part_acc,
-                       part_ml, splits, D, static_cast<__nv_bfloat16*>(out), B, hkv, L, kv_len_dev);
+                       part_ml, splits, D, static_cast<__nv_bfloat16*>(out), B, hkv, L, blocks_per_sm(G, D), kv_len_dev);
 }
 
 }  // namespace cdeep
