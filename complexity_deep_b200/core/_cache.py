@@ -6,18 +6,18 @@ rebuilt whenever a caller mutates a source parameter in place (``_version``), re
 """
 from __future__ import annotations
 
-from typing import Callable, Dict, Sequence, Tuple
+from typing import Callable, Dict, List, Sequence, Tuple
 
 import torch
 
 
-def _key(tensors: Sequence[torch.Tensor]) -> Tuple:
-    return tuple((t.data_ptr(), t._version, t.dtype, t.device, tuple(t.shape)) for t in tensors)
+def _key(tensors: Sequence[torch.Tensor]) -> List[Tuple]:
+    return [(t.data_ptr(), t._version, t.dtype, t.device, t.shape) for t in tensors]
 
 
 class DerivedCache:
     def __init__(self) -> None:
-        self._slots: Dict[str, Tuple[Tuple, object]] = {}
+        self._slots: Dict[str, Tuple[List[Tuple], object]] = {}
 
     def get(self, name: str, sources: Sequence[torch.Tensor], make: Callable[[], object]):
         key = _key(sources)

@@ -207,6 +207,10 @@ class ComplexityAttention(nn.Module):
                               self.k_norm.weight if self.use_qk_norm else None, cos, sin, 1e-6, S,
                               past_len, hq, hkv, D)
 
+        if (S > 1 and not use_cache
+                and self._prefill_kernel_applies(B, S, attention_mask, past_key_value)):
+            return ops.attention_prefill(qkv, B, S, hq, hkv, D), None   # nobody needs k and v by themselves
+
         q = qkv[:, : hq * D].view(B, S, hq, D).transpose(1, 2)
         k = qkv[:, hq * D: (hq + hkv) * D].view(B, S, hkv, D).transpose(1, 2)
         v = qkv[:, (hq + hkv) * D:].view(B, S, hkv, D).transpose(1, 2)

@@ -8,6 +8,7 @@ back to PyTorch operators.
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
 from dataclasses import dataclass
 from typing import Optional, Tuple
@@ -19,8 +20,13 @@ from . import _lib
 BF16 = torch.bfloat16
 
 
+# the handle of the calling thread's current stream on its current device: what
+# torch.cuda.current_stream().cuda_stream gives, without building a Stream object (0.2 us instead of 3.3 a launch)
+_current_device, _raw_stream = torch._C._cuda_getDevice, torch._C._cuda_getCurrentRawStream
+
+
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    return _raw_stream(_current_device())
 
 
 def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
@@ -28,6 +34,8 @@ def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
 
 
 def _need(t: torch.Tensor, name: str, dtype=BF16) -> None:
+    if isinstance(t, torch.Tensor) and t.is_cuda and t.dtype is dtype and t.is_contiguous():
+        return
     if not isinstance(t, torch.Tensor) or not t.is_cuda:
         raise RuntimeError(
             f"{name}: expected a CUDA tensor; the complexity_deep_b200 kernels have no CPU path")
@@ -154,14 +162,14 @@ def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float,
     """
     lib = _lib.load()
     H = x.shape[-1]
-    x2 = x.reshape(-1, H)
+    x2 = x if x.dim() == 2 else x.reshape(-1, H)
     _need(x2, "x")
     _need(weight, "weight")
     T = x2.shape[0]
     if x_lo is not None:
         if residual is not None or want_sum:
             raise RuntimeError("x_lo cannot be combined with residual / want_sum")
-        lo2 = x_lo.reshape(-1, H)
+        lo2 = x_lo if x_lo.dim() == 2 and x_lo.shape[1] == H else x_lo.reshape(-1, H)
         _need(lo2, "x_lo")
         if lo2.shape[0] != T:
             raise RuntimeError("x_lo does not match x")
@@ -174,7 +182,7 @@ def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float,
             _lib.check(lib.cd_rmsnorm_split(x2.data_ptr(), lo2.data_ptr(), weight.data_ptr(),
                                             float(eps), out.data_ptr(), _ptr(dst_rows), T, H,
                                             _stream()), "cd_rmsnorm_split")
-        return out.view(x.shape)
+        return out if x2 is x else out.view(x.shape)
     res2 = None
     if residual is not None:
         res2 = residual.reshape(-1, H)
@@ -325,6 +333,11 @@ def attention_prefill(qkv: torch.Tensor, batch: int, seq_len: int, hq: int, hkv:
 
 
 # --------------------------------------------------------------------------- weights
+@functools.lru_cache(maxsize=None)
+def _sm_count(device: int) -> int:
+    return torch.cuda.get_device_properties(device).multi_processor_count
+
+
 def choose_block_n(width: int, rows: Optional[int] = None, groups: int = 1,
                    sm_count: Optional[int] = None) -> int:
     """Accumulator-tile width for the SwiGLU up-projection of an expert `width` wide.
@@ -340,8 +353,7 @@ def choose_block_n(width: int, rows: Optional[int] = None, groups: int = 1,
     """
     if rows is not None and rows <= 512:
         if sm_count is None:
-            sm_count = (torch.cuda.get_device_properties(torch.cuda.current_device())
-                        .multi_processor_count if torch.cuda.is_available() else 148)
+            sm_count = _sm_count(_current_device()) if torch.cuda.is_available() else 148
         m_tiles = max(groups, -(-rows // 128))
         for bn in (32, 64, 128, 256):
             if m_tiles * -(-width // (bn // 2)) <= sm_count:
