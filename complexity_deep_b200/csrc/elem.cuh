@@ -78,6 +78,16 @@ __device__ __forceinline__ void pdl_enter() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// Asks for `bytes` (a multiple of 16, at a 16-byte boundary) in L2. Reads nothing into the program, so it may run ahead
+// of kernels that still write there.
+__device__ __forceinline__ void prefetch_l2_bulk(const void* p, uint32_t bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+}
+// The same for a block's `bytes` (a multiple of 512), dealt to its first warp.
+__device__ __forceinline__ void prefetch_l2_warp(const void* p, uint32_t bytes) {
+  if (threadIdx.x < 32) prefetch_l2_bulk(static_cast<const char*>(p) + threadIdx.x * (bytes / 32), bytes / 32);
+}
+
 __device__ __forceinline__ float exp2_approx(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));

@@ -90,6 +90,30 @@ window_decode_scores_kernel(const DecodeParams p) {
   T* ring_k = static_cast<T*>(a.ring_k) + (b * slots * a.G + c) * dp;
   const long long stride = static_cast<long long>(a.G) * dp;
   const bool has_new = r.nk > 0 && r.n0 + r.nk == r.count;
+  // the values of this block's keys are asked for in L2 now: the keys alone leave the memory idle most of the time
+  {
+    const T* v = static_cast<const T*>(a.ring_v) + (b * slots * a.G + c) * static_cast<long long>(vp);
+    if (blockIdx.y % groups == 0)
+      for (int n = tid; n < r.nk; n += kThreads)
+        prefetch_l2_bulk(v + static_cast<long long>(r.slot(r.n0 + n)) * a.G * vp, static_cast<uint32_t>(vp * sizeof(T)));
+  }
+  // Rows in flight per lane; the first ones are on their way before the query is there.
+  constexpr int kAhead = DC * sizeof(T) <= 4 ? 4 : 2;
+  constexpr int kStep = kWarps * 4;             // rows of the block per step
+  Raw8<T> kf[kAhead][DC];
+  auto load_row = [&](int base, int u) {
+    const int n = min(base + u * kStep + warp * 4 + rg, r.nk - 1);          // rows past the end are not used
+    const T* k = ring_k + static_cast<long long>(r.slot(r.n0 + n)) * stride;
+#pragma unroll
+    for (int e = 0; e < DC; ++e) {
+      const int d = (e * 8 + sub) * 8;
+      raw_load(k + (d < dp ? d : 0), kf[u][e]);                             // past the head: the query is zero
+    }
+  };
+  if (r.nk > 0) {
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) load_row(0, u);
+  }
 
   auto rms_scale = [&](const T* x) {
     float ss = 0.f;
@@ -127,12 +151,10 @@ window_decode_scores_kernel(const DecodeParams p) {
 #pragma unroll
       for (int y = 0; y < 8; ++y) qf[x][e][y] = (x < nh && d < dp) ? sm[x * dp + d + y] : 0.f;
     }
-  // Rows in flight per lane.  The kAhead x REP scores of a lane group are finished by its lanes: lane
-  // `sub` takes the head sub % REP and, in `kRounds` rounds, row sub / REP + round * (8 / REP).
-  constexpr int kAhead = DC * sizeof(T) <= 4 ? 4 : 2;
+  // The kAhead x REP scores of a lane group are finished by its lanes: lane `sub` takes the head sub % REP and, in
+  // `kRounds` rounds, row sub / REP + round * (8 / REP).
   constexpr int kRowsRound = 8 / REP < kAhead ? 8 / REP : kAhead;
   constexpr int kRounds = kAhead / kRowsRound;
-  constexpr int kStep = kWarps * 4;             // rows of the block per step
   const int my_head = sub % REP, my_row = sub / REP;
   float r1 = 0.f, r2 = 0.f, m = -FLT_MAX, l = 0.f;
   if (my_head < nh) {
@@ -141,16 +163,10 @@ window_decode_scores_kernel(const DecodeParams p) {
   }
   float* out = p.scores + (static_cast<long long>(b) * a.H + h0 + (my_head < nh ? my_head : 0)) * p.n_max;
   for (int base = 0; base < r.nk; base += kStep * kAhead) {
-    Raw8<T> kf[kAhead][DC];
 #pragma unroll
     for (int u = 0; u < kAhead; ++u) {
-      const int n = min(base + u * kStep + warp * 4 + rg, r.nk - 1);      // rows past the end are not used
-      const T* k = ring_k + static_cast<long long>(r.slot(r.n0 + n)) * stride;
-#pragma unroll
-      for (int e = 0; e < DC; ++e) {
-        const int d = (e * 8 + sub) * 8;
-        raw_load(k + (d < dp ? d : 0), kf[u][e]);                         // past the head: the query is zero
-      }
+      // of the first rows only the new token's is loaded again: it was written after they were asked for
+      if (base > 0 || (has_new && base + u * kStep + warp * 4 + rg >= r.nk - 1)) load_row(base, u);
     }
     float s[kAhead][REP];
 #pragma unroll
@@ -260,7 +276,7 @@ __host__ __device__ inline int values_smem_floats(int vp) {
 }
 
 template <typename T, int REP>
-__global__ void __launch_bounds__(kThreads, REP <= 2 && sizeof(T) == 2 ? 4 : 2)
+__global__ void __launch_bounds__(kThreads, REP <= 2 && sizeof(T) == 2 ? 3 : 2)
 window_decode_values_kernel(const DecodeParams p) {
   extern __shared__ float sm[];
   pdl_enter();
@@ -285,7 +301,7 @@ window_decode_values_kernel(const DecodeParams p) {
   for (int x = 0; x < REP; ++x)
 #pragma unroll
     for (int e = 0; e < 8; ++e) acc[x][e] = 0.f;
-  constexpr int kAhead = 4;
+  constexpr int kAhead = REP <= 2 && sizeof(T) == 2 ? 6 : 4;
   if (active) {
     for (int at = row; at < r.nk; at += rows * kAhead) {
       Raw8<T> vf[kAhead];
@@ -332,12 +348,27 @@ window_decode_values_kernel(const DecodeParams p) {
   if (p.splits > 1) cluster.sync();     // the other blocks read this block's shared memory until here
 }
 
+// Splits of the keys of a (head group, sequence): those whose last wave ends first. A block costs about 4 us of its own
+// (position, query, first keys, statistics) and, with three on an SM, the time that its keys take at the SM's share of
+// the memory's rate (44 bytes per ns). One B200, 32 sequences, 4 key heads of 128, 516 keys, scores / values us: 8 splits
+// (1 024 blocks, three waves of 64 keys each, the rule before) 15.0 / 15.4, 3 splits (one wave) 12.4 / 8.8, the
+// prefetch of the values included in the first.
+constexpr int kMostSplits = 8;             // of a portable cluster
 int choose_splits(const WindowAttnParams& a, int rep_block) {
-  const int rep = a.H / a.G;
+  const int rep = a.H / a.G, keys = a.keep + a.window;
   const long long blocks = static_cast<long long>(a.B) * a.G * ((rep + rep_block - 1) / rep_block);
-  int s = 1;
-  while (s < 8 && blocks * s < 148 * 6 && (a.keep + a.window) / (2 * s) >= 64) s *= 2;
-  return s;
+  const long long wave = 3LL * current_sm_count();
+  const double key_us = 2.0 * (a.dp > a.vp ? a.dp : a.vp) * 3 / 44e3;
+  int best = 1;
+  double best_us = 1e30;
+  for (int s = 1; s <= kMostSplits && (s == 1 || keys / s >= 48); ++s) {
+    const double us = static_cast<double>((blocks * s + wave - 1) / wave) * (4.0 + (keys + s - 1) / s * key_us);
+    if (us < 0.98 * best_us) {
+      best = s;
+      best_us = us;
+    }
+  }
+  return best;
 }
 
 int rep_block(const WindowAttnParams& a) {
