@@ -359,7 +359,7 @@ __global__ void __launch_bounds__(256, 2)
 qk_norm_rope_vec_kernel(__nv_bfloat16* __restrict__ qkv, const __nv_bfloat16* __restrict__ q_w,
                         const __nv_bfloat16* __restrict__ k_w, const float* __restrict__ cos_t,
                         const float* __restrict__ sin_t, float eps, int T, int S, int pos0, int hq,
-                        int hkv, int D, KvAppend app) {
+                        int hkv, int D, int iters, KvAppend app) {
   griddep_wait();               // the previous kernel's writes are visible from here
   griddep_launch_dependents();  // the next kernel may be scheduled
   const int heads = hq + hkv;
@@ -403,14 +403,15 @@ qk_norm_rope_vec_kernel(__nv_bfloat16* __restrict__ qkv, const __nv_bfloat16* __
   // All loads of the token are issued before any arithmetic (up to kMaxIter heads per lane
   // group) so enough bytes are in flight to cover HBM latency.
   constexpr int kMaxIter = 3;
-  for (int hb = 0; hb < heads; hb += groups * kMaxIter) {   // uniform trip count across the warp
+  const int stride = gridDim.y * groups * iters;
+  for (int hb = blockIdx.y * groups * iters; hb < heads; hb += stride) {   // uniform trip count across the warp
     uint4 a[kMaxIter], b[kMaxIter];
 #pragma unroll
     for (int i = 0; i < kMaxIter; ++i) {
       const int h = hb + i * groups + g;
       a[i] = make_uint4(0, 0, 0, 0);
       b[i] = make_uint4(0, 0, 0, 0);
-      if (h < heads) {
+      if (i < iters && h < heads) {
         a[i] = *reinterpret_cast<const uint4*>(row + static_cast<size_t>(h) * D + j);
         b[i] = *reinterpret_cast<const uint4*>(row + static_cast<size_t>(h) * D + half + j);
       }
@@ -418,7 +419,7 @@ qk_norm_rope_vec_kernel(__nv_bfloat16* __restrict__ qkv, const __nv_bfloat16* __
 #pragma unroll
     for (int i = 0; i < kMaxIter; ++i) {
       const int h = hb + i * groups + g;
-      if (hb + i * groups >= heads) break;                  // uniform
+      if (i >= iters || hb + i * groups >= heads) break;    // uniform
       const bool active = h < heads;
       const uint32_t aw[4] = {a[i].x, a[i].y, a[i].z, a[i].w};
       const uint32_t bw[4] = {b[i].x, b[i].y, b[i].z, b[i].w};
@@ -465,7 +466,7 @@ qk_norm_rope_vec_kernel(__nv_bfloat16* __restrict__ qkv, const __nv_bfloat16* __
   }
   if (kAppend) {   // the row's v heads, 16 bytes per lane and step
     const __nv_bfloat16* vsrc = row + static_cast<size_t>(heads) * D;
-    for (int c = lane * 8; c < hkv * D; c += 256) {
+    for (int c = (blockIdx.y * 32 + lane) * 8; c < hkv * D; c += 256 * gridDim.y) {
       const int vh = c / D;
       __nv_bfloat16* vdst = app.v_cache + t * app.stride_b + vh * app.stride_h +
                             pos * app.stride_t + (c - vh * D);
@@ -555,11 +556,15 @@ cudaError_t launch_qk_norm_rope(void* qkv, const void* q_w, const void* k_w, con
   auto qw = static_cast<const __nv_bfloat16*>(q_w);
   auto kw = static_cast<const __nv_bfloat16*>(k_w);
   if ((D & 15) == 0 && lph >= 1 && lph <= 32 && (lph & (lph - 1)) == 0 && aligned) {
-    const unsigned nblocks = static_cast<unsigned>((T + 7) / 8);  // one warp per token
-    return append ? launch_kernel(qk_norm_rope_vec_kernel<true>, dim3(nblocks), dim3(256), 0, stream,
-                                  qb, qw, kw, cos_t, sin_t, eps, T, S, pos0, hq, hkv, D, app)
-                  : launch_kernel(qk_norm_rope_vec_kernel<false>, dim3(nblocks), dim3(256), 0, stream,
-                                  qb, qw, kw, cos_t, sin_t, eps, T, S, pos0, hq, hkv, D, app);
+    const unsigned nblocks = static_cast<unsigned>((T + 7) / 8);  // a token per warp
+    const int groups = 32 / lph;
+    const bool few = T < 4 * current_sm_count();
+    const int iters = few ? 1 : 3;
+    const dim3 grid(nblocks, few ? (hq + hkv + groups - 1) / groups : 1);
+    return append ? launch_kernel(qk_norm_rope_vec_kernel<true>, grid, dim3(256), 0, stream, qb, qw,
+                                  kw, cos_t, sin_t, eps, T, S, pos0, hq, hkv, D, iters, app)
+                  : launch_kernel(qk_norm_rope_vec_kernel<false>, grid, dim3(256), 0, stream, qb, qw,
+                                  kw, cos_t, sin_t, eps, T, S, pos0, hq, hkv, D, iters, app);
   }
   const long long warps = static_cast<long long>(T) * (hq + hkv);
   const int wpb = 8;
