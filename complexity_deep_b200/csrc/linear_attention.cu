@@ -12,13 +12,33 @@ namespace {
 constexpr int kThreads = 256;
 
 // ---------------------------------------------------------------- decode
+// A block per head and sequence. A thread loads up to kRows rows of four columns of the state before anything else (a
+// state of 128 x 128 is on its way whole while the decay is computed); a block asks for its state in L2 ahead of the
+// kernel before it, and for that of the block that takes its place. 32 sequences, 4 heads of 128 x 128: 6.0 us, with
+// four rows at a time behind the decay 12.7.
+constexpr int kRows = 16;
 template <typename T>
-__global__ void __launch_bounds__(kThreads)
-gla_step_kernel(const LinearAttnParams p) {
+__global__ void __launch_bounds__(kThreads, 2)
+gla_step_kernel(const LinearAttnParams p, int resident) {
   extern __shared__ float sm[];
-  pdl_enter();
   const int h = blockIdx.x, b = blockIdx.y, tid = threadIdx.x;
   const int dkp = p.dkp, dvp = p.dvp;
+  // columns in groups of four; the rows of the state are dealt to the row groups
+  const int cgs = dvp / 4;                 // dvp <= 1024
+  const int rgs = kThreads / cgs;
+  const int rg = tid / cgs, col = (tid - rg * cgs) * 4;
+  float* S = p.state + (static_cast<long long>(b) * p.H + h) * dkp * dvp;
+  const uint32_t state_bytes = static_cast<uint32_t>(dkp) * dvp * 4;
+  prefetch_l2_warp(S, state_bytes);
+  pdl_enter();
+  if (b * p.H + h + resident < p.B * p.H) prefetch_l2_warp(S + static_cast<long long>(resident) * dkp * dvp, state_bytes);
+  float4 first[kRows];
+#pragma unroll
+  for (int i = 0; i < kRows; ++i) {
+    const int r = rg + i * rgs;
+    first[i] = rg < rgs && r < dkp ? *reinterpret_cast<const float4*>(S + static_cast<long long>(r) * dvp + col)
+                                   : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
   float* sq = sm;                // [dkp]
   float* sk = sq + dkp;          // [dkp]
   float* sa = sk + dkp;          // [dkp]
@@ -36,29 +56,26 @@ gla_step_kernel(const LinearAttnParams p) {
     sv[c] = to_f32(static_cast<const T*>(p.v)[row * p.ldp + static_cast<long long>(h) * dvp + c]);
   __syncthreads();
 
-  // columns in groups of four; the rows of the state are dealt to the row groups
-  const int cgs = dvp / 4;                 // dvp <= 1024
-  const int rgs = kThreads / cgs;
-  const int rg = tid / cgs, col = (tid - rg * cgs) * 4;
-  float* S = p.state + (static_cast<long long>(b) * p.H + h) * dkp * dvp;
   float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
   if (rg < rgs) {
     const float4 v = *reinterpret_cast<const float4*>(sv + col);
-#pragma unroll 4
-    for (int r = rg; r < dkp; r += rgs) {
-      float4* ptr = reinterpret_cast<float4*>(S + static_cast<long long>(r) * dvp + col);
-      float4 s = *ptr;
+    auto row_of = [&](int r, float4 s) {
       const float a = sa[r], k = sk[r], q = sq[r];
       s.x = fmaf(a, s.x, k * v.x);
       s.y = fmaf(a, s.y, k * v.y);
       s.z = fmaf(a, s.z, k * v.z);
       s.w = fmaf(a, s.w, k * v.w);
-      *ptr = s;
+      *reinterpret_cast<float4*>(S + static_cast<long long>(r) * dvp + col) = s;
       o.x = fmaf(q, s.x, o.x);
       o.y = fmaf(q, s.y, o.y);
       o.z = fmaf(q, s.z, o.z);
       o.w = fmaf(q, s.w, o.w);
-    }
+    };
+#pragma unroll
+    for (int i = 0; i < kRows; ++i)
+      if (rg + i * rgs < dkp) row_of(rg + i * rgs, first[i]);
+#pragma unroll 4
+    for (int r = rg + kRows * rgs; r < dkp; r += rgs) row_of(r, *reinterpret_cast<const float4*>(S + static_cast<long long>(r) * dvp + col));
     *reinterpret_cast<float4*>(so + tid * 4) = o;    // = [rg][dvp]
   }
   __syncthreads();
@@ -285,7 +302,7 @@ cudaError_t launch_sequence(const LinearAttnParams& p, cudaStream_t st) {
 template <typename T>
 cudaError_t launch_step(const LinearAttnParams& p, cudaStream_t st) {
   const size_t bytes = (3 * p.dkp + p.dvp + kThreads * 4) * sizeof(float);
-  return launch_kernel(gla_step_kernel<T>, dim3(p.H, p.B), dim3(kThreads), bytes, st, p);
+  return launch_kernel(gla_step_kernel<T>, dim3(p.H, p.B), dim3(kThreads), bytes, st, p, 2 * current_sm_count());
 }
 
 }  // namespace
