@@ -168,13 +168,33 @@ cudaError_t launch_decay(const LinearAttnParams& p, cudaStream_t st) {
 }
 
 constexpr int kSteps = 16;      // tokens staged in shared memory at a time
-constexpr int kCols = 32;       // state columns per block
 
-// M rows of the state per thread (dkp <= 32 M), four columns each
-template <typename T, int M>
-__global__ void __launch_bounds__(kThreads)
+// CW neighbouring columns of a row
+template <int CW> struct Cols { float v[CW]; };
+template <int CW> __device__ __forceinline__ Cols<CW> cols_load(const float* p) {
+  Cols<CW> r;
+  if constexpr (CW == 4) *reinterpret_cast<float4*>(r.v) = *reinterpret_cast<const float4*>(p);
+  else if constexpr (CW == 2) *reinterpret_cast<float2*>(r.v) = *reinterpret_cast<const float2*>(p);
+  else r.v[0] = *p;
+  return r;
+}
+template <int CW> __device__ __forceinline__ void cols_store(float* p, const Cols<CW>& r) {
+  if constexpr (CW == 4) *reinterpret_cast<float4*>(p) = *reinterpret_cast<const float4*>(r.v);
+  else if constexpr (CW == 2) *reinterpret_cast<float2*>(p) = *reinterpret_cast<const float2*>(r.v);
+  else *p = r.v[0];
+}
+
+// M rows of the state per thread (dkp <= 32 M), CW columns each; a block has 8 CW columns. Columns do not meet, so with
+// few sequences a block takes fewer of them. The next tokens' inputs are on their way while kSteps are walked (as many
+// as registers hold: M <= 8). Bound by the chain of steps: 2 sequences of 509 tokens, 4 heads of 128 x 128,
+// 135 us; with 32 columns a block (32 blocks) and loads waited for at every 16 tokens 332.
+template <typename T, int M, int CW>
+__global__ void __launch_bounds__(kThreads, M <= 4 ? 2 : 1)
 gla_sequence_kernel(const LinearAttnParams p) {
-  extern __shared__ float sm[];
+  constexpr int kCols = 8 * CW;
+  constexpr int kTok = kSteps / 8;           // tokens that a warp stages
+  constexpr bool kEarly = M <= 8;
+  extern __shared__ __align__(16) float sm[];
   pdl_enter();
   const int h = blockIdx.y, b = blockIdx.z, col0 = blockIdx.x * kCols;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -184,60 +204,87 @@ gla_sequence_kernel(const LinearAttnParams p) {
   float* sa = sk + kSteps * dkp;
   float* sv = sa + kSteps * dkp;             // [kSteps][kCols]
   float* so = sv + kSteps * kCols;           // [kSteps][8 warps][kCols]
-  const int cl = (lane & 7) * 4;             // this thread's columns within the block
+  const int cl = (lane & 7) * CW;            // this thread's columns within the block
   const int rg = warp * 4 + (lane >> 3);     // rows rg, rg + 32, ...
   const bool col_ok = col0 + cl < dvp;       // dvp is a multiple of 8
   float* S = p.state + (static_cast<long long>(b) * p.H + h) * dkp * dvp;
-  float4 s[M];
+  Cols<CW> s[M];
 #pragma unroll
   for (int m = 0; m < M; ++m) {
     const int r = rg + 32 * m;
-    s[m] = (r < dkp && col_ok) ? *reinterpret_cast<const float4*>(S + static_cast<long long>(r) * dvp + col0 + cl)
-                               : make_float4(0.f, 0.f, 0.f, 0.f);
+    if (r < dkp && col_ok) {
+      s[m] = cols_load<CW>(S + static_cast<long long>(r) * dvp + col0 + cl);
+    } else {
+#pragma unroll
+      for (int e = 0; e < CW; ++e) s[m].v[e] = 0.f;
+    }
   }
   const long long row0 = static_cast<long long>(b) * p.S;
+  T rq[kTok][M], rk[kTok][M], rv[kTok];
+  float ra[kTok][M];
+  auto fetch = [&](int t0) {                 // a warp takes whole tokens, lanes their channels
+#pragma unroll
+    for (int u = 0; u < kTok; ++u) {
+      const int t = t0 + warp + 8 * u;
+      if (t >= p.S) continue;
+      const long long at = (row0 + t) * p.ldp;
+#pragma unroll
+      for (int m = 0; m < M; ++m) {
+        const int c = lane + 32 * m;
+        if (c >= dkp) continue;
+        rq[u][m] = static_cast<const T*>(p.q)[at + static_cast<long long>(h) * dkp + c];
+        rk[u][m] = static_cast<const T*>(p.k)[at + static_cast<long long>(h) * dkp + c];
+        ra[u][m] = p.log_decay[(row0 + t) * ch + h * dkp + c];
+      }
+      if (lane < kCols && col0 + lane < dvp) rv[u] = static_cast<const T*>(p.v)[at + static_cast<long long>(h) * dvp + col0 + lane];
+    }
+  };
+  auto put = [&](int t0) {
+#pragma unroll
+    for (int u = 0; u < kTok; ++u) {
+      const int x = warp + 8 * u;
+      if (t0 + x >= p.S) continue;
+#pragma unroll
+      for (int m = 0; m < M; ++m) {
+        const int c = lane + 32 * m;
+        if (c >= dkp) continue;
+        sq[x * dkp + c] = to_f32(rq[u][m]) * p.q_scale;
+        sk[x * dkp + c] = to_f32(rk[u][m]);
+        sa[x * dkp + c] = expf(ra[u][m]);
+      }
+      if (lane < kCols) sv[x * kCols + lane] = col0 + lane < dvp ? to_f32(rv[u]) : 0.f;
+    }
+  };
+  if (kEarly) fetch(0);
   for (int t0 = 0; t0 < p.S; t0 += kSteps) {
     const int n = min(kSteps, p.S - t0);
-    for (int idx = tid; idx < n * dkp; idx += kThreads) {
-      const int t = idx / dkp, c = idx - t * dkp;
-      const long long off = (row0 + t0 + t) * p.ldp + static_cast<long long>(h) * dkp + c;
-      sq[idx] = to_f32(static_cast<const T*>(p.q)[off]) * p.q_scale;
-      sk[idx] = to_f32(static_cast<const T*>(p.k)[off]);
-      sa[idx] = expf(p.log_decay[(row0 + t0 + t) * ch + h * dkp + c]);
-    }
-    for (int idx = tid; idx < n * kCols; idx += kThreads) {
-      const int t = idx / kCols, c = idx - t * kCols;
-      sv[idx] = col0 + c < dvp
-                    ? to_f32(static_cast<const T*>(p.v)[(row0 + t0 + t) * p.ldp + static_cast<long long>(h) * dvp + col0 + c])
-                    : 0.f;
-    }
+    if (!kEarly) fetch(t0);
+    put(t0);
     __syncthreads();
+    if (kEarly) fetch(t0 + kSteps);
+#pragma unroll 4
     for (int t = 0; t < n; ++t) {
-      const float4 v = *reinterpret_cast<const float4*>(sv + t * kCols + cl);
-      float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+      const Cols<CW> v = cols_load<CW>(sv + t * kCols + cl);
+      Cols<CW> o;
+#pragma unroll
+      for (int e = 0; e < CW; ++e) o.v[e] = 0.f;
 #pragma unroll
       for (int m = 0; m < M; ++m) {
         const int r = rg + 32 * m;
         if (r < dkp) {
           const float a = sa[t * dkp + r], k = sk[t * dkp + r], q = sq[t * dkp + r];
-          s[m].x = fmaf(a, s[m].x, k * v.x);
-          s[m].y = fmaf(a, s[m].y, k * v.y);
-          s[m].z = fmaf(a, s[m].z, k * v.z);
-          s[m].w = fmaf(a, s[m].w, k * v.w);
-          o.x = fmaf(q, s[m].x, o.x);
-          o.y = fmaf(q, s[m].y, o.y);
-          o.z = fmaf(q, s[m].z, o.z);
-          o.w = fmaf(q, s[m].w, o.w);
+#pragma unroll
+          for (int e = 0; e < CW; ++e) {
+            s[m].v[e] = fmaf(a, s[m].v[e], k * v.v[e]);
+            o.v[e] = fmaf(q, s[m].v[e], o.v[e]);
+          }
         }
       }
 #pragma unroll
-      for (int d = 8; d < 32; d <<= 1) {
-        o.x += __shfl_xor_sync(0xffffffffu, o.x, d);
-        o.y += __shfl_xor_sync(0xffffffffu, o.y, d);
-        o.z += __shfl_xor_sync(0xffffffffu, o.z, d);
-        o.w += __shfl_xor_sync(0xffffffffu, o.w, d);
-      }
-      if (lane < 8) *reinterpret_cast<float4*>(so + (t * 8 + warp) * kCols + cl) = o;
+      for (int d = 8; d < 32; d <<= 1)
+#pragma unroll
+        for (int e = 0; e < CW; ++e) o.v[e] += __shfl_xor_sync(0xffffffffu, o.v[e], d);
+      if (lane < 8) cols_store<CW>(so + (t * 8 + warp) * kCols + cl, o);
     }
     __syncthreads();
     for (int idx = tid; idx < n * kCols; idx += kThreads) {
@@ -249,16 +296,16 @@ gla_sequence_kernel(const LinearAttnParams p) {
         p.o_raw[(row0 + t0 + t) * (p.H * dvp) + static_cast<long long>(h) * dvp + col0 + c] = a;
       }
     }
-    __syncthreads();
+    // no barrier here: what is put next was last read before the barrier above, and `so` is written again only behind
+    // the one that follows the next put
   }
 #pragma unroll
   for (int m = 0; m < M; ++m) {
     const int r = rg + 32 * m;
-    if (r < dkp && col_ok) *reinterpret_cast<float4*>(S + static_cast<long long>(r) * dvp + col0 + cl) = s[m];
+    if (r < dkp && col_ok) cols_store<CW>(S + static_cast<long long>(r) * dvp + col0 + cl, s[m]);
   }
 }
 
-// head norm and gate on the raw outputs; one warp per (row, head)
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
 gla_finish_kernel(const LinearAttnParams p) {
@@ -279,23 +326,30 @@ gla_finish_kernel(const LinearAttnParams p) {
                          p.out_scale);
 }
 
+template <typename T, int M, int CW>
+cudaError_t launch_sequence_of(const LinearAttnParams& p, cudaStream_t st) {
+  const dim3 grid((p.dvp + 8 * CW - 1) / (8 * CW), p.H, p.B);
+  const int bytes = (3 * kSteps * p.dkp + kSteps * 9 * 8 * CW) * static_cast<int>(sizeof(float));
+  const cudaError_t e = allow_smem<gla_sequence_kernel<T, M, CW>>(bytes);
+  if (e != cudaSuccess) return e;
+  return launch_kernel(gla_sequence_kernel<T, M, CW>, grid, dim3(kThreads), bytes, st, p);
+}
+// The widest columns that still give every SM a block.
+template <typename T, int M>
+cudaError_t launch_sequence_m(const LinearAttnParams& p, cudaStream_t st) {
+  const long long heads = static_cast<long long>(p.B) * p.H;
+  const int sms = current_sm_count();
+  if (heads * ((p.dvp + 31) / 32) >= sms) return launch_sequence_of<T, M, 4>(p, st);
+  if (heads * ((p.dvp + 15) / 16) >= sms) return launch_sequence_of<T, M, 2>(p, st);
+  return launch_sequence_of<T, M, 1>(p, st);
+}
 template <typename T>
 cudaError_t launch_sequence(const LinearAttnParams& p, cudaStream_t st) {
-  const dim3 grid((p.dvp + kCols - 1) / kCols, p.H, p.B), block(kThreads);
-  const size_t bytes = (3 * kSteps * p.dkp + kSteps * kCols + kSteps * 8 * kCols) * sizeof(float);
-#define CDEEP_GLA_SEQ(M)                                                                                     \
-  {                                                                                                          \
-    cudaError_t e = cudaFuncSetAttribute(gla_sequence_kernel<T, M>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                                         static_cast<int>(bytes));                                           \
-    if (e != cudaSuccess) return e;                                                                          \
-    return launch_kernel(gla_sequence_kernel<T, M>, grid, block, bytes, st, p);                              \
-  }
-  if (p.dkp <= 32) CDEEP_GLA_SEQ(1)
-  if (p.dkp <= 64) CDEEP_GLA_SEQ(2)
-  if (p.dkp <= 128) CDEEP_GLA_SEQ(4)
-  if (p.dkp <= 256) CDEEP_GLA_SEQ(8)
-  if (p.dkp <= 512) CDEEP_GLA_SEQ(16)
-#undef CDEEP_GLA_SEQ
+  if (p.dkp <= 32) return launch_sequence_m<T, 1>(p, st);
+  if (p.dkp <= 64) return launch_sequence_m<T, 2>(p, st);
+  if (p.dkp <= 128) return launch_sequence_m<T, 4>(p, st);
+  if (p.dkp <= 256) return launch_sequence_m<T, 8>(p, st);
+  if (p.dkp <= 512) return launch_sequence_m<T, 16>(p, st);
   return cudaErrorInvalidValue;
 }
 
