@@ -7,7 +7,7 @@
 // permutation is a stable counting sort of the expert ids; there is no atomic whose order
 // could change the result, and two runs give identical bytes.
 //
-// Two launches:
+// Up to kSmallTokens tokens: one block (route_small). More, two launches:
 //   route_lookup_hist : ids -> expert_ids, and one histogram per block of kTokPerBlock tokens
 //   route_rank        : totals + offsets from the block histograms, then each warp ranks a
 //                       contiguous slice of its block with match/ballot, in row order.
@@ -127,6 +127,100 @@ route_rank_kernel(const int* __restrict__ expert_ids, const int* __restrict__ bl
   }
 }
 
+// The whole dispatch of a decode step or a short prompt by one block: a warp owns a contiguous slice of the tokens (a
+// multiple of 32 of them) and keeps their experts in registers; histograms of the slices, their scan, and the ranks
+// follow without going through memory. Bound by latency: ids, table, four barriers. Rugedra 2048 wide, 64 sequences,
+// 7 dispatches of 512 rows a step: 30.4 ms for 16 steps with the two kernels below (2.3 + 6.0 us), 29.7 with this one.
+constexpr int kSmallThreads = 1024;
+constexpr int kSmallWarps = kSmallThreads / 32;
+constexpr int kSmallTokens = 4096;
+constexpr int kSmallPer = kSmallTokens / kSmallThreads;   // tokens per thread
+constexpr int kSmallExperts = 256;
+
+__global__ void __launch_bounds__(kSmallThreads)
+route_small_kernel(const long long* __restrict__ ids, const long long* __restrict__ table, int V, int E, int T,
+                   int* __restrict__ expert_ids, int* __restrict__ counts, int* __restrict__ offsets,
+                   int* __restrict__ perm, int* __restrict__ inv_perm) {
+  extern __shared__ int s_hist[];                         // [warps][E], then the slices' first positions
+  __shared__ int s_warp[kSmallExperts / 32];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  for (int k = tid; k < kSmallWarps * E; k += kSmallThreads) s_hist[k] = 0;
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const int rounds = (T + kSmallThreads - 1) / kSmallThreads;
+  const int base = warp * rounds * 32;
+  long long id[kSmallPer];
+  int e[kSmallPer];
+#pragma unroll
+  for (int k = 0; k < kSmallPer; ++k) {
+    const int i = base + k * 32 + lane;
+    id[k] = k < rounds && i < T ? ids[i] : 0;
+  }
+#pragma unroll
+  for (int k = 0; k < kSmallPer; ++k) {
+    const int i = base + k * 32 + lane;
+    e[k] = E;                                             // no token
+    if (k < rounds && i < T) {
+      const long long x = table[id[k] < 0 ? 0 : (id[k] > V - 1 ? V - 1 : id[k])];   // clamped to the table
+      e[k] = static_cast<int>(x < 0 ? 0 : (x > E - 1 ? E - 1 : x));                 // memory safety only
+      expert_ids[i] = e[k];
+    }
+  }
+  __syncthreads();                                        // the histograms are zero
+  int* mine = s_hist + warp * E;
+  unsigned peers[kSmallPer];
+#pragma unroll
+  for (int k = 0; k < kSmallPer; ++k) {
+    if (k >= rounds) break;                               // uniform
+    peers[k] = __match_any_sync(0xffffffffu, e[k]);
+    if (e[k] < E && lane == __ffs(peers[k]) - 1) mine[e[k]] += __popc(peers[k]);
+    __syncwarp();
+  }
+  __syncthreads();
+  // a thread per expert: its total over the slices, the scan over the experts, the slices' first positions
+  int total = 0;
+  if (tid < E) {
+#pragma unroll
+    for (int w = 0; w < kSmallWarps; ++w) total += s_hist[w * E + tid];
+  }
+  int incl = total;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, incl, d);
+    if (lane >= d) incl += v;
+  }
+  if (lane == 31 && warp < kSmallExperts / 32) s_warp[warp] = incl;
+  __syncthreads();
+  if (tid < E) {
+    int run = incl - total;
+    for (int w = 0; w < warp; ++w) run += s_warp[w];
+    counts[tid] = total;
+    offsets[tid] = run;
+    if (tid == E - 1) offsets[E] = run + total;
+#pragma unroll
+    for (int w = 0; w < kSmallWarps; ++w) {
+      const int c = s_hist[w * E + tid];
+      s_hist[w * E + tid] = run;
+      run += c;
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < kSmallPer; ++k) {
+    if (k >= rounds) break;
+    const int i = base + k * 32 + lane;
+    const unsigned lower = peers[k] & ((1u << lane) - 1u);
+    if (e[k] < E) {
+      const int pos = mine[e[k]] + __popc(lower);
+      perm[pos] = i;
+      inv_perm[i] = pos;
+    }
+    __syncwarp();
+    if (e[k] < E && lower == 0) mine[e[k]] += __popc(peers[k]);
+    __syncwarp();
+  }
+}
+
 size_t route_workspace_bytes(int T, int E) {
   const size_t nb = (static_cast<size_t>(T) + kTokPerBlock - 1) / kTokPerBlock;
   return (nb > 0 ? nb : 1) * static_cast<size_t>(E) * sizeof(int);
@@ -135,6 +229,9 @@ size_t route_workspace_bytes(int T, int E) {
 cudaError_t launch_route(const long long* ids, const long long* table, int V, int E, int T,
                          int* expert_ids, int* counts, int* offsets, int* perm, int* inv_perm,
                          int* block_hist, cudaStream_t stream) {
+  if (T > 0 && T <= kSmallTokens)                       // E is at most kSmallExperts at every entry
+    return launch_kernel(route_small_kernel, dim3(1), dim3(kSmallThreads), kSmallWarps * E * sizeof(int), stream, ids,
+                         table, V, E, T, expert_ids, counts, offsets, perm, inv_perm);
   const int nb = (T + kTokPerBlock - 1) / kTokPerBlock;
   const int blocks = nb > 0 ? nb : 1;  // T == 0 still writes zero counts and offsets
   route_lookup_hist_kernel<<<blocks, kRouteThreads, E * sizeof(int), stream>>>(
