@@ -89,6 +89,32 @@ struct AttnSmem {
   static constexpr int kDynamic = kTotal + 1024;
 };
 
+// two fp32 operations in one instruction, each rounded as its scalar form, and the maximum of three: the softmax warps
+// are bound by issue
+__device__ __forceinline__ unsigned long long pair2(float lo, float hi) {
+  unsigned long long v;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+  return v;
+}
+__device__ __forceinline__ void unpair2(unsigned long long v, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ unsigned long long fma_x2(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ unsigned long long add_x2(unsigned long long a, unsigned long long b) {
+  unsigned long long d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float d;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
+
 __device__ __forceinline__ float fast_exp2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -369,12 +395,14 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
               float m0 = __uint_as_float(cur[0]), m1 = __uint_as_float(cur[1]);
               float m2 = __uint_as_float(cur[2]), m3 = __uint_as_float(cur[3]);
 #pragma unroll
-              for (int i = 4; i < 32; i += 4) {
-                m0 = fmaxf(m0, __uint_as_float(cur[i]));
-                m1 = fmaxf(m1, __uint_as_float(cur[i + 1]));
-                m2 = fmaxf(m2, __uint_as_float(cur[i + 2]));
-                m3 = fmaxf(m3, __uint_as_float(cur[i + 3]));
+              for (int i = 4; i < 28; i += 8) {
+                m0 = max3(m0, __uint_as_float(cur[i]), __uint_as_float(cur[i + 4]));
+                m1 = max3(m1, __uint_as_float(cur[i + 1]), __uint_as_float(cur[i + 5]));
+                m2 = max3(m2, __uint_as_float(cur[i + 2]), __uint_as_float(cur[i + 6]));
+                m3 = max3(m3, __uint_as_float(cur[i + 3]), __uint_as_float(cur[i + 7]));
               }
+              m0 = max3(m0, __uint_as_float(cur[28]), __uint_as_float(cur[29]));
+              m1 = max3(m1, __uint_as_float(cur[30]), __uint_as_float(cur[31]));
               m_tile = fmaxf(m_tile, fmaxf(fmaxf(m0, m1), fmaxf(m2, m3)));
             } else {
 #pragma unroll
@@ -408,7 +436,8 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
         const float m_scaled = m_ref * p.scale_log2;
         {
           uint32_t va[32], vb[32];
-          float l0 = 0.f, l1 = 0.f;
+          unsigned long long l01 = 0ull;
+          const unsigned long long scale2 = pair2(p.scale_log2, p.scale_log2), minus2 = pair2(-m_scaled, -m_scaled);
           tmem_ld32(s_tmem, va);
 #pragma unroll
           for (int c = 0; c < 4; ++c) {
@@ -419,19 +448,22 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
             uint32_t pk[16];
 #pragma unroll
             for (int i = 0; i < 16; ++i) {
-              float e0 = fast_exp2(fmaf(__uint_as_float(cur[2 * i]), p.scale_log2, -m_scaled));
-              float e1 = fast_exp2(fmaf(__uint_as_float(cur[2 * i + 1]), p.scale_log2, -m_scaled));
+              float e0, e1;
+              unpair2(fma_x2(pair2(__uint_as_float(cur[2 * i]), __uint_as_float(cur[2 * i + 1])), scale2, minus2), e0, e1);
+              e0 = fast_exp2(e0);
+              e1 = fast_exp2(e1);
               if (diagonal) {
                 if (c * 32 + 2 * i >= n_vis) e0 = 0.f;
                 if (c * 32 + 2 * i + 1 >= n_vis) e1 = 0.f;
               }
-              l0 += e0;
-              l1 += e1;
+              l01 = add_x2(l01, pair2(e0, e1));
               const __nv_bfloat162 b2 = __floats2bfloat162_rn(e0, e1);
               pk[i] = *reinterpret_cast<const uint32_t*>(&b2);
             }
             tmem_st16(s_tmem + c * 16, pk);
           }
+          float l0, l1;
+          unpair2(l01, l0, l1);
           l_sum += l0 + l1;
         }
         tmem_st_wait();
