@@ -11,7 +11,6 @@
 //   * A block asks for its weights in L2 BEFORE it waits for the kernel ahead of it. A prefetch reads nothing into
 //     the program, so it may run ahead of whatever still writes; it takes the DRAM latency out of the step.
 //   * The partial sums are added in the order of the warps: results do not depend on timing.
-//   * Once it has started, a block asks for the weights of the block that will follow it on the SM.
 // Row groups (experts) are walked in passes of at most 32 rows of one group; empty groups end at once.
 // Bound by: L2 to SM traffic (weights once, the rows once per block: 7 to 9 TB/s) from 16 rows on, before that by
 // the launch (2.1 us at K = N = 768, one row; the tile kernel 6.8). The other figures stand at few_rows_taken.
@@ -35,7 +34,7 @@ struct FewParams {
   int half;                        // gated units: rows of a gate block, up rows follow (packed layout)
   int tiles, tiles2;               // blocks per group, of the second problem
   int prefetch;                    // ask for the block's own weights ahead of the kernel before
-  int ahead;                       // blocks on the device at a time
+  int sms;                         // of the device
 };
 
 __device__ __forceinline__ uint4 load_stream(const bf16* p) {
@@ -305,12 +304,6 @@ __global__ void __launch_bounds__(WK * 32, (NTMAX >= 8 ? 8 : 16) / WK) few_rows_
     m_lo = g.seg_offsets[at.group];
     m_hi = g.seg_offsets[at.group + 1];
   }
-  // the weights of the block that takes this one's place are asked for now
-  if (p.ahead > 0 && blockIdx.x + p.ahead < gridDim.x) {
-    const Block next = locate<EPI, MT>(p, blockIdx.x + p.ahead);
-    if (next.second || !g.seg_offsets || g.seg_offsets[next.group] < g.seg_offsets[next.group + 1])
-      prefetch_block<EPI, MT>(p, next);
-  }
   if (kChecks && g.seg_offsets) {
     // checking build: a segment table that is not 0 <= s[0] <= s[1] <= ... <= M stores nothing
     bool bad = false;
@@ -347,8 +340,10 @@ cudaError_t launch_few(const FewParams& p, cudaStream_t stream) {
   cudaError_t e = allow_smem<few_rows_kernel<EPI, MT, NTMAX, WK>>(smem);
   if (e != cudaSuccess) return e;
   FewParams q = p;
-  q.ahead = p.ahead * (NTMAX >= 8 ? 8 : 16) / WK;
   const unsigned grid = static_cast<unsigned>(p.tiles * p.g.num_groups + p.tiles2);
+  // Beyond one wave the asking ahead gets in the way of the reads themselves: 64 experts of 2 x 704 x 2048, 256 rows 100 us
+  // with it (each block asking for the next one's as well), 73 without; N 32000, 8 rows 39 / 32.
+  if (grid > static_cast<unsigned>(p.sms * (NTMAX >= 8 ? 8 : 16) / WK)) q.prefetch = 0;
   return launch_kernel(few_rows_kernel<EPI, MT, NTMAX, WK>, dim3(grid), dim3(WK * 32), smem, stream, q);
 }
 
@@ -363,7 +358,7 @@ cudaError_t launch_warps(const FewParams& p, cudaStream_t stream) {
 template <int EPI, int MT>
 cudaError_t launch_rows(const FewParams& p, cudaStream_t stream) {
   const long long blocks = static_cast<long long>(p.tiles) * p.g.num_groups + p.tiles2;
-  return blocks > 2LL * p.ahead ? launch_warps<EPI, MT, 4>(p, stream) : launch_warps<EPI, MT, 8>(p, stream);
+  return blocks > 2LL * p.sms ? launch_warps<EPI, MT, 4>(p, stream) : launch_warps<EPI, MT, 8>(p, stream);
 }
 
 template <int EPI>
@@ -377,17 +372,18 @@ cudaError_t launch_store(const FewParams& p, int mt, cudaStream_t stream) {
 static int store_mt(long long cols, int num_groups, int sm_count) { return num_groups * ((cols + 31) / 32) >= 2LL * sm_count ? 2 : 1; }
 
 // Which calls stream (us on one B200, this kernel / the tile kernel):
-//   row groups: up to 64 rows, or 4 per group. 64 experts of 2 x 704 x 2048: 104 rows 64 / 80, 512 rows 94 / 84 (8 rows
-//     of an expert fill half of a product, and the tile kernel reads the weights at the same rate whatever the rows);
-//     8 experts and a shared one: 32 rows 14 / 26, 64 rows 15 / 26.
+//   row groups: up to 64 rows, or 4 per group, or 8 for gated units. 64 experts of 2 x 704 x 2048, cold: 384 rows 69 / 89,
+//     512 rows 70 / 89 (half of them in one group 105 / 88), 1024 rows 79 / 90 (179 / 90: a pass per 32 rows of a group,
+//     hence the line); their down projections 46 / 46; 32 experts of 2 x 704 x 1024, 256 rows 28 / 44. 8 experts and a
+//     shared one: 32 rows 14 / 26, 64 rows 15 / 26.
 //   dense: up to 64 rows, unless the tokens, which every block reads again, cost more than the tile kernel's chains.
 //     K 2048, N 2048: 32 rows 5.5 / 11.6, 64 rows 7.1 / 11.6; K 4096, N 4096: 32 rows 12.9 / 16.1, 48 rows 17.6 / 16.1;
 //     K 2048, N 32000: 8 rows 29 / 37, 32 rows 41 / 27. The estimates below put the line between these: both sides in
 //     bytes per ns at the rates that they reach, 4.9 us and 0.21 us per 64 of K for a chain.
 bool few_rows_taken(int M, int num_groups, bool second, int kind, int cols, int K, int sm_count) {
-  if (num_groups > 1 || second) return M <= 64 || (!second && M <= 4 * num_groups);
-  if (M > 64) return false;
   const bool gated = kind == kEpiSwiGLU || kind == kEpiGlu;
+  if (num_groups > 1 || second) return M <= 64 || (!second && M <= (gated ? 8 : 4) * num_groups);
+  if (M > 64) return false;
   const int per_block = gated ? 16 : 16 * store_mt(cols, 1, sm_count);
   const long long weights = 2LL * cols * K * (gated ? 2 : 1);
   const long long tokens = 2LL * M * K * ((cols + per_block - 1) / per_block);
@@ -412,7 +408,7 @@ cudaError_t launch_few_rows(const GemmParams& g, int kind, const GemmOperand& op
   p.tiles2 = second ? (second->out_cols + 15) / 16 : 0;
   // of a grouped call only as much is asked for ahead of time as its rows are sure to use
   p.prefetch = g.num_groups == 1 || g.M >= 2 * g.num_groups;
-  p.ahead = sm_count;
+  p.sms = sm_count;
   if (kind == kEpiSwiGLU || kind == kEpiGlu) {
     p.tiles = (g.out_cols + 15) / 16;
     return kind == kEpiSwiGLU ? launch_rows<kEpiSwiGLU, 2>(p, stream) : launch_rows<kEpiGlu, 2>(p, stream);
