@@ -372,18 +372,18 @@ cudaError_t launch_store(const FewParams& p, int mt, cudaStream_t stream) {
 static int store_mt(long long cols, int num_groups, int sm_count) { return num_groups * ((cols + 31) / 32) >= 2LL * sm_count ? 2 : 1; }
 
 // Which calls stream (us on one B200, this kernel / the tile kernel):
-//   row groups: up to 64 rows, or 4 per group, or 8 for gated units. 64 experts of 2 x 704 x 2048, cold: 384 rows 69 / 89,
-//     512 rows 70 / 89 (half of them in one group 105 / 88), 1024 rows 79 / 90 (179 / 90: a pass per 32 rows of a group,
-//     hence the line); their down projections 46 / 46; 32 experts of 2 x 704 x 1024, 256 rows 28 / 44. 8 experts and a
+//   row groups: up to 64 rows, or 8 per group. 64 experts of 2 x 704 x 2048, cold: 384 rows 69 / 89, 512 rows 70 / 89
+//     (half of them in one group 105 / 88), 1024 rows 79 / 90 (179 / 90: a pass per 32 rows of a group, hence the line);
+//     their down projections 46 / 46, in a step behind one another 16 steps of Rugedra 26.0 / 26.7 ms; 32 experts of 2 x 704 x 1024, 256 rows 28 / 44. 8 experts and a
 //     shared one: 32 rows 14 / 26, 64 rows 15 / 26.
 //   dense: up to 64 rows, unless the tokens, which every block reads again, cost more than the tile kernel's chains.
 //     K 2048, N 2048: 32 rows 5.5 / 11.6, 64 rows 7.1 / 11.6; K 4096, N 4096: 32 rows 12.9 / 16.1, 48 rows 17.6 / 16.1;
 //     K 2048, N 32000: 8 rows 29 / 37, 32 rows 41 / 27. The estimates below put the line between these: both sides in
 //     bytes per ns at the rates that they reach, 4.9 us and 0.21 us per 64 of K for a chain.
 bool few_rows_taken(int M, int num_groups, bool second, int kind, int cols, int K, int sm_count) {
-  const bool gated = kind == kEpiSwiGLU || kind == kEpiGlu;
-  if (num_groups > 1 || second) return M <= 64 || (!second && M <= (gated ? 8 : 4) * num_groups);
+  if (num_groups > 1 || second) return M <= 64 || (!second && M <= 8 * num_groups);
   if (M > 64) return false;
+  const bool gated = kind == kEpiSwiGLU || kind == kEpiGlu;
   const int per_block = gated ? 16 : 16 * store_mt(cols, 1, sm_count);
   const long long weights = 2LL * cols * K * (gated ? 2 : 1);
   const long long tokens = 2LL * M * K * ((cols + per_block - 1) / per_block);

@@ -1,5 +1,5 @@
-"""Row groups that stream their weights with more than 64 rows in all (csrc/gemm_few_rows.cu): up to 8 a group on average for
-gated units, most of them in one group among them, at the last call that streams and the first that does not."""
+"""Row groups that stream their weights with more than 64 rows in all (csrc/gemm_few_rows.cu): up to 8 a group on average,
+most of them in one group among them, at the last call that streams and the first that does not."""
 import pytest
 
 import test_gpu_n_few_rows as few
