@@ -38,8 +38,9 @@ struct KeyRange {
   int kept, first, slot0;      // keys n < kept: slot n; else slot0 + (n - kept), wrapped once
   int wrap;                    // slots from `wrap` on are lower by `window`
   int window;
-  __device__ __forceinline__ KeyRange(const WindowAttnParams& p, int split, int splits) {
-    i = window_pos0(p);
+  __device__ __forceinline__ KeyRange(const WindowAttnParams& p, int split, int splits) : KeyRange(p, window_pos0(p), split, splits) {}
+  __device__ __forceinline__ KeyRange(const WindowAttnParams& p, int pos, int split, int splits) {
+    i = pos;
     const WindowKeys keys(i, p.window, p.keep);
     kept = keys.kept;
     first = keys.first;
@@ -78,25 +79,31 @@ __global__ void __launch_bounds__(kThreads, REP * DC <= 4 && sizeof(T) == 2 ? 3 
 window_decode_scores_kernel(const DecodeParams p) {
   extern __shared__ float sm[];        // [REP][dp] queries
   __shared__ float s_m[kWarps][REP], s_l[kWarps][REP];
-  pdl_enter();
   const WindowAttnParams& a = p.a;
   const int split = blockIdx.x, b = blockIdx.z, rep = a.H / a.G, groups = (rep + REP - 1) / REP;
   const int c = blockIdx.y / groups, h0 = c * rep + (blockIdx.y % groups) * REP;
   const int nh = min(REP, (c + 1) * rep - h0);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, sub = lane & 7, rg = lane >> 3;
   const int dp = a.dp, vp = a.vp;
+  // The rows of this block's keys and values are asked for in L2 before the wait for the kernel ahead: a prefetch reads
+  // nothing into the program. The position may still be an earlier one here; it only chooses slots of the ring, and is
+  // read again below.
+  if (blockIdx.y % groups == 0) {
+    const int pos = a.pos_dev ? *reinterpret_cast<const volatile int*>(a.pos_dev) : a.pos0;
+    const KeyRange hint(a, min(max(pos, 0), 1 << 30), split, p.splits);
+    const long long row = b * static_cast<long long>(a.keep + a.window);
+    for (int n = tid; n < hint.nk; n += kThreads) {
+      const long long at = (row + hint.slot(hint.n0 + n)) * a.G + c;
+      prefetch_l2_bulk(static_cast<const T*>(a.ring_k) + at * dp, static_cast<uint32_t>(dp * sizeof(T)));
+      prefetch_l2_bulk(static_cast<const T*>(a.ring_v) + at * vp, static_cast<uint32_t>(vp * sizeof(T)));
+    }
+  }
+  pdl_enter();
   const KeyRange r(a, split, p.splits);
   const long long slots = a.keep + a.window;
   T* ring_k = static_cast<T*>(a.ring_k) + (b * slots * a.G + c) * dp;
   const long long stride = static_cast<long long>(a.G) * dp;
   const bool has_new = r.nk > 0 && r.n0 + r.nk == r.count;
-  // the values of this block's keys are asked for in L2 now: the keys alone leave the memory idle most of the time
-  {
-    const T* v = static_cast<const T*>(a.ring_v) + (b * slots * a.G + c) * static_cast<long long>(vp);
-    if (blockIdx.y % groups == 0)
-      for (int n = tid; n < r.nk; n += kThreads)
-        prefetch_l2_bulk(v + static_cast<long long>(r.slot(r.n0 + n)) * a.G * vp, static_cast<uint32_t>(vp * sizeof(T)));
-  }
   // Rows in flight per lane; the first ones are on their way before the query is there.
   constexpr int kAhead = DC * sizeof(T) <= 4 ? 4 : 2;
   constexpr int kStep = kWarps * 4;             // rows of the block per step
@@ -352,7 +359,7 @@ window_decode_values_kernel(const DecodeParams p) {
 // (position, query, first keys, statistics) and, with three on an SM, the time that its keys take at the SM's share of
 // the memory's rate (44 bytes per ns). One B200, 32 sequences, 4 key heads of 128, 516 keys, scores / values us: 8 splits
 // (1 024 blocks, three waves of 64 keys each, the rule before) 15.0 / 15.4, 3 splits (one wave) 12.4 / 8.8, the
-// prefetch of the values included in the first.
+// prefetch of the rows included in the first.
 constexpr int kMostSplits = 8;             // of a portable cluster
 int choose_splits(const WindowAttnParams& a, int rep_block) {
   const int rep = a.H / a.G, keys = a.keep + a.window;
