@@ -1,6 +1,6 @@
 // Matrix products of few rows (decode steps, short prompts): out[r, n] = epilogue(sum_k A[r, k] W[n, k]).
 //
-// Such a call is a read of the weights: 2 bytes per weight against at most 64 rows of work. The tile kernel
+// Such a call is a read of the weights: 2 bytes per weight against at most 64 rows of work (8 of a row group). The tile kernel
 // (gemm_sm100.cuh) runs it as chains of 128-row tensor-core tiles with barriers, tensor memory and an
 // issuing thread between them: 4.9 us before its first result and 0.21 us per 64 elements of K, whatever the
 // rows. Here a block takes 16 (or 32) weight rows and its eight warps a share of K each; weights and rows go
