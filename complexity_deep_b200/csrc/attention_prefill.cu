@@ -539,13 +539,8 @@ cudaError_t launch_one(const CUtensorMap& q, const CUtensorMap& kv, const CUtens
   const int sms = current_sm_count();
   const dim3 grid(static_cast<unsigned>(items < sms ? items : sms), 1, 1);
   constexpr int bytes = AttnSmem<KB, VB>::kDynamic;
-  static bool attr_done = false;
-  if (!attr_done) {
-    cudaError_t e = cudaFuncSetAttribute(attention_prefill_kernel<KB, VB, kLatent>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (e != cudaSuccess) return e;
-    attr_done = true;
-  }
+  const cudaError_t e = allow_smem<attention_prefill_kernel<KB, VB, kLatent>>(bytes);
+  if (e != cudaSuccess) return e;
   return launch_kernel(attention_prefill_kernel<KB, VB, kLatent>, grid, dim3(kAttnThreads), bytes, stream, q, kv, rot, p);
 }
 

@@ -1,10 +1,10 @@
 // Internal launch functions shared by the translation units of libcdeep.so.
 #pragma once
-#include <atomic>
 #include <cstddef>
 #include <cstdlib>
 #include <cuda_runtime.h>
 #include "../../include/cdeep.h"
+#include "smem_limit.h"
 
 namespace cdeep {
 
@@ -35,14 +35,16 @@ inline cudaError_t launch_kernel(void (*kern)(P...), dim3 grid, dim3 block, size
   return cudaLaunchKernelEx(&cfg, kern, static_cast<A&&>(args)...);
 }
 
-// Raises a kernel's limit of dynamic shared memory; asks the driver only when it grows.
+// Raises a kernel's limit of dynamic shared memory on the current device; asks the driver only when it grows.
 template <auto kKernel>
 inline cudaError_t allow_smem(int bytes) {
-  static std::atomic<int> allowed{0};
-  if (bytes <= allowed.load(std::memory_order_relaxed)) return cudaSuccess;
-  const cudaError_t e = cudaFuncSetAttribute(kKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  if (e == cudaSuccess) allowed.store(bytes, std::memory_order_relaxed);
-  return e;
+  static SmemLimit limit;
+  int device = 0;
+  const cudaError_t e = cudaGetDevice(&device);
+  if (e != cudaSuccess) return e;
+  return static_cast<cudaError_t>(limit.raise(device, bytes, [](int n) {
+    return static_cast<int>(cudaFuncSetAttribute(kKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, n));
+  }));
 }
 
 size_t route_workspace_bytes(int T, int E);
