@@ -2,8 +2,9 @@
 // matrix product of models that run entirely in fp32 (no reduced-precision mode anywhere on that path).
 //
 // With `seg` the grid's third axis is the group: its rows [seg[g], seg[g + 1]) of a meet the g-th N rows of b.
-// Every output is one chain of fused multiply-adds over k in ascending order, whatever the tile: results depend on
-// neither the number of rows nor the tile that was chosen.
+// Every output is one chain of fused multiply-adds over k in ascending order, whatever the tile, and its last factor and
+// the residual are one more (written as such, so that no compiler chooses): results depend on neither the number of rows
+// nor the tile nor the width of the stores.
 //   * Both operands lie transposed in shared memory, two stages; the next stage is on its way in registers while one
 //     is multiplied. A thread holds TM x TN outputs; products go in pairs of columns (fma.rn.f32x2: half the
 //     instructions; 1303 against 1543 us with single ones for 1018 x 1024 x 32000).
@@ -155,30 +156,33 @@ linear_f32_kernel(const LinearF32 p) {
       float v[4];
       unpair(acc[i][2 * c], v[0], v[1]);
       unpair(acc[i][2 * c + 1], v[2], v[3]);
+      if (p.act == 1) {
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        if (p.act == 1) v[j] = fmaxf(v[j], 0.f) * fmaxf(v[j], 0.f);
-        v[j] *= p.scale;
+        for (int j = 0; j < 4; ++j) v[j] = fmaxf(v[j], 0.f) * fmaxf(v[j], 0.f);
       }
       const size_t at = static_cast<size_t>(m) * N + n;
       if (p.vec && n + 4 <= N) {
+        float f[4] = {p.scale, p.scale, p.scale, p.scale}, r[4];
         if (p.col_scale) {
-          const float4 q = *reinterpret_cast<const float4*>(p.col_scale + n);
-          v[0] *= q.x; v[1] *= q.y; v[2] *= q.z; v[3] *= q.w;
+#pragma unroll
+          for (int j = 0; j < 4; ++j) v[j] *= p.scale;
+          *reinterpret_cast<float4*>(f) = *reinterpret_cast<const float4*>(p.col_scale + n);
         }
-        if (p.residual) {
-          const float4 q = *reinterpret_cast<const float4*>(p.residual + at);
-          v[0] += q.x; v[1] += q.y; v[2] += q.z; v[3] += q.w;
-        }
+        if (p.residual) *reinterpret_cast<float4*>(r) = *reinterpret_cast<const float4*>(p.residual + at);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) v[j] = p.residual ? fmaf(v[j], f[j], r[j]) : v[j] * f[j];
         *reinterpret_cast<float4*>(p.out + at) = make_float4(v[0], v[1], v[2], v[3]);
         continue;
       }
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         if (n + j >= N) break;
-        if (p.col_scale) v[j] *= p.col_scale[n + j];
-        if (p.residual) v[j] += p.residual[at + j];
-        p.out[at + j] = v[j];
+        float f = p.scale;
+        if (p.col_scale) {
+          v[j] *= p.scale;
+          f = p.col_scale[n + j];
+        }
+        p.out[at + j] = p.residual ? fmaf(v[j], f, p.residual[at + j]) : v[j] * f;
       }
     }
   }

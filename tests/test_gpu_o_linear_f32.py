@@ -3,6 +3,7 @@
 Tolerance: a chain of K fused multiply-adds is off by at most K 2^-24 sum |x| |w| (1 + tiny), scale, column factor and
 residual by one rounding each. Every output is one chain over k, whatever the tile, so that a row by itself and the
 same row among many (which take other tiles) agree to the bit."""
+import numpy as np
 import pytest
 import torch
 
@@ -48,3 +49,22 @@ def test_row_groups(counts, K, N):
     for e, (a, b) in enumerate(zip(seg[:-1], seg[1:])):
         xd, wd = x[a:b].double(), w[e].double()
         _near(got[a:b], xd @ wd.t(), (xd.abs() @ wd.abs().t()) * (K + 2) * U)
+
+
+@pytest.mark.parametrize("T,K,N", [(5, 40, 31), (130, 64, 1000), (600, 24, 1028), (7, 516, 66)])
+def test_factors_and_residual_round_as_one_multiply_add(T, K, N):
+    """Behind the sum come the scale, the column factor and the residual; the last factor and the residual round once,
+    whether the columns are stored by fours or singly. 80-bit numbers hold the product exactly."""
+    from complexity_deep_b200 import ops
+    g = torch.Generator().manual_seed(T + N)
+    x, w = torch.randn(T, K, generator=g).cuda(), torch.randn(N, K, generator=g).cuda()
+    res, col = torch.randn(T, N, generator=g), torch.randn(N, generator=g)
+    y, scale = ops.project(x, w).cpu().numpy(), np.float32(0.7)
+    wide = lambda a: a.numpy().astype(np.longdouble)
+    for c in (None, col):
+        first, last = (y, np.longdouble(scale)) if c is None else (y * scale, wide(c))
+        want = first.astype(np.longdouble) * last
+        got = ops.linear_to_f32(x, w, residual=res.cuda(), col_scale=None if c is None else c.cuda(), scale=0.7)
+        assert np.array_equal(got.cpu().numpy(), (want + wide(res)).astype(np.float32))
+        got = ops.linear_to_f32(x, w, col_scale=None if c is None else c.cuda(), scale=0.7)
+        assert np.array_equal(got.cpu().numpy(), want.astype(np.float32))
