@@ -297,3 +297,17 @@ print("ok")
     proc = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True,
                           env={**__import__("os").environ, "PYTHONPATH": ROOT})
     assert proc.returncode == 0 and proc.stdout.strip() == "ok", proc.stderr
+
+
+def test_import_with_a_torch_without_cuda():
+    """A torch that was built without CUDA has no _cuda_* functions; the package still imports and plans."""
+    import subprocess
+    import sys
+    from conftest import ROOT
+    code = ("import torch\n"
+            "for name in [n for n in dir(torch._C) if n.startswith('_cuda_getDevice') or n == '_cuda_getCurrentRawStream']:\n"
+            "    delattr(torch._C, name)\n"
+            "torch.cuda.is_available = lambda: False\n"
+            "from complexity_deep_b200 import ops\n"
+            "assert ops.choose_block_n(704, 32, 8) in (32, 64, 128, 256)\n")
+    subprocess.run([sys.executable, "-c", code], cwd=ROOT, check=True, timeout=300)
