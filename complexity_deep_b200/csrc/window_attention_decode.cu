@@ -38,9 +38,8 @@ struct KeyRange {
   int kept, first, slot0;      // keys n < kept: slot n; else slot0 + (n - kept), wrapped once
   int wrap;                    // slots from `wrap` on are lower by `window`
   int window;
-  __device__ __forceinline__ KeyRange(const WindowAttnParams& p, int split, int splits) : KeyRange(p, window_pos0(p), split, splits) {}
-  __device__ __forceinline__ KeyRange(const WindowAttnParams& p, int pos, int split, int splits) {
-    i = pos;
+  __device__ __forceinline__ KeyRange(const WindowAttnParams& p, int split, int splits) {
+    i = window_pos0(p);
     const WindowKeys keys(i, p.window, p.keep);
     kept = keys.kept;
     first = keys.first;
@@ -73,54 +72,27 @@ __device__ __forceinline__ float group8_add(float v) {
   return v;
 }
 
-// REP query heads per block; DC chunks of 8 elements per lane (head width up to 64 DC)
+// REP query heads per block; DC chunks of 8 elements per lane (head width up to 64 DC). Keys are read behind the query, and
+// nothing is asked for in L2 ahead of the kernel before. With the first keys loaded ahead of the query and the rows of the
+// keys and values asked for ahead of time, steps of Pimezen took, us, with / without: 2048 wide, 1028 keys, 64 sequences
+// 1 890 / 1 689, 32 1 426 / 1 341; 1024 wide, 516 keys, 64 790 / 753, 32 566 / 547, 1 344 / 341.
 template <typename T, int REP, int DC>
 __global__ void __launch_bounds__(kThreads, REP * DC <= 4 && sizeof(T) == 2 ? 3 : 1)
 window_decode_scores_kernel(const DecodeParams p) {
   extern __shared__ float sm[];        // [REP][dp] queries
   __shared__ float s_m[kWarps][REP], s_l[kWarps][REP];
+  pdl_enter();
   const WindowAttnParams& a = p.a;
   const int split = blockIdx.x, b = blockIdx.z, rep = a.H / a.G, groups = (rep + REP - 1) / REP;
   const int c = blockIdx.y / groups, h0 = c * rep + (blockIdx.y % groups) * REP;
   const int nh = min(REP, (c + 1) * rep - h0);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, sub = lane & 7, rg = lane >> 3;
   const int dp = a.dp, vp = a.vp;
-  // The rows of this block's keys and values are asked for in L2 before the wait for the kernel ahead: a prefetch reads
-  // nothing into the program. The position may still be an earlier one here; it only chooses slots of the ring, and is
-  // read again below.
-  if (blockIdx.y % groups == 0) {
-    const int pos = a.pos_dev ? *reinterpret_cast<const volatile int*>(a.pos_dev) : a.pos0;
-    const KeyRange hint(a, min(max(pos, 0), 1 << 30), split, p.splits);
-    const long long row = b * static_cast<long long>(a.keep + a.window);
-    for (int n = tid; n < hint.nk; n += kThreads) {
-      const long long at = (row + hint.slot(hint.n0 + n)) * a.G + c;
-      prefetch_l2_bulk(static_cast<const T*>(a.ring_k) + at * dp, static_cast<uint32_t>(dp * sizeof(T)));
-      prefetch_l2_bulk(static_cast<const T*>(a.ring_v) + at * vp, static_cast<uint32_t>(vp * sizeof(T)));
-    }
-  }
-  pdl_enter();
   const KeyRange r(a, split, p.splits);
   const long long slots = a.keep + a.window;
   T* ring_k = static_cast<T*>(a.ring_k) + (b * slots * a.G + c) * dp;
   const long long stride = static_cast<long long>(a.G) * dp;
   const bool has_new = r.nk > 0 && r.n0 + r.nk == r.count;
-  // Rows in flight per lane; the first ones are on their way before the query is there.
-  constexpr int kAhead = DC * sizeof(T) <= 4 ? 4 : 2;
-  constexpr int kStep = kWarps * 4;             // rows of the block per step
-  Raw8<T> kf[kAhead][DC];
-  auto load_row = [&](int base, int u) {
-    const int n = min(base + u * kStep + warp * 4 + rg, r.nk - 1);          // rows past the end are not used
-    const T* k = ring_k + static_cast<long long>(r.slot(r.n0 + n)) * stride;
-#pragma unroll
-    for (int e = 0; e < DC; ++e) {
-      const int d = (e * 8 + sub) * 8;
-      raw_load(k + (d < dp ? d : 0), kf[u][e]);                             // past the head: the query is zero
-    }
-  };
-  if (r.nk > 0) {
-#pragma unroll
-    for (int u = 0; u < kAhead; ++u) load_row(0, u);
-  }
 
   auto rms_scale = [&](const T* x) {
     float ss = 0.f;
@@ -158,10 +130,12 @@ window_decode_scores_kernel(const DecodeParams p) {
 #pragma unroll
       for (int y = 0; y < 8; ++y) qf[x][e][y] = (x < nh && d < dp) ? sm[x * dp + d + y] : 0.f;
     }
-  // The kAhead x REP scores of a lane group are finished by its lanes: lane `sub` takes the head sub % REP and, in
-  // `kRounds` rounds, row sub / REP + round * (8 / REP).
+  // Rows in flight per lane.  The kAhead x REP scores of a lane group are finished by its lanes: lane
+  // `sub` takes the head sub % REP and, in `kRounds` rounds, row sub / REP + round * (8 / REP).
+  constexpr int kAhead = DC * sizeof(T) <= 4 ? 4 : 2;
   constexpr int kRowsRound = 8 / REP < kAhead ? 8 / REP : kAhead;
   constexpr int kRounds = kAhead / kRowsRound;
+  constexpr int kStep = kWarps * 4;             // rows of the block per step
   const int my_head = sub % REP, my_row = sub / REP;
   float r1 = 0.f, r2 = 0.f, m = -FLT_MAX, l = 0.f;
   if (my_head < nh) {
@@ -170,10 +144,16 @@ window_decode_scores_kernel(const DecodeParams p) {
   }
   float* out = p.scores + (static_cast<long long>(b) * a.H + h0 + (my_head < nh ? my_head : 0)) * p.n_max;
   for (int base = 0; base < r.nk; base += kStep * kAhead) {
+    Raw8<T> kf[kAhead][DC];
 #pragma unroll
     for (int u = 0; u < kAhead; ++u) {
-      // of the first rows only the new token's is loaded again: it was written after they were asked for
-      if (base > 0 || (has_new && base + u * kStep + warp * 4 + rg >= r.nk - 1)) load_row(base, u);
+      const int n = min(base + u * kStep + warp * 4 + rg, r.nk - 1);      // rows past the end are not used
+      const T* k = ring_k + static_cast<long long>(r.slot(r.n0 + n)) * stride;
+#pragma unroll
+      for (int e = 0; e < DC; ++e) {
+        const int d = (e * 8 + sub) * 8;
+        raw_load(k + (d < dp ? d : 0), kf[u][e]);                         // past the head: the query is zero
+      }
     }
     float s[kAhead][REP];
 #pragma unroll
@@ -282,8 +262,9 @@ __host__ __device__ inline int values_smem_floats(int vp) {
   return REP * 8 * kThreads + REP * vp;          // the threads' sums [REP * 8][kThreads], the block's output [REP][vp]
 }
 
-template <typename T, int REP>
-__global__ void __launch_bounds__(kThreads, REP <= 2 && sizeof(T) == 2 ? 3 : 2)
+// kAhead rows in flight per thread, kPerSm blocks on an SM
+template <typename T, int REP, int kAhead, int kPerSm>
+__global__ void __launch_bounds__(kThreads, kPerSm)
 window_decode_values_kernel(const DecodeParams p) {
   extern __shared__ float sm[];
   pdl_enter();
@@ -308,7 +289,6 @@ window_decode_values_kernel(const DecodeParams p) {
   for (int x = 0; x < REP; ++x)
 #pragma unroll
     for (int e = 0; e < 8; ++e) acc[x][e] = 0.f;
-  constexpr int kAhead = REP <= 2 && sizeof(T) == 2 ? 6 : 4;
   if (active) {
     for (int at = row; at < r.nk; at += rows * kAhead) {
       Raw8<T> vf[kAhead];
@@ -358,8 +338,7 @@ window_decode_values_kernel(const DecodeParams p) {
 // Splits of the keys of a (head group, sequence): those whose last wave ends first. A block costs about 4 us of its own
 // (position, query, first keys, statistics) and, with three on an SM, the time that its keys take at the SM's share of
 // the memory's rate (44 bytes per ns). One B200, 32 sequences, 4 key heads of 128, 516 keys, scores / values us: 8 splits
-// (1 024 blocks, three waves of 64 keys each, the rule before) 15.0 / 15.4, 3 splits (one wave) 12.4 / 8.8, the
-// prefetch of the rows included in the first.
+// (1 024 blocks, three waves of 64 keys each, the rule before) 15.0 / 15.4, 3 splits (one wave) 9.4 / 8.9.
 constexpr int kMostSplits = 8;             // of a portable cluster
 int choose_splits(const WindowAttnParams& a, int rep_block) {
   const int rep = a.H / a.G, keys = a.keep + a.window;
@@ -388,23 +367,11 @@ cudaError_t launch_scores(const DecodeParams& p, dim3 grid, cudaStream_t st) {
   return launch_kernel(window_decode_scores_kernel<T, REP, DC>, grid, dim3(kThreads), REP * p.a.dp * sizeof(float), st, p);
 }
 
-template <typename T, int REP>
-cudaError_t launch_both(const DecodeParams& p, cudaStream_t st) {
-  const int rep = p.a.H / p.a.G;
-  const dim3 grid(p.splits, p.a.G * ((rep + REP - 1) / REP), p.a.B);
-  cudaError_t e = p.a.dp <= 64    ? launch_scores<T, REP, 1>(p, grid, st)
-                  : p.a.dp <= 128 ? launch_scores<T, REP, 2>(p, grid, st)
-                                  : launch_scores<T, REP, 4>(p, grid, st);
-  if (e != cudaSuccess) return e;
-  const int mix_bytes = p.a.H * (2 + kMixKeys) * static_cast<int>(sizeof(float));
-  e = cudaFuncSetAttribute(window_decode_mix_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, mix_bytes);
-  if (e != cudaSuccess) return e;
-  e = launch_kernel(window_decode_mix_kernel<T>, dim3((p.n_max + kMixKeys - 1) / kMixKeys, p.a.B), dim3(kThreads),
-                    mix_bytes, st, p);
-  if (e != cudaSuccess) return e;
+template <typename T, int REP, int kAhead, int kPerSm>
+cudaError_t launch_values(const DecodeParams& p, dim3 grid, cudaStream_t st) {
   const int bytes = values_smem_floats<REP>(p.a.vp) * static_cast<int>(sizeof(float));
-  auto kern = window_decode_values_kernel<T, REP>;
-  e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  auto kern = window_decode_values_kernel<T, REP, kAhead, kPerSm>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
@@ -421,6 +388,31 @@ cudaError_t launch_both(const DecodeParams& p, cudaStream_t st) {
   cfg.attrs = attr;
   cfg.numAttrs = 2;
   return cudaLaunchKernelEx(&cfg, kern, p);
+}
+
+template <typename T, int REP>
+cudaError_t launch_both(const DecodeParams& p, cudaStream_t st) {
+  const int rep = p.a.H / p.a.G;
+  const dim3 grid(p.splits, p.a.G * ((rep + REP - 1) / REP), p.a.B);
+  cudaError_t e = p.a.dp <= 64    ? launch_scores<T, REP, 1>(p, grid, st)
+                  : p.a.dp <= 128 ? launch_scores<T, REP, 2>(p, grid, st)
+                                  : launch_scores<T, REP, 4>(p, grid, st);
+  if (e != cudaSuccess) return e;
+  const int mix_bytes = p.a.H * (2 + kMixKeys) * static_cast<int>(sizeof(float));
+  e = cudaFuncSetAttribute(window_decode_mix_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, mix_bytes);
+  if (e != cudaSuccess) return e;
+  e = launch_kernel(window_decode_mix_kernel<T>, dim3((p.n_max + kMixKeys - 1) / kMixKeys, p.a.B), dim3(kThreads),
+                    mix_bytes, st, p);
+  if (e != cudaSuccess) return e;
+  if constexpr (REP <= 2 && sizeof(T) == 2) {
+    // six rows in flight and three blocks on an SM, unless four blocks on an SM end a wave earlier: 32 sequences of 516 keys
+    // (one wave of either) 8.9 us, with four and four 10.1; 64 of 1028 (1 024 blocks) 41.5 / 37.3
+    const long long blocks = static_cast<long long>(grid.x) * grid.y * grid.z, sms = current_sm_count();
+    if ((blocks + 3 * sms - 1) / (3 * sms) <= (blocks + 4 * sms - 1) / (4 * sms)) return launch_values<T, REP, 6, 3>(p, grid, st);
+    return launch_values<T, REP, 4, 4>(p, grid, st);
+  } else {
+    return launch_values<T, REP, 4, 2>(p, grid, st);
+  }
 }
 
 template <typename T>

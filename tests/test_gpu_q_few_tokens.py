@@ -53,13 +53,14 @@ def test_rotary_embedding_does_not_depend_on_the_number_of_tokens(hq, hkv, D):
 
 @pytest.mark.parametrize("dtype", [BF, F32], ids=["bf16", "fp32"])
 @pytest.mark.parametrize("B,H,G,size,keep", [(148, 2, 1, 150, 3), (100, 1, 1, 195, 0), (44, 4, 2, 260, 4), (60, 2, 1, 340, 2),
-                                             (1, 4, 1, 400, 5), (20, 5, 1, 300, 1)])
+                                             (1, 4, 1, 400, 5), (20, 5, 1, 300, 1), (63, 8, 8, 20, 1), (75, 12, 6, 24, 0)])
 def test_window_decode_splits(B, H, G, size, keep, dtype):
     w = Window(dtype, size + keep + 6, H, G, 16, 16, size, keep, B, seed=B)
     assert _rel(w.run([w.T - 5] + [1] * 5), w.reference()) <= TOL[dtype]
 
 
-@pytest.mark.parametrize("B,H,dk,dv", [(1, 1, 160, 16), (2, 2, 48, 80), (40, 4, 32, 32), (3, 5, 272, 48), (80, 4, 128, 32), (1, 2, 512, 144)])
+@pytest.mark.parametrize("B,H,dk,dv", [(1, 1, 160, 16), (2, 2, 48, 80), (40, 4, 32, 32), (3, 5, 272, 48), (80, 4, 128, 32), (1, 2, 512, 144),
+                                       (74, 4, 144, 48), (75, 4, 144, 48), (99, 3, 32, 272)])
 def test_linear_attention_forms_agree(B, H, dk, dv):
     """Token by token from a carried state (one kernel) and all tokens at once in 32 bits (another) against 64 bits."""
     from complexity_deep_b200 import ops
