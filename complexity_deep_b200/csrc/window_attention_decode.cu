@@ -72,12 +72,18 @@ __device__ __forceinline__ float group8_add(float v) {
   return v;
 }
 
+// Blocks that an SM holds at a time, by the registers of the two kernels that walk the keys.
+__host__ __device__ constexpr int scores_per_sm(int size, int REP, int DC) {
+  return REP * DC > 4 || (size == 4 && DC > 2) ? 1 : size == 4 ? 2 : 3;
+}
+__host__ __device__ constexpr int values_per_sm(int size, int REP) { return size == 2 && REP <= 2 ? 3 : 2; }
+
 // REP query heads per block; DC chunks of 8 elements per lane (head width up to 64 DC). Keys are read behind the query, and
 // nothing is asked for in L2 ahead of the kernel before. With the first keys loaded ahead of the query and the rows of the
 // keys and values asked for ahead of time, steps of Pimezen took, us, with / without: 2048 wide, 1028 keys, 64 sequences
 // 1 890 / 1 689, 32 1 426 / 1 341; 1024 wide, 516 keys, 64 790 / 753, 32 566 / 547, 1 344 / 341.
 template <typename T, int REP, int DC>
-__global__ void __launch_bounds__(kThreads, REP * DC <= 4 && sizeof(T) == 2 ? 3 : 1)
+__global__ void __launch_bounds__(kThreads, scores_per_sm(sizeof(T), REP, DC))
 window_decode_scores_kernel(const DecodeParams p) {
   extern __shared__ float sm[];        // [REP][dp] queries
   __shared__ float s_m[kWarps][REP], s_l[kWarps][REP];
@@ -335,19 +341,30 @@ window_decode_values_kernel(const DecodeParams p) {
   if (p.splits > 1) cluster.sync();     // the other blocks read this block's shared memory until here
 }
 
-// Splits of the keys of a (head group, sequence): those whose last wave ends first. A block costs about 4 us of its own
-// (position, query, first keys, statistics) and, with three on an SM, the time that its keys take at the SM's share of
-// the memory's rate (44 bytes per ns). One B200, 32 sequences, 4 key heads of 128, 516 keys, scores / values us: 8 splits
-// (1 024 blocks, three waves of 64 keys each, the rule before) 15.0 / 15.4, 3 splits (one wave) 9.4 / 8.9.
+int rep_block(const WindowAttnParams& a) {
+  const int rep = a.H / a.G;
+  return rep <= 1 ? 1 : rep <= 2 ? 2 : 4;
+}
+
+// Splits of the keys of a (head group, sequence): those whose last wave ends first, a wave being what the SMs hold of the
+// kernel that they hold less of. A block costs about 4 us of its own (position, query, first keys, statistics) and, with
+// the others on its SM, the time that its keys take at the SM's share of the memory's rate (44 bytes per ns); below 64
+// keys a block it gets slower whatever the waves (5 splits of 304 keys 15.0, 4 of them 12.3). One B200, us of the three kernels,
+// this rule / powers of two up to 888 blocks / three blocks of 16 bits an SM whatever the kernel holds, 516 keys:
+//   32 sequences x 4 key heads of 128, 2 query heads each   22 / 34 / 22, in 32 bits 27 / 49 / 34
+//   24 x 4 of 128, 4 query heads each                       31 / 52 / 38
+//   32 x 2 of 256, 2 query heads each                       26 / 35 / 30
 constexpr int kMostSplits = 8;             // of a portable cluster
-int choose_splits(const WindowAttnParams& a, int rep_block) {
-  const int rep = a.H / a.G, keys = a.keep + a.window;
-  const long long blocks = static_cast<long long>(a.B) * a.G * ((rep + rep_block - 1) / rep_block);
-  const long long wave = 3LL * current_sm_count();
-  const double key_us = 2.0 * (a.dp > a.vp ? a.dp : a.vp) * 3 / 44e3;
+int choose_splits(const WindowAttnParams& a, int size) {
+  const int rep = a.H / a.G, heads = rep_block(a), keys = a.keep + a.window;
+  const long long blocks = static_cast<long long>(a.B) * a.G * ((rep + heads - 1) / heads);
+  const int scores = scores_per_sm(size, heads, a.dp <= 64 ? 1 : a.dp <= 128 ? 2 : 4), values = values_per_sm(size, heads);
+  const int per_sm = scores < values ? scores : values;
+  const long long wave = static_cast<long long>(per_sm) * current_sm_count();
+  const double key_us = static_cast<double>(size) * (a.dp > a.vp ? a.dp : a.vp) * per_sm / 44e3;
   int best = 1;
   double best_us = 1e30;
-  for (int s = 1; s <= kMostSplits && (s == 1 || keys / s >= 48); ++s) {
+  for (int s = 1; s <= kMostSplits && (s == 1 || keys / s >= 64); ++s) {
     const double us = static_cast<double>((blocks * s + wave - 1) / wave) * (4.0 + (keys + s - 1) / s * key_us);
     if (us < 0.98 * best_us) {
       best = s;
@@ -355,11 +372,6 @@ int choose_splits(const WindowAttnParams& a, int rep_block) {
     }
   }
   return best;
-}
-
-int rep_block(const WindowAttnParams& a) {
-  const int rep = a.H / a.G;
-  return rep <= 1 ? 1 : rep <= 2 ? 2 : 4;
 }
 
 template <typename T, int REP, int DC>
@@ -408,10 +420,10 @@ cudaError_t launch_both(const DecodeParams& p, cudaStream_t st) {
     // six rows in flight and three blocks on an SM, unless four blocks on an SM end a wave earlier: 32 sequences of 516 keys
     // (one wave of either) 8.9 us, with four and four 10.1; 64 of 1028 (1 024 blocks) 41.5 / 37.3
     const long long blocks = static_cast<long long>(grid.x) * grid.y * grid.z, sms = current_sm_count();
-    if ((blocks + 3 * sms - 1) / (3 * sms) <= (blocks + 4 * sms - 1) / (4 * sms)) return launch_values<T, REP, 6, 3>(p, grid, st);
+    if ((blocks + 3 * sms - 1) / (3 * sms) <= (blocks + 4 * sms - 1) / (4 * sms)) return launch_values<T, REP, 6, values_per_sm(sizeof(T), REP)>(p, grid, st);
     return launch_values<T, REP, 4, 4>(p, grid, st);
   } else {
-    return launch_values<T, REP, 4, 2>(p, grid, st);
+    return launch_values<T, REP, 4, values_per_sm(sizeof(T), REP)>(p, grid, st);
   }
 }
 
@@ -431,14 +443,14 @@ bool window_decode_supported(const WindowAttnParams& a) {
 }
 
 size_t window_decode_workspace_bytes(const WindowAttnParams& a) {
-  return static_cast<size_t>(a.B) * a.H * (a.keep + a.window + 2 * choose_splits(a, rep_block(a))) * sizeof(float);
+  return static_cast<size_t>(a.B) * a.H * (a.keep + a.window + 2 * kMostSplits) * sizeof(float);    // of either storage type
 }
 
 cudaError_t launch_window_decode(const WindowAttnParams& a, void* ws, int fp32, cudaStream_t st) {
   if (a.B == 0) return cudaSuccess;
   DecodeParams p;
   p.a = a;
-  p.splits = choose_splits(a, rep_block(a));
+  p.splits = choose_splits(a, fp32 ? 4 : 2);
   p.n_max = a.keep + a.window;
   p.scores = static_cast<float*>(ws);
   p.stats = p.scores + static_cast<size_t>(a.B) * a.H * p.n_max;

@@ -59,6 +59,15 @@ def test_window_decode_splits(B, H, G, size, keep, dtype):
     assert _rel(w.run([w.T - 5] + [1] * 5), w.reference()) <= TOL[dtype]
 
 
+@pytest.mark.parametrize("dtype", [BF, F32], ids=["bf16", "fp32"])
+@pytest.mark.parametrize("B,H,G,dim,vdim,size,keep", [(75, 4, 1, 72, 40, 127, 1), (37, 8, 2, 130, 16, 255, 1), (149, 2, 1, 40, 72, 64, 0),
+                                                      (20, 5, 5, 200, 30, 129, 0)])
+def test_window_decode_splits_by_what_an_sm_holds(B, H, G, dim, vdim, size, keep, dtype):
+    """Kernels of which an SM holds one, two or three blocks: heads of each width, one to four query heads a block."""
+    w = Window(dtype, size + keep + 3, H, G, dim, vdim, size, keep, B, seed=B)
+    assert _rel(w.run([w.T - 2] + [1] * 2), w.reference()) <= TOL[dtype]
+
+
 @pytest.mark.parametrize("B,H,dk,dv", [(1, 1, 160, 16), (2, 2, 48, 80), (40, 4, 32, 32), (3, 5, 272, 48), (80, 4, 128, 32), (1, 2, 512, 144),
                                        (74, 4, 144, 48), (75, 4, 144, 48), (99, 3, 32, 272)])
 def test_linear_attention_forms_agree(B, H, dk, dv):
