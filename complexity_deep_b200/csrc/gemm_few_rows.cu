@@ -37,10 +37,25 @@ struct FewParams {
   int sms;                         // of the device
 };
 
-__device__ __forceinline__ uint4 load_stream(const bf16* p) {
+// Weights and rows may have been written by the kernel ahead, which can still run when this one starts: neither takes the
+// read-only path. The weights' loads keep their place behind the wait as volatile; a row's load, which the compiler is free
+// to place (volatile as well, or as plain C++, steps took 1 to 3 % longer), depends on a value that the wait gives.
+__device__ __forceinline__ uint4 load_weights(const bf16* p) {
   uint4 v;
-  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  asm volatile("ld.global.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
   return v;
+}
+__device__ __forceinline__ uint4 load_row(const bf16* p) {
+  uint4 v;
+  asm("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+// Zero, known only once the kernel ahead has ended.
+__device__ __forceinline__ uint32_t zero_after_wait() {
+  uint32_t z;
+  pdl_enter();
+  asm volatile("mov.u32 %0, 0;" : "=r"(z) : : "memory");
+  return z;
 }
 __device__ __forceinline__ void prefetch_row(const void* p, uint32_t bytes) {
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
@@ -57,7 +72,7 @@ constexpr int kRowFloats = 16 * MT + 4;                    // partial sums of a 
 // One pass: the block's weight rows against the tokens [m0, m0 + 8 NT) of a group that ends at m_end.
 template <int EPI, int MT, int NT, int WK>
 __device__ __forceinline__ void few_pass(const FewParams& p, float* red, const Weights& wt, const int (&w_row)[MT][2], int n_steps0,
-                                         int n_steps, int m0, int m_end, int col0, bool second) {
+                                         int n_steps, int m0, int m_end, int col0, bool second, uint32_t after) {
   constexpr bool kGated = EPI == kEpiSwiGLU || EPI == kEpiGlu;
   constexpr bool kSplit = EPI == kEpiStoreSplit;
   constexpr bool kF32 = EPI == kEpiStoreF32;
@@ -118,16 +133,16 @@ __device__ __forceinline__ void few_pass(const FewParams& p, float* red, const W
 #pragma unroll
     for (int m = 0; m < MT; ++m)
 #pragma unroll
-      for (int h = 0; h < 2; ++h) v[m][h] = in ? load_stream(base + w_row[m][h] * ld) : zero;
+      for (int h = 0; h < 2; ++h) v[m][h] = in ? load_weights(base + w_row[m][h] * ld) : zero;
   };
   auto load_t = [&](int s, uint4 (&v)[NT]) {
     const bool one = s >= n_steps0;
     const int k = (one ? s - n_steps0 : s) * kStep + q8;
     const bool in = s < s_hi && k < (one ? g.K1 : g.K0);
-    const bf16* base = (one ? p.a1 : p.a0) + k;
+    const bf16* base = (one ? p.a1 : p.a0) + k + after;
     const long long ld = one ? p.lda1 : p.lda0;
 #pragma unroll
-    for (int n = 0; n < NT; ++n) v[n] = in ? __ldg(reinterpret_cast<const uint4*>(base + t_row[n] * ld)) : zero;
+    for (int n = 0; n < NT; ++n) v[n] = in ? load_row(base + t_row[n] * ld) : zero;
   };
   float acc[MT][NT][4];
 #pragma unroll
@@ -297,7 +312,7 @@ __global__ void __launch_bounds__(WK * 32, (NTMAX >= 8 ? 8 : 16) / WK) few_rows_
 #pragma unroll
     for (int h = 0; h < 2; ++h) w_row[m][h] = weight_row<EPI>(p, at, m, (lane >> 2) + h * 8);
   if (p.prefetch) prefetch_block<EPI, MT>(p, at);
-  pdl_enter();
+  const uint32_t after = zero_after_wait();
 
   int m_lo = 0, m_hi = g.M;
   if (g.seg_offsets && !at.second) {
@@ -322,14 +337,14 @@ __global__ void __launch_bounds__(WK * 32, (NTMAX >= 8 ? 8 : 16) / WK) few_rows_
     const int left = m_hi - m0;
     if (m0 > m_lo) __syncthreads();                        // the sums of the pass before are read
     if constexpr (NTMAX == 1) {
-      few_pass<EPI, MT, 1, WK>(p, red, wt, w_row, n_steps0, n_steps, m0, m_hi, at.col0, at.second);
+      few_pass<EPI, MT, 1, WK>(p, red, wt, w_row, n_steps0, n_steps, m0, m_hi, at.col0, at.second, after);
     } else if constexpr (NTMAX == 4) {
-      if (left <= 8) few_pass<EPI, MT, 1, WK>(p, red, wt, w_row, n_steps0, n_steps, m0, m_hi, at.col0, at.second);
-      else if (left <= 16) few_pass<EPI, MT, 2, WK>(p, red, wt, w_row, n_steps0, n_steps, m0, m_hi, at.col0, at.second);
-      else few_pass<EPI, MT, 4, WK>(p, red, wt, w_row, n_steps0, n_steps, m0, m_hi, at.col0, at.second);
+      if (left <= 8) few_pass<EPI, MT, 1, WK>(p, red, wt, w_row, n_steps0, n_steps, m0, m_hi, at.col0, at.second, after);
+      else if (left <= 16) few_pass<EPI, MT, 2, WK>(p, red, wt, w_row, n_steps0, n_steps, m0, m_hi, at.col0, at.second, after);
+      else few_pass<EPI, MT, 4, WK>(p, red, wt, w_row, n_steps0, n_steps, m0, m_hi, at.col0, at.second, after);
     } else {
-      if (left <= 48) few_pass<EPI, MT, 6, WK>(p, red, wt, w_row, n_steps0, n_steps, m0, m_hi, at.col0, at.second);
-      else few_pass<EPI, MT, 8, WK>(p, red, wt, w_row, n_steps0, n_steps, m0, m_hi, at.col0, at.second);
+      if (left <= 48) few_pass<EPI, MT, 6, WK>(p, red, wt, w_row, n_steps0, n_steps, m0, m_hi, at.col0, at.second, after);
+      else few_pass<EPI, MT, 8, WK>(p, red, wt, w_row, n_steps0, n_steps, m0, m_hi, at.col0, at.second, after);
     }
   }
 }
