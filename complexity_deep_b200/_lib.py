@@ -108,6 +108,9 @@ SIGNATURES = {
     "cd_moe_down": (c_int, [c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int,
                             c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int,
                             c_void_p]),
+    "cd_moe_down_bounded": (c_int, [c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int,
+                                    c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
+                                    c_void_p]),
     "cd_peer_put_i32": (c_int, [c_void_p, c_int, c_void_p, c_int, c_longlong, c_void_p]),
     "cd_ep_plan": (c_int, [c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_longlong, c_int, c_void_p,
                            c_void_p, c_void_p, c_void_p]),
@@ -139,6 +142,8 @@ SIGNATURES = {
                               c_int, c_int, c_int, c_int, c_void_p]),
     "cd_glu_up": (c_int, [c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_float, c_float,
                           c_float, c_void_p]),
+    "cd_glu_up_bounded": (c_int, [c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_float,
+                                  c_float, c_float, c_int, c_void_p]),
     "cd_glu_f32": (c_int, [c_void_p, c_void_p, c_int, c_int, c_float, c_float, c_float, c_void_p]),
     "cd_window_attention_supported": (c_int, [ctypes.POINTER(WindowAttn)]),
     "cd_window_attention_norm": _WINDOW_FN,

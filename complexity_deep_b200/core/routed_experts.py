@@ -42,7 +42,7 @@ class RoutedExperts(nn.Module):
             self.router.weight.detach(), round_up(self.experts, ROW_ALIGN), x.shape[1]).contiguous())
         return ops.route_top(ops.linear_to_f32(x, w, tag="router"), self.experts, self.top, self.groups, self.keep)
 
-    def _up(self, x: torch.Tensor, seg: torch.Tensor) -> torch.Tensor:
+    def _up(self, x: torch.Tensor, seg: torch.Tensor, most_rows: int) -> torch.Tensor:
         src = (self.gate_proj, self.up_proj)
         rows = round_up(self.gate_proj.shape[1], ROW_ALIGN)
         width = x.shape[1]
@@ -53,7 +53,8 @@ class RoutedExperts(nn.Module):
         bn = ops.choose_block_n(rows, x.shape[0], self.experts)
         w = self._derived.get(f"gate_up_{bn}", src, lambda: ops.pack_gate_up(
             self._pad(self.gate_proj, rows, width), self._pad(self.up_proj, rows, width), bn))
-        return ops.glu_up(x, w, rows, bn, self.alpha, self.limit, self.offset, seg_offsets=seg)
+        return ops.glu_up(x, w, rows, bn, self.alpha, self.limit, self.offset, seg_offsets=seg,
+                          most_rows=most_rows)
 
     def run(self, x: torch.Tensor, stream: torch.Tensor, layer_scale=None, scale: float = 1.0) -> torch.Tensor:
         """stream += scale * experts(x), in place; x [T, width padded], stream fp32."""
@@ -63,11 +64,12 @@ class RoutedExperts(nn.Module):
         table = self._derived.get("table", (self.router.weight,), lambda: torch.arange(
             self.experts, dtype=torch.int64, device=x.device))
         r = ops.route(ids, table, self.experts)
-        h = self._up(ops.gather_div(x, r.perm, self.top), r.offsets)
+        tokens = x.shape[0]                                  # a token chooses an expert once: the most that one gets
+        h = self._up(ops.gather_div(x, r.perm, self.top), r.offsets, tokens)
         down = self._derived.get("down", (self.down_proj,), lambda: self._pad(
             self.down_proj, stream.shape[1], h.shape[1]))
         if x.dtype == torch.float32:
             y = ops.grouped_linear_f32(h, down, r.offsets, "moe_down")
         else:
-            y = ops.moe_down(h, down, None, None, r.offsets, self.experts, None, None)
+            y = ops.moe_down(h, down, None, None, r.offsets, self.experts, None, None, most_rows=tokens)
         return ops.combine_top_(stream, y, r.inv_perm, weights, scale)

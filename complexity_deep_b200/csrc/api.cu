@@ -281,11 +281,11 @@ int cd_moe_up_pair(const void* x_sorted, const int32_t* seg_offsets, int num_gro
                      as_stream(stream), &sec);
 }
 
-int cd_moe_down(const void* h_routed, int I_e, const void* wd_routed, const void* h_shared,
-                int I_s, const void* wd_shared, const int32_t* seg_offsets, int E,
-                const int32_t* row_map, const void* residual, const void* residual_lo, void* out,
-                void* out_lo, int T, int H, void* stream) {
-  if (T < 0 || H < 8 || (H & 7) || I_e < 8 || (I_e & 7) || E < 1) return CD_ERR_INVALID;
+int cd_moe_down_bounded(const void* h_routed, int I_e, const void* wd_routed, const void* h_shared,
+                        int I_s, const void* wd_shared, const int32_t* seg_offsets, int E,
+                        const int32_t* row_map, const void* residual, const void* residual_lo,
+                        void* out, void* out_lo, int T, int H, int most_rows, void* stream) {
+  if (most_rows < 0 || T < 0 || H < 8 || (H & 7) || I_e < 8 || (I_e & 7) || E < 1) return CD_ERR_INVALID;
   if ((h_shared == nullptr) != (wd_shared == nullptr)) return CD_ERR_INVALID;
   if (h_shared && (I_s < 8 || (I_s & 7))) return CD_ERR_INVALID;
   GemmOperand op0{};
@@ -318,7 +318,16 @@ int cd_moe_down(const void* h_routed, int I_e, const void* wd_routed, const void
   epi.residual_lo = residual_lo;
   epi.out_lo = out_lo;
   return launch_gemm(T, H, E, seg_offsets, op0, h_shared ? &op1 : nullptr, epi,
-                     choose_store_block_n(T, H, E, current_sm_count()), as_stream(stream));
+                     choose_store_block_n(T, H, E, current_sm_count()), as_stream(stream), nullptr,
+                     most_rows);
+}
+
+int cd_moe_down(const void* h_routed, int I_e, const void* wd_routed, const void* h_shared,
+                int I_s, const void* wd_shared, const int32_t* seg_offsets, int E,
+                const int32_t* row_map, const void* residual, const void* residual_lo, void* out,
+                void* out_lo, int T, int H, void* stream) {
+  return cd_moe_down_bounded(h_routed, I_e, wd_routed, h_shared, I_s, wd_shared, seg_offsets, E,
+                             row_map, residual, residual_lo, out, out_lo, T, H, 0, stream);
 }
 
 int cd_push_rows(const void* x, const int32_t* src_rows, const int32_t* offsets,
@@ -645,9 +654,9 @@ int cd_linear_f32(const float* x, int64_t ldx, const float* w, const float* resi
   return e == cudaSuccess ? CD_OK : cuda_fail(e, "linear_f32 launch");
 }
 
-int cd_glu_up(const void* x, const int32_t* seg_offsets, int groups, const void* packed_w, void* h, int T, int H, int I,
-              int block_n, float alpha, float limit, float offset, void* stream) {
-  if (T < 0 || H < 8 || I < 8 || (H & 7) || (I & 7) || groups < 1) return CD_ERR_INVALID;
+int cd_glu_up_bounded(const void* x, const int32_t* seg_offsets, int groups, const void* packed_w, void* h, int T, int H,
+                      int I, int block_n, float alpha, float limit, float offset, int most_rows, void* stream) {
+  if (most_rows < 0 || T < 0 || H < 8 || I < 8 || (H & 7) || (I & 7) || groups < 1) return CD_ERR_INVALID;
   const int rows = cd_gate_up_packed_rows(I, block_n);
   if (rows == 0) return CD_ERR_INVALID;
   GemmOperand op{};
@@ -666,7 +675,12 @@ int cd_glu_up(const void* x, const int32_t* seg_offsets, int groups, const void*
   epi.glu_alpha = alpha;
   epi.glu_limit = limit;
   epi.glu_offset = offset;
-  return launch_gemm(T, rows, groups, seg_offsets, op, nullptr, epi, block_n, as_stream(stream));
+  return launch_gemm(T, rows, groups, seg_offsets, op, nullptr, epi, block_n, as_stream(stream), nullptr, most_rows);
+}
+
+int cd_glu_up(const void* x, const int32_t* seg_offsets, int groups, const void* packed_w, void* h, int T, int H, int I,
+              int block_n, float alpha, float limit, float offset, void* stream) {
+  return cd_glu_up_bounded(x, seg_offsets, groups, packed_w, h, T, H, I, block_n, alpha, limit, offset, 0, stream);
 }
 
 int cd_glu_f32(const float* gu, float* h, int T, int I, float alpha, float limit, float offset, void* stream) {

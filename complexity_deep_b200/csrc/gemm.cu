@@ -292,7 +292,7 @@ ClusterSplitPlan plan_cluster_split(int M, int N, int kb64, int unsplit_bn, int 
 }  // namespace
 
 // gemm_few_rows.cu
-bool few_rows_taken(int M, int num_groups, bool second, int kind, int cols, int K, int sm_count);
+bool few_rows_taken(int M, int num_groups, int most_rows, bool second, int kind, int cols, int K, int sm_count);
 cudaError_t launch_few_rows(const GemmParams& g, int kind, const GemmOperand& op0, const GemmOperand* op1, const GemmSecond* second,
                             int block_n, int sm_count, cudaStream_t stream);
 
@@ -391,7 +391,7 @@ int splitk_ranges_dense(int M, int N, int K) {
 
 int launch_gemm(int M, int N, int num_groups, const int* seg_offsets, const GemmOperand& op0,
                 const GemmOperand* op1, const GemmEpilogueArgs& epi, int block_n,
-                cudaStream_t stream, const GemmSecond* second) {
+                cudaStream_t stream, const GemmSecond* second, int most_rows) {
   if (M < 0 || N <= 0 || num_groups < 1) return CD_ERR_INVALID;
   if (num_groups > kMaxGroups) {
     snprintf(g_cuda_err, sizeof(g_cuda_err), "grouped GEMM: %d row groups, at most %d are supported",
@@ -496,7 +496,7 @@ int launch_gemm(int M, int N, int num_groups, const int* seg_offsets, const Gemm
   const int kind = epi.rope_cos ? static_cast<int>(kEpiStoreRope)
                    : (epi.out_lo || epi.residual_lo) ? static_cast<int>(kEpiStoreSplit) : epi.kind;
   if (kind != kEpiStoreRope && !epi.selftest_stall &&
-      few_rows_taken(M, num_groups, second != nullptr, kind, epi.out_cols, op0.K + (op1 ? op1->K : 0), di->sm_count)) {
+      few_rows_taken(M, num_groups, most_rows, second != nullptr, kind, epi.out_cols, op0.K + (op1 ? op1->K : 0), di->sm_count)) {
     cudaError_t e = launch_few_rows(p, kind, op0, op1, second, block_n, di->sm_count, stream);
     return e == cudaSuccess ? CD_OK : cuda_fail(e, "few-row gemm launch");
   }

@@ -1,6 +1,6 @@
 // Matrix products of few rows (decode steps, short prompts): out[r, n] = epilogue(sum_k A[r, k] W[n, k]).
 //
-// Such a call is a read of the weights: 2 bytes per weight against at most 64 rows of work (8 of a row group). The tile kernel
+// Such a call is a read of the weights: 2 bytes per weight against at most 64 rows of work. The tile kernel
 // (gemm_sm100.cuh) runs it as chains of 128-row tensor-core tiles with barriers, tensor memory and an
 // issuing thread between them: 4.9 us before its first result and 0.21 us per 64 elements of K, whatever the
 // rows. Here a block takes 16 (or 32) weight rows and its eight warps a share of K each; weights and rows go
@@ -387,16 +387,18 @@ cudaError_t launch_store(const FewParams& p, int mt, cudaStream_t stream) {
 static int store_mt(long long cols, int num_groups, int sm_count) { return num_groups * ((cols + 31) / 32) >= 2LL * sm_count ? 2 : 1; }
 
 // Which calls stream (us on one B200, this kernel / the tile kernel):
-//   row groups: up to 64 rows, or 8 per group. 64 experts of 2 x 704 x 2048, cold: 384 rows 69 / 89, 512 rows 70 / 89
-//     (half of them in one group 105 / 88), 1024 rows 79 / 90 (179 / 90: a pass per 32 rows of a group, hence the line);
-//     their down projections 46 / 46, in a step behind one another 16 steps of Rugedra 26.0 / 26.7 ms; 32 experts of 2 x 704 x 1024, 256 rows 28 / 44. 8 experts and a
-//     shared one: 32 rows 14 / 26, 64 rows 15 / 26.
+//   row groups: up to 64 rows; up to 8 per group on average where the caller knows that no group has more than 64 (two
+//     passes; the sizes themselves are on the device). 64 experts of 2 x 704 x 2048, cold, 512 rows: evenly dealt 69 / 90,
+//     64 in each of 8 groups 35 / 39, their down projections 46 / 47 and 23 / 22; 1024 rows 79 / 90. Without a bound on a group a pass
+//     per 32 of its rows reads the weights again: half of 512 rows in one group 100 / 90 and 55 / 47, all of them 152 / 31
+//     and 80 / 20; 128 experts, 1024 rows in one 174 / 27. 32 experts of 2 x 704 x 1024, 256 rows 27 / 44. 8 experts and a
+//     shared one: 32 rows 14 / 26, 64 rows 15 / 26; 65 rows in one group 33 / 39 and 19 / 21.
 //   dense: up to 64 rows, unless the tokens, which every block reads again, cost more than the tile kernel's chains.
 //     K 2048, N 2048: 32 rows 5.5 / 11.6, 64 rows 7.1 / 11.6; K 4096, N 4096: 32 rows 12.9 / 16.1, 48 rows 17.6 / 16.1;
 //     K 2048, N 32000: 8 rows 29 / 37, 32 rows 41 / 27. The estimates below put the line between these: both sides in
 //     bytes per ns at the rates that they reach, 4.9 us and 0.21 us per 64 of K for a chain.
-bool few_rows_taken(int M, int num_groups, bool second, int kind, int cols, int K, int sm_count) {
-  if (num_groups > 1 || second) return M <= 64 || (!second && M <= 8 * num_groups);
+bool few_rows_taken(int M, int num_groups, int most_rows, bool second, int kind, int cols, int K, int sm_count) {
+  if (num_groups > 1 || second) return M <= 64 || (!second && M <= 8 * num_groups && most_rows > 0 && most_rows <= 64);
   if (M > 64) return false;
   const bool gated = kind == kEpiSwiGLU || kind == kEpiGlu;
   const int per_block = gated ? 16 : 16 * store_mt(cols, 1, sm_count);

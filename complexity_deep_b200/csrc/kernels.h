@@ -225,10 +225,10 @@ struct GemmSecond {
   int out_cols;
 };
 
-// Returns a CD_* status code.
+// Returns a CD_* status code. most_rows: no row group has more rows (0: not known; it only chooses the kernel).
 int launch_gemm(int M, int N, int num_groups, const int* seg_offsets, const GemmOperand& op0,
                 const GemmOperand* op1, const GemmEpilogueArgs& epi, int block_n,
-                cudaStream_t stream, const GemmSecond* second = nullptr);
+                cudaStream_t stream, const GemmSecond* second = nullptr, int most_rows = 0);
 
 int choose_store_block_n(int M, int N, int num_groups, int sm_count);  // SM count of the current device
 int current_sm_count();

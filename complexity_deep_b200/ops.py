@@ -461,9 +461,10 @@ def moe_down(h_routed: torch.Tensor, wd_routed: torch.Tensor, h_shared: Optional
              wd_shared: Optional[torch.Tensor], seg_offsets: Optional[torch.Tensor],
              num_experts: int, row_map: Optional[torch.Tensor],
              residual: Optional[torch.Tensor], residual_lo: Optional[torch.Tensor] = None,
-             want_lo: bool = False):
+             want_lo: bool = False, most_rows: int = 0):
     """wd_routed: [E, H, I_e] (feature rows, I_e contiguous); wd_shared: [H, I_s].
-    `residual_lo` / `want_lo`: split-bf16 residual stream; with want_lo returns (out, out_lo)."""
+    `residual_lo` / `want_lo`: split-bf16 residual stream; with want_lo returns (out, out_lo).
+    `most_rows`: no expert has more rows (0: not known)."""
     lib = _lib.load()
     _need(h_routed, "h_routed")
     _need(wd_routed, "routed down weights")
@@ -493,10 +494,10 @@ def moe_down(h_routed: torch.Tensor, wd_routed: torch.Tensor, h_shared: Optional
     lo2, out_lo = _split_args(res2, residual_lo, T, H, want_lo, h_routed.device)
     out = torch.empty(T, H, dtype=BF16, device=h_routed.device)
     with _Span("moe_down"):
-        _lib.check(lib.cd_moe_down(h_routed.data_ptr(), I_e, wd_routed.data_ptr(), _ptr(h_shared),
-                                   I_s, _ptr(wd_shared), _ptr(seg_offsets), E, _ptr(row_map),
-                                   _ptr(res2), _ptr(lo2), out.data_ptr(), _ptr(out_lo), T, H,
-                                   _stream()), "cd_moe_down")
+        _lib.check(lib.cd_moe_down_bounded(h_routed.data_ptr(), I_e, wd_routed.data_ptr(), _ptr(h_shared),
+                                           I_s, _ptr(wd_shared), _ptr(seg_offsets), E, _ptr(row_map),
+                                           _ptr(res2), _ptr(lo2), out.data_ptr(), _ptr(out_lo), T, H,
+                                           most_rows, _stream()), "cd_moe_down")
     return (out, out_lo) if want_lo else out
 
 
@@ -927,9 +928,10 @@ def grouped_linear_f32(x: torch.Tensor, w: torch.Tensor, seg_offsets: torch.Tens
 
 
 def glu_up(x: torch.Tensor, packed_w: torch.Tensor, width: int, block_n: int, alpha: float,
-           limit: float, offset: float, seg_offsets: Optional[torch.Tensor] = None) -> torch.Tensor:
+           limit: float, offset: float, seg_offsets: Optional[torch.Tensor] = None,
+           most_rows: int = 0) -> torch.Tensor:
     """Clamped gated unit on packed gate / up weights (pack_gate_up); with several groups the row
-    ranges of x come from seg_offsets."""
+    ranges of x come from seg_offsets, and `most_rows` says that none is longer (0: not known)."""
     lib = _lib.load()
     _need(x, "x")
     _need(packed_w, "packed gate/up weights")
@@ -943,8 +945,9 @@ def glu_up(x: torch.Tensor, packed_w: torch.Tensor, width: int, block_n: int, al
         raise RuntimeError("seg_offsets do not match the groups")
     h = torch.empty(T, width, dtype=BF16, device=x.device)
     with _Span("glu_up" if seg_offsets is None else "glu_up_routed"):
-        _lib.check(lib.cd_glu_up(x.data_ptr(), _ptr(seg_offsets), G, packed_w.data_ptr(), h.data_ptr(), T, H, width,
-                                 block_n, float(alpha), float(limit), float(offset), _stream()), "cd_glu_up")
+        _lib.check(lib.cd_glu_up_bounded(x.data_ptr(), _ptr(seg_offsets), G, packed_w.data_ptr(), h.data_ptr(), T, H,
+                                         width, block_n, float(alpha), float(limit), float(offset), most_rows,
+                                         _stream()), "cd_glu_up")
     return h
 
 

@@ -270,6 +270,13 @@ int cd_moe_down(const void* h_routed, int I_e, const void* wd_routed, const void
                 int I_s, const void* wd_shared, const int32_t* seg_offsets, int E,
                 const int32_t* row_map, const void* residual, const void* residual_lo, void* out,
                 void* out_lo, int T, int H, void* stream);
+/* cd_moe_down of which the caller knows that no group has more than most_rows rows (0: not known). The
+ * sizes of the groups are on the device, so this is what the choice between a kernel for few rows of
+ * many groups and the tile kernel goes by; the result is right whatever is said. */
+int cd_moe_down_bounded(const void* h_routed, int I_e, const void* wd_routed, const void* h_shared,
+                        int I_s, const void* wd_shared, const int32_t* seg_offsets, int E,
+                        const int32_t* row_map, const void* residual, const void* residual_lo,
+                        void* out, void* out_lo, int T, int H, int most_rows, void* stream);
 
 /* ---- expert-parallel combine ---------------------------------------------------------------
  * Home-GPU half of the layer when the routed experts live on other GPUs: the shared expert's
@@ -411,6 +418,9 @@ int cd_linear_f32(const float* x, int64_t ldx, const float* w, const float* resi
  * h = g sigmoid(alpha g) (u + offset), g = min(x Wg^T, limit), u = clamp(x Wu^T, -limit, limit). */
 int cd_glu_up(const void* x, const int32_t* seg_offsets, int groups, const void* packed_w, void* h, int T,
               int H, int I, int block_n, float alpha, float limit, float offset, void* stream);
+/* cd_glu_up with a bound on the rows of a group (as cd_moe_down_bounded). */
+int cd_glu_up_bounded(const void* x, const int32_t* seg_offsets, int groups, const void* packed_w, void* h, int T,
+                      int H, int I, int block_n, float alpha, float limit, float offset, int most_rows, void* stream);
 /* The same function of fp32 pre-activations gu [T, 2 I] (gate columns, then up). */
 int cd_glu_f32(const float* gu, float* h, int T, int I, float alpha, float limit, float offset,
                void* stream);

@@ -66,6 +66,10 @@ def test_store_epilogues(T, K, N):
     ([1, 0, 2], 40, 24, 32, 40), ([0, 9, 17, 0, 33], 72, 104, 64, 0), ([8, 8, 0, 16, 32], 264, 136, 128, 72),
     ([0] * 30 + [40, 1], 104, 200, 256, 0), ([5] + [0] * 63, 64, 48, 64, 0), ([3, 61], 520, 344, 256, 128)])
 def test_row_groups(counts, H, I, bn, shared):
+    check_row_groups(counts, H, I, bn, shared, 0)
+
+
+def check_row_groups(counts, H, I, bn, shared, most):
     """Groups of experts, empty ones among them: both gated units, the down projection with its scattered rows, its
     residual pair and a shared expert."""
     from complexity_deep_b200 import ops
@@ -82,7 +86,7 @@ def test_row_groups(counts, H, I, bn, shared):
     _near(ops.moe_up(cx, cseg, E, packed, I, bn), F.silu(gv) * uv, slack)
     limit, alpha = 1.5, 1.702
     lg, lu = gv.clamp(max=limit), uv.clamp(-limit, limit)
-    _near(ops.glu_up(cx, packed, I, bn, alpha, limit, 1.0, seg_offsets=cseg), lg * torch.sigmoid(alpha * lg) * (lu + 1.0),
+    _near(ops.glu_up(cx, packed, I, bn, alpha, limit, 1.0, seg_offsets=cseg, most_rows=most), lg * torch.sigmoid(alpha * lg) * (lu + 1.0),
           2 * gs * (limit + 1) + us * limit + (lg * (lu + 1)).abs() * 2.0 ** -19 + 1e-6)
     h = _rand(g, T, I)
     rows = torch.randperm(T, generator=g).int()
@@ -97,7 +101,8 @@ def test_row_groups(counts, H, I, bn, shared):
         hs, ws = hs.cuda(), ws.cuda()
     want, bound = torch.zeros(T, H, dtype=torch.float64), torch.zeros(T, H, dtype=torch.float64)
     want[rows.long()], bound[rows.long()] = y, s
-    a, b = ops.moe_down(h.cuda(), down.cuda(), hs, ws, cseg, E, rows.cuda(), hi.cuda(), residual_lo=lo.cuda(), want_lo=True)
+    a, b = ops.moe_down(h.cuda(), down.cuda(), hs, ws, cseg, E, rows.cuda(), hi.cuda(), residual_lo=lo.cuda(), want_lo=True,
+                        most_rows=most)
     want = want + hi.double() + lo.double()
     bound = bound + hi.abs().double() * 2.0 ** -21
     _near(a, want, bound)
