@@ -102,6 +102,8 @@ SIGNATURES = {
                           c_int, c_void_p]),
     "cd_moe_up_pair": (c_int, [c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p,
                                c_void_p, c_int, c_int, c_int, c_int, c_void_p]),
+    "cd_moe_up_pair_layouts": (c_int, [c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_void_p,
+                                       c_void_p, c_int, c_int, c_int, c_int, c_void_p]),
     "cd_pack_gate_up": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
                                 c_void_p]),
     "cd_pack_down": (c_int, [c_void_p, c_void_p, c_int, c_int, c_int, c_void_p]),

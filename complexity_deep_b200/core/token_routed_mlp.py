@@ -151,9 +151,9 @@ class TokenRoutedMLP(nn.Module):
                                      feature_major=False))
         return packed, bn
 
-    def _packed_shared(self, rows: Optional[int] = None, bn: Optional[int] = None):
+    def _packed_shared(self, rows: Optional[int] = None):
         g, u = self.shared_gate.weight, self.shared_up.weight
-        bn = bn or ops.choose_block_n(g.shape[0], rows)
+        bn = ops.choose_block_n(g.shape[0], rows)
         packed = self._derived.get(
             f"shared_gate_up_{bn}", (g, u),
             lambda: ops.pack_gate_up(g.detach()[None].contiguous(), u.detach()[None].contiguous(), bn))
@@ -177,15 +177,14 @@ class TokenRoutedMLP(nn.Module):
         packed_r, bn_r = self._packed_routed(rows)
         h_s = wd_s = None
         if self.use_shared_expert:
-            # up to 64 rows stream the weights whatever their layout: the shared expert takes the routed ones', so
-            # that both go in one launch
-            packed_s, bn_s = self._packed_shared(rows, bn_r if rows <= 64 else None)
+            packed_s, bn_s = self._packed_shared(rows)
             wd_s = self.shared_down.weight.detach()
             I_s = self.shared_gate.weight.shape[0]
-        if self.use_shared_expert and bn_s == bn_r:
-            # routed and shared up-projections share one launch (one tail instead of two)
+        if self.use_shared_expert and (bn_s == bn_r or rows <= 64):
+            # routed and shared up-projections share one launch (one tail instead of two); up to 64 rows stream the
+            # weights whatever the two layouts
             h_r, h_s = ops.moe_up_pair(x_sorted, routing.offsets, self.num_experts, packed_r,
-                                       self.expert_intermediate_size, packed_s, I_s, bn_r)
+                                       self.expert_intermediate_size, packed_s, I_s, bn_r, bn_s)
         else:
             h_r = ops.moe_up(x_sorted, routing.offsets, self.num_experts, packed_r,
                              self.expert_intermediate_size, bn_r)

@@ -249,13 +249,13 @@ int cd_moe_up(const void* x_sorted, const int32_t* seg_offsets, int num_groups,
                      as_stream(stream));
 }
 
-int cd_moe_up_pair(const void* x_sorted, const int32_t* seg_offsets, int num_groups,
-                   const void* packed_w, void* h, int I, const void* packed_shared, void* h_shared,
-                   int I_s, int T, int H, int block_n, void* stream) {
+int cd_moe_up_pair_layouts(const void* x_sorted, const int32_t* seg_offsets, int num_groups,
+                           const void* packed_w, void* h, int I, int block_n, const void* packed_shared,
+                           void* h_shared, int I_s, int block_n_shared, int T, int H, void* stream) {
   if (T < 0 || H < 8 || I < 8 || I_s < 8 || (H & 7) || (I & 7) || (I_s & 7) || num_groups < 1)
     return CD_ERR_INVALID;
   const int rows = cd_gate_up_packed_rows(I, block_n);
-  const int rows_s = cd_gate_up_packed_rows(I_s, block_n);
+  const int rows_s = cd_gate_up_packed_rows(I_s, block_n_shared);
   if (rows == 0 || rows_s == 0 || !packed_shared || !h_shared) return CD_ERR_INVALID;
   GemmOperand op{};
   op.a = x_sorted;
@@ -277,8 +277,16 @@ int cd_moe_up_pair(const void* x_sorted, const int32_t* seg_offsets, int num_gro
   sec.out = h_shared;
   sec.ldo = I_s;
   sec.out_cols = I_s;
+  sec.block_n = block_n_shared;
   return launch_gemm(T, rows, num_groups, seg_offsets, op, nullptr, epi, block_n,
                      as_stream(stream), &sec);
+}
+
+int cd_moe_up_pair(const void* x_sorted, const int32_t* seg_offsets, int num_groups,
+                   const void* packed_w, void* h, int I, const void* packed_shared, void* h_shared,
+                   int I_s, int T, int H, int block_n, void* stream) {
+  return cd_moe_up_pair_layouts(x_sorted, seg_offsets, num_groups, packed_w, h, I, block_n, packed_shared,
+                                h_shared, I_s, block_n, T, H, stream);
 }
 
 int cd_moe_down_bounded(const void* h_routed, int I_e, const void* wd_routed, const void* h_shared,

@@ -500,6 +500,10 @@ int launch_gemm(int M, int N, int num_groups, const int* seg_offsets, const Gemm
     cudaError_t e = launch_few_rows(p, kind, op0, op1, second, block_n, di->sm_count, stream);
     return e == cudaSuccess ? CD_OK : cuda_fail(e, "few-row gemm launch");
   }
+  if (second && second->block_n != block_n) {
+    snprintf(g_cuda_err, sizeof(g_cuda_err), "tiles of two widths in one launch: %d and %d", block_n, second->block_n);
+    return CD_ERR_UNSUPPORTED;
+  }
 
   // dense store-epilogue calls of few rows may take the cluster form of split-K (128-wide tiles)
   int csk_splits = 1;

@@ -31,7 +31,7 @@ struct FewParams {
   GemmParams g;                    // shapes and epilogue, as the tile kernel takes them
   const bf16 *a0, *b0, *a1, *b1;   // a1 / b1: second K segment, or b1 the second problem's weights
   long long lda0, ldb0, lda1, ldb1;
-  int half;                        // gated units: rows of a gate block, up rows follow (packed layout)
+  int half, half2;                 // gated units: rows of a gate block, up rows follow (packed layout); the second problem's
   int tiles, tiles2;               // blocks per group, of the second problem
   int prefetch;                    // ask for the block's own weights ahead of the kernel before
   int sms;                         // of the device
@@ -281,8 +281,8 @@ template <int EPI>
 __device__ __forceinline__ int weight_row(const FewParams& p, const Block& b, int m, int i) {
   const int last = (b.second ? p.g.N2 : p.g.N) - 1;
   if constexpr (EPI == kEpiSwiGLU || EPI == kEpiGlu) {
-    const int j = b.col0 + i, blk = j / p.half;
-    return min(blk * 2 * p.half + m * p.half + (j - blk * p.half), last);
+    const int half = b.second ? p.half2 : p.half, j = b.col0 + i, blk = j / half;
+    return min(blk * 2 * half + m * half + (j - blk * half), last);
   } else {
     return min(b.col0 + m * 16 + i, last);
   }
@@ -422,6 +422,7 @@ cudaError_t launch_few_rows(const GemmParams& g, int kind, const GemmOperand& op
   p.lda1 = op1 ? op1->lda : op0.lda;
   p.ldb1 = op1 ? op1->ldb : second ? second->ldb : op0.ldb;
   p.half = block_n / 2;
+  p.half2 = second ? second->block_n / 2 : p.half;
   p.tiles2 = second ? (second->out_cols + 15) / 16 : 0;
   // of a grouped call only as much is asked for ahead of time as its rows are sure to use
   p.prefetch = g.num_groups == 1 || g.M >= 2 * g.num_groups;

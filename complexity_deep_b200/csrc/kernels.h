@@ -223,6 +223,7 @@ struct GemmSecond {
   void* out;
   int ldo;
   int out_cols;
+  int block_n;        // tile width that its rows are packed for; another one than the first problem's only where the call streams
 };
 
 // Returns a CD_* status code. most_rows: no row group has more rows (0: not known; it only chooses the kernel).

@@ -420,9 +420,11 @@ def moe_up(x_sorted: torch.Tensor, seg_offsets: Optional[torch.Tensor], num_grou
 
 def moe_up_pair(x_sorted: torch.Tensor, seg_offsets: torch.Tensor, num_groups: int,
                 packed_w: torch.Tensor, width: int, packed_shared: torch.Tensor,
-                width_shared: int, block_n: int) -> Tuple[torch.Tensor, torch.Tensor]:
+                width_shared: int, block_n: int, block_n_shared: Optional[int] = None
+                ) -> Tuple[torch.Tensor, torch.Tensor]:
     """Routed (grouped) and shared (dense) SwiGLU up-projections of the same rows in one
-    launch; returns (h_routed [T, width], h_shared [T, width_shared])."""
+    launch; returns (h_routed [T, width], h_shared [T, width_shared]).  The shared weights may be
+    packed for a width of their own where at most 64 rows come."""
     lib = _lib.load()
     _need(x_sorted, "x_sorted")
     _need(packed_w, "packed gate/up weights")
@@ -430,16 +432,17 @@ def moe_up_pair(x_sorted: torch.Tensor, seg_offsets: torch.Tensor, num_groups: i
     _need(seg_offsets, "seg_offsets", torch.int32)
     T, H = x_sorted.shape
     rows = lib.cd_gate_up_packed_rows(width, block_n)
-    rows_s = lib.cd_gate_up_packed_rows(width_shared, block_n)
+    bn_s = block_n_shared or block_n
+    rows_s = lib.cd_gate_up_packed_rows(width_shared, bn_s)
     if tuple(packed_w.shape) != (num_groups, rows, H) or tuple(packed_shared.shape) != (1, rows_s, H):
         raise RuntimeError("packed weights do not match the widths / tile width")
     h = torch.empty(T, width, dtype=BF16, device=x_sorted.device)
     h_s = torch.empty(T, width_shared, dtype=BF16, device=x_sorted.device)
     with _Span("moe_up_pair"):
-        _lib.check(lib.cd_moe_up_pair(x_sorted.data_ptr(), seg_offsets.data_ptr(), num_groups,
-                                      packed_w.data_ptr(), h.data_ptr(), width,
-                                      packed_shared.data_ptr(), h_s.data_ptr(), width_shared, T, H,
-                                      block_n, _stream()), "cd_moe_up_pair")
+        _lib.check(lib.cd_moe_up_pair_layouts(x_sorted.data_ptr(), seg_offsets.data_ptr(), num_groups,
+                                              packed_w.data_ptr(), h.data_ptr(), width, block_n,
+                                              packed_shared.data_ptr(), h_s.data_ptr(), width_shared, bn_s,
+                                              T, H, _stream()), "cd_moe_up_pair")
     return h, h_s
 
 

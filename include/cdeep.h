@@ -240,6 +240,11 @@ int cd_moe_up(const void* x_sorted, const int32_t* seg_offsets, int num_groups,
 int cd_moe_up_pair(const void* x_sorted, const int32_t* seg_offsets, int num_groups,
                    const void* packed_w, void* h, int I, const void* packed_shared, void* h_shared,
                    int I_s, int T, int H, int block_n, void* stream);
+/* The same with each weight set packed for a width of its own. Where those differ, calls of more than 64
+ * rows (which take tiles, of one width) return CD_ERR_UNSUPPORTED. */
+int cd_moe_up_pair_layouts(const void* x_sorted, const int32_t* seg_offsets, int num_groups,
+                           const void* packed_w, void* h, int I, int block_n, const void* packed_shared,
+                           void* h_shared, int I_s, int block_n_shared, int T, int H, void* stream);
 
 /* ---- one-off weight layout transforms ------------------------------------------------------
  * What a host has to do once per weight version to get from the reference's parameter layouts

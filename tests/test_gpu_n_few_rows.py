@@ -118,3 +118,33 @@ def test_rows_do_not_depend_on_their_neighbours():
     full = ops.linear(x, w)
     for n in (1, 8, 9, 20, 33, 50):
         assert torch.equal(ops.linear(x[:n].contiguous(), w), full[:n]), n
+
+
+@pytest.mark.parametrize("rows,I,Is,bn,bn_s", [(1, 40, 104, 32, 256), (17, 136, 24, 256, 32), (64, 200, 328, 64, 128)])
+def test_routed_and_shared_weights_of_two_layouts(rows, I, Is, bn, bn_s):
+    """In one launch the bits of the same weights packed alike; calls of more than 64 rows refuse two layouts."""
+    from complexity_deep_b200 import ops
+    E, H = 4, 72
+    g = torch.Generator().manual_seed(rows)
+    x = _rand(g, 65, H).cuda()
+    seg = torch.tensor([0, rows // 3, rows // 3, rows - rows // 2, rows], dtype=torch.int32).cuda()
+    gate, up, sg, su = (_rand(g, *s, scale=0.1).cuda() for s in ((E, I, H), (E, I, H), (1, Is, H), (1, Is, H)))
+    routed, shared = ops.pack_gate_up(gate, up, bn), ops.pack_gate_up(sg, su, bn_s)
+    got = ops.moe_up_pair(x[:rows], seg, E, routed, I, shared, Is, bn, bn_s)
+    want = ops.moe_up_pair(x[:rows], seg, E, routed, I, ops.pack_gate_up(sg, su, bn), Is, bn)
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+    whole = torch.tensor([0, 65, 65, 65, 65], dtype=torch.int32).cuda()
+    with pytest.raises(RuntimeError):
+        ops.moe_up_pair(x, whole, E, routed, I, shared, Is, bn, bn_s)
+
+
+def test_a_layer_packs_its_shared_expert_once_for_decoding_and_short_prompts():
+    from complexity_deep_b200 import ops
+    from complexity_deep_b200.core.token_routed_mlp import TokenRoutedMLP
+    mlp = TokenRoutedMLP(hidden_size=768, intermediate_size=2816, num_experts=4, vocab_size=100).to("cuda", BF)
+    assert len({ops.choose_block_n(mlp.shared_gate.weight.shape[0], n) for n in (1, 64, 100)}) == 1
+    assert ops.choose_block_n(mlp.expert_intermediate_size, 1, 4) != ops.choose_block_n(mlp.shared_gate.weight.shape[0], 1)
+    with torch.no_grad():
+        for n in (1, 64, 100):
+            mlp(torch.zeros(1, n, 768, dtype=BF, device="cuda"), torch.zeros(1, n, dtype=torch.long, device="cuda"))
+    assert sum(name.startswith("shared_gate_up") for name in mlp._derived._slots) == 1
