@@ -379,6 +379,7 @@ int splitk_ranges_dense(int M, int N, int K) {
   int st;
   DeviceInfo* di = device_info(&st);
   if (!di || M <= 0 || N <= 0 || K <= 0) return 1;
+  if (few_rows_taken(M, 1, M, false, kEpiStore, N, K, di->sm_count)) return 1;
   const int bn = store_block_n_impl(M, N, 1, di->sm_count);
   if (choose_cta_group(M, bn, di->sm_count) != 1) return 1;
   if (bn <= 128 && choose_cta_group(M, 128, di->sm_count) == 1) {

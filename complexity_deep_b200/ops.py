@@ -624,9 +624,10 @@ _SPLIT_K_AUTO = os.environ.get("CDEEP_SPLIT_K", "0") == "1"
 
 
 def split_k(enable: bool = True, device: Optional[torch.device] = None) -> None:
-    """Registers (or withdraws) the workspace that lets the few-row projections of a decode step
-    cut their K loop over several CTAs (cd_splitk_workspace_set).  The workspace is shared by
-    every call on the device: keep launches that may split on one stream."""
+    """Registers (or withdraws) the workspace that lets projections of some 65 to 512 rows cut their
+    K loop over several CTAs (cd_splitk_workspace_set); fewer rows mostly stream their weights and
+    have no use for it.  The workspace is shared by every call on the device: keep launches that may
+    split on one stream."""
     lib = _lib.load()
     dev = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
     with torch.cuda.device(dev):
@@ -642,13 +643,13 @@ def split_k(enable: bool = True, device: Optional[torch.device] = None) -> None:
 
 
 def split_k_config(flags: int = -1) -> int:
-    """Which forms of split-K the few-row projections may take (cd_splitk_config): bit 0 the
+    """Which forms of split-K projections on tiles may take (cd_splitk_config): bit 0 the
     cluster form, bit 1 the workspace form; negative = query.  Returns the previous flags."""
     return _lib.load().cd_splitk_config(int(flags))
 
 
 def _split_k_auto(x: torch.Tensor) -> None:
-    # first few-row projection on a device: register the workspace (not while a graph is being
+    # first projection of few rows on a device: register the workspace (not while a graph is being
     # captured; the model's warm-up pass before the capture comes through here)
     if (_SPLIT_K_AUTO and x.shape[0] <= _SPLIT_K_ROWS and x.device.index not in _SPLIT_K_WS
             and not torch.cuda.is_current_stream_capturing()):

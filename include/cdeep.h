@@ -45,8 +45,8 @@ const char* cd_last_cuda_error(void);
  * cd_moe_up_pair, cd_moe_down and cd_moe_down_push return CD_ERR_UNSUPPORTED (text in
  * cd_last_cuda_error) beyond it.  The dispatch entry points accept up to 256 experts. */
 int cd_max_groups(void);
-/* Split-K for projections of few rows (decode; no counterpart in the reference).  A dense
- * projection whose output tiles would leave most SMs idle cuts the K loop of every tile into
+/* Split-K for projections of some 65 to 512 rows (no counterpart in the reference; fewer rows mostly
+ * take a kernel without tiles).  A dense projection whose output tiles would leave most SMs idle cuts the K loop of every tile into
  * ranges computed by different CTAs, which then combine their fp32 partial tiles and run the same
  * fused epilogue; results differ from the unsplit launch only by the order of the fp32 additions,
  * and do not depend on timing.  Two forms:
@@ -67,9 +67,9 @@ int cd_splitk_config(int flags);
 size_t cd_splitk_workspace_bytes(void);
 int cd_splitk_workspace_set(void* workspace, size_t bytes, void* stream);
 /* Number of K ranges cd_linear (or cd_mu_proj; cd_mu_qkv with K = the sum of its two K extents)
- * would use for a [T, K] x [N, K]^T call on the current device as it is set up now (1 = unsplit),
- * where the tile kernel takes the call: calls of at most 64 rows mostly stream their weights through a
- * kernel without tiles (csrc/gemm_few_rows.cu), whose blocks share K out among their own warps. */
+ * would use for a [T, K] x [N, K]^T call on the current device as it is set up now (1 = unsplit;
+ * also where the call streams its weights through the kernel without tiles, csrc/gemm_few_rows.cu, as
+ * most of at most 64 rows do: its blocks share K out among their own warps). */
 int cd_splitk_ranges(int T, int K, int N);
 /* 1 when this library is the checking build (libcdeep_checks.so, compiled with -DCDEEP_CHECKS),
  * else 0.  The checking build validates what its kernels read from device memory before using it

@@ -134,7 +134,7 @@ def test_pack_kernels_match_layout(G, I, H, bn):
 @pytest.mark.parametrize("T,H,I,bn", [(128, 64, 128, 256), (200, 128, 64, 128), (77, 256, 40, 128),
                                       (1000, 768, 512, 256), (512, 2048, 704, 128),
                                       (512, 2048, 704, 256), (300, 512, 200, 256),
-                                      (32, 2048, 704, 32), (200, 256, 72, 64), (8, 64, 16, 32)])
+                                      (32, 2048, 704, 32), (200, 256, 72, 64), (8, 64, 16, 32), (96, 2048, 704, 32)])
 def test_moe_up_dense(T, H, I, bn):
     from complexity_deep_b200 import ops
     g = torch.Generator().manual_seed(11)
@@ -159,7 +159,7 @@ def _segments(g, T, E, empty=()):
 @pytest.mark.parametrize("T,H,I,E,bn,empty", [(300, 64, 64, 4, 128, ()), (1000, 128, 136, 8, 256, (2,)),
                                               (4096, 768, 512, 4, 256, ()), (517, 256, 72, 32, 128, (0, 31)),
                                               (129, 64, 64, 4, 128, (1, 2, 3)),
-                                              (256, 256, 88, 8, 32, (3,)), (40, 128, 48, 4, 64, ())])
+                                              (256, 256, 88, 8, 32, (3,)), (40, 128, 48, 4, 64, ()), (100, 128, 48, 4, 64, ())])
 def test_moe_up_grouped_ragged(T, H, I, E, bn, empty):
     from complexity_deep_b200 import ops
     g = torch.Generator().manual_seed(13)
@@ -372,7 +372,7 @@ def _split(v):
 
 
 @pytest.mark.parametrize("T,K,N", [(128, 64, 256), (300, 128, 264), (1000, 768, 1024),
-                                   (4096, 2048, 2048), (40, 256, 96), (129, 1032, 520)])
+                                   (4096, 2048, 2048), (40, 256, 96), (72, 256, 96), (129, 1032, 520)])
 @pytest.mark.parametrize("res_lo", [False, True])
 def test_linear_split_residual_stream(T, K, N, res_lo):
     """cd_linear with the residual as a split-bf16 pair and the result stored as one: hi must be
@@ -443,7 +443,8 @@ def test_moe_combine_split_residual_stream():
 @pytest.mark.parametrize("T,H,I,Is,E,bn,empty", [
     (300, 64, 64, 64, 4, 128, ()), (1000, 128, 136, 200, 8, 256, (2,)),
     (4096, 768, 512, 512, 4, 256, ()), (517, 256, 72, 40, 32, 128, (0, 31)),
-    (8192, 2048, 704, 704, 8, 256, ()), (256, 256, 88, 88, 8, 32, (3,)), (40, 128, 48, 112, 4, 64, ())])
+    (8192, 2048, 704, 704, 8, 256, ()), (256, 256, 88, 88, 8, 32, (3,)), (40, 128, 48, 112, 4, 64, ()),
+    (100, 128, 48, 112, 4, 64, ())])
 def test_moe_up_pair_routed_and_shared_one_launch(T, H, I, Is, E, bn, empty):
     """cd_moe_up_pair = cd_moe_up over the groups + cd_moe_up of the shared expert, same bits."""
     from complexity_deep_b200 import ops
@@ -481,10 +482,10 @@ def _noise_bound(ref):
     return ref.abs() * 2.0 ** -7 + 1e-5 * float(ref.pow(2).mean().sqrt())
 
 
-@pytest.mark.parametrize("T,K,N,with_res", [(32, 4096, 2048, False), (128, 5632, 2048, True),
-                                            (8, 3072, 1024, True), (100, 8192, 512, False),
-                                            (256, 4096, 1024, True), (17, 4096 + 64, 264, False),
-                                            (200, 6144, 1024, True), (32, 2048, 2048, True),
+@pytest.mark.parametrize("T,K,N,with_res", [(96, 4096, 2048, False), (128, 5632, 2048, True),
+                                            (72, 3072, 1024, True), (100, 8192, 512, False),
+                                            (256, 4096, 1024, True), (81, 4096 + 64, 264, False),
+                                            (200, 6144, 1024, True), (96, 2048, 2048, True),
                                             (32, 8192, 6144, True)])   # the last: two ranges per cluster
 def test_linear_split_k_forms_match_unsplit_and_fp32(split_k_modes, T, K, N, with_res):
     """The same call unsplit, with the cluster form and with the workspace form of split-K: all
@@ -517,14 +518,14 @@ def test_linear_split_k_forms_match_unsplit_and_fp32(split_k_modes, T, K, N, wit
 
 
 def test_split_k_through_the_fused_epilogues(split_k_modes):
-    """Split-K in front of every fused epilogue a few-row call can take: the mu K-concatenation,
+    """Split-K in front of every fused epilogue it can meet: the mu K-concatenation,
     mu_proj's clamped bias and output clamp, the split-bf16 residual stream (both forms), and the
     dense SwiGLU (workspace form)."""
     ops = split_k_modes
     from complexity_deep_b200 import _lib
     lib = _lib.load()
     g = torch.Generator().manual_seed(99)
-    T, H = 48, 3072
+    T, H = 112, 3072                   # calls of up to 64 rows stream instead
     x, mu = _rand(g, T, H).cuda(), _rand(g, T, H).cuda()
     w, wm = _rand(g, 768, H, scale=0.05).cuda(), _rand(g, 768, H, scale=0.05).cuda()
     wp, mu_param = _rand(g, H, H, scale=0.05).cuda(), (_rand(g, H) * 3).cuda()

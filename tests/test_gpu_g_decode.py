@@ -78,8 +78,10 @@ def test_attention_module_decode_step_uses_cache_in_place():
 
 
 @pytest.mark.parametrize("T,K,N", [(32, 2048, 4096), (8, 256, 2048), (256, 2048, 2048),
-                                   (64, 768, 40), (200, 512, 1000), (1, 64, 32)])
+                                   (64, 768, 40), (200, 512, 1000), (1, 64, 32), (96, 2048, 4096),
+                                   (72, 256, 2048), (100, 768, 40)])
 def test_few_rows_use_narrow_tiles(T, K, N):
+    """Up to 64 rows stream; the narrow tiles take what lies above (32 to 128 columns wide)."""
     from complexity_deep_b200 import ops
     g = torch.Generator().manual_seed(T + N)
     x = torch.randn(T, K, generator=g).to(BF)

@@ -32,7 +32,9 @@ ROWS = [1, 7, 8, 9, 16, 17, 32, 33, 48, 49, 64]
 
 
 @pytest.mark.parametrize("T,K,N", [(t, k, n) for t, (k, n) in zip(ROWS, [
-    (8, 8), (40, 24), (72, 40), (768, 264), (1032, 16), (96, 32), (2048, 2056), (264, 1280), (32, 48), (520, 72), (64, 9504)])])
+    (8, 8), (40, 24), (72, 40), (768, 264), (1032, 16), (96, 32), (2048, 2056), (264, 1280), (32, 48), (520, 72), (64, 9504)])]
+    + [(17, 264, 264), (48, 776, 776), (64, 40, 40)]                                  # square: mu_proj as well
+    + [(1, 72, 9480), (8, 64, 9496), (9, 40, 9448), (17, 72, 9512), (33, 24, 9480)])   # 32 weight rows a block, the last not full
 def test_store_epilogues(T, K, N):
     from complexity_deep_b200 import ops
     g = torch.Generator().manual_seed(T * 1000 + N)
