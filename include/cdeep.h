@@ -35,7 +35,7 @@ extern "C" {
 #define CD_ERR_BOUNDS 5       /* checking build only: an index / address / segment table read from device
                                  memory was out of range (reported by cd_status_fetch) */
 
-/* ABI version of this header (bumped on any signature change; currently 3). */
+/* ABI version of this header (bumped on any signature change; currently 4). */
 int cd_version(void);
 /* Static text for a CD_* code. */
 const char* cd_error_string(int status);
