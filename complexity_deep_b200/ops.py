@@ -20,12 +20,15 @@ from . import _lib
 BF16 = torch.bfloat16
 
 
+# the handle of the calling thread's current stream on its current device: what
+# torch.cuda.current_stream().cuda_stream gives, without building a Stream object (0.2 us instead of 3.3 a launch).
+# A torch without CUDA has neither function and still imports this module.
+_current_device = getattr(torch._C, "_cuda_getDevice", None)
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def _stream() -> int:
-    # the handle of the calling thread's current stream on its current device: what
-    # torch.cuda.current_stream().cuda_stream gives, without building a Stream object (0.2 us instead of 3.3 a launch).
-    # Looked up here because a torch without CUDA has neither function and must still import this module.
-    c = torch._C
-    return c._cuda_getCurrentRawStream(c._cuda_getDevice())
+    return _raw_stream(_current_device())
 
 
 def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
@@ -352,7 +355,7 @@ def choose_block_n(width: int, rows: Optional[int] = None, groups: int = 1,
     """
     if rows is not None and rows <= 512:
         if sm_count is None:
-            sm_count = _sm_count(torch.cuda.current_device()) if torch.cuda.is_available() else 148
+            sm_count = _sm_count(_current_device()) if torch.cuda.is_available() else 148
         m_tiles = max(groups, -(-rows // 128))
         for bn in (32, 64, 128, 256):
             if m_tiles * -(-width // (bn // 2)) <= sm_count:
