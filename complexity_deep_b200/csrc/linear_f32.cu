@@ -146,6 +146,8 @@ linear_f32_kernel(const LinearF32 p) {
       __syncthreads();
     }
   }
+  // scale and column factor, or the scale alone, then the residual (-0 changes nothing)
+  const float first = p.col_scale ? p.scale : 1.f;
 #pragma unroll
   for (int i = 0; i < TM; ++i) {
     const int m = m0 + (i >> 2) * 4 * L::kRowThreads + ty * 4 + (i & 3);
@@ -162,27 +164,17 @@ linear_f32_kernel(const LinearF32 p) {
       }
       const size_t at = static_cast<size_t>(m) * N + n;
       if (p.vec && n + 4 <= N) {
-        float f[4] = {p.scale, p.scale, p.scale, p.scale}, r[4];
-        if (p.col_scale) {
-#pragma unroll
-          for (int j = 0; j < 4; ++j) v[j] *= p.scale;
-          *reinterpret_cast<float4*>(f) = *reinterpret_cast<const float4*>(p.col_scale + n);
-        }
-        if (p.residual) *reinterpret_cast<float4*>(r) = *reinterpret_cast<const float4*>(p.residual + at);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) v[j] = p.residual ? fmaf(v[j], f[j], r[j]) : v[j] * f[j];
-        *reinterpret_cast<float4*>(p.out + at) = make_float4(v[0], v[1], v[2], v[3]);
+        float4 f = make_float4(p.scale, p.scale, p.scale, p.scale), r = make_float4(-0.f, -0.f, -0.f, -0.f);
+        if (p.col_scale) f = *reinterpret_cast<const float4*>(p.col_scale + n);
+        if (p.residual) r = *reinterpret_cast<const float4*>(p.residual + at);
+        *reinterpret_cast<float4*>(p.out + at) = make_float4(fmaf(v[0] * first, f.x, r.x), fmaf(v[1] * first, f.y, r.y),
+                                                             fmaf(v[2] * first, f.z, r.z), fmaf(v[3] * first, f.w, r.w));
         continue;
       }
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         if (n + j >= N) break;
-        float f = p.scale;
-        if (p.col_scale) {
-          v[j] *= p.scale;
-          f = p.col_scale[n + j];
-        }
-        p.out[at + j] = p.residual ? fmaf(v[j], f, p.residual[at + j]) : v[j] * f;
+        p.out[at + j] = fmaf(v[j] * first, p.col_scale ? p.col_scale[n + j] : p.scale, p.residual ? p.residual[at + j] : -0.f);
       }
     }
   }
