@@ -246,26 +246,35 @@ __device__ __forceinline__ void block_add(float (&v)[N], float* s) {
   }
 }
 
-// One of the values that a step needs before its recurrence: a channel of q, k or v after convolution and
-// silu, or a decay.  Loaded before it is used, so that a thread has several on the way.
-template <typename T>
-struct StepItem {
-  T x[kWindow], w[kWindow];
-  float z;
+// Two neighbouring elements as loaded.
+template <typename T> struct Raw2;
+template <> struct Raw2<bf16> {
+  uint32_t v;
+  __device__ __forceinline__ float2 get() const { return make_float2(bf_lo(v), bf_hi(v)); }
 };
+template <> struct Raw2<float> {
+  float2 v;
+  __device__ __forceinline__ float2 get() const { return v; }
+};
+template <typename T>
+__device__ __forceinline__ Raw2<T> load2(const T* p) { return *reinterpret_cast<const Raw2<T>*>(p); }
 
 // A block per head and sequence does the whole step: convolution, norms, decay, recurrence, head norm,
 // gate.  A thread keeps RP rows of four columns of the state in registers (loaded before anything
 // else), so the state is read and written once: with a = (g S)^T k and o = (g S)^T q from one pass,
 // u = beta (v - a), the new state is g S + k u^T and the result o + (k . q) u.
-template <typename T, int RP>
+// Bound by: instructions. A step of 64 sequences x 16 heads of 128 x 128 was 1 990 instructions a warp and 42 us for its 134 MB
+// (21 at the copy bandwidth), whether an SM held two, three or four blocks; with the head's widths known to the compiler
+// (D = 128 for both; 0: any) and two channels of the convolution at a time it is 30. The state partly in shared
+// memory, for three blocks an SM, gained nothing more and cost steps of few sequences 2 %.
+template <typename T, int RP, int D>
 __global__ void __launch_bounds__(kThreads, RP <= 16 ? 2 : 1)
 delta_step_kernel(const DeltaParams p) {
   extern __shared__ float sm[];
   __shared__ float s_red[3 * kThreads / 32];
   pdl_enter();
   const int h = blockIdx.x, b = blockIdx.y, rep = p.H / p.G, g = h / rep, tid = threadIdx.x;
-  const int dkp = p.dkp, dvp = p.dvp, C = delta_channels(p);
+  const int dkp = D ? D : p.dkp, dvp = D ? D : p.dvp, C = 2 * p.G * dkp + p.H * dvp;
   float* sq = sm;                  // [dkp]
   float* sk = sq + dkp;
   float* sg = sk + dkp;            // decays
@@ -285,59 +294,52 @@ delta_step_kernel(const DeltaParams p) {
   const int pos = first_position(p);
   T* ring = static_cast<T*>(p.ring) + static_cast<long long>(b) * p.taps * C;
   const T* taps = static_cast<const T*>(p.taps_w);
+  const int slot = pos % p.taps;
   int back[kWindow];                      // offset in the ring of the input j tokens back, -1: none
 #pragma unroll
-  for (int j = 0; j < kWindow; ++j) back[j] = j < p.taps && j <= pos ? (pos - j) % p.taps * C : -1;
+  for (int j = 0; j < kWindow; ++j) back[j] = j < p.taps && j <= pos ? (slot >= j ? slot - j : slot - j + p.taps) * C : -1;
   const bool first = h % rep == 0;        // the block that brings the ring up to date for its q / k head
   const float rate = p.rate[h];
   const float* zg = p.zg + b * p.ldz;
-  // items: q, k, v channels, decays
+  // q, k, v after convolution and silu, and the decays, two neighbours at a time (all widths are even)
   const int n_k = dkp, n_v = 2 * dkp, n_g = n_v + dvp, total = n_g + dkp;
-  auto channel_of = [&](int i) { return i < n_v ? (i < n_k ? g * dkp + i : (p.G + g) * dkp + i - n_k) : 2 * p.G * dkp + h * dvp + i - n_v; };
-  auto load = [&](int i, StepItem<T>& r) {
-    if (i >= total) return;
+  for (int i = 2 * tid; i < total; i += 2 * kThreads) {
     if (i >= n_g) {
       const int c = h * dkp + i - n_g;
-      r.z = zg[c] + p.dt_bias[c];
-      return;
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const float z = zg[c + e] + p.dt_bias[c + e];
+        sg[i - n_g + e] = sizeof(T) == 2 ? exp2_approx(-rate * 1.4426950408889634f * softplus_fast(z))
+                                         : expf(-rate * softplus_precise(z));
+      }
+      continue;
     }
     const T* in = i < n_k ? static_cast<const T*>(p.q) + g * dkp + i
                           : i < n_v ? static_cast<const T*>(p.k) + g * dkp + i - n_k
                                     : static_cast<const T*>(p.v) + h * dvp + i - n_v;
-    const int ch = channel_of(i);
-    r.x[0] = in[b * p.ldp];
-    r.w[0] = taps[(p.taps - 1) * C + ch];
+    const int ch = i < n_v ? (i < n_k ? g * dkp + i : (p.G + g) * dkp + i - n_k) : 2 * p.G * dkp + h * dvp + i - n_v;
+    Raw2<T> x[kWindow], w[kWindow];
+    x[0] = load2(in + b * p.ldp);
 #pragma unroll
-    for (int j = 1; j < kWindow; ++j) {
-      r.x[j] = back[j] >= 0 ? ring[back[j] + ch] : from_f32<T>(0.f);
-      r.w[j] = back[j] >= 0 ? taps[(p.taps - 1 - j) * C + ch] : from_f32<T>(0.f);
+    for (int j = 0; j < kWindow; ++j) {
+      if (j > 0) x[j] = back[j] >= 0 ? load2(ring + back[j] + ch) : Raw2<T>{};
+      w[j] = back[j] >= 0 ? load2(taps + (p.taps - 1 - j) * C + ch) : Raw2<T>{};
     }
-  };
-  auto finish = [&](int i, const StepItem<T>& r) {
-    if (i >= total) return;
-    if (i >= n_g) {
-      sg[i - n_g] = sizeof(T) == 2 ? exp2_approx(-rate * 1.4426950408889634f * softplus_fast(r.z))
-                                   : expf(-rate * softplus_precise(r.z));
-      return;
-    }
-    const int ch = channel_of(i);
-    float y = 0.f;
+    float2 y = make_float2(0.f, 0.f);
     for (int j = p.taps - 1; j >= kWindow; --j)             // more taps than the window holds
-      if (j <= pos)
-        y = fmaf(to_f32(taps[(p.taps - 1 - j) * C + ch]), to_f32(ring[(pos - j) % p.taps * C + ch]), y);
+      if (j <= pos) {
+        const float2 u = load2(taps + (p.taps - 1 - j) * C + ch).get(), v = load2(ring + (pos - j) % p.taps * C + ch).get();
+        y = make_float2(fmaf(u.x, v.x, y.x), fmaf(u.y, v.y, y.y));
+      }
 #pragma unroll
-    for (int j = kWindow - 1; j >= 0; --j) y = fmaf(to_f32(r.w[j]), to_f32(r.x[j]), y);
-    y = to_f32(from_f32<T>(sizeof(T) == 2 ? silu_fast(y) : silu_precise(y)));
-    if (i < n_v) sq[i] = y;               // k follows q
-    else sv[i - n_v] = y;
-    if (i >= n_v || first) ring[back[0] + ch] = r.x[0];
-  };
-  for (int i = tid; i < total; i += 2 * kThreads) {
-    StepItem<T> r0, r1;
-    load(i, r0);
-    load(i + kThreads, r1);
-    finish(i, r0);
-    finish(i + kThreads, r1);
+    for (int j = kWindow - 1; j >= 0; --j) {
+      const float2 u = w[j].get(), v = x[j].get();
+      y = make_float2(fmaf(u.x, v.x, y.x), fmaf(u.y, v.y, y.y));
+    }
+    const float y0 = to_f32(from_f32<T>(sizeof(T) == 2 ? silu_fast(y.x) : silu_precise(y.x)));
+    const float y1 = to_f32(from_f32<T>(sizeof(T) == 2 ? silu_fast(y.y) : silu_precise(y.y)));
+    *reinterpret_cast<float2*>((i < n_v ? sq + i : sv + i - n_v)) = make_float2(y0, y1);      // k follows q
+    if (i >= n_v || first) *reinterpret_cast<Raw2<T>*>(ring + back[0] + ch) = x[0];
   }
   __syncthreads();
   float sums[3] = {0.f, 0.f, 0.f};        // |q|^2, |k|^2, k . q
@@ -516,10 +518,11 @@ cudaError_t launch_step(const DeltaParams& p, cudaStream_t st) {
   const int rgs = kThreads / (p.dvp / 4), rp = step_rows(p);
   const size_t bytes = (3 * p.dkp + 2 * p.dvp + 2 * rgs * p.dvp) * sizeof(float);
   const dim3 grid(p.H, p.B), block(kThreads);
-  if (rp <= 4) return launch_kernel(delta_step_kernel<T, 4>, grid, block, bytes, st, p);
-  if (rp <= 8) return launch_kernel(delta_step_kernel<T, 8>, grid, block, bytes, st, p);
-  if (rp <= 16) return launch_kernel(delta_step_kernel<T, 16>, grid, block, bytes, st, p);
-  if (rp <= 32) return launch_kernel(delta_step_kernel<T, 32>, grid, block, bytes, st, p);
+  if (p.dkp == 128 && p.dvp == 128) return launch_kernel(delta_step_kernel<T, 16, 128>, grid, block, bytes, st, p);
+  if (rp <= 4) return launch_kernel(delta_step_kernel<T, 4, 0>, grid, block, bytes, st, p);
+  if (rp <= 8) return launch_kernel(delta_step_kernel<T, 8, 0>, grid, block, bytes, st, p);
+  if (rp <= 16) return launch_kernel(delta_step_kernel<T, 16, 0>, grid, block, bytes, st, p);
+  if (rp <= 32) return launch_kernel(delta_step_kernel<T, 32, 0>, grid, block, bytes, st, p);
   return cudaErrorInvalidValue;
 }
 
