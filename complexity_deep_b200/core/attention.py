@@ -246,8 +246,8 @@ class ComplexityAttention(nn.Module):
 
     def _attend_static(self, x2, mu2, past: StaticKVLayer, S, attention_mask) -> torch.Tensor:
         """Decode step on a StaticKVCache: projection, then one kernel that normalises and
-        rotates q / k at the device-side position and appends k / v to the cache, then the
-        split-KV attention over the device-side length."""
+        rotates q / k at the device-side position, appends k / v to the cache and attends over
+        the device-side length."""
         hq, hkv, D = self.num_heads, self.num_kv_heads, self.head_dim
         if S != 1 or attention_mask is not None:
             raise RuntimeError("a StaticKVCache takes one new token per sequence and no mask "
@@ -258,11 +258,9 @@ class ComplexityAttention(nn.Module):
         cache = past.cache
         cos, sin = self.rotary_emb.tables_fp32(cache.capacity)
         qkv = ops.mu_qkv(x2, mu2, self._w_qkv(), self._w_mu() if mu2 is not None else None)
-        ops.decode_rope_append(qkv, self.q_norm.weight if self.use_qk_norm else None,
-                               self.k_norm.weight if self.use_qk_norm else None, cos, sin, 1e-6,
-                               hq, hkv, D, past.k, past.v, cache.state[0:1])
-        return ops.decode_attention(qkv, past.k, past.v, None, hq, hkv, D,
-                                    kv_len_dev=cache.state[1:2])
+        return ops.decode_step_attention(qkv, self.q_norm.weight if self.use_qk_norm else None,
+                                         self.k_norm.weight if self.use_qk_norm else None, cos, sin, 1e-6,
+                                         hq, hkv, D, past.k, past.v, cache.state[0:1], cache.state[1:2])
 
     def _prefill_kernel_applies(self, B, S, attention_mask, past_key_value) -> bool:
         if attention_mask is not None or past_key_value is not None or not _PREFILL_KERNEL:

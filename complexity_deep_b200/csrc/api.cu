@@ -165,8 +165,8 @@ int cd_decode_rope_append(void* qkv, const void* q_w, const void* k_w, const flo
 }
 
 size_t cd_decode_attention_workspace_bytes(int B, int hq, int hkv, int L, int D) {
-  if (B < 1 || hq < 1 || hkv < 1 || L < 1 || D < 1 || hq % hkv) return 0;
-  return decode_attention_workspace_bytes(B, hq, hkv, L, D);
+  (void)B, (void)hq, (void)hkv, (void)L, (void)D;
+  return 0;
 }
 
 int cd_decode_attention(const void* q, long long q_stride_b, const void* k, const void* v,
@@ -177,15 +177,35 @@ int cd_decode_attention(const void* q, long long q_stride_b, const void* k, cons
   if (B < 1 || hq < 1 || hkv < 1 || L < 1 || hq % hkv) return CD_ERR_INVALID;
   if (D != 64 && D != 128) return CD_ERR_UNSUPPORTED;
   if (hq / hkv > 4) return CD_ERR_UNSUPPORTED;
-  if (!q || !k || !v || !out || !ws) return CD_ERR_INVALID;
+  (void)ws, (void)ws_bytes;
+  if (!q || !k || !v || !out) return CD_ERR_INVALID;
   if (!aligned16(q) || !aligned16(k) || !aligned16(v) || !aligned16(out)) return CD_ERR_INVALID;
   if ((q_stride_b & 7) || (kv_stride_b & 7) || (kv_stride_h & 7) || (kv_stride_t & 7))
     return CD_ERR_INVALID;
-  if (ws_bytes < decode_attention_workspace_bytes(B, hq, hkv, L, D)) return CD_ERR_INVALID;
   cudaError_t e = launch_decode_attention(q, q_stride_b, k, v, kv_stride_b, kv_stride_h,
                                           kv_stride_t, mask, mask_stride_b, scale, B, hq, hkv, L,
-                                          D, out, ws, as_stream(stream), kv_len_dev);
+                                          D, out, as_stream(stream), kv_len_dev);
   return e == cudaSuccess ? CD_OK : cuda_fail(e, "decode attention launch");
+}
+
+int cd_decode_step_attention(const void* qkv, const void* q_w, const void* k_w, const float* cos_t,
+                             const float* sin_t, float eps, float scale, int B, int hq, int hkv, int D,
+                             void* k_cache, void* v_cache, long long kv_stride_b, long long kv_stride_h,
+                             long long kv_stride_t, int capacity, const int32_t* pos_dev,
+                             const int32_t* kv_len_dev, void* out, void* stream) {
+  if (B < 1 || hq < 1 || hkv < 1 || capacity < 1 || hq % hkv) return CD_ERR_INVALID;
+  if (D != 64 && D != 128) return CD_ERR_UNSUPPORTED;
+  if (hq / hkv > 4) return CD_ERR_UNSUPPORTED;
+  if (!qkv || !cos_t || !sin_t || !k_cache || !v_cache || !pos_dev || !kv_len_dev || !out) return CD_ERR_INVALID;
+  if ((q_w == nullptr) != (k_w == nullptr)) return CD_ERR_INVALID;
+  if (!aligned16(qkv) || !aligned16(k_cache) || !aligned16(v_cache) || !aligned16(out) || !aligned16(cos_t) ||
+      !aligned16(sin_t) || (q_w && (!aligned16(q_w) || !aligned16(k_w))))
+    return CD_ERR_INVALID;
+  if ((kv_stride_b & 7) || (kv_stride_h & 7) || (kv_stride_t & 7)) return CD_ERR_INVALID;
+  cudaError_t e = launch_decode_step_attention(qkv, q_w, k_w, cos_t, sin_t, eps, k_cache, v_cache, kv_stride_b,
+                                               kv_stride_h, kv_stride_t, capacity, pos_dev, kv_len_dev, scale, B, hq,
+                                               hkv, D, out, as_stream(stream));
+  return e == cudaSuccess ? CD_OK : cuda_fail(e, "decode step attention launch");
 }
 
 int cd_attention_prefill_supported(int B, int S, int hq, int hkv, int D) {

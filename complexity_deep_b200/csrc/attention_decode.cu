@@ -12,7 +12,19 @@
 // covers 128 contiguous bytes of the row (whole sectors, no re-fetch); a warp streams 4 rows
 // per step; every lane group
 // keeps an online-softmax state (running max, sum, weighted V) per query head, merged across
-// the block through shared memory and across splits by a second small kernel.
+// the block through shared memory. The splits of a pair are one thread-block cluster and
+// merge through one another's shared memory, each block a share of the columns.
+//
+// A decode step (kStep) hands over the raw projections: every block normalises and rotates the query
+// heads of its group itself (8 lanes a head, as many as the rows need anyway), and the one
+// whose rows include the new token does so for its key, writes key and value into the cache
+// and takes the row behind all others, from shared memory.
+//
+// Bound by HBM for a full device (B 32, 8 kv heads, 2 064 rows of 128: 270 MB), by the launch and the chain of one
+// block before that. A step used to be three launches (rotation and append, partial sums to memory, their sum), each
+// with its own start, end and round trip through L2. us, cold L2, three launches / this one: 1 sequence x 4 kv heads x 302
+// rows of 3 x 64 9.3 / 5.6, 1 x 8 x 2 064 of 2 x 128 11.9 / 10.4, 8 x 8 x 1 000 16.4 / 13.7, 32 x 8 x 2 064 52.0 / 49.9,
+// 64 x 8 x 2 064 103 / 91.
 #include <cfloat>
 #include <cstdint>
 #include <cuda_bf16.h>
@@ -26,7 +38,8 @@ namespace {
 constexpr int kAttnThreads = 128;
 constexpr int kMaxGroup = 4;    // query heads per KV head handled by one block (the entry point refuses more)
 constexpr int kLanesPerRow = 8;
-constexpr int kMaxSplits = 64;
+constexpr int kMaxSplits = 16;  // of a pair: the largest cluster that there is
+constexpr int kPortable = 8;    // the largest that every launch may ask for
 
 __device__ __forceinline__ float lo_f(uint32_t v) { return __uint_as_float(v << 16); }
 __device__ __forceinline__ float hi_f(uint32_t v) { return __uint_as_float(v & 0xffff0000u); }
@@ -34,30 +47,48 @@ __device__ __forceinline__ float hi_f(uint32_t v) { return __uint_as_float(v & 0
 // Blocks that an SM holds at a time, by the registers of G query heads of D dimensions.
 __host__ __device__ constexpr int blocks_per_sm(int G, int D) { return G * D > 384 ? 2 : G * D > 256 ? 3 : 4; }
 
-// Blocks per (batch, kv head) pair.  Also evaluated on the device when the cache length is
-// read from device memory, so both forms split (and therefore round) identically; never falls as L grows.
-// kSms is a tuning constant (a B200's 148 SMs), not a limit: any other SM count only changes how many
-// blocks share the work.
-//   Two splits of every pair fit the device at once: as many as do, down to 48 rows a block, in one wave (at most 32:
-//   the combining kernel reads them all). us, this rule / at least 512 rows a block and up to four waves, partial and
-//   combine, cold L2: 1 sequence x 4 kv heads x 302 rows 11 / 17; 1 x 8 x 2064 13 / 24; 8 x 8 x 1000 18 / 24;
-//   32 x 8 x 2064 64 / 73 (1 280 blocks are 2.2 waves).
-//   More pairs: several waves of at least 512 rows a block keep the last one short.
-constexpr int kSms = 148;
-__host__ __device__ inline int choose_splits(int B, int hkv, int L, int per_sm) {
-  const int pairs = B * hkv, one_wave = per_sm * kSms / pairs;
-  int splits, max_splits;
-  if (one_wave >= 2) {
-    splits = one_wave < 32 ? one_wave : 32;
-    max_splits = (L + 47) / 48;
-  } else {
-    splits = (16 * kSms + pairs - 1) / pairs;
-    max_splits = (L + 511) / 512;
+// How the rows of a (batch, kv head) pair are split over the blocks of a cluster: at most `most` blocks of at least
+// `min_rows` rows, and more than eight only of 72 rows or more.  Evaluated on the device as well when the cache length is read
+// from there, so both forms split (and therefore round) identically; never falls as L grows.
+struct Split {
+  int most, min_rows;
+  __host__ __device__ int of(int L) const {
+    int n = (L + min_rows - 1) / min_rows;
+    if (n > kPortable) n = max(kPortable, (L + 71) / 72);
+    return max(1, min(most, n));
   }
-  if (splits > max_splits) splits = max_splits;
-  if (splits < 1) splits = 1;
-  if (splits > kMaxSplits) splits = kMaxSplits;
-  return splits;
+};
+// Clusters of 1 .. 16 blocks that a B200 holds at a time (cudaOccupancyMaxActiveClusters: a cluster lies within one GPC,
+// so the SMs that are left over in each go unused), by blocks per SM. Tuning constants: other figures only change how many
+// blocks share the work.
+constexpr int kSms = 148;
+constexpr short kActive[3][kMaxSplits] = {{296, 148, 93, 71, 56, 45, 37, 33, 30, 26, 21, 21, 17, 14, 14, 14},
+                                          {444, 222, 142, 104, 82, 71, 56, 48, 45, 41, 31, 31, 28, 24, 24, 21},
+                                          {592, 296, 187, 142, 112, 93, 78, 71, 60, 56, 45, 42, 38, 35, 31, 31}};
+//   Two blocks of every pair fit the device at once: the largest cluster of which one per pair fits; 9 to 12 blocks are no
+//   better than eight, and all sixteen worth it for eight pairs only. us, cold L2, heads of 2 x 128 and 2 064 rows, by the
+//   size of the cluster: 8 pairs 8: 12.0, 13: 9.8, 16: 9.3; 16 pairs 8: 13.2, 13: 10.7, 16: 12.3; 32 pairs 8: 14.3, 11:
+//   14.3, 13: 13.5, 16: 19.2; 64 pairs 7: 18.9, 8: 18.2, 9: 26; 96 pairs 4: 27.3, 5: 23.2, 6: 32.6; 128 pairs 3: 33, 4:
+//   28.3, 5: 38.6; 256 pairs 1: 66, 2: 47.7, 3: 60. Down to 48 rows a block: 4 pairs of 302 rows of 3 x 64, 3: 6.9, 5: 5.3,
+//   7: 4.8; above eight blocks the larger launch costs more (32 pairs of 400 rows 7: 7.3, 9: 8.3).
+//   More pairs: the size whose waves are fullest, each block more costing some 5 % (320 pairs 1: 84, 2: 81, 3: 65, 4: 73,
+//   5: 66; 512 pairs 1: 86, 2: 93, 5: 105, 8: 121).
+inline Split choose_split(int B, int hkv, int per_sm) {
+  const long long pairs = static_cast<long long>(B) * hkv;
+  const short(&active)[kMaxSplits] = kActive[per_sm - 2];
+  if (pairs <= active[1]) {
+    int fit = 2;
+    while (fit < kMaxSplits && pairs <= active[fit]) ++fit;
+    return {fit >= 13 ? (pairs <= 8 ? kMaxSplits : 13) : fit > kPortable ? kPortable : fit, 48};
+  }
+  int best = 1;
+  long long best_score = -1;
+  for (int c = 1; c <= 5; ++c) {
+    const long long waves = (pairs + active[c - 1] - 1) / active[c - 1];
+    const long long score = 1000 * pairs * c / (waves * per_sm * kSms) - 50 * (c - 1);
+    if (score > best_score) best = c, best_score = score;
+  }
+  return {best, 256};
 }
 
 __host__ __device__ inline int chunk_rows(int L, int splits) {
@@ -81,25 +112,119 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// *p of this block, read from the block of rank `rank` of the cluster
+__device__ __forceinline__ float peer_load(const float* p, int rank) {
+  uint32_t a;
+  float v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(p))), "r"(rank));
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+  return v;
+}
+
+// What a decode step brings besides the query: norm weights (or none), rotation tables, where the new row goes.
+struct StepArgs {
+  const __nv_bfloat16 *q_w, *k_w;
+  const float *cos_t, *sin_t;
+  float eps;
+  __nv_bfloat16 *k_cache, *v_cache;
+  const int* pos_dev;
+  int capacity;
+};
+
+// One head by 8 lanes: RMSNorm and rotation as qk_norm_rope_vec_kernel computes them, rounded to bf16. Lane `sub` holds
+// columns j .. j + 7 and D / 2 + j ..; of 64 columns two lanes hold the same ones, and each returns the half that it
+// owns in the row layout (dims 8 sub of every 64).
+template <int D>
+__device__ __forceinline__ int rope_col(int sub) { return (sub & (D / 16 - 1)) * 8; }
+struct Halves {
+  uint4 a, b;
+};
+template <int D>
+__device__ __forceinline__ Halves load_halves(const __nv_bfloat16* p, int sub) {
+  const __nv_bfloat16* x = p + rope_col<D>(sub);
+  return {*reinterpret_cast<const uint4*>(x), *reinterpret_cast<const uint4*>(x + D / 2)};
+}
+struct Angles {                  // cosines and sines of the two halves
+  float c1[8], s1[8], c2[8], s2[8];
+};
+template <int D>
+__device__ __forceinline__ void load_angles(Angles& t, const float* cs, const float* sn, int sub) {
+  const int j = rope_col<D>(sub);
+#pragma unroll
+  for (int v = 0; v < 2; ++v) {
+    *reinterpret_cast<float4*>(t.c1 + 4 * v) = *reinterpret_cast<const float4*>(cs + j + 4 * v);
+    *reinterpret_cast<float4*>(t.s1 + 4 * v) = *reinterpret_cast<const float4*>(sn + j + 4 * v);
+    *reinterpret_cast<float4*>(t.c2 + 4 * v) = *reinterpret_cast<const float4*>(cs + D / 2 + j + 4 * v);
+    *reinterpret_cast<float4*>(t.s2 + 4 * v) = *reinterpret_cast<const float4*>(sn + D / 2 + j + 4 * v);
+  }
+}
+template <int D>
+__device__ __forceinline__ void norm_rope(const Halves& x, const Halves& w, bool normed, const Angles& t, float eps, bool rotate,
+                                          int sub, uint4 (&out)[D / 64]) {
+  constexpr int kLanes = D / 16;
+  const uint32_t aw[4] = {x.a.x, x.a.y, x.a.z, x.a.w}, bw[4] = {x.b.x, x.b.y, x.b.z, x.b.w};
+  float x1[8], x2[8], ss = 0.f;
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    x1[2 * e] = lo_f(aw[e]); x1[2 * e + 1] = hi_f(aw[e]);
+    x2[2 * e] = lo_f(bw[e]); x2[2 * e + 1] = hi_f(bw[e]);
+    ss += x1[2 * e] * x1[2 * e] + x1[2 * e + 1] * x1[2 * e + 1] + x2[2 * e] * x2[2 * e] + x2[2 * e + 1] * x2[2 * e + 1];
+  }
+#pragma unroll
+  for (int o = kLanes >> 1; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+  uint4 lo = x.a, hi = x.b;
+  if (rotate) {
+    if (normed) {
+      const float rstd = rsqrtf(ss / static_cast<float>(D) + eps);
+      const uint32_t w1[4] = {w.a.x, w.a.y, w.a.z, w.a.w}, w2[4] = {w.b.x, w.b.y, w.b.z, w.b.w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        x1[2 * e] *= rstd * lo_f(w1[e]); x1[2 * e + 1] *= rstd * hi_f(w1[e]);
+        x2[2 * e] *= rstd * lo_f(w2[e]); x2[2 * e + 1] *= rstd * hi_f(w2[e]);
+      }
+    }
+    uint32_t o1[4], o2[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int i = 2 * e, k = 2 * e + 1;
+      const __nv_bfloat162 p1 = __floats2bfloat162_rn(x1[i] * t.c1[i] - x2[i] * t.s1[i], x1[k] * t.c1[k] - x2[k] * t.s1[k]);
+      const __nv_bfloat162 p2 = __floats2bfloat162_rn(x2[i] * t.c2[i] + x1[i] * t.s2[i], x2[k] * t.c2[k] + x1[k] * t.s2[k]);
+      o1[e] = *reinterpret_cast<const uint32_t*>(&p1);
+      o2[e] = *reinterpret_cast<const uint32_t*>(&p2);
+    }
+    lo = make_uint4(o1[0], o1[1], o1[2], o1[3]);
+    hi = make_uint4(o2[0], o2[1], o2[2], o2[3]);
+  }
+  if constexpr (D == 64) {
+    out[0] = sub < kLanes ? lo : hi;
+  } else {
+    out[0] = lo;
+    out[1] = hi;
+  }
+}
+
 constexpr int kStages = 4;   // row steps staged in shared memory per thread (3 in flight)
 
 // DPL = dimensions per lane = D / 8 (8 or 16 -> D = 64 or 128), G = query heads per KV head.
 // len_dev (optional): the number of cached rows is min(L, *len_dev) and the split of the rows
-// over blocks is recomputed from it; the grid and the workspace layout stay those of L.
+// over blocks is recomputed from it; the grid stays that of L, and blocks beyond the split only
+// take part in the cluster's barriers.
 //
 // A row step = 16 cached rows of the block (4 warps x 4 lane groups), 2 * DPL bytes of K and
 // of V per lane.  Every lane copies its own slices of the next kStages - 1 steps into a
 // private slot of shared memory with cp.async (bytes in flight without holding registers:
 // 4 blocks per SM keep ~100 KB on the way) and reads them back with 16-byte loads, so no
 // block-level synchronisation is needed inside the loop.
-template <int DPL, int G>
+template <int DPL, int G, bool kStep>
 __global__ void __launch_bounds__(kAttnThreads, blocks_per_sm(G, DPL * kLanesPerRow))
-decode_attn_partial_kernel(const __nv_bfloat16* __restrict__ q, long long q_stride_b,
-                           const __nv_bfloat16* __restrict__ k, const __nv_bfloat16* __restrict__ v,
-                           long long kv_stride_b, long long kv_stride_h, long long kv_stride_t,
-                           const __nv_bfloat16* __restrict__ mask, long long mask_stride_b,
-                           float scale, int L, int chunk, int hq, float* __restrict__ part_acc,
-                           float* __restrict__ part_ml, const int* __restrict__ len_dev) {
+decode_attn_kernel(const __nv_bfloat16* __restrict__ q, long long q_stride_b,
+                   const __nv_bfloat16* k, const __nv_bfloat16* v,
+                   long long kv_stride_b, long long kv_stride_h, long long kv_stride_t,
+                   const __nv_bfloat16* __restrict__ mask, long long mask_stride_b,
+                   float scale, int L, Split rule, __nv_bfloat16* __restrict__ out,
+                   const int* __restrict__ len_dev, StepArgs st) {
   constexpr int D = DPL * kLanesPerRow;
   constexpr int kV = DPL / 8;                               // 16-byte pieces of K (and of V) per lane
   constexpr int kStepBytes = kAttnThreads * 2 * kV * 16;    // one row step of the block
@@ -107,39 +232,38 @@ decode_attn_partial_kernel(const __nv_bfloat16* __restrict__ q, long long q_stri
   constexpr int kSmemBytes = kStages * kStepBytes > kMergeBytes ? kStages * kStepBytes : kMergeBytes;
   __shared__ __align__(16) unsigned char s_raw[kSmemBytes];
   __shared__ float s_m[16][G], s_l[16][G];
+  __shared__ float s_part[G * D + 2 * G];                   // this block's sums, then its maxima and sums of weights
+  __shared__ uint4 s_new[2 * kV][kStep ? kLanesPerRow : 1];
 
   griddep_wait();
   griddep_launch_dependents();
-  const int split = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
-  const int splits = gridDim.x;
-  if (len_dev) {
-    L = max(0, min(L, __ldg(len_dev)));
-    const int live = choose_splits(gridDim.z, gridDim.y, L, blocks_per_sm(G, D));
-    if (split >= live) return;       // whole block; the combine kernel skips these slots
-    chunk = chunk_rows(L, live);
-  }
+  const int split = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z, hkv = gridDim.y;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int sub = lane & 7;          // which D/8 slice of the row
   const int rgrp = lane >> 3;        // which of the warp's 4 concurrent rows
-  const int t_begin = split * chunk;
-  const int t_end = min(L, t_begin + chunk);
-
-  // query fragments of the G heads, pre-scaled
-  float qf[G][DPL];
+  // all that a step needs besides the cache is asked for before the first rows, whose copies end the reach of a load
+  const __nv_bfloat16* row = q + b * q_stride_b;
+  Halves qx[G], qw = {};
+  Angles ang;
+  int pos = -1;                      // the row that this step brings
+  if constexpr (kStep) {
+    pos = __ldg(st.pos_dev);
 #pragma unroll
-  for (int g = 0; g < G; ++g) {
-    const __nv_bfloat16* qp = q + b * q_stride_b + static_cast<long long>(kvh * G + g) * D + sub * 8;
-#pragma unroll
-    for (int i = 0; i < DPL; i += 8) {
-      const uint4 w = *reinterpret_cast<const uint4*>(qp + i * 8);
-      const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        qf[g][i + 2 * e] = lo_f(ww[e]) * scale;
-        qf[g][i + 2 * e + 1] = hi_f(ww[e]) * scale;
-      }
-    }
+    for (int g = 0; g < G; ++g) qx[g] = load_halves<D>(row + static_cast<long long>(kvh * G + g) * D, sub);
+    if (st.q_w) qw = load_halves<D>(st.q_w, sub);
   }
+  if (len_dev) L = max(0, min(L, __ldg(len_dev)));
+  const int splits = rule.of(L);
+  const int chunk = chunk_rows(L, splits);
+  const int t_begin = min(L, split * chunk);
+  const int t_end = min(L, t_begin + chunk);
+  bool owner = false;                // of the new row: the warp whose rows include it, or beyond all rows the first
+  if constexpr (kStep) {
+    if (pos < 0 || pos >= st.capacity) pos = -1;
+    owner = pos >= 0 && (pos < L ? pos >= t_begin && pos < t_end && warp == (((pos - t_begin) >> 2) & 3) : split + warp == 0);
+    load_angles<D>(ang, st.cos_t + static_cast<long long>(max(pos, 0)) * D, st.sin_t + static_cast<long long>(max(pos, 0)) * D, sub);
+  }
+
   float m_run[G], l_run[G], acc[G][DPL];
 #pragma unroll
   for (int g = 0; g < G; ++g) {
@@ -150,7 +274,7 @@ decode_attn_partial_kernel(const __nv_bfloat16* __restrict__ q, long long q_stri
   }
   const __nv_bfloat16* kb = k + b * kv_stride_b + kvh * kv_stride_h + sub * 8;
   const __nv_bfloat16* vb = v + b * kv_stride_b + kvh * kv_stride_h + sub * 8;
-  const __nv_bfloat16* mb = mask ? mask + b * mask_stride_b : nullptr;
+  const __nv_bfloat16* mb = !kStep && mask ? mask + b * mask_stride_b : nullptr;
 
   // slot of (stage, piece) for this thread: consecutive threads are 16 bytes apart, so both
   // the asynchronous writes and the reads are free of bank conflicts
@@ -161,7 +285,7 @@ decode_attn_partial_kernel(const __nv_bfloat16* __restrict__ q, long long q_stri
   const int n_steps = (t_end - t_begin + 15) >> 4;          // same for the whole block
   auto issue = [&](int step) {
     const int t = t_lane + step * 16;
-    if (step < n_steps && t < t_end) {
+    if (step < n_steps && t < t_end && (!kStep || t != pos)) {
       const int stage = step % kStages;
 #pragma unroll
       for (int i = 0; i < kV; ++i) {
@@ -174,6 +298,49 @@ decode_attn_partial_kernel(const __nv_bfloat16* __restrict__ q, long long q_stri
 #pragma unroll
   for (int s0 = 0; s0 < kStages - 1; ++s0) issue(s0);
 
+  // query fragments of the G heads, pre-scaled
+  float qf[G][DPL];
+#pragma unroll
+  for (int g = 0; g < G; ++g) {
+    uint4 w[kV];
+    if constexpr (kStep) {
+      norm_rope<D>(qx[g], qw, st.q_w != nullptr, ang, st.eps, pos >= 0, sub, w);
+    } else {
+#pragma unroll
+      for (int i = 0; i < kV; ++i) w[i] = *reinterpret_cast<const uint4*>(row + static_cast<long long>(kvh * G + g) * D + i * 64 + sub * 8);
+    }
+#pragma unroll
+    for (int i = 0; i < kV; ++i) {
+      const uint32_t ww[4] = {w[i].x, w[i].y, w[i].z, w[i].w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        qf[g][i * 8 + 2 * e] = lo_f(ww[e]) * scale;
+        qf[g][i * 8 + 2 * e + 1] = hi_f(ww[e]) * scale;
+      }
+    }
+  }
+  if constexpr (kStep) {
+    if (owner) {                       // the new row into the cache; its own step comes behind all others'
+      uint4 w[kV];
+      Halves kw = {};
+      if (st.k_w) kw = load_halves<D>(st.k_w, sub);
+      norm_rope<D>(load_halves<D>(row + static_cast<long long>(hkv * G + kvh) * D, sub), kw, st.k_w != nullptr, ang, st.eps, true,
+                   sub, w);
+      const __nv_bfloat16* vp = row + static_cast<long long>(hkv * (G + 1) + kvh) * D + sub * 8;
+      if (rgrp == 0) {
+#pragma unroll
+        for (int i = 0; i < kV; ++i) {
+          const uint4 x = *reinterpret_cast<const uint4*>(vp + i * 64);
+          const long long at = b * kv_stride_b + kvh * kv_stride_h + pos * kv_stride_t + i * 64 + sub * 8;
+          s_new[i][sub] = w[i];
+          s_new[kV + i][sub] = x;
+          *reinterpret_cast<uint4*>(st.k_cache + at) = w[i];
+          *reinterpret_cast<uint4*>(st.v_cache + at) = x;
+        }
+      }
+    }
+  }
+
   // Additive mask: once per 8 steps lane l fetches the value of row group (l & 3) of step
   // (window + l / 4) of this warp, one window ahead of its use; a step then takes its value
   // from the owning lane with a shuffle, so no step waits for a global load.
@@ -183,31 +350,13 @@ decode_attn_partial_kernel(const __nv_bfloat16* __restrict__ q, long long q_stri
   };
   float mwin = mask_window(0), mwin_next = mask_window(8);
 
-  for (int step = 0; step < n_steps; ++step) {
-    issue(step + kStages - 1);
-    float madd = 0.f;
-    if (mb) {                                               // uniform
-      const int j = step & 7;
-      if (j == 0 && step > 0) {
-        mwin = mwin_next;
-        mwin_next = mask_window(step + 8);
-      }
-      madd = __shfl_sync(0xffffffffu, mwin, (j << 2) | rgrp);
-    }
-    cp_async_wait<kStages - 1>();                           // this step's group has landed
-    const int t = t_lane + step * 16;
-    const bool valid = t < t_end;
-    const int stage = step % kStages;
+  // one row per lane group: its scores, and its share of the weighted sums
+  auto take = [&](const uint4 (&kr)[kV], const uint4 (&vr)[kV], bool valid, float madd) {
     float kf[DPL], vf[DPL];
 #pragma unroll
     for (int i = 0; i < kV; ++i) {
-      uint4 kr = make_uint4(0, 0, 0, 0), vr = kr;
-      if (valid) {
-        kr = *slot(stage, i);
-        vr = *slot(stage, kV + i);
-      }
-      const uint32_t kw[4] = {kr.x, kr.y, kr.z, kr.w};
-      const uint32_t vw[4] = {vr.x, vr.y, vr.z, vr.w};
+      const uint32_t kw[4] = {kr[i].x, kr[i].y, kr[i].z, kr[i].w};
+      const uint32_t vw[4] = {vr[i].x, vr[i].y, vr[i].z, vr[i].w};
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         kf[i * 8 + 2 * e] = lo_f(kw[e]); kf[i * 8 + 2 * e + 1] = hi_f(kw[e]);
@@ -238,6 +387,43 @@ decode_attn_partial_kernel(const __nv_bfloat16* __restrict__ q, long long q_stri
         for (int i = 0; i < DPL; ++i) acc[g][i] += pr * vf[i];
       }
     }
+  };
+  for (int step = 0; step < n_steps; ++step) {
+    issue(step + kStages - 1);
+    float madd = 0.f;
+    if (mb) {                                               // uniform
+      const int j = step & 7;
+      if (j == 0 && step > 0) {
+        mwin = mwin_next;
+        mwin_next = mask_window(step + 8);
+      }
+      madd = __shfl_sync(0xffffffffu, mwin, (j << 2) | rgrp);
+    }
+    cp_async_wait<kStages - 1>();                           // this step's group has landed
+    const int t = t_lane + step * 16, stage = step % kStages;
+    const bool valid = t < t_end && (!kStep || t != pos);
+    uint4 kr[kV], vr[kV];
+#pragma unroll
+    for (int i = 0; i < kV; ++i) {
+      kr[i] = vr[i] = make_uint4(0, 0, 0, 0);
+      if (valid) {
+        kr[i] = *slot(stage, i);
+        vr[i] = *slot(stage, kV + i);
+      }
+    }
+    take(kr, vr, valid, madd);
+  }
+  if constexpr (kStep) {
+    if (owner && pos < L) {
+      uint4 kr[kV], vr[kV];
+      __syncwarp();
+#pragma unroll
+      for (int i = 0; i < kV; ++i) {
+        kr[i] = s_new[i][sub];
+        vr[i] = s_new[kV + i][sub];
+      }
+      take(kr, vr, rgrp == ((pos - t_begin) & 3), 0.f);   // as the last row its sums are those of a cache that already holds it
+    }
   }
   cp_async_wait<0>();
   __syncthreads();                     // every lane is done with its slots: re-use them
@@ -267,119 +453,120 @@ decode_attn_partial_kernel(const __nv_bfloat16* __restrict__ q, long long q_stri
       l += s_l[s][g] * w;
       a += s_acc[s][g][d] * w;
     }
-    const long long row = (static_cast<long long>(b) * hq + kvh * G + g) * splits + split;
-    part_acc[row * D + d] = a;
+    s_part[idx] = a;
     if (d == 0) {
-      part_ml[row * 2] = m;
-      part_ml[row * 2 + 1] = l;
+      s_part[G * D + g] = m;
+      s_part[G * D + G + g] = l;
     }
+  }
+
+  // the splits of the pair: out = sum_s w_s acc_s / sum_s w_s l_s, w_s = exp(m_s - max m), every block a share of the columns
+  if (gridDim.x > 1) {
+    __syncwarp();
+    cluster_arrive();
+    cluster_wait();
+  } else {
+    __syncthreads();
+  }
+  for (int idx = split * kAttnThreads + threadIdx.x; idx < G * D; idx += gridDim.x * kAttnThreads) {
+    const int g = idx / D;
+    float ms[kMaxSplits], ls[kMaxSplits], as[kMaxSplits], m = -FLT_MAX;
+#pragma unroll
+    for (int s = 0; s < kMaxSplits; ++s) {
+      ms[s] = -FLT_MAX;
+      ls[s] = as[s] = 0.f;
+      if (s < splits) {
+        ms[s] = peer_load(&s_part[G * D + g], s);
+        ls[s] = peer_load(&s_part[G * D + G + g], s);
+        as[s] = peer_load(&s_part[idx], s);
+      }
+      m = fmaxf(m, ms[s]);
+    }
+    float l = 0.f, a = 0.f;
+#pragma unroll
+    for (int s = 0; s < kMaxSplits; ++s) {
+      const float w = ms[s] > -FLT_MAX ? __expf(ms[s] - m) : 0.f;
+      l += ls[s] * w;
+      a += as[s] * w;
+    }
+    out[(static_cast<long long>(b) * hkv + kvh) * G * D + idx] = __float2bfloat16_rn(l > 0.f ? a / l : 0.f);
+  }
+  if (gridDim.x > 1) {                 // nobody leaves while its sums are being read
+    __syncwarp();
+    cluster_arrive();
+    cluster_wait();
   }
 }
 
-// out[b, h, :] = sum_s w_s acc_s / sum_s w_s l_s, w_s = exp(m_s - max m). The weights of the (at most 64) splits are
-// found by one warp, a lane per split, so that what follows is one chain of independent loads per column.
-__global__ void __launch_bounds__(128)
-decode_attn_combine_kernel(const float* __restrict__ part_acc, const float* __restrict__ part_ml,
-                           int splits, int D, __nv_bfloat16* __restrict__ out, int B, int hkv,
-                           int L, int per_sm, const int* __restrict__ len_dev) {
-  __shared__ float s_w[kMaxSplits];
-  __shared__ float s_sum;
-  griddep_wait();
-  griddep_launch_dependents();
-  const long long row0 = static_cast<long long>(blockIdx.x) * splits;   // (b, h)
-  if (len_dev) splits = choose_splits(B, hkv, max(0, min(L, __ldg(len_dev))), per_sm);
-  const int lane = threadIdx.x & 31;
-  if (threadIdx.x < 32) {
-    float ms[kMaxSplits / 32], ls[kMaxSplits / 32], m = -FLT_MAX, sum = 0.f;
-#pragma unroll
-    for (int i = 0; i < kMaxSplits / 32; ++i) {
-      const int s = lane + 32 * i;
-      ms[i] = s < splits ? part_ml[(row0 + s) * 2] : -FLT_MAX;
-      ls[i] = s < splits ? part_ml[(row0 + s) * 2 + 1] : 0.f;
-      m = fmaxf(m, ms[i]);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-#pragma unroll
-    for (int i = 0; i < kMaxSplits / 32; ++i) {
-      const float w = ms[i] > -FLT_MAX ? __expf(ms[i] - m) : 0.f;
-      s_w[lane + 32 * i] = w;
-      sum += ls[i] * w;
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-    if (lane == 0) s_sum = sum;
+template <int DPL, int G, bool kStep>
+cudaError_t launch_one(dim3 grid, cudaStream_t stream, const __nv_bfloat16* q, long long qsb, const __nv_bfloat16* k,
+                       const __nv_bfloat16* v, long long sb, long long sh, long long stt, const __nv_bfloat16* mask,
+                       long long msb, float scale, int L, Split rule, __nv_bfloat16* out, const int* len_dev,
+                       const StepArgs& step) {
+  auto* kernel = decode_attn_kernel<DPL, G, kStep>;
+  if (grid.x > kPortable) {
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e != cudaSuccess) return e;
   }
-  __syncthreads();
-  const float l = s_sum;
-  for (int d = threadIdx.x; d < D; d += blockDim.x) {
-    float a = 0.f;
-#pragma unroll 8
-    for (int s = 0; s < splits; ++s) a += part_acc[(row0 + s) * D + d] * s_w[s];
-    out[static_cast<long long>(blockIdx.x) * D + d] = __float2bfloat16_rn(l > 0.f ? a / l : 0.f);
-  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(kAttnThreads);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = grid.x;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = grid.x > 1 ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, kernel, q, qsb, k, v, sb, sh, stt, mask, msb, scale, L, rule, out, len_dev, step);
 }
 
-template <int DPL>
-cudaError_t launch_partial(int G, dim3 grid, cudaStream_t st, const __nv_bfloat16* q,
-                           long long qsb, const __nv_bfloat16* k, const __nv_bfloat16* v,
-                           long long sb, long long sh, long long stt, const __nv_bfloat16* mask,
-                           long long msb, float scale, int L, int chunk, int hq, float* pa,
-                           float* pml, const int* len_dev) {
-#define CDEEP_ATTN_CASE(GG)                                                                     \
-  case GG:                                                                                      \
-    return launch_kernel(decode_attn_partial_kernel<DPL, GG>, grid, dim3(kAttnThreads), 0, st,  \
-                         q, qsb, k, v, sb, sh, stt, mask, msb, scale, L, chunk, hq, pa, pml,    \
-                         len_dev);
-  switch (G) {
-    CDEEP_ATTN_CASE(1)
-    CDEEP_ATTN_CASE(2)
-    CDEEP_ATTN_CASE(3)
-    CDEEP_ATTN_CASE(4)
-    default:
-      return cudaErrorInvalidValue;
-  }
+template <bool kStep>
+cudaError_t launch_any(const void* q, long long qsb, const void* k, const void* v, long long sb, long long sh, long long stt,
+                       const void* mask, long long msb, float scale, int B, int hq, int hkv, int L, int D, void* out,
+                       cudaStream_t stream, const int* len_dev, const StepArgs& step) {
+  const int G = hq / hkv;
+  const Split rule = choose_split(B, hkv, blocks_per_sm(G, D));
+  const dim3 grid(rule.of(L), hkv, B);
+  auto b16 = [](const void* p) { return static_cast<const __nv_bfloat16*>(p); };
+#define CDEEP_ATTN_CASE(DPL, GG)                                                                                        \
+  if (D == 8 * DPL && G == GG)                                                                                          \
+    return launch_one<DPL, GG, kStep>(grid, stream, b16(q), qsb, b16(k), b16(v), sb, sh, stt, b16(mask), msb, scale, L, \
+                                      rule, static_cast<__nv_bfloat16*>(out), len_dev, step);
+  CDEEP_ATTN_CASE(8, 1) CDEEP_ATTN_CASE(8, 2) CDEEP_ATTN_CASE(8, 3) CDEEP_ATTN_CASE(8, 4)
+  CDEEP_ATTN_CASE(16, 1) CDEEP_ATTN_CASE(16, 2) CDEEP_ATTN_CASE(16, 3) CDEEP_ATTN_CASE(16, 4)
 #undef CDEEP_ATTN_CASE
-  return cudaGetLastError();
+  return cudaErrorInvalidValue;
 }
 
 }  // namespace
 
-size_t decode_attention_workspace_bytes(int B, int hq, int hkv, int L, int D) {
-  const size_t splits = choose_splits(B, hkv, L, blocks_per_sm(hq / hkv, D));
-  return static_cast<size_t>(B) * hq * splits * (D + 2) * sizeof(float);
+cudaError_t launch_decode_attention(const void* q, long long q_stride_b, const void* k, const void* v, long long kv_stride_b,
+                                    long long kv_stride_h, long long kv_stride_t, const void* mask, long long mask_stride_b,
+                                    float scale, int B, int hq, int hkv, int L, int D, void* out, cudaStream_t stream,
+                                    const int* kv_len_dev) {
+  return launch_any<false>(q, q_stride_b, k, v, kv_stride_b, kv_stride_h, kv_stride_t, mask, mask_stride_b, scale, B, hq, hkv,
+                           L, D, out, stream, kv_len_dev, StepArgs{});
 }
 
-cudaError_t launch_decode_attention(const void* q, long long q_stride_b, const void* k,
-                                    const void* v, long long kv_stride_b, long long kv_stride_h,
-                                    long long kv_stride_t, const void* mask,
-                                    long long mask_stride_b, float scale, int B, int hq, int hkv,
-                                    int L, int D, void* out, void* ws, cudaStream_t stream,
-                                    const int* kv_len_dev) {
-  const int G = hq / hkv;
-  const int splits = choose_splits(B, hkv, L, blocks_per_sm(G, D));
-  const int chunk = chunk_rows(L, splits);
-  float* part_acc = static_cast<float*>(ws);
-  float* part_ml = part_acc + static_cast<size_t>(B) * hq * splits * D;
-  dim3 grid(splits, hkv, B);
-  auto qb = static_cast<const __nv_bfloat16*>(q);
-  auto kb = static_cast<const __nv_bfloat16*>(k);
-  auto vb = static_cast<const __nv_bfloat16*>(v);
-  auto mb = static_cast<const __nv_bfloat16*>(mask);
-  cudaError_t e;
-  if (D == 128)
-    e = launch_partial<16>(G, grid, stream, qb, q_stride_b, kb, vb, kv_stride_b, kv_stride_h,
-                           kv_stride_t, mb, mask_stride_b, scale, L, chunk, hq, part_acc, part_ml,
-                           kv_len_dev);
-  else if (D == 64)
-    e = launch_partial<8>(G, grid, stream, qb, q_stride_b, kb, vb, kv_stride_b, kv_stride_h,
-                          kv_stride_t, mb, mask_stride_b, scale, L, chunk, hq, part_acc, part_ml,
-                           kv_len_dev);
-  else
-    return cudaErrorInvalidValue;
-  if (e != cudaSuccess) return e;
-  return launch_kernel(decode_attn_combine_kernel, dim3(B * hq), dim3(128), 0, stream, part_acc,
-                       part_ml, splits, D, static_cast<__nv_bfloat16*>(out), B, hkv, L, blocks_per_sm(G, D), kv_len_dev);
+cudaError_t launch_decode_step_attention(const void* qkv, const void* q_w, const void* k_w, const float* cos_t, const float* sin_t,
+                                         float eps, void* k_cache, void* v_cache, long long kv_stride_b, long long kv_stride_h,
+                                         long long kv_stride_t, int capacity, const int* pos_dev, const int* kv_len_dev,
+                                         float scale, int B, int hq, int hkv, int D, void* out, cudaStream_t stream) {
+  StepArgs st;
+  st.q_w = static_cast<const __nv_bfloat16*>(q_w);
+  st.k_w = static_cast<const __nv_bfloat16*>(k_w);
+  st.cos_t = cos_t;
+  st.sin_t = sin_t;
+  st.eps = eps;
+  st.k_cache = static_cast<__nv_bfloat16*>(k_cache);
+  st.v_cache = static_cast<__nv_bfloat16*>(v_cache);
+  st.pos_dev = pos_dev;
+  st.capacity = capacity;
+  return launch_any<true>(qkv, static_cast<long long>(hq + 2 * hkv) * D, k_cache, v_cache, kv_stride_b, kv_stride_h, kv_stride_t,
+                          nullptr, 0, scale, B, hq, hkv, capacity, D, out, stream, kv_len_dev, st);
 }
 
 }  // namespace cdeep

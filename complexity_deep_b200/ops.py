@@ -241,14 +241,7 @@ def qk_norm_rope_(qkv: torch.Tensor, q_w: Optional[torch.Tensor], k_w: Optional[
     return qkv
 
 
-def decode_rope_append(qkv: torch.Tensor, q_w: Optional[torch.Tensor],
-                       k_w: Optional[torch.Tensor], cos: torch.Tensor, sin: torch.Tensor,
-                       eps: float, hq: int, hkv: int, head_dim: int, k_cache: torch.Tensor,
-                       v_cache: torch.Tensor, pos_dev: torch.Tensor) -> torch.Tensor:
-    """Decode step (one row of qkv per sequence): Q/K RMSNorm + RoPE in place at the position
-    held by the device scalar `pos_dev` (int32), and the row's rotated k and its v written
-    into k_cache / v_cache [B, hkv, capacity, D] at that position."""
-    lib = _lib.load()
+def _check_decode_step(qkv, q_w, k_w, cos, sin, hq, hkv, head_dim, k_cache, v_cache, pos_dev) -> None:
     _need(qkv, "qkv")
     _need(cos, "cos", torch.float32)
     _need(sin, "sin", torch.float32)
@@ -268,6 +261,18 @@ def decode_rope_append(qkv: torch.Tensor, q_w: Optional[torch.Tensor],
         raise RuntimeError("cos/sin tables must cover the cache capacity")
     if pos_dev.dtype != torch.int32 or not pos_dev.is_cuda or pos_dev.numel() != 1:
         raise RuntimeError("pos_dev: expected one int32 on the device")
+
+
+def decode_rope_append(qkv: torch.Tensor, q_w: Optional[torch.Tensor],
+                       k_w: Optional[torch.Tensor], cos: torch.Tensor, sin: torch.Tensor,
+                       eps: float, hq: int, hkv: int, head_dim: int, k_cache: torch.Tensor,
+                       v_cache: torch.Tensor, pos_dev: torch.Tensor) -> torch.Tensor:
+    """Decode step (one row of qkv per sequence): Q/K RMSNorm + RoPE in place at the position
+    held by the device scalar `pos_dev` (int32), and the row's rotated k and its v written
+    into k_cache / v_cache [B, hkv, capacity, D] at that position."""
+    lib = _lib.load()
+    _check_decode_step(qkv, q_w, k_w, cos, sin, hq, hkv, head_dim, k_cache, v_cache, pos_dev)
+    B, D, cap = qkv.shape[0], head_dim, k_cache.shape[2]
     with _Span("decode_rope_append"):
         _lib.check(lib.cd_decode_rope_append(
             qkv.data_ptr(), _ptr(q_w), _ptr(k_w), cos.data_ptr(), sin.data_ptr(), float(eps), B,
@@ -303,14 +308,36 @@ def decode_attention(qkv: torch.Tensor, k: torch.Tensor, v: torch.Tensor,
     if kv_len_dev is not None and (kv_len_dev.dtype != torch.int32 or not kv_len_dev.is_cuda
                                    or kv_len_dev.numel() != 1):
         raise RuntimeError("kv_len_dev: expected one int32 on the device")
-    ws_bytes = lib.cd_decode_attention_workspace_bytes(B, hq, hkv, L, D)
-    ws = torch.empty(ws_bytes, dtype=torch.uint8, device=qkv.device)
     out = torch.empty(B, hq * D, dtype=BF16, device=qkv.device)
-    with _Span("decode_attention", 2):
+    with _Span("decode_attention"):
         _lib.check(lib.cd_decode_attention(
             qkv.data_ptr(), qkv.stride(0), k.data_ptr(), v.data_ptr(), k.stride(0), k.stride(1),
             k.stride(2), mptr, mstride, float(head_dim) ** -0.5, B, hq, hkv, L, _ptr(kv_len_dev),
-            D, out.data_ptr(), ws.data_ptr(), ws_bytes, _stream()), "cd_decode_attention")
+            D, out.data_ptr(), None, 0, _stream()), "cd_decode_attention")
+    return out
+
+
+def decode_step_attention(qkv: torch.Tensor, q_w: Optional[torch.Tensor], k_w: Optional[torch.Tensor],
+                          cos: torch.Tensor, sin: torch.Tensor, eps: float, hq: int, hkv: int, head_dim: int,
+                          k_cache: torch.Tensor, v_cache: torch.Tensor, pos_dev: torch.Tensor,
+                          kv_len_dev: torch.Tensor) -> torch.Tensor:
+    """``decode_rope_append`` and ``decode_attention`` over the first `kv_len_dev` tokens of the caches in one launch;
+    qkv stays as it is.  Returns [B, hq * D]."""
+    lib = _lib.load()
+    _check_decode_step(qkv, q_w, k_w, cos, sin, hq, hkv, head_dim, k_cache, v_cache, pos_dev)
+    if kv_len_dev.dtype != torch.int32 or not kv_len_dev.is_cuda or kv_len_dev.numel() != 1:
+        raise RuntimeError("kv_len_dev: expected one int32 on the device")
+    B, D = qkv.shape[0], head_dim
+    if (cos.data_ptr() | sin.data_ptr() | (_ptr(q_w) or 0) | (_ptr(k_w) or 0)) & 15:   # tables or weights off a 16-byte boundary
+        rotated = decode_rope_append(qkv.clone(), q_w, k_w, cos, sin, eps, hq, hkv, D, k_cache, v_cache, pos_dev)
+        return decode_attention(rotated, k_cache, v_cache, None, hq, hkv, D, kv_len_dev=kv_len_dev)
+    out = torch.empty(B, hq * D, dtype=BF16, device=qkv.device)
+    with _Span("decode_attention"):
+        _lib.check(lib.cd_decode_step_attention(
+            qkv.data_ptr(), _ptr(q_w), _ptr(k_w), cos.data_ptr(), sin.data_ptr(), float(eps), float(D) ** -0.5, B, hq, hkv,
+            D, k_cache.data_ptr(), v_cache.data_ptr(), k_cache.stride(0), k_cache.stride(1), k_cache.stride(2),
+            k_cache.shape[2], pos_dev.data_ptr(), kv_len_dev.data_ptr(), out.data_ptr(), _stream()),
+            "cd_decode_step_attention")
     return out
 
 

@@ -188,7 +188,8 @@ int cd_decode_rope_append(void* qkv, const void* q_w, const void* k_w, const flo
  * projection buffer).  k, v: element strides (batch, kv head, token), D contiguous — the
  * cache is read in place, whatever buffer it lives in.  mask: bf16 additive [B, L] with row
  * stride mask_stride_b (0 = one row for all), or NULL.  out: [B, hq * D] bf16.
- * ws: cd_decode_attention_workspace_bytes(...) bytes.  D is 64 or 128, G <= 4; all strides
+ * ws: not used any more (NULL will do; cd_decode_attention_workspace_bytes is 0): the blocks of a
+ * pair meet in one another's shared memory.  D is 64 or 128, G <= 4; all strides
  * multiples of 8 elements.  kv_len_dev (may be NULL): a device scalar; when given, only the
  * first min(L, *kv_len_dev) cached tokens are attended (L then is the capacity the launch is
  * sized for), with the same split of the rows over blocks, hence the same bits, as a call
@@ -199,6 +200,15 @@ int cd_decode_attention(const void* q, long long q_stride_b, const void* k, cons
                         const void* mask, long long mask_stride_b, float scale, int B, int hq,
                         int hkv, int L, const int32_t* kv_len_dev, int D, void* out, void* ws,
                         size_t ws_bytes, void* stream);
+
+/* cd_decode_rope_append followed by cd_decode_attention over the first *kv_len_dev tokens of the
+ * caches (of `capacity` tokens each), as one launch: what both give, but for qkv, which stays as it
+ * is.  D is 64 or 128, G <= 4; cos_t, sin_t and the norm weights on 16-byte boundaries. */
+int cd_decode_step_attention(const void* qkv, const void* q_w, const void* k_w, const float* cos_t,
+                             const float* sin_t, float eps, float scale, int B, int hq, int hkv, int D,
+                             void* k_cache, void* v_cache, long long kv_stride_b, long long kv_stride_h,
+                             long long kv_stride_t, int capacity, const int32_t* pos_dev,
+                             const int32_t* kv_len_dev, void* out, void* stream);
 
 /* ---- causal self-attention over a prompt (prefill) --------------------------------------------
  * Replaces, for a prompt without cached keys and without an additive mask,

@@ -1,0 +1,59 @@
+"""A decode step's attention in one launch (cd_decode_step_attention) against the two calls that it stands for: rotation
+and append, then attention over the cache.  Every cluster size from one block a pair to sixteen, the new row first, last
+and in the middle of a block's rows, caches with strides of their own, a position outside the cache (nothing is written).
+
+Both round q and k to bf16 after the same arithmetic, so the caches must agree to the bit and the result to two units of
+bf16's last place (a fused multiply-add may be contracted differently)."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _inputs(B, hkv, G, D, cap, norm, seed):
+    g = torch.Generator().manual_seed(seed)
+    r = lambda *s: torch.randn(*s, generator=g).to(torch.bfloat16).cuda()
+    ang = torch.rand(cap, D // 2, generator=g) * 6
+    ang = torch.cat([ang, ang], 1)
+    w = (r(D), r(D)) if norm else (None, None)
+    return r(B, (G + 2) * hkv * D), r(B, hkv, cap, D), r(B, hkv, cap, D), ang.cos().cuda(), ang.sin().cuda(), w
+
+
+def _check(B, hkv, G, D, cap, pos, length, norm=True, token_major=False):
+    from complexity_deep_b200 import ops
+    qkv, k, v, cos, sin, (qw, kw) = _inputs(B, hkv, G, D, cap, norm, B + 7 * pos + cap)
+    if token_major:                                      # same values, another order in memory
+        k, v = (t.transpose(1, 2).contiguous().transpose(1, 2) for t in (k, v))
+    state = torch.tensor([pos, length], dtype=torch.int32, device="cuda")
+    hq = hkv * G
+    k1, v1 = k.clone(memory_format=torch.preserve_format), v.clone(memory_format=torch.preserve_format)
+    rot = ops.decode_rope_append(qkv.clone(), qw, kw, cos, sin, 1e-6, hq, hkv, D, k1, v1, state[:1])
+    want = ops.decode_attention(rot, k1, v1, None, hq, hkv, D, kv_len_dev=state[1:])
+    before = qkv.clone()
+    got = ops.decode_step_attention(qkv, qw, kw, cos, sin, 1e-6, hq, hkv, D, k, v, state[:1], state[1:])
+    assert torch.equal(qkv, before) and torch.equal(k, k1) and torch.equal(v, v1)
+    # two units of the last place, or what a bf16 unit of q or k moves a score by (2^-8 of at most ~6)
+    assert bool(((got.float() - want.float()).abs() <= want.float().abs() * 2.0 ** -7 + 2.0 ** -7).all())
+    if pos + 1 == length:                                # against 64 bits on the rotated rows
+        q = rot[:, : hq * D].double().view(B, hkv, G, D)
+        s = torch.einsum("bhgd,bhld->bhgl", q, k1[:, :, :length].double()) * D ** -0.5
+        ref = torch.einsum("bhgl,bhld->bhgd", s.softmax(-1), v1[:, :, :length].double()).reshape(B, hq * D)
+        assert bool(((got.double() - ref).abs() <= ref.abs() * 2.0 ** -8 + 2.0 ** -8).all())
+
+
+@pytest.mark.parametrize("splits", range(1, 17))
+def test_cluster_sizes(splits):
+    _check(1, 2, 2, 64, 48 * splits, 48 * splits - 1, 48 * splits)
+
+
+@pytest.mark.parametrize("B,hkv,G,D,cap,pos", [(1, 4, 3, 64, 320, 0), (1, 4, 3, 64, 320, 16), (1, 4, 3, 64, 320, 47), (2, 1, 4, 128, 700, 699),
+                                               (3, 2, 1, 128, 130, 64), (32, 8, 2, 128, 300, 255), (40, 8, 2, 64, 520, 519),
+                                               (64, 8, 1, 128, 1100, 1023)])
+def test_positions(B, hkv, G, D, cap, pos):
+    for norm in (True, False):
+        _check(B, hkv, G, D, cap, pos, pos + 1, norm, token_major=pos % 2 == 1)
+
+
+@pytest.mark.parametrize("pos,length", [(-1, 40), (200, 200), (130, 60), (5, 0), (10, 190)])
+def test_position_outside_the_rows_attended(pos, length):
+    _check(2, 2, 2, 64, 200, pos, length)
