@@ -55,6 +55,16 @@ class DeltaAttn(ctypes.Structure):
                 + [(n, c_int) for n in ("B", "S", "H", "G", "dk", "dkp", "dv", "dvp", "taps", "pos0")])
 
 
+class Block(ctypes.Structure):
+    """cd_block of include/cdeep.h."""
+    _fields_ = ([(n, c_void_p) for n in ("x", "x_lo", "mu", "ln1", "ln2", "w_qkv", "w_mu", "q_norm", "k_norm", "w_o", "w_up",
+                                         "w_up_s", "w_down", "w_down_s", "w_mu_proj", "mu_param", "cos_t", "sin_t",
+                                         "offsets", "perm", "inv_perm", "normed", "qkv", "attn", "h1", "h1_lo",
+                                         "x_sorted", "h_r", "h_s", "out", "out_lo", "mu_out")]
+                + [(n, c_float) for n in ("eps1", "eps2", "eps_qk", "scale", "mu_min", "mu_max", "clamp_lo", "clamp_hi")]
+                + [(n, c_int) for n in ("B", "S", "H", "hq", "hkv", "D", "E", "I", "I_s", "bn", "bn_s")])
+
+
 _WINDOW_FN = (c_int, [ctypes.POINTER(WindowAttn), c_int, c_void_p])
 _LATENT_FN = (c_int, [ctypes.POINTER(LatentAttn), c_int, c_void_p])
 _DELTA_FN = (c_int, [ctypes.POINTER(DeltaAttn), c_int, c_void_p])
@@ -134,6 +144,7 @@ SIGNATURES = {
                                c_int, c_int, c_int, c_void_p]),
     "cd_mu_proj": (c_int, [c_void_p, c_void_p, c_void_p, c_float, c_float, c_int, c_float, c_float,
                            c_void_p, c_int, c_int, c_void_p]),
+    "cd_complexity_block": (c_int, [ctypes.POINTER(Block), c_void_p]),
     "cd_linear": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int,
                           c_int, c_int, c_void_p]),
     "cd_embed_rows": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p]),

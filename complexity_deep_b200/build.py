@@ -15,7 +15,7 @@ LIB_PATH = os.path.join(PKG_DIR, "libcdeep.so")
 # the checking build: same sources with -DCDEEP_CHECKS (device-side validation of indices that
 # kernels read from device memory; see include/cdeep.h, cd_checks_enabled)
 CHECKS_LIB_PATH = os.path.join(PKG_DIR, "libcdeep_checks.so")
-SOURCES = ["api.cu", "gemm.cu", "gemm_few_rows.cu", "route.cu", "rowwise.cu", "attention_decode.cu", "attention_prefill.cu", "pack.cu", "ep_plan.cu",
+SOURCES = ["api.cu", "block.cu", "gemm.cu", "gemm_few_rows.cu", "route.cu", "rowwise.cu", "attention_decode.cu", "attention_prefill.cu", "pack.cu", "ep_plan.cu",
            "stream_f32.cu", "linear_f32.cu", "window_attention.cu", "window_attention_decode.cu", "window_attention_prefill.cu",
            "linear_attention.cu", "linear_attention_chunk.cu", "latent_attention.cu", "latent_decode.cu",
            "delta_rule.cu", "delta_rule_chunk.cu", "routed_experts.cu"]

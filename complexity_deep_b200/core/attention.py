@@ -180,11 +180,13 @@ class ComplexityAttention(nn.Module):
 
     # ------------------------------------------------------------------ stacked weights
     def _w_qkv(self) -> torch.Tensor:
-        src = (self.q_proj.weight, self.k_proj.weight, self.v_proj.weight)
+        m = self._modules
+        src = (m["q_proj"].weight, m["k_proj"].weight, m["v_proj"].weight)
         return self._derived.get("w_qkv", src, lambda: torch.cat([w.detach() for w in src], 0))
 
     def _w_mu(self) -> torch.Tensor:
-        src = (self.mu_to_q.weight, self.mu_to_k.weight, self.mu_to_v.weight)
+        m = self._modules
+        src = (m["mu_to_q"].weight, m["mu_to_k"].weight, m["mu_to_v"].weight)
         return self._derived.get("w_mu", src, lambda: torch.cat([w.detach() for w in src], 0))
 
     # ------------------------------------------------------------------ forward

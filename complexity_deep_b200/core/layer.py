@@ -170,7 +170,12 @@ class TransformerBlock(nn.Module):
         mu_prev: Optional[torch.Tensor] = None,
     ) -> Tuple[torch.Tensor, Optional[Tuple[torch.Tensor, torch.Tensor]], Optional[torch.Tensor]]:
         ops.forward_only(hidden_states, "TransformerBlock")
-        if self._fusable(token_ids):
+        fusable = self._fusable(token_ids)
+        if fusable and attention_mask is None and past_key_value is None:
+            done = self._forward_native(hidden_states, use_cache, token_ids, mu_prev)
+            if done is not None:
+                return done
+        if fusable:
             hidden_states, new_kv = self._forward_fused(
                 hidden_states, attention_mask, past_key_value, use_cache, token_ids, mu_prev)
         else:
@@ -201,6 +206,53 @@ class TransformerBlock(nn.Module):
             else:
                 mu_contextual = self.mu_guidance(hidden_states)
         return hidden_states, new_kv, mu_contextual
+
+    def _forward_native(self, hidden_states, use_cache, token_ids, mu_prev):
+        """A prompt's block in the model's layer loop as one call into the library (cd_complexity_block): the launches of
+        `_forward_fused` and `mu_proj` in the same order, without Python between them.  None, before anything is launched,
+        where something about the call is not as plain as that takes it; the general route then runs or refuses it."""
+        stream, req, mods = SplitStream.current, MuClampRequest.current, self._modules
+        attn, mlp, mg = mods["self_attn"], mods["mlp"], mods.get("mu_guidance")
+        if (stream is None or req is None or mu_prev is None or mg is None or ops.PROFILE.enabled or self.expert_parallel is not None
+                or type(mlp) is not TokenRoutedMLP or not mlp.use_shared_expert or type(attn) is not ComplexityAttention
+                or _has_hooks(self) or _has_hooks(mg)):
+            return None
+        B, S, H = hidden_states.shape
+        T = B * S
+        # longer prompts keep the GPU busy either way, and the general route gives intermediate results back as it goes
+        if S < 2 or T > 16384 or token_ids.numel() != T or not attn._prefill_kernel_applies(B, S, None, None):
+            return None
+        if hidden_states.dtype is not ops.BF16 or mu_prev.shape != hidden_states.shape:
+            return None
+        hq, hkv, D = attn.num_heads, attn.num_kv_heads, attn.head_dim
+        N, E, I = (hq + 2 * hkv) * D, mlp.num_experts, mlp.expert_intermediate_size
+        ln1, ln2 = mods["input_layernorm"], mods["post_attention_layernorm"]
+        packed, bn = mlp._packed_routed(T)
+        packed_s, bn_s = mlp._packed_shared(T)
+        I_s = mlp._modules["shared_gate"].weight.shape[0]
+        wanted = [(hidden_states, (B, S, H)), (ln1.weight, (H,)), (ln2.weight, (H,)), (attn._w_qkv(), (N, H)), (attn._w_mu(), (N, H)),
+                  (attn._modules["o_proj"].weight, (H, hq * D)), (packed, (E, ops.packed_rows(I, bn), H)),
+                  (packed_s, (1, ops.packed_rows(I_s, bn_s), H)), (mlp._down_routed(), (E, H, I)),
+                  (mlp._modules["shared_down"].weight, (H, I_s)), (mg._modules["mu_proj"].weight, (H, H)), (mg.mu, (H,))]
+        if attn.use_qk_norm:
+            wanted += [(attn._modules["q_norm"].weight, (D,)), (attn._modules["k_norm"].weight, (D,))]
+        if not ops.all_plain(wanted):
+            return None
+        # `take` hands the low part out once: from here on the block runs
+        lo0 = stream.take(hidden_states)
+        routing = mlp.routing(token_ids)
+        cos, sin = attn._modules["rotary_emb"].tables_fp32(S)
+        mu2 = mu_prev.reshape(T, H).contiguous()           # materialises a broadcast mu_init
+        out, out_lo, mu, qkv = ops.complexity_block(
+            [t for t, _ in wanted], lo0, mu2, routing, cos, sin, (B, S, H, hq, hkv, D, E, I, I_s, bn, bn_s),
+            (ln1.eps, ln2.eps, 1e-6, mg.mu_min, mg.mu_max) + req.range)
+        out = out.view(B, S, H)
+        stream.put(out, out_lo)
+        req.applied = True
+        kv = None
+        if use_cache:
+            kv = tuple(qkv[:, a:a + hkv * D].view(B, S, hkv, D).transpose(1, 2) for a in (hq * D, (hq + hkv) * D))
+        return out, kv, mu.view(B, S, H)
 
     def _forward_fused(self, hidden_states, attention_mask, past_key_value, use_cache, token_ids,
                        mu_prev):

@@ -382,7 +382,8 @@ def choose_block_n(width: int, rows: Optional[int] = None, groups: int = 1,
     """
     if rows is not None and rows <= 512:
         if sm_count is None:
-            sm_count = _sm_count(_current_device()) if torch.cuda.is_available() else 148
+            on_gpu = torch.cuda.is_initialized() or torch.cuda.is_available()     # the second asks the driver each time
+            sm_count = _sm_count(_current_device()) if on_gpu else 148
         m_tiles = max(groups, -(-rows // 128))
         for bn in (32, 64, 128, 256):
             if m_tiles * -(-width // (bn // 2)) <= sm_count:
@@ -791,6 +792,68 @@ def linear(x: torch.Tensor, w: torch.Tensor, residual: Optional[torch.Tensor] = 
         _lib.check(lib.cd_linear(x.data_ptr(), w.data_ptr(), _ptr(residual), _ptr(lo2),
                                  out.data_ptr(), _ptr(out_lo), T, K, N, _stream()), "cd_linear")
     return (out, out_lo) if want_lo else out
+
+
+def packed_rows(width: int, block_n: int) -> int:
+    """Rows of `pack_gate_up`'s result for one expert."""
+    half = block_n // 2
+    return -(-width // half) * block_n
+
+
+def all_plain(wanted) -> bool:
+    """Every tensor of the (tensor, shape) pairs a contiguous bf16 CUDA tensor of that shape on the current device?"""
+    device = _current_device()
+    for t, shape in wanted:
+        if t.dtype is not BF16 or t.shape != shape or not t.is_cuda or not t.is_contiguous() or t.get_device() != device:
+            return False
+    return True
+
+
+def complexity_block(tensors, x_lo: Optional[torch.Tensor], mu: torch.Tensor, routing: Routing, cos: torch.Tensor,
+                     sin: torch.Tensor, sizes, constants):
+    """One block of a prompt (cd_complexity_block).  `tensors`, checked by the caller (`all_plain`): hidden states, ln1, ln2,
+    w_qkv, w_mu, w_o, packed gate/up of the routed and of the shared experts, their down weights, mu_proj, mu and, with Q/K
+    norm, its two weights.  `sizes`: B, S, H, hq, hkv, D, E, I, I_s, block_n of the two packed layouts; `constants`: the three
+    eps, mu_min, mu_max and the clamp's bounds.  Returns (out, out_lo, mu, qkv), rows of tokens."""
+    lib = _lib.load()
+    B, S, H, hq, hkv, D, E, I, I_s, bn, bn_s = sizes
+    T, N = B * S, (hq + 2 * hkv) * D
+    x = tensors[0]
+    _need(mu, "mu_prev")
+    if x_lo is not None:
+        _need(x_lo, "x_lo")
+        if x_lo.numel() != T * H:
+            raise RuntimeError("x_lo does not match x")
+    for t, n in ((routing.perm, T), (routing.inv_perm, T), (routing.offsets, E + 1)):
+        _need(t, "routing", torch.int32)
+        if t.numel() != n:
+            raise ValueError(f"routing made for {routing.perm.numel()} tokens, not {T}")
+    _need(cos, "cos", torch.float32)
+    _need(sin, "sin", torch.float32)
+    if cos.shape[0] < S or cos.shape[1] != D or sin.shape != cos.shape:
+        raise RuntimeError("cos/sin tables too short for the requested positions")
+    _split_k_auto(x.view(T, H))
+    new = functools.partial(torch.empty, dtype=BF16, device=x.device)
+    out, out_lo, mu_out, qkv = new(T, H), new(T, H), new(T, H), new(T, N)
+    # intermediate results, each on a boundary of its own
+    widths = (H, hq * D, H, H, H, I, I_s)
+    at, places = 0, []
+    for w in widths:
+        places.append(at)
+        at += -(-T * w // 128) * 128
+    scratch = new(at)
+    base = scratch.data_ptr()
+    normed, attn, h1, h1_lo, x_sorted, h_r, h_s = (base + 2 * a for a in places)
+    p = [t.data_ptr() for t in tensors]
+    q_norm, k_norm = (p[12], p[13]) if len(p) > 12 else (None, None)
+    eps1, eps2, eps_qk, mu_min, mu_max, clamp_lo, clamp_hi = constants
+    block = _lib.Block(p[0], _ptr(x_lo), mu.data_ptr(), p[1], p[2], p[3], p[4], q_norm, k_norm, p[5], p[6], p[7], p[8], p[9],
+                       p[10], p[11], cos.data_ptr(), sin.data_ptr(), routing.offsets.data_ptr(), routing.perm.data_ptr(),
+                       routing.inv_perm.data_ptr(), normed, qkv.data_ptr(), attn, h1, h1_lo, x_sorted, h_r, h_s,
+                       out.data_ptr(), out_lo.data_ptr(), mu_out.data_ptr(), eps1, eps2, eps_qk, float(D) ** -0.5, mu_min,
+                       mu_max, clamp_lo, clamp_hi, B, S, H, hq, hkv, D, E, I, I_s, bn, bn_s)
+    _lib.check(lib.cd_complexity_block(ctypes.byref(block), _stream()), "cd_complexity_block")
+    return out, out_lo, mu_out, qkv
 
 
 # --------------------------------------------------------------------------- fp32 residual stream

@@ -390,6 +390,32 @@ int cd_mu_qkv_rope(const void* x, const void* mu_prev, const void* w, const void
 int cd_mu_proj(const void* h, const void* w, const void* mu_param, float mu_min, float mu_max,
                int clamp_out, float out_lo, float out_hi, void* out, int T, int H, void* stream);
 
+/* ---- one decoder block of a prompt ----------------------------------------------------------
+ * complexity_deep/core/layer.py:143-190 for a prompt without cache and mask, with token-routed and
+ * shared experts and mu guidance, as the calls above in this order: cd_rmsnorm_split (ln1),
+ * cd_mu_qkv_rope (or cd_mu_qkv and cd_qk_norm_rope), cd_attention_prefill, cd_linear (o_proj with the
+ * residual), cd_rmsnorm_split (ln2, rows to expert order), cd_moe_up_pair_layouts (or cd_moe_up twice),
+ * cd_moe_down, cd_mu_proj with its clamp.  Every pointer is what that call takes; the first error
+ * ends the sequence and is returned. */
+typedef struct cd_block {
+  const void *x, *x_lo;            /* [B * S, H] residual stream and its low part (may be NULL) */
+  const void* mu;                  /* [B * S, H] or NULL, with w_mu */
+  const void *ln1, *ln2;           /* [H] */
+  const void *w_qkv, *w_mu;        /* [(hq + 2 hkv) * D, H] */
+  const void *q_norm, *k_norm;     /* [D] or both NULL */
+  const void* w_o;                 /* [H, hq * D] */
+  const void *w_up, *w_up_s;       /* packed for tiles of bn / bn_s */
+  const void *w_down, *w_down_s;   /* [E, H, I], [H, I_s] */
+  const void *w_mu_proj, *mu_param;
+  const float *cos_t, *sin_t;      /* [>= S, D] */
+  const int32_t *offsets, *perm, *inv_perm;                       /* of cd_route */
+  void *normed, *qkv, *attn, *h1, *h1_lo, *x_sorted, *h_r, *h_s;  /* intermediate results */
+  void *out, *out_lo, *mu_out;     /* [B * S, H] */
+  float eps1, eps2, eps_qk, scale, mu_min, mu_max, clamp_lo, clamp_hi;
+  int B, S, H, hq, hkv, D, E, I, I_s, bn, bn_s;
+} cd_block;
+int cd_complexity_block(const cd_block* block, void* stream);
+
 /* ---- plain projection with optional residual ---------------------------------------------
  * out[t, :N] = x[t, :K] @ w^T (+ residual[t, :N]);  w = nn.Linear weight [N, K].
  * Replaces o_proj + residual (complexity_deep/core/attention.py:181 with layer.py:174) and
