@@ -168,6 +168,8 @@ SIGNATURES = {
     "cd_window_attention_decode": (c_int, [ctypes.POINTER(WindowAttn), c_void_p, c_size_t, c_int, c_void_p]),
     "cd_window_attention_prefill_supported": (c_int, [ctypes.POINTER(WindowAttn)]),
     "cd_window_attention_prefill": (c_int, [ctypes.POINTER(WindowAttn), c_void_p]),
+    "cd_window_attention_prefill_workspace_bytes": (c_size_t, [ctypes.POINTER(WindowAttn)]),
+    "cd_window_attention_prefill_ws": (c_int, [ctypes.POINTER(WindowAttn), c_void_p, c_size_t, c_void_p]),
     "cd_window_attention_append": _WINDOW_FN,
     "cd_gla_supported": (c_int, [ctypes.POINTER(LinearAttn)]),
     "cd_gla_step": _GLA_FN,

@@ -764,11 +764,21 @@ int cd_window_attention_prefill_supported(const cd_window_attn* a) {
   return window_args_ok(a) == CD_OK && window_prefill_supported(*a) ? 1 : 0;
 }
 
+size_t cd_window_attention_prefill_workspace_bytes(const cd_window_attn* a) {
+  return window_args_ok(a) == CD_OK && window_prefill_supported(*a) ? window_prefill_workspace_bytes(*a) : 0;
+}
+
 int cd_window_attention_prefill(const cd_window_attn* a, void* stream) {
+  return cd_window_attention_prefill_ws(a, nullptr, 0, stream);
+}
+
+int cd_window_attention_prefill_ws(const cd_window_attn* a, void* ws, size_t ws_bytes, void* stream) {
   if (window_args_ok(a) != CD_OK || !a->r1 || !a->r2 || !a->talk || !a->ring_k || !a->ring_v || !a->out || !a->normed)
     return CD_ERR_INVALID;
   if (!window_prefill_supported(*a)) return CD_ERR_UNSUPPORTED;
-  cudaError_t e = launch_window_prefill(*a, as_stream(stream));
+  const size_t need = window_prefill_workspace_bytes(*a);
+  if (ws && (!aligned16(ws) || ws_bytes < need)) return CD_ERR_INVALID;
+  cudaError_t e = launch_window_prefill(*a, need ? static_cast<float*>(ws) : nullptr, as_stream(stream));
   return e == cudaSuccess ? CD_OK : cuda_fail(e, "window attention prefill launch");
 }
 

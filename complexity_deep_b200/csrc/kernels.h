@@ -136,7 +136,8 @@ bool window_decode_supported(const cd_window_attn& p);
 size_t window_decode_workspace_bytes(const cd_window_attn& p);
 cudaError_t launch_window_decode(const cd_window_attn& p, void* ws, int fp32, cudaStream_t stream);
 bool window_prefill_supported(const cd_window_attn& p);
-cudaError_t launch_window_prefill(const cd_window_attn& p, cudaStream_t stream);
+size_t window_prefill_workspace_bytes(const cd_window_attn& p);   // 0: takes none
+cudaError_t launch_window_prefill(const cd_window_attn& p, float* lse, cudaStream_t stream);
 bool linear_attention_supported(int dkp, int dvp);
 cudaError_t launch_gla_step(const cd_linear_attn& p, int fp32, cudaStream_t stream);
 cudaError_t launch_gla_decay(const cd_linear_attn& p, int fp32, cudaStream_t stream);

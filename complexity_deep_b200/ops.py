@@ -1116,8 +1116,11 @@ def window_attention_(proj: dict, out: torch.Tensor, weights: dict, ring_k: torc
         _lib.check(lib.cd_window_attention_norm(ref, fp32, _stream()), "cd_window_attention_norm")
     a.normed = 1
     if not fp32 and lib.cd_window_attention_prefill_supported(ref):
-        with _Span("window_attention_prefill"):
-            _lib.check(lib.cd_window_attention_prefill(ref, _stream()), "cd_window_attention_prefill")
+        ws_bytes = lib.cd_window_attention_prefill_workspace_bytes(ref)
+        ws = torch.empty(ws_bytes, dtype=torch.uint8, device=out.device) if ws_bytes else None
+        with _Span("window_attention_prefill", 2 if ws_bytes else 1):
+            _lib.check(lib.cd_window_attention_prefill_ws(ref, _ptr(ws), ws_bytes, _stream()),
+                       "cd_window_attention_prefill")
     else:
         with _Span("window_attention_rows"):
             _lib.check(lib.cd_window_attention_rows(ref, fp32, _stream()), "cd_window_attention_rows")

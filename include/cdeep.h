@@ -510,6 +510,10 @@ int cd_window_attention_rows(const cd_window_attn* h_args, int fp32, void* strea
  * Not every head layout fits (cd_window_attention_prefill_supported); the form above takes any. */
 int cd_window_attention_prefill_supported(const cd_window_attn* h_args);
 int cd_window_attention_prefill(const cd_window_attn* h_args, void* stream);
+/* The same with the heads' normalisers found by a kernel of their own, for which it needs a workspace (size 0: it has no
+ * use for one; NULL: as above). */
+size_t cd_window_attention_prefill_workspace_bytes(const cd_window_attn* h_args);
+int cd_window_attention_prefill_ws(const cd_window_attn* h_args, void* workspace, size_t bytes, void* stream);
 /* Writes the call's normed keys and values into the ring (after the attention of the call). */
 int cd_window_attention_append(const cd_window_attn* h_args, int fp32, void* stream);
 
