@@ -1,16 +1,17 @@
 // Window attention of one new token per sequence (decoding), bound by the two passes over the ring.
 // The heads' weights are mixed after the softmax, so the values cannot be weighted before the
-// normalisers of all heads are known; three kernels:
+// normalisers of all heads are known; two kernels or three:
 //
 //   scores   grid (splits, key heads x query-head groups, sequences): a block streams its share of the
 //            keys of one key head for up to four query heads; 8 lanes share a key.  Scores (scaled,
 //            biased) go to a workspace that stays in L2, with every block's softmax statistics.  The
 //            block that holds the new token norms its key and writes key and value into the ring.
-//   mix      grid (64 keys, sequences): combines the statistics, replaces the scores of all heads by
-//            their mixed weights.
 //   values   grid as for the scores, the splits of a (head group, sequence) form a thread-block
-//            cluster: streams its share of the values; the parts are added through distributed shared
-//            memory.
+//            cluster: asks for its first values, combines the statistics, makes the mixed weights of its own heads
+//            and keys from the scores of all heads, streams its share of the values; the parts are added through
+//            distributed shared memory.
+//   mix      grid (64 keys, sequences): where the blocks of the values are more than one wave, it makes the mixed weights
+//            of all heads between the two, since every key head's blocks would do so again (see launch_both).
 #include <cfloat>
 #include <cooperative_groups.h>
 #include "kernels.h"
@@ -29,7 +30,7 @@ struct DecodeParams {
   WindowAttnParams a;
   int splits;
   int n_max;        // keep + window
-  float* scores;    // [B, H, n_max], then the mixed weights
+  float* scores;    // [B, H, n_max]; where the mixing kernel ran, the mixed weights
   float* stats;     // [B, H, splits, 2]
 };
 
@@ -222,17 +223,17 @@ window_decode_scores_kernel(const DecodeParams p) {
   }
 }
 
-constexpr int kMixKeys = 64;       // keys per block of the mixing kernel
+constexpr int kMixBlock = 64;       // keys per block of the mixing kernel
 
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
 window_decode_mix_kernel(const DecodeParams p) {
-  extern __shared__ float sm[];        // [H] maximum, [H] 1 / sum, [H][kMixKeys] weights
+  extern __shared__ float sm[];        // [H] maximum, [H] 1 / sum, [H][kMixBlock] weights
   pdl_enter();
   const WindowAttnParams& a = p.a;
-  const int H = a.H, b = blockIdx.y, n0 = blockIdx.x * kMixKeys;
+  const int H = a.H, b = blockIdx.y, n0 = blockIdx.x * kMixBlock;
   const KeyRange r(a, 0, 1);
-  const int n = min(kMixKeys, r.count - n0);
+  const int n = min(kMixBlock, r.count - n0);
   if (n <= 0) return;
   for (int h = threadIdx.x; h < H; h += kThreads) {
     const float* st = p.stats + (static_cast<long long>(b) * H + h) * p.splits * 2;
@@ -249,27 +250,31 @@ window_decode_mix_kernel(const DecodeParams p) {
   __syncthreads();
   float* scores = p.scores + static_cast<long long>(b) * H * p.n_max + n0;
   float* w = sm + 2 * H;
-  for (int x = threadIdx.x; x < H * kMixKeys; x += kThreads) {
-    const int h = x / kMixKeys, k = x - h * kMixKeys;
+  for (int x = threadIdx.x; x < H * kMixBlock; x += kThreads) {
+    const int h = x / kMixBlock, k = x - h * kMixBlock;
     w[x] = k < n ? score_exp<T>(scores[static_cast<long long>(h) * p.n_max + k] - sm[h]) * sm[H + h] : 0.f;
   }
   __syncthreads();
   const T* talk = static_cast<const T*>(a.talk);
-  for (int x = threadIdx.x; x < H * kMixKeys; x += kThreads) {
-    const int h = x / kMixKeys, k = x - h * kMixKeys;
+  for (int x = threadIdx.x; x < H * kMixBlock; x += kThreads) {
+    const int h = x / kMixBlock, k = x - h * kMixBlock;
     float v = 0.f;
-    for (int g = 0; g < H; ++g) v = fmaf(to_f32(talk[h * H + g]), w[g * kMixKeys + k], v);
+    for (int g = 0; g < H; ++g) v = fmaf(to_f32(talk[h * H + g]), w[g * kMixBlock + k], v);
     if (k < n) scores[static_cast<long long>(h) * p.n_max + k] = v;
   }
 }
 
+constexpr int kMixKeys = 512;      // keys whose mixed weights a block of the values has at a time
+
 template <int REP>
 __host__ __device__ inline int values_smem_floats(int vp) {
-  return REP * 8 * kThreads + REP * vp;          // the threads' sums [REP * 8][kThreads], the block's output [REP][vp]
+  // the threads' sums [REP * 8][kThreads] (before that [H] maxima, [H] 1 / sums, [REP][kMixKeys] weights; H <= 256), the
+  // block's output [REP][vp]
+  return REP * 8 * kThreads + REP * vp;
 }
 
 // kAhead rows in flight per thread, kPerSm blocks on an SM
-template <typename T, int REP, int kAhead, int kPerSm>
+template <typename T, int REP, int kAhead, int kPerSm, bool kMix>
 __global__ void __launch_bounds__(kThreads, kPerSm)
 window_decode_values_kernel(const DecodeParams p) {
   extern __shared__ float sm[];
@@ -289,35 +294,78 @@ window_decode_values_kernel(const DecodeParams p) {
   const int cols = vp / 8, rows = kThreads / cols;               // vp <= 1024
   const int row = tid / cols, col = (tid - row * cols) * 8;
   const bool active = row < rows;
-  const float* weights = p.scores + (static_cast<long long>(b) * a.H + h0) * p.n_max + r.n0;
+  static_assert(2 * 256 + REP * kMixKeys <= REP * 8 * kThreads, "the weights lie where the sums come");
+  const int H = a.H;
+  float *s_max = sm, *s_inv = sm + H, *s_w = sm + 2 * H;
+  Raw8<T> vf[kAhead];
+  // rows at, at + rows, ... of the split; past its end the last one, with weight zero
+  auto ask = [&](int at, int u) { raw_load(ring_v + static_cast<long long>(r.slot(r.n0 + min(at + u * rows, r.nk - 1))) * stride + col, vf[u]); };
+  if (active && r.nk > 0) {
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) ask(row, u);
+  }
+  for (int h = tid; kMix && h < H; h += kThreads) {
+    const float* st = p.stats + (static_cast<long long>(b) * H + h) * p.splits * 2;
+    float m = -FLT_MAX, l = 0.f;
+    for (int s = 0; s < p.splits; ++s) {
+      if (st[2 * s + 1] <= 0.f) continue;          // a split without keys
+      const float mn = fmaxf(m, st[2 * s]);
+      l = l * expf(m - mn) + st[2 * s + 1] * expf(st[2 * s] - mn);
+      m = mn;
+    }
+    s_max[h] = m;
+    s_inv[h] = 1.0f / l;
+  }
+  __syncthreads();
   float acc[REP][8];
 #pragma unroll
   for (int x = 0; x < REP; ++x)
 #pragma unroll
     for (int e = 0; e < 8; ++e) acc[x][e] = 0.f;
-  if (active) {
-    for (int at = row; at < r.nk; at += rows * kAhead) {
-      Raw8<T> vf[kAhead];
-      float w[kAhead][REP];
-#pragma unroll
-      for (int u = 0; u < kAhead; ++u) {
-        const int k = at + u * rows;
-        const int kc = min(k, r.nk - 1);                         // past the end: weight zero
-        raw_load(ring_v + static_cast<long long>(r.slot(r.n0 + kc)) * stride + col, vf[u]);
+  const T* talk = static_cast<const T*>(a.talk) + static_cast<long long>(h0) * H;
+  for (int k0 = 0; k0 < r.nk; k0 += kMixKeys) {
+    const int n = min(kMixKeys, r.nk - k0);
+    for (int k = tid; k < n; k += kThreads) {
+      const float* score = p.scores + static_cast<long long>(b) * H * p.n_max + r.n0 + k0 + k;
+      float v[REP] = {};
+      if constexpr (!kMix) {
 #pragma unroll
         for (int x = 0; x < REP; ++x)
-          w[u][x] = k < r.nk && x < nh ? weights[static_cast<long long>(x) * p.n_max + k] : 0.f;
+          if (x < nh) v[x] = score[static_cast<long long>(h0 + x) * p.n_max];
+      }
+#pragma unroll 8
+      for (int g = 0; kMix && g < H; ++g) {
+        const float w = score_exp<T>(score[static_cast<long long>(g) * p.n_max] - s_max[g]) * s_inv[g];
+#pragma unroll
+        for (int x = 0; x < REP; ++x)
+          if (x < nh) v[x] = fmaf(to_f32(talk[x * H + g]), w, v[x]);
       }
 #pragma unroll
-      for (int u = 0; u < kAhead; ++u) {
-        float f[8];
-        raw_unpack(vf[u], f);
+      for (int x = 0; x < REP; ++x) s_w[x * kMixKeys + k] = v[x];
+    }
+    __syncthreads();
+    if (active) {
+      if (k0 > 0) {
 #pragma unroll
-        for (int x = 0; x < REP; ++x)
+        for (int u = 0; u < kAhead; ++u) ask(k0 + row, u);
+      }
+      for (int at = row; at < n; at += rows * kAhead) {
 #pragma unroll
-          for (int e = 0; e < 8; ++e) acc[x][e] = fmaf(w[u][x], f[e], acc[x][e]);
+        for (int u = 0; u < kAhead; ++u) {
+          float f[8];
+          raw_unpack(vf[u], f);
+          if (at + rows * kAhead < n) ask(k0 + at + rows * kAhead, u);
+          const int k = at + u * rows;
+#pragma unroll
+          for (int x = 0; x < REP; ++x) {
+            const float w = k < n ? s_w[x * kMixKeys + k] : 0.f;
+#pragma unroll
+            for (int e = 0; e < 8; ++e) acc[x][e] = fmaf(w, f[e], acc[x][e]);
+          }
+        }
       }
     }
+    __syncthreads();
   }
 #pragma unroll
   for (int x = 0; x < REP; ++x)
@@ -349,7 +397,7 @@ int rep_block(const WindowAttnParams& a) {
 // Splits of the keys of a (head group, sequence): those whose last wave ends first, a wave being what the SMs hold of the
 // kernel that they hold less of. A block costs about 4 us of its own (position, query, first keys, statistics) and, with
 // the others on its SM, the time that its keys take at the SM's share of the memory's rate (44 bytes per ns); below 64
-// keys a block it gets slower whatever the waves (5 splits of 304 keys 15.0, 4 of them 12.3). One B200, us of the three kernels,
+// keys a block it gets slower whatever the waves (5 splits of 304 keys 15.0, 4 of them 12.3). One B200, us of scores, mixing and values,
 // this rule / powers of two up to 888 blocks / three blocks of 16 bits an SM whatever the kernel holds, 516 keys:
 //   32 sequences x 4 key heads of 128, 2 query heads each   22 / 34 / 22, in 32 bits 27 / 49 / 34
 //   24 x 4 of 128, 4 query heads each                       31 / 52 / 38
@@ -379,10 +427,10 @@ cudaError_t launch_scores(const DecodeParams& p, dim3 grid, cudaStream_t st) {
   return launch_kernel(window_decode_scores_kernel<T, REP, DC>, grid, dim3(kThreads), REP * p.a.dp * sizeof(float), st, p);
 }
 
-template <typename T, int REP, int kAhead, int kPerSm>
+template <typename T, int REP, int kAhead, int kPerSm, bool kMix = false>
 cudaError_t launch_values(const DecodeParams& p, dim3 grid, cudaStream_t st) {
   const int bytes = values_smem_floats<REP>(p.a.vp) * static_cast<int>(sizeof(float));
-  auto kern = window_decode_values_kernel<T, REP, kAhead, kPerSm>;
+  auto kern = window_decode_values_kernel<T, REP, kAhead, kPerSm, kMix>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
@@ -410,16 +458,21 @@ cudaError_t launch_both(const DecodeParams& p, cudaStream_t st) {
                   : p.a.dp <= 128 ? launch_scores<T, REP, 2>(p, grid, st)
                                   : launch_scores<T, REP, 4>(p, grid, st);
   if (e != cudaSuccess) return e;
-  const int mix_bytes = p.a.H * (2 + kMixKeys) * static_cast<int>(sizeof(float));
+  // Blocks of one wave make the mixed weights of their heads and keys themselves: each key head's blocks again, H exponentials a
+  // key, but a launch and the weights' way through memory less. Steps of Pimezen, us, with the mixing kernel / without: 1024
+  // wide, 32 sequences 484 / 477, 1 319 / 308; 2048 wide, 16 sequences of 300 keys 641 / 587, 64 of 1 028 (two waves) 1 666 / 1 760.
+  const long long blocks = static_cast<long long>(grid.x) * grid.y * grid.z, sms = current_sm_count();
+  constexpr int kAhead = REP <= 2 && sizeof(T) == 2 ? 6 : 4;
+  if (blocks <= values_per_sm(sizeof(T), REP) * sms) return launch_values<T, REP, kAhead, values_per_sm(sizeof(T), REP), true>(p, grid, st);
+  const int mix_bytes = p.a.H * (2 + kMixBlock) * static_cast<int>(sizeof(float));
   e = cudaFuncSetAttribute(window_decode_mix_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, mix_bytes);
   if (e != cudaSuccess) return e;
-  e = launch_kernel(window_decode_mix_kernel<T>, dim3((p.n_max + kMixKeys - 1) / kMixKeys, p.a.B), dim3(kThreads),
+  e = launch_kernel(window_decode_mix_kernel<T>, dim3((p.n_max + kMixBlock - 1) / kMixBlock, p.a.B), dim3(kThreads),
                     mix_bytes, st, p);
   if (e != cudaSuccess) return e;
   if constexpr (REP <= 2 && sizeof(T) == 2) {
     // six rows in flight and three blocks on an SM, unless four blocks on an SM end a wave earlier: 32 sequences of 516 keys
     // (one wave of either) 8.9 us, with four and four 10.1; 64 of 1028 (1 024 blocks) 41.5 / 37.3
-    const long long blocks = static_cast<long long>(grid.x) * grid.y * grid.z, sms = current_sm_count();
     if ((blocks + 3 * sms - 1) / (3 * sms) <= (blocks + 4 * sms - 1) / (4 * sms)) return launch_values<T, REP, 6, values_per_sm(sizeof(T), REP)>(p, grid, st);
     return launch_values<T, REP, 4, 4>(p, grid, st);
   } else {
