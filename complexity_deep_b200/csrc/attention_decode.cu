@@ -66,7 +66,8 @@ constexpr short kActive[3][kMaxSplits] = {{296, 148, 93, 71, 56, 45, 37, 33, 30,
                                           {444, 222, 142, 104, 82, 71, 56, 48, 45, 41, 31, 31, 28, 24, 24, 21},
                                           {592, 296, 187, 142, 112, 93, 78, 71, 60, 56, 45, 42, 38, 35, 31, 31}};
 //   Two blocks of every pair fit the device at once: the largest cluster of which one per pair fits; 9 to 12 blocks are no
-//   better than eight, and all sixteen worth it for eight pairs only. us, cold L2, heads of 2 x 128 and 2 064 rows, by the
+//   better than eight, 13 only up to 24 pairs (beside other kernels' blocks a large cluster waits for room: steps of the 18-layer model
+//   with 8 sequences, 32 pairs, 669 us with 13, 617 with eight; 1B-class with 3, 24 pairs, 1 198 / 1 211), all sixteen for eight pairs. us, cold L2, heads of 2 x 128 and 2 064 rows, by the
 //   size of the cluster: 8 pairs 8: 12.0, 13: 9.8, 16: 9.3; 16 pairs 8: 13.2, 13: 10.7, 16: 12.3; 32 pairs 8: 14.3, 11:
 //   14.3, 13: 13.5, 16: 19.2; 64 pairs 7: 18.9, 8: 18.2, 9: 26; 96 pairs 4: 27.3, 5: 23.2, 6: 32.6; 128 pairs 3: 33, 4:
 //   28.3, 5: 38.6; 256 pairs 1: 66, 2: 47.7, 3: 60. Down to 48 rows a block: 4 pairs of 302 rows of 3 x 64, 3: 6.9, 5: 5.3,
@@ -79,7 +80,7 @@ inline Split choose_split(int B, int hkv, int per_sm) {
   if (pairs <= active[1]) {
     int fit = 2;
     while (fit < kMaxSplits && pairs <= active[fit]) ++fit;
-    return {fit >= 13 ? (pairs <= 8 ? kMaxSplits : 13) : fit > kPortable ? kPortable : fit, 48};
+    return {pairs <= 8 && fit == kMaxSplits ? kMaxSplits : pairs <= 24 && fit >= 13 ? 13 : fit > kPortable ? kPortable : fit, 48};
   }
   int best = 1;
   long long best_score = -1;
