@@ -1116,7 +1116,10 @@ def window_attention_(proj: dict, out: torch.Tensor, weights: dict, ring_k: torc
         _lib.check(lib.cd_window_attention_norm(ref, fp32, _stream()), "cd_window_attention_norm")
     a.normed = 1
     if not fp32 and lib.cd_window_attention_prefill_supported(ref):
-        ws_bytes = lib.cd_window_attention_prefill_workspace_bytes(ref)
+        # up to 256 keys the first pass inside the kernel is a few tiles, less than another launch and its workspace cost a
+        # caller that is bound by the host (a 4-layer model's short prompts 987 us, 1 007 with them)
+        seen = min(window + keep, pos0 + seq_len) if pos_dev is None else window + keep
+        ws_bytes = lib.cd_window_attention_prefill_workspace_bytes(ref) if seen > 256 else 0
         ws = torch.empty(ws_bytes, dtype=torch.uint8, device=out.device) if ws_bytes else None
         with _Span("window_attention_prefill", 2 if ws_bytes else 1):
             _lib.check(lib.cd_window_attention_prefill_ws(ref, _ptr(ws), ws_bytes, _stream()),
