@@ -395,7 +395,7 @@ window_tile_kernel(const WindowAttnParams p, int cap) {
     float m = -FLT_MAX, l = 0.f;
     for (int n = lane; n < nk; n += 32) m = fmaxf(m, s[n]);
     m = warp_max(m);
-    for (int n = lane; n < nk; n += 32) l += s[n] > -FLT_MAX ? expf(s[n] - m) : 0.f;
+    for (int n = lane; n < nk; n += 32) l += s[n] != -FLT_MAX ? expf(s[n] - m) : 0.f;
     l = warp_add(l);
     if (lane == 0) {
       sm[L.stat + x] = m;
@@ -416,7 +416,7 @@ window_tile_kernel(const WindowAttnParams p, int cap) {
     }
     const float inv = 1.0f / l;
     float* s = sm + L.s + x * cap;
-    for (int n = lane; n < nk; n += 32) s[n] = s[n] > -FLT_MAX ? expf(s[n] - m) * inv : 0.f;
+    for (int n = lane; n < nk; n += 32) s[n] = s[n] != -FLT_MAX ? expf(s[n] - m) * inv : 0.f;
   }
   __syncthreads();
 
