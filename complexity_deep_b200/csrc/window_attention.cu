@@ -3,6 +3,7 @@
 // latter serves prompts in 32-bit storage and head layouts that the kernels of
 // window_attention_prefill.cu (prompts in bf16) and window_attention_decode.cu do not take.
 #include <cfloat>
+#include <type_traits>
 #include <cooperative_groups.h>
 #include "kernels.h"
 #include "window_attention.cuh"
@@ -312,6 +313,7 @@ window_tile_kernel(const WindowAttnParams p, int cap) {
   const int chunk = (count + CL - 1) / CL;
   const int n0 = min(rank * chunk, count);
   const int nk = min(chunk, count - n0);        // keys of this block (0 possible)
+  auto sees = [&](int qi, int j) { return j <= i0 + qi && (i0 + qi - j < p.window || j < p.keep); };
 
   // queries, pre-scaled (those past the end repeat the last one and are not stored), and the mixing matrix
   for (int x = tid; x < kTileQ * H * dp; x += kThreads) {
@@ -376,13 +378,10 @@ window_tile_kernel(const WindowAttnParams p, int cap) {
 #pragma unroll
           for (int qi = 0; qi < kTileQ; ++qi)
 #pragma unroll
-            for (int y = 0; y < 2; ++y) {
-              const int d = i0 + qi - j[y];
-              const bool seen = d >= 0 && (d < p.window || j[y] < p.keep);
+            for (int y = 0; y < 2; ++y)
               if (n + y * pairs < nk)
                 sm[L.s + (qi * H + h) * cap + n + y * pairs] =
-                    seen ? acc[y][qi][r] - r1 * log1pf(r2 * static_cast<float>(d)) : -FLT_MAX;
-            }
+                    sees(qi, j[y]) ? acc[y][qi][r] - r1 * log1pf(r2 * static_cast<float>(i0 + qi - j[y])) : -FLT_MAX;
         }
       }
     }
@@ -420,6 +419,23 @@ window_tile_kernel(const WindowAttnParams p, int cap) {
   }
   __syncthreads();
 
+  // A value that only some of the queries see has weight zero for the others, which keeps it out as long as it is finite: the few
+  // keys at both ends of the tile's window are looked at.
+  bool odd = false;
+  for (int x = tid; x < 2 * (kTileQ - 1) * (G * vp / 8); x += kThreads) {
+    const int y = x / (G * vp / 8), col = (x - y * (G * vp / 8)) * 8;
+    const int n = (y < kTileQ - 1 ? keys.kept + y : count - 2 * (kTileQ - 1) + y) - n0;
+    if (n < 0 || n >= nk) continue;
+    const int j = keys.position(n0 + n);
+    float f[8];
+    load8(j >= pos0 ? new_v + (j - pos0) * p.ldp + col
+                    : ring_v + static_cast<long long>(window_slot(j, p.window, p.keep)) * G * vp + col, f);
+    float zero = 0.f;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) zero = fmaf(f[e], 0.f, zero);
+    odd |= zero != 0.f;                  // infinities and NaN times zero are NaN
+  }
+
   // mixed weights
   for (int item = tid; item < nk * kTileQ; item += kThreads) {
     const int qi = item / nk, n = item - qi * nk;
@@ -436,7 +452,7 @@ window_tile_kernel(const WindowAttnParams p, int cap) {
       s[h * cap] = a;
     }
   }
-  __syncthreads();
+  const bool check_seen = __syncthreads_or(odd);
 
   // values: a thread takes eight columns of a key head and every `groups`-th key
   const int vchunks = G * vp / 8;
@@ -456,24 +472,29 @@ window_tile_kernel(const WindowAttnParams p, int cap) {
                                  : ring_v + (static_cast<long long>(window_slot(j, p.window, p.keep)) * G + c) * vp + d;
           load8(v, next);
         };
-        int n = groups > 1 ? grp : 0;
-        if (n < nk) ask(n);
-        for (; n < nk; n += groups) {
+        auto walk = [&](auto check) {
+          int n = groups > 1 ? grp : 0;
+          if (n < nk) ask(n);
+          for (; n < nk; n += groups) {
 #pragma unroll
-          for (int e = 0; e < 8; ++e) f[e] = next[e];
-          if (n + groups < nk) ask(n + groups);
+            for (int e = 0; e < 8; ++e) f[e] = next[e];
+            if (n + groups < nk) ask(n + groups);
 #pragma unroll
-          for (int r = 0; r < kTileRep; ++r) {
-            if (r0 + r < rep) {
+            for (int r = 0; r < kTileRep; ++r) {
+              if (r0 + r < rep) {
 #pragma unroll
-              for (int qi = 0; qi < kTileQ; ++qi) {
-                const float w = sm[L.s + (qi * H + c * rep + r0 + r) * cap + n];
+                for (int qi = 0; qi < kTileQ; ++qi) {
+                  if (decltype(check)::value && !sees(qi, keys.position(n0 + n))) continue;
+                  const float w = sm[L.s + (qi * H + c * rep + r0 + r) * cap + n];
 #pragma unroll
-                for (int e = 0; e < 8; ++e) acc[qi][r][e] += w * f[e];
+                  for (int e = 0; e < 8; ++e) acc[qi][r][e] += w * f[e];
+                }
               }
             }
           }
-        }
+        };
+        if (check_seen) walk(std::true_type{});
+        else walk(std::false_type{});
       }
 #pragma unroll
       for (int qi = 0; qi < kTileQ; ++qi) {

@@ -97,3 +97,18 @@ def test_nan_reaches_the_queries_that_see_it(S, what):
     assert bool(got[hit].isnan().all()) and bool(got[~hit].isfinite().all())
     if what != "bias":
         assert torch.equal(got[~hit], clean[~hit])
+
+
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+@pytest.mark.parametrize("S", [145, 401])
+def test_a_value_reaches_only_the_queries_that_see_it(S, bad):
+    """Queries of a tile ahead of a key, or beyond its window, give it weight zero: infinities and NaN must not come through that."""
+    H, G, dim, window, keep, at = 8, 4, 128, 256, 4, 70           # the third query of a tile, and the third beyond the window
+    proj, q, k, v, ring_k, ring_v, r1, r2, talk = _inputs(1, S, H, G, dim, dim, window, keep, torch.float32, S)
+    clean = _run(proj, q, k, v, ring_k, ring_v, r1, r2, talk, window, keep, 0)[0]
+    v[0, at, 1, 9] = bad
+    got = _run(proj, q, k, v, ring_k, ring_v, r1, r2, talk, window, keep, 0)[0]
+    i = torch.arange(S, device="cuda")
+    hit = torch.zeros_like(clean, dtype=torch.bool)
+    hit[(i >= at) & (i - at < window), 2:4, 9] = True
+    assert not bool(got[hit].isfinite().any()) and torch.equal(got[~hit], clean[~hit])
