@@ -142,6 +142,7 @@ int cd_qk_norm_rope(void* qkv, const void* q_w, const void* k_w, const float* co
   if (T < 0 || S < 1 || pos0 < 0 || hq < 1 || hkv < 1 || D < 4 || (D & 3)) return CD_ERR_INVALID;
   if (!cos_t || !sin_t || (T > 0 && !qkv)) return CD_ERR_INVALID;
   if ((q_w == nullptr) != (k_w == nullptr)) return CD_ERR_INVALID;
+  if (reinterpret_cast<uintptr_t>(qkv) & 3) return CD_ERR_INVALID;   // pairs of elements
   cudaError_t e = launch_qk_norm_rope(qkv, q_w, k_w, cos_t, sin_t, eps, T, S, pos0, hq, hkv, D,
                                       as_stream(stream));
   return e == cudaSuccess ? CD_OK : cuda_fail(e, "qk_norm_rope launch");

@@ -330,9 +330,9 @@ qk_norm_rope_kernel(__nv_bfloat16* __restrict__ qkv, const __nv_bfloat16* __rest
     const uint32_t b = *reinterpret_cast<const uint32_t*>(head + half + j);
     float a0 = lo_f(a) * rstd, a1 = hi_f(a) * rstd, b0 = lo_f(b) * rstd, b1 = hi_f(b) * rstd;
     if (nw) {
-      const uint32_t wa = *reinterpret_cast<const uint32_t*>(nw + j);
-      const uint32_t wb = *reinterpret_cast<const uint32_t*>(nw + half + j);
-      a0 *= lo_f(wa); a1 *= hi_f(wa); b0 *= lo_f(wb); b1 *= hi_f(wb);
+      // one by one: weights may lie at any element
+      a0 *= __bfloat162float(nw[j]); a1 *= __bfloat162float(nw[j + 1]);
+      b0 *= __bfloat162float(nw[half + j]); b1 *= __bfloat162float(nw[half + j + 1]);
     }
     // out = x * cos + rotate_half(x) * sin, rotate_half(x) = [-x2, x1]
     const float o_a0 = a0 * cs[j] - b0 * sn[j];

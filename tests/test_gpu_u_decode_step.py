@@ -57,3 +57,23 @@ def test_positions(B, hkv, G, D, cap, pos):
 @pytest.mark.parametrize("pos,length", [(-1, 40), (200, 200), (130, 60), (5, 0), (10, 190)])
 def test_position_outside_the_rows_attended(pos, length):
     _check(2, 2, 2, 64, 200, pos, length)
+
+
+@pytest.mark.parametrize("what", ["cos", "weight"])
+def test_off_a_16_byte_boundary(what):
+    from complexity_deep_b200 import ops
+    B, hkv, G, D, cap, pos = 2, 2, 2, 64, 200, 77
+    qkv, k, v, cos, sin, (qw, kw) = _inputs(B, hkv, G, D, cap, True, 5)
+    state = torch.tensor([pos, pos + 1], dtype=torch.int32, device="cuda")
+    k1, v1 = k.clone(), v.clone()
+    want = ops.decode_step_attention(qkv, qw, kw, cos, sin, 1e-6, hkv * G, hkv, D, k1, v1, state[:1], state[1:])
+    move = lambda t: torch.cat([t.new_zeros(1), t.flatten()])[1:].view(t.shape)      # the same values one element further on
+    if what == "cos":
+        cos = move(cos)
+    else:
+        qw = move(qw)
+    before = qkv.clone()
+    got = ops.decode_step_attention(qkv, qw, kw, cos, sin, 1e-6, hkv * G, hkv, D, k, v, state[:1], state[1:])
+    assert torch.equal(k, k1) and torch.equal(v, v1) and torch.equal(qkv, before)
+    # what a rounding of q to bf16 moves a score by (2^-8 of at most ~6), as above
+    assert bool(((got.float() - want.float()).abs() <= want.float().abs() * 2.0 ** -7 + 2.0 ** -7).all())
