@@ -10,8 +10,8 @@
 //     operands use the same permutation, and the four lanes of a row read 64 consecutive bytes.
 //   * A block asks for its weights in L2 BEFORE it waits for the kernel ahead of it. A prefetch reads nothing into
 //     the program, so it may run ahead of whatever still writes; it takes the DRAM latency out of the step.
-//   * The partial sums are added in the order of the warps: results do not depend on timing, nor on the rows beside a row, but
-//     for K of 2048 on and few enough blocks, where calls of more than 32 rows take eight shares of K for sixteen.
+//   * The partial sums are added in the order of their shares of K, whose number depends on the weights alone: results depend
+//     neither on timing nor on the rows beside a row.
 // Row groups (experts) are walked in passes of at most 32 rows of one group; empty groups end at once.
 // Bound by: L2 to SM traffic (weights once, the rows once per block: 7 to 9 TB/s) from 16 rows on, before that by
 // the launch (2.1 us at K = N = 768, one row; the tile kernel 6.8). The other figures stand at few_rows_taken.
@@ -77,8 +77,9 @@ __device__ __forceinline__ FewRun few_run(int s_lo, int s_hi, int off, int K, in
 
 // acc += tokens x weights over a run of steps. wp: this lane's weight rows at the run's first step, tp: its token rows
 // (kA steps in flight). Nothing but the loads and the products is left in the loop: a warp is one chain of a few
-// hundred instructions, and with two warps a scheduler each of them costs some eight cycles. us, with bounds and addresses found step by step / so (eight warps a block): K = N = 2048, one row
-// 4.4 / 3.9, 64 rows 6.7 / 6.2; K 5632, N 2048, one row 11.2 / 8.1; K 768, N 1280 3.3 / 2.9.
+// hundred instructions, and with two warps a scheduler each of them costs some eight cycles. us, with bounds and addresses
+// found step by step / so (eight warps a block): K = N = 2048, one row 4.4 / 3.9, 64 rows 6.7 / 6.2; K 5632, N 2048, one row
+// 11.2 / 8.1; K 768, N 1280 3.3 / 2.9.
 template <int MT, int NT, int kU, int kA>
 __device__ __forceinline__ void few_walk(float (&acc)[MT][NT][4], const bf16* (&wp)[MT][2], const bf16* (&tp)[NT],
                                          const FewRun& run) {
@@ -227,8 +228,9 @@ struct Weights {                   // of the block's group, one matrix per K seg
 template <int MT>
 constexpr int kRowFloats = 16 * MT + 4;                    // partial sums of a token: the accumulators' writes hit 32 banks
 
-// One pass: the block's weight rows against the tokens [m0, m0 + 8 NT) of a group that ends at m_end.
-template <int EPI, int MT, int NT, int WK, bool kDeep>
+// One pass: the block's weight rows against the tokens [m0, m0 + 8 NT) of a group that ends at m_end. K is cut into WK x SUB shares,
+// SUB behind one another for each warp.
+template <int EPI, int MT, int NT, int WK, int SUB, bool kDeep>
 __device__ __forceinline__ void few_pass(const FewParams& p, float* red, const Weights& wt, const int (&w_row)[MT][2], int n_steps0,
                                          int n_steps, int m0, int m_end, int col0, bool second) {
   constexpr bool kGated = EPI == kEpiSwiGLU || EPI == kEpiGlu;
@@ -249,36 +251,38 @@ __device__ __forceinline__ void few_pass(const FewParams& p, float* red, const W
     items[i] = few_fetch<EPI>(g, item < 8 * NT * kQuads ? m0 + item / kQuads : m_end, m_end, col0 + (item % kQuads) * 4, out_cols);
   }
 
-  float acc[MT][NT][4];
-#pragma unroll
-  for (int m = 0; m < MT; ++m)
-#pragma unroll
-    for (int n = 0; n < NT; ++n)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) acc[m][n][e] = 0.f;
-  // this warp's steps, segment by segment
-  const int s_lo = warp * n_steps / WK, s_hi = (warp + 1) * n_steps / WK;
 #pragma unroll 1
-  for (int seg = 0; seg < (g.K1 > 0 ? 2 : 1); ++seg) {
-    const FewRun run = few_run(s_lo, s_hi, seg ? n_steps0 : 0, seg ? g.K1 : g.K0, q8);
-    if (run.n == 0) continue;
-    const long long k = run.first * kStep + q8;
-    const bf16 *wp[MT][2], *tp[NT];
+  for (int sub = 0; sub < SUB; ++sub) {
+    const int share = warp * SUB + sub;
+    float acc[MT][NT][4];
 #pragma unroll
     for (int m = 0; m < MT; ++m)
 #pragma unroll
-      for (int h = 0; h < 2; ++h) wp[m][h] = (seg ? wt.b1 + w_row[m][h] * wt.ld1 : wt.b0 + w_row[m][h] * wt.ld0) + k;
+      for (int n = 0; n < NT; ++n)
 #pragma unroll
-    for (int n = 0; n < NT; ++n) {
-      const int row = min(m0 + n * 8 + (lane >> 2), m_end - 1);                       // rows past the end are not stored
-      tp[n] = (seg ? p.a1 + row * p.lda1 : p.a0 + row * p.lda0) + k;
+        for (int e = 0; e < 4; ++e) acc[m][n][e] = 0.f;
+    // this share's steps, segment by segment
+    const int s_lo = share * n_steps / (WK * SUB), s_hi = (share + 1) * n_steps / (WK * SUB);
+#pragma unroll 1
+    for (int seg = 0; seg < (g.K1 > 0 ? 2 : 1); ++seg) {
+      const FewRun run = few_run(s_lo, s_hi, seg ? n_steps0 : 0, seg ? g.K1 : g.K0, q8);
+      if (run.n == 0) continue;
+      const long long k = run.first * kStep + q8;
+      const bf16 *wp[MT][2], *tp[NT];
+#pragma unroll
+      for (int m = 0; m < MT; ++m)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) wp[m][h] = (seg ? wt.b1 + w_row[m][h] * wt.ld1 : wt.b0 + w_row[m][h] * wt.ld0) + k;
+#pragma unroll
+      for (int n = 0; n < NT; ++n) {
+        const int row = min(m0 + n * 8 + (lane >> 2), m_end - 1);                       // rows past the end are not stored
+        tp[n] = (seg ? p.a1 + row * p.lda1 : p.a0 + row * p.lda0) + k;
+      }
+      few_walk<MT, NT, kU, kAhead>(acc, wp, tp, run);
     }
-    few_walk<MT, NT, kU, kAhead>(acc, wp, tp, run);
-  }
 
-  // partial sums: [warp][token][feature]
-  {
-    float* mine = red + warp * (8 * NT * kRow);
+    // partial sums: [share][token][feature]
+    float* mine = red + share * (8 * NT * kRow);
 #pragma unroll
     for (int m = 0; m < MT; ++m)
 #pragma unroll
@@ -299,7 +303,7 @@ __device__ __forceinline__ void few_pass(const FewParams& p, float* red, const W
     float f[4] = {0.f, 0.f, 0.f, 0.f}, u[4] = {0.f, 0.f, 0.f, 0.f};
     const float* src = red + tok * kRow + quad * 4;
 #pragma unroll
-    for (int w_ = 0; w_ < WK; ++w_) {
+    for (int w_ = 0; w_ < WK * SUB; ++w_) {
       const float4 v = *reinterpret_cast<const float4*>(src + w_ * (8 * NT * kRow));
       f[0] += v.x; f[1] += v.y; f[2] += v.z; f[3] += v.w;
       if constexpr (kGated) {
@@ -359,7 +363,7 @@ template <int N> struct Int { static constexpr int value = N; };
 // kManyGroups: in several waves of blocks, where nothing is asked for ahead of time and four steps of weights in flight take its
 // place (64 experts, 512 rows, both products: steps of the 2048 wide model 25.8 -> 25.3 ms; in one wave they cost 1 %).
 enum Kind { kWhole, kGroups, kManyGroups };
-template <int EPI, int MT, int NTMAX, int WK, int KIND>
+template <int EPI, int MT, int NTMAX, int WK, int KIND, int SUB>
 __global__ void __launch_bounds__(WK * 32, NTMAX >= 8 ? 8 / WK : 16 / WK) few_rows_kernel(const __grid_constant__ FewParams p) {
   static_assert((EPI != kEpiSwiGLU && EPI != kEpiGlu) || MT == 2, "a gated unit takes its gate rows and its up rows together");
   extern __shared__ float4 smem4[];
@@ -399,7 +403,9 @@ __global__ void __launch_bounds__(WK * 32, NTMAX >= 8 ? 8 / WK : 16 / WK) few_ro
   for (int m0 = m_lo; m0 < m_hi; m0 += 8 * NTMAX) {
     const int left = m_hi - m0;
     if (m0 > m_lo) __syncthreads();                        // the sums of the pass before are read
-    auto pass = [&](auto nt) { few_pass<EPI, MT, decltype(nt)::value, WK, KIND == kManyGroups>(p, red, wt, w_row, n_steps0, n_steps, m0, m_hi, at.col0, at.second); };
+    auto pass = [&](auto nt) {
+      few_pass<EPI, MT, decltype(nt)::value, WK, SUB, KIND == kManyGroups>(p, red, wt, w_row, n_steps0, n_steps, m0, m_hi, at.col0, at.second);
+    };
     if constexpr (KIND == kWhole) {
       if constexpr (NTMAX == 8) {
         if (left <= 48) pass(Int<6>());
@@ -415,22 +421,27 @@ __global__ void __launch_bounds__(WK * 32, NTMAX >= 8 ? 8 / WK : 16 / WK) few_ro
   }
 }
 
-template <int EPI, int MT, int NTMAX, int WK, int KIND = kWhole>
+template <int EPI, int MT, int NTMAX, int WK, int KIND = kWhole, int SUB = 1>
 cudaError_t launch_few(const FewParams& p, cudaStream_t stream) {
-  constexpr int smem = WK * 8 * NTMAX * kRowFloats<MT> * 4;
-  cudaError_t e = allow_smem<few_rows_kernel<EPI, MT, NTMAX, WK, KIND>>(smem);
+  constexpr int smem = WK * SUB * 8 * NTMAX * kRowFloats<MT> * 4;
+  cudaError_t e = allow_smem<few_rows_kernel<EPI, MT, NTMAX, WK, KIND, SUB>>(smem);
   if (e != cudaSuccess) return e;
   FewParams q = p;
   const unsigned grid = static_cast<unsigned>(p.tiles * p.g.num_groups + p.tiles2);
   // Beyond one wave the asking ahead gets in the way of the reads themselves: 64 experts of 2 x 704 x 2048, 256 rows 100 us
   // with it (each block asking for the next one's as well), 73 without; N 32000, 8 rows 39 / 32.
   if (grid > static_cast<unsigned>(p.sms * (NTMAX >= 8 ? 8 : 16) / WK)) q.prefetch = 0;
-  return launch_kernel(few_rows_kernel<EPI, MT, NTMAX, WK, KIND>, dim3(grid), dim3(WK * 32), smem, stream, q);
+  return launch_kernel(few_rows_kernel<EPI, MT, NTMAX, WK, KIND, SUB>, dim3(grid), dim3(WK * 32), smem, stream, q);
 }
 
 template <int EPI, int MT, int WK>
 cudaError_t launch_warps(const FewParams& p, cudaStream_t stream) {
   if constexpr (WK == 16) {
+    // sixteen shares whatever the number of rows, so that a row's bits do not depend on it: 49 and more do not fit the registers
+    // of sixteen warps, and eight take two shares each
+    if (p.g.M > 32 && p.g.num_groups > 1) return launch_few<EPI, MT, 4, WK, kGroups>(p, stream);
+    if (p.g.M > 48) return launch_few<EPI, MT, 8, 8, kWhole, 2>(p, stream);
+    if (p.g.M > 32) return launch_few<EPI, MT, 6, WK>(p, stream);
     return p.g.M <= 8 ? launch_few<EPI, MT, 1, WK>(p, stream) : p.g.M <= 16 ? launch_few<EPI, MT, 2, WK>(p, stream) : launch_few<EPI, MT, 4, WK>(p, stream);
   } else {
     if (p.g.M <= 8) return launch_few<EPI, MT, 1, WK>(p, stream);
@@ -444,16 +455,17 @@ cudaError_t launch_warps(const FewParams& p, cudaStream_t stream) {
 }
 // More blocks than the two of eight warps that an SM holds: four warps each and four on an SM, since a block is then
 // mostly its own start and end (64 experts of 704 x 2048, 8 rows: 14.5 us with eight warps, 9.4 with four). Fewer
-// blocks: eight warps, a shorter chain. No more blocks than SMs, and a long K: sixteen, since eight warps with four steps in
-// flight do not keep an SM's share of the bandwidth busy (N 2048, one row, us with eight / sixteen: K 2048 3.9 / 3.3, 4096 6.2 /
-// 4.8, 5632 8.1 / 6.1; 32 rows 5.5 / 4.7, 8.6 / 7.3, 11.1 / 8.9). Of a shorter K the sixteen sums cost more than they bring
-// (K = N = 1024, 16 rows 2.7 / 3.1), of few blocks as well (N 64, K 2048 3.2 / 3.6), and 33 rows and more do not fit the registers.
+// blocks: eight warps, a shorter chain. No more blocks than SMs, and a long K (64 steps of both segments together): sixteen
+// shares, since eight warps with four steps in flight do not keep an SM's share of the bandwidth busy (N 2048, one row, us with
+// eight / sixteen: K 2048 3.9 / 3.3, 4096 6.2 / 4.8, 5632 8.1 / 6.1; 32 rows 5.5 / 4.7, 8.6 / 7.3, 11.1 / 8.9; replayed, where
+// eight shares were faster: 33 rows 4.6 / 4.8, 7.1 / 7.0, 9.0 / 8.7, 64 rows 5.6 / 6.5, 8.6 / 9.4, 11.0 / 11.9). Of a shorter K
+// the sixteen sums cost more than they bring (K = N = 1024, 16 rows 2.7 / 3.1), of few blocks as well (N 64, K 2048 3.2 / 3.6).
 template <int EPI, int MT>
 cudaError_t launch_rows(const FewParams& p, cudaStream_t stream) {
   const long long blocks = static_cast<long long>(p.tiles) * p.g.num_groups + p.tiles2;
   const int n_steps = (p.g.K0 + kStep - 1) / kStep + (p.g.K1 + kStep - 1) / kStep;
   if constexpr (MT == 1)
-    if (blocks <= p.sms && 4 * blocks >= p.sms && n_steps >= 64 && p.g.M <= 32) return launch_warps<EPI, MT, 16>(p, stream);
+    if (blocks <= p.sms && 4 * blocks >= p.sms && n_steps >= 64) return launch_warps<EPI, MT, 16>(p, stream);
   return blocks > 2LL * p.sms ? launch_warps<EPI, MT, 4>(p, stream) : launch_warps<EPI, MT, 8>(p, stream);
 }
 
@@ -475,7 +487,7 @@ static int store_mt(long long cols, int num_groups, int sm_count) { return num_g
 //     and 80 / 20; 128 experts, 1024 rows in one 174 / 27. 32 experts of 2 x 704 x 1024, 256 rows 27 / 44. 8 experts and a
 //     shared one: 32 rows 14 / 26, 64 rows 15 / 26; 65 rows in one group 33 / 39 and 19 / 21.
 //   dense: up to 64 rows, unless the tokens, which every block reads again, cost more than the tile kernel's chains.
-//     K 2048, N 2048: 32 rows 4.8 / 11.6, 64 rows 6.2 / 11.6; K 4096, N 4096: 32 rows 11.3 / 16.2, 40 rows 19.1 / 16.2;
+//     K 2048, N 2048: 32 rows 4.8 / 11.6, 64 rows 7.0 / 11.6; K 4096, N 4096: 32 rows 11.3 / 16.2, 40 rows 19.1 / 16.2;
 //     K 2048, N 6272: 32 rows 10.3 / 12.7, 40 rows 17.9 / 12.7; K 2048, N 32000: 16 rows 26 / 37, 32 rows 34 / 30. The
 //     estimates below put the line between these: both sides in bytes per ns at the rates that they reach (from 33 rows
 //     on a block has an SM to itself, and more blocks than SMs lose), 4.9 us and 0.21 us per 64 of K for a chain.
