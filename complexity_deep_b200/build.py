@@ -19,7 +19,7 @@ SOURCES = ["api.cu", "block.cu", "gemm.cu", "gemm_few_rows.cu", "route.cu", "row
            "stream_f32.cu", "linear_f32.cu", "window_attention.cu", "window_attention_decode.cu", "window_attention_prefill.cu",
            "linear_attention.cu", "linear_attention_chunk.cu", "latent_attention.cu", "latent_decode.cu",
            "delta_rule.cu", "delta_rule_chunk.cu", "routed_experts.cu"]
-HEADERS = ["ptx.cuh", "checks.cuh", "gemm_sm100.cuh", "kernels.h", "smem_limit.h", "elem.cuh", "mma.cuh", "window_attention.cuh", "linear_attention.cuh",
+HEADERS = ["ptx.cuh", "checks.cuh", "gemm_sm100.cuh", "kernels.h", "smem_limit.h", "decode_split.h", "elem.cuh", "mma.cuh", "window_attention.cuh", "linear_attention.cuh",
            "latent_attention.cuh", "delta_rule.cuh",
            os.path.join("..", "..", "include", "cdeep.h")]
 

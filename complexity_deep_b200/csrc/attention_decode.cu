@@ -29,6 +29,7 @@
 #include <cstdint>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
+#include "decode_split.h"
 #include "kernels.h"
 
 namespace cdeep {
@@ -36,10 +37,7 @@ namespace cdeep {
 namespace {
 
 constexpr int kAttnThreads = 128;
-constexpr int kMaxGroup = 4;    // query heads per KV head handled by one block (the entry point refuses more)
 constexpr int kLanesPerRow = 8;
-constexpr int kMaxSplits = 16;  // of a pair: the largest cluster that there is
-constexpr int kPortable = 8;    // the largest that every launch may ask for
 
 __device__ __forceinline__ float lo_f(uint32_t v) { return __uint_as_float(v << 16); }
 __device__ __forceinline__ float hi_f(uint32_t v) { return __uint_as_float(v & 0xffff0000u); }
@@ -47,34 +45,23 @@ __device__ __forceinline__ float hi_f(uint32_t v) { return __uint_as_float(v & 0
 // Blocks that an SM holds at a time, by the registers of G query heads of D dimensions.
 __host__ __device__ constexpr int blocks_per_sm(int G, int D) { return G * D > 384 ? 2 : G * D > 256 ? 3 : 4; }
 
-// How the rows of a (batch, kv head) pair are split over the blocks of a cluster: at most `most` blocks of at least
-// `min_rows` rows, and more than eight only of 72 rows or more.  Evaluated on the device as well when the cache length is read
-// from there, so both forms split (and therefore round) identically; never falls as L grows.
-struct Split {
-  int most, min_rows;
-  __host__ __device__ int of(int L) const {
-    int n = (L + min_rows - 1) / min_rows;
-    if (n > kPortable) n = max(kPortable, (L + 71) / 72);
-    return max(1, min(most, n));
-  }
-};
 // Clusters of 1 .. 16 blocks that a B200 holds at a time (cudaOccupancyMaxActiveClusters: a cluster lies within one GPC,
-// so the SMs that are left over in each go unused), by blocks per SM. Tuning constants: other figures only change how many
-// blocks share the work.
+// so the SMs that are left over in each go unused), by blocks per SM.
 constexpr int kSms = 148;
 constexpr short kActive[3][kMaxSplits] = {{296, 148, 93, 71, 56, 45, 37, 33, 30, 26, 21, 21, 17, 14, 14, 14},
                                           {444, 222, 142, 104, 82, 71, 56, 48, 45, 41, 31, 31, 28, 24, 24, 21},
                                           {592, 296, 187, 142, 112, 93, 78, 71, 60, 56, 45, 42, 38, 35, 31, 31}};
-//   Two blocks of every pair fit the device at once: the largest cluster of which one per pair fits; 9 to 12 blocks are no
-//   better than eight, 13 only up to 24 pairs (beside other kernels' blocks a large cluster waits for room: steps of the 18-layer model
-//   with 8 sequences, 32 pairs, 669 us with 13, 617 with eight; 1B-class with 3, 24 pairs, 1 198 / 1 211), all sixteen for eight pairs. us, cold L2, heads of 2 x 128 and 2 064 rows, by the
-//   size of the cluster: 8 pairs 8: 12.0, 13: 9.8, 16: 9.3; 16 pairs 8: 13.2, 13: 10.7, 16: 12.3; 32 pairs 8: 14.3, 11:
-//   14.3, 13: 13.5, 16: 19.2; 64 pairs 7: 18.9, 8: 18.2, 9: 26; 96 pairs 4: 27.3, 5: 23.2, 6: 32.6; 128 pairs 3: 33, 4:
-//   28.3, 5: 38.6; 256 pairs 1: 66, 2: 47.7, 3: 60. Down to 48 rows a block: 4 pairs of 302 rows of 3 x 64, 3: 6.9, 5: 5.3,
-//   7: 4.8; above eight blocks the larger launch costs more (32 pairs of 400 rows 7: 7.3, 9: 8.3).
+//   Two blocks of every pair fit the device at once: the largest cluster of which one per pair fits, and of more than eight
+//   blocks 13 up to 24 pairs (beside other kernels' blocks a large cluster waits for room: steps of the 18-layer model with
+//   8 sequences, 32 pairs, 669 us with 13, 617 with eight; 1B-class with 3, 24 pairs, 1 198 / 1 211) and 16 up to eight. us,
+//   cold L2, heads of 2 x 128 and 2 064 rows, by the size of the cluster: 8 pairs 8: 14.1, 13: 12.3, 16: 12.1; 16 pairs 8: 16.2,
+//   13: 13.9, 16: 14.2; 24 pairs 8: 16.2, 13: 15.0, 16: 16.2; 32 pairs 8: 16.3, 10: 16.3, 13: 16.6, 16: 22.5; another
+//   kernel's blocks aside, 64 pairs 7: 18.9, 8: 18.2, 9: 26; 96 pairs 4: 27.3, 5: 23.2, 6: 32.6; 128 pairs 3: 33, 4: 28.3,
+//   5: 38.6; 256 pairs 1: 66, 2: 47.7, 3: 60. Down to 48 rows a block: 4 pairs of 302 rows of 3 x 64 4: 8.6, 5: 8.2, 8: 8.0,
+//   of 800 rows 8: 10.1, 12: 10.1, 13: 8.1; 8 pairs of 1 000 of 2 x 128 8: 10.9, 16: 10.0; 24 pairs of 800 8: 11.4, 13: 12.0.
 //   More pairs: the size whose waves are fullest, each block more costing some 5 % (320 pairs 1: 84, 2: 81, 3: 65, 4: 73,
 //   5: 66; 512 pairs 1: 86, 2: 93, 5: 105, 8: 121).
-inline Split choose_split(int B, int hkv, int per_sm) {
+inline DecodeSplit choose_split(int B, int hkv, int per_sm) {
   const long long pairs = static_cast<long long>(B) * hkv;
   const short(&active)[kMaxSplits] = kActive[per_sm - 2];
   if (pairs <= active[1]) {
@@ -90,10 +77,6 @@ inline Split choose_split(int B, int hkv, int per_sm) {
     if (score > best_score) best = c, best_score = score;
   }
   return {best, 256};
-}
-
-__host__ __device__ inline int chunk_rows(int L, int splits) {
-  return (((L + splits - 1) / splits) + 15) / 16 * 16;
 }
 
 // programmatic dependent launch: wait for the previous kernel of the stream before touching
@@ -224,7 +207,7 @@ decode_attn_kernel(const __nv_bfloat16* __restrict__ q, long long q_stride_b,
                    const __nv_bfloat16* k, const __nv_bfloat16* v,
                    long long kv_stride_b, long long kv_stride_h, long long kv_stride_t,
                    const __nv_bfloat16* __restrict__ mask, long long mask_stride_b,
-                   float scale, int L, Split rule, __nv_bfloat16* __restrict__ out,
+                   float scale, int L, DecodeSplit rule, __nv_bfloat16* __restrict__ out,
                    const int* __restrict__ len_dev, StepArgs st) {
   constexpr int D = DPL * kLanesPerRow;
   constexpr int kV = DPL / 8;                               // 16-byte pieces of K (and of V) per lane
@@ -254,8 +237,8 @@ decode_attn_kernel(const __nv_bfloat16* __restrict__ q, long long q_stride_b,
     if (st.q_w) qw = load_halves<D>(st.q_w, sub);
   }
   if (len_dev) L = max(0, min(L, __ldg(len_dev)));
-  const int splits = rule.of(L);
-  const int chunk = chunk_rows(L, splits);
+  const int splits = rule.blocks(L);
+  const int chunk = rule.chunk(L);
   const int t_begin = min(L, split * chunk);
   const int t_end = min(L, t_begin + chunk);
   bool owner = false;                // of the new row: the warp whose rows include it, or beyond all rows the first
@@ -502,7 +485,7 @@ decode_attn_kernel(const __nv_bfloat16* __restrict__ q, long long q_stride_b,
 template <int DPL, int G, bool kStep>
 cudaError_t launch_one(dim3 grid, cudaStream_t stream, const __nv_bfloat16* q, long long qsb, const __nv_bfloat16* k,
                        const __nv_bfloat16* v, long long sb, long long sh, long long stt, const __nv_bfloat16* mask,
-                       long long msb, float scale, int L, Split rule, __nv_bfloat16* out, const int* len_dev,
+                       long long msb, float scale, int L, DecodeSplit rule, __nv_bfloat16* out, const int* len_dev,
                        const StepArgs& step) {
   auto* kernel = decode_attn_kernel<DPL, G, kStep>;
   if (grid.x > kPortable) {
@@ -529,8 +512,8 @@ cudaError_t launch_any(const void* q, long long qsb, const void* k, const void* 
                        const void* mask, long long msb, float scale, int B, int hq, int hkv, int L, int D, void* out,
                        cudaStream_t stream, const int* len_dev, const StepArgs& step) {
   const int G = hq / hkv;
-  const Split rule = choose_split(B, hkv, blocks_per_sm(G, D));
-  const dim3 grid(rule.of(L), hkv, B);
+  const DecodeSplit rule = choose_split(B, hkv, blocks_per_sm(G, D));
+  const dim3 grid(len_dev ? rule.bound(L) : rule.blocks(L), hkv, B);
   auto b16 = [](const void* p) { return static_cast<const __nv_bfloat16*>(p); };
 #define CDEEP_ATTN_CASE(DPL, GG)                                                                                        \
   if (D == 8 * DPL && G == GG)                                                                                          \

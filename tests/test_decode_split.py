@@ -1,0 +1,47 @@
+"""How decode attention shares out a cache (csrc/decode_split.h), compiled for the host: every block counted has rows, whole row
+steps but for the last one's, never more blocks than a launch sized for a longer cache, and more than eight only where all of
+them have the least rows."""
+import os
+import shutil
+import subprocess
+
+import pytest
+
+from conftest import ROOT
+
+PROGRAM = r"""
+#include <cassert>
+#include "decode_split.h"
+using namespace cdeep;
+int main() {
+  const int least[] = {48, 256};
+  for (int most = 1; most <= kMaxSplits; ++most)
+    for (int min_rows : least) {
+      if (min_rows > 48 && most > 5) continue;
+      const DecodeSplit rule{most, min_rows};
+      assert(rule.blocks(0) == 1 && rule.bound(0) == 1);
+      int before = 1;
+      for (int L = 1; L <= 6000; ++L) {
+        const int bound = rule.bound(L), chunk = rule.chunk(L), blocks = rule.blocks(L);
+        assert(bound >= before && bound <= most && blocks >= 1 && blocks <= bound);
+        assert(chunk % 16 == 0 && (blocks - 1) * chunk < L && L <= blocks * chunk);
+        assert(bound <= kPortable || (bound == most && L > min_rows * (most - 1)));
+        before = bound;
+      }
+      assert(before == most);
+    }
+  return 0;
+}
+"""
+
+
+def test_every_block_has_rows(tmp_path):
+    gxx = shutil.which("g++")
+    if gxx is None:
+        pytest.skip("no C++ compiler")
+    src = tmp_path / "split.cpp"
+    src.write_text(PROGRAM)
+    exe = str(tmp_path / "split")
+    subprocess.run([gxx, "-std=c++17", "-O1", "-I", os.path.join(ROOT, "complexity_deep_b200", "csrc"), str(src), "-o", exe],
+                   check=True)
+    subprocess.run([exe], check=True, timeout=60)

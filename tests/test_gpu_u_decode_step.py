@@ -1,6 +1,8 @@
 """A decode step's attention in one launch (cd_decode_step_attention) against the two calls that it stands for: rotation
-and append, then attention over the cache.  Every cluster size from one block a pair to sixteen, the new row first, last
-and in the middle of a block's rows, caches with strides of their own, a position outside the cache (nothing is written).
+and append, then attention over the cache.  Every cluster size that csrc/decode_split.h gives (one to eight blocks a pair, 13 and
+16), lengths far below the capacity that a launch is sized for, caches of several thousand rows, the new row first, last
+and in the middle of a block's rows, caches with strides of their own, a position outside the cache (nothing is written),
+tables and weights off a 16-byte boundary (the two calls run).
 
 Both round q and k to bf16 after the same arithmetic, so the caches must agree to the bit and the result to two units of
 bf16's last place (a fused multiply-add may be contracted differently)."""
@@ -41,9 +43,24 @@ def _check(B, hkv, G, D, cap, pos, length, norm=True, token_major=False):
         assert bool(((got.double() - ref).abs() <= ref.abs() * 2.0 ** -8 + 2.0 ** -8).all())
 
 
-@pytest.mark.parametrize("splits", range(1, 17))
-def test_cluster_sizes(splits):
-    _check(1, 2, 2, 64, 48 * splits, 48 * splits - 1, 48 * splits)
+# one to eight blocks of 48 rows; 16 blocks of a pair (up to eight pairs) of 80 and of 144 rows, 13 (up to 24 pairs) of 80 and of 96;
+# eight just below both
+@pytest.mark.parametrize("B,hkv,G,D,cap", [(1, 2, 2, 64, 48 * n) for n in range(1, 9)] + [
+    (1, 2, 2, 64, 1151), (1, 2, 2, 64, 1280), (2, 4, 1, 128, 2300), (1, 4, 3, 64, 2064), (2, 8, 2, 128, 935), (2, 8, 2, 128, 1040),
+    (3, 8, 2, 64, 1248), (1, 12, 4, 64, 937)])
+def test_cluster_sizes(B, hkv, G, D, cap):
+    _check(B, hkv, G, D, cap, cap - 1, cap)
+
+
+@pytest.mark.parametrize("length", [1, 16, 47, 385, 900, 1152, 1500, 4000])
+def test_lengths_below_the_capacity(length):
+    _check(1, 4, 2, 128, 4096, length - 1, length)
+    _check(2, 8, 3, 64, 4096, length - 1, length)
+
+
+@pytest.mark.parametrize("B,hkv,G,D,cap,pos", [(1, 2, 3, 64, 9000, 8999), (1, 8, 2, 128, 8200, 5000), (4, 8, 2, 128, 4100, 4099), (40, 8, 1, 64, 3000, 2999)])
+def test_long_caches(B, hkv, G, D, cap, pos):
+    _check(B, hkv, G, D, cap, pos, pos + 1)
 
 
 @pytest.mark.parametrize("B,hkv,G,D,cap,pos", [(1, 4, 3, 64, 320, 0), (1, 4, 3, 64, 320, 16), (1, 4, 3, 64, 320, 47), (2, 1, 4, 128, 700, 699),
