@@ -46,7 +46,8 @@ __device__ __forceinline__ float hi_f(uint32_t v) { return __uint_as_float(v & 0
 __host__ __device__ constexpr int blocks_per_sm(int G, int D) { return G * D > 384 ? 2 : G * D > 256 ? 3 : 4; }
 
 // Clusters of 1 .. 16 blocks that a B200 holds at a time (cudaOccupancyMaxActiveClusters: a cluster lies within one GPC,
-// so the SMs that are left over in each go unused), by blocks per SM.
+// so the SMs that are left over in each go unused), by blocks per SM. Other devices take other sizes better; which of more than
+// eight blocks they take at all they are asked (allow_clusters).
 constexpr int kSms = 148;
 constexpr short kActive[3][kMaxSplits] = {{296, 148, 93, 71, 56, 45, 37, 33, 30, 26, 21, 21, 17, 14, 14, 14},
                                           {444, 222, 142, 104, 82, 71, 56, 48, 45, 41, 31, 31, 28, 24, 24, 21},
@@ -482,29 +483,58 @@ decode_attn_kernel(const __nv_bfloat16* __restrict__ q, long long q_stride_b,
   }
 }
 
+// Clusters of more than eight blocks are asked for only where the device holds one.
+template <auto kKernel>
+cudaError_t allow_clusters(DecodeSplit& rule) {
+  static DeviceNumber largest;
+  int device = 0;
+  const cudaError_t e = cudaGetDevice(&device);
+  if (e != cudaSuccess) return e;
+  const int most = largest.get(device, [] {
+    return largest_cluster([](int blocks) {
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(blocks);
+      cfg.blockDim = dim3(kAttnThreads);
+      cudaLaunchAttribute attr;
+      attr.id = cudaLaunchAttributeClusterDimension;
+      attr.val.clusterDim.x = blocks;
+      attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+      cfg.attrs = &attr;
+      cfg.numAttrs = 1;
+      int clusters = 0;
+      if (cudaFuncSetAttribute(kKernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+          cudaOccupancyMaxActiveClusters(&clusters, kKernel, &cfg) != cudaSuccess)
+        cudaGetLastError();              // not a size for this device
+      return clusters > 0;
+    });
+  });
+  if (rule.most > most) rule.most = most;
+  return cudaSuccess;
+}
+
 template <int DPL, int G, bool kStep>
-cudaError_t launch_one(dim3 grid, cudaStream_t stream, const __nv_bfloat16* q, long long qsb, const __nv_bfloat16* k,
+cudaError_t launch_one(int B, int hkv, cudaStream_t stream, const __nv_bfloat16* q, long long qsb, const __nv_bfloat16* k,
                        const __nv_bfloat16* v, long long sb, long long sh, long long stt, const __nv_bfloat16* mask,
                        long long msb, float scale, int L, DecodeSplit rule, __nv_bfloat16* out, const int* len_dev,
                        const StepArgs& step) {
-  auto* kernel = decode_attn_kernel<DPL, G, kStep>;
-  if (grid.x > kPortable) {
-    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  constexpr auto kKernel = decode_attn_kernel<DPL, G, kStep>;
+  if (rule.most > kPortable) {
+    const cudaError_t e = allow_clusters<kKernel>(rule);
     if (e != cudaSuccess) return e;
   }
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
+  cfg.gridDim = dim3(len_dev ? rule.bound(L) : rule.blocks(L), hkv, B);
   cfg.blockDim = dim3(kAttnThreads);
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
   attr[1].id = cudaLaunchAttributeClusterDimension;
-  attr[1].val.clusterDim.x = grid.x;
+  attr[1].val.clusterDim.x = cfg.gridDim.x;
   attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = grid.x > 1 ? 2 : 1;
-  return cudaLaunchKernelEx(&cfg, kernel, q, qsb, k, v, sb, sh, stt, mask, msb, scale, L, rule, out, len_dev, step);
+  cfg.numAttrs = cfg.gridDim.x > 1 ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, kKernel, q, qsb, k, v, sb, sh, stt, mask, msb, scale, L, rule, out, len_dev, step);
 }
 
 template <bool kStep>
@@ -513,11 +543,10 @@ cudaError_t launch_any(const void* q, long long qsb, const void* k, const void* 
                        cudaStream_t stream, const int* len_dev, const StepArgs& step) {
   const int G = hq / hkv;
   const DecodeSplit rule = choose_split(B, hkv, blocks_per_sm(G, D));
-  const dim3 grid(len_dev ? rule.bound(L) : rule.blocks(L), hkv, B);
   auto b16 = [](const void* p) { return static_cast<const __nv_bfloat16*>(p); };
-#define CDEEP_ATTN_CASE(DPL, GG)                                                                                        \
-  if (D == 8 * DPL && G == GG)                                                                                          \
-    return launch_one<DPL, GG, kStep>(grid, stream, b16(q), qsb, b16(k), b16(v), sb, sh, stt, b16(mask), msb, scale, L, \
+#define CDEEP_ATTN_CASE(DPL, GG)                                                                                           \
+  if (D == 8 * DPL && G == GG)                                                                                             \
+    return launch_one<DPL, GG, kStep>(B, hkv, stream, b16(q), qsb, b16(k), b16(v), sb, sh, stt, b16(mask), msb, scale, L,  \
                                       rule, static_cast<__nv_bfloat16*>(out), len_dev, step);
   CDEEP_ATTN_CASE(8, 1) CDEEP_ATTN_CASE(8, 2) CDEEP_ATTN_CASE(8, 3) CDEEP_ATTN_CASE(8, 4)
   CDEEP_ATTN_CASE(16, 1) CDEEP_ATTN_CASE(16, 2) CDEEP_ATTN_CASE(16, 3) CDEEP_ATTN_CASE(16, 4)

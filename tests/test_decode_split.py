@@ -1,6 +1,6 @@
 """How decode attention shares out a cache (csrc/decode_split.h), compiled for the host: every block counted has rows, whole row
 steps but for the last one's, never more blocks than a launch sized for a longer cache, and more than eight only where all of
-them have the least rows."""
+them have the least rows, on devices (here ones that only answer) that hold such a cluster."""
 import os
 import shutil
 import subprocess
@@ -11,6 +11,8 @@ from conftest import ROOT
 
 PROGRAM = r"""
 #include <cassert>
+#include <thread>
+#include <vector>
 #include "decode_split.h"
 using namespace cdeep;
 int main() {
@@ -30,6 +32,26 @@ int main() {
       }
       assert(before == most);
     }
+  DeviceNumber number;
+  int asked = 0, holds = 16;
+  auto most = [&](int device) { return number.get(device, [&] { return largest_cluster([&](int n) { ++asked; return n <= holds; }); }); };
+  assert(most(0) == 16 && asked == 1);
+  holds = 8;
+  assert(most(0) == 16 && asked == 1);          // of a device that was asked
+  assert(most(1) == 8 && asked == 3);           // another one
+  assert(most(1) == 8 && asked == 3);
+  holds = 14;
+  assert(most(2) == 13 && most(1000) == 13 && most(-1) == 13);
+  DeviceNumber none;                            // nothing at all is an answer, too
+  for (int i = 0; i < 2; ++i) assert(none.get(3, [&] { ++asked; return 0; }) == 0);
+  assert(asked == 10);
+  DeviceNumber shared;
+  std::vector<std::thread> threads;
+  for (int t = 0; t < 8; ++t)
+    threads.emplace_back([&] {
+      for (int i = 0; i < 2000; ++i) assert(shared.get(i % 64, [] { return 13; }) == 13);
+    });
+  for (auto& t : threads) t.join();
   return 0;
 }
 """
@@ -42,6 +64,6 @@ def test_every_block_has_rows(tmp_path):
     src = tmp_path / "split.cpp"
     src.write_text(PROGRAM)
     exe = str(tmp_path / "split")
-    subprocess.run([gxx, "-std=c++17", "-O1", "-I", os.path.join(ROOT, "complexity_deep_b200", "csrc"), str(src), "-o", exe],
+    subprocess.run([gxx, "-std=c++17", "-O1", "-pthread", "-I", os.path.join(ROOT, "complexity_deep_b200", "csrc"), str(src), "-o", exe],
                    check=True)
     subprocess.run([exe], check=True, timeout=60)
