@@ -60,24 +60,21 @@ constexpr short kActive[3][kMaxSplits] = {{296, 148, 93, 71, 56, 45, 37, 33, 30,
 //   kernel's blocks aside, 64 pairs 7: 18.9, 8: 18.2, 9: 26; 96 pairs 4: 27.3, 5: 23.2, 6: 32.6; 128 pairs 3: 33, 4: 28.3,
 //   5: 38.6; 256 pairs 1: 66, 2: 47.7, 3: 60. Down to 48 rows a block: 4 pairs of 302 rows of 3 x 64 4: 8.6, 5: 8.2, 8: 8.0,
 //   of 800 rows 8: 10.1, 12: 10.1, 13: 8.1; 8 pairs of 1 000 of 2 x 128 8: 10.9, 16: 10.0; 24 pairs of 800 8: 11.4, 13: 12.0.
-//   More pairs: the size whose waves are fullest, each block more costing some 5 % (320 pairs 1: 84, 2: 81, 3: 65, 4: 73,
-//   5: 66; 512 pairs 1: 86, 2: 93, 5: 105, 8: 121).
+//   More pairs: split_of_waves. us, cold L2, 2 x 128, one block / two / three / four a pair: 384 pairs of 300 rows 21 / 29 / 33 / 34,
+//   of 2 064 86 / 109 / 105 / 96; 640 of 300 39 / 41 / 47 / 54, of 1 024 100 / 90 / 87 / 94, of 4 096 310 / 262 / 252 / 244; 768 of
+//   300 41 / 45 / 55 / 64, of 2 064 188 / 161 / 171 / 171; 2 048 of 300 83 / 103 / 128 / 153, of 4 096 671 / 663 / 687 / 695.
 inline DecodeSplit choose_split(int B, int hkv, int per_sm) {
   const long long pairs = static_cast<long long>(B) * hkv;
   const short(&active)[kMaxSplits] = kActive[per_sm - 2];
   if (pairs <= active[1]) {
     int fit = 2;
     while (fit < kMaxSplits && pairs <= active[fit]) ++fit;
-    return {pairs <= 8 && fit == kMaxSplits ? kMaxSplits : pairs <= 24 && fit >= 13 ? 13 : fit > kPortable ? kPortable : fit, 48};
+    DecodeSplit r;
+    r.most = pairs <= 8 && fit == kMaxSplits ? kMaxSplits : pairs <= 24 && fit >= 13 ? 13 : fit > kPortable ? kPortable : fit;
+    r.large_from = r.most * (pairs > 16 ? 64 : 48);
+    return r;
   }
-  int best = 1;
-  long long best_score = -1;
-  for (int c = 1; c <= 5; ++c) {
-    const long long waves = (pairs + active[c - 1] - 1) / active[c - 1];
-    const long long score = 1000 * pairs * c / (waves * per_sm * kSms) - 50 * (c - 1);
-    if (score > best_score) best = c, best_score = score;
-  }
-  return {best, 256};
+  return split_of_waves(pairs, active);
 }
 
 // programmatic dependent launch: wait for the previous kernel of the stream before touching

@@ -1,6 +1,6 @@
 """How decode attention shares out a cache (csrc/decode_split.h), compiled for the host: every block counted has rows, whole row
-steps but for the last one's, never more blocks than a launch sized for a longer cache, and more than eight only where all of
-them have the least rows, on devices (here ones that only answer) that hold such a cluster."""
+steps but for the last one's, never more blocks than a launch sized for a longer cache, more than eight only where all of
+them have the least rows, on devices (here ones that only answer) that hold such a cluster, and one of a short cache whose pairs fill the device."""
 import os
 import shutil
 import subprocess
@@ -15,23 +15,32 @@ PROGRAM = r"""
 #include <vector>
 #include "decode_split.h"
 using namespace cdeep;
+static void check(const DecodeSplit& rule, int most, int rows) {
+  assert(rule.blocks(0) == 1 && rule.bound(0) == 1);
+  int before = 1;
+  for (int L = 1; L <= rows; ++L) {
+    const int bound = rule.bound(L), chunk = rule.chunk(L), blocks = rule.blocks(L);
+    assert(bound >= before && bound <= most && blocks >= 1 && blocks <= bound);
+    assert(chunk % 16 == 0 && (blocks - 1) * chunk < L && L <= blocks * chunk);
+    before = bound;
+  }
+  assert(before == most);
+}
 int main() {
-  const int least[] = {48, 256};
-  for (int most = 1; most <= kMaxSplits; ++most)
-    for (int min_rows : least) {
-      if (min_rows > 48 && most > 5) continue;
-      const DecodeSplit rule{most, min_rows};
-      assert(rule.blocks(0) == 1 && rule.bound(0) == 1);
-      int before = 1;
-      for (int L = 1; L <= 6000; ++L) {
-        const int bound = rule.bound(L), chunk = rule.chunk(L), blocks = rule.blocks(L);
-        assert(bound >= before && bound <= most && blocks >= 1 && blocks <= bound);
-        assert(chunk % 16 == 0 && (blocks - 1) * chunk < L && L <= blocks * chunk);
-        assert(bound <= kPortable || (bound == most && L > min_rows * (most - 1)));
-        before = bound;
-      }
-      assert(before == most);
-    }
+  for (int most = 1; most <= kMaxSplits; ++most) {
+    DecodeSplit rule;
+    rule.most = most;
+    rule.large_from = 48 * most;
+    check(rule, most, 6000);
+    for (int L = 1; L <= 6000; ++L) assert(rule.bound(L) <= kPortable || (rule.bound(L) == most && L > 48 * (most - 1)));
+  }
+  const short active[] = {592, 296, 187, 142, 112};
+  for (int pairs = 297; pairs <= 3000; ++pairs) {
+    const DecodeSplit rule = split_of_waves(pairs, active);
+    check(rule, rule.most, 1 << 16);
+    assert(rule.most <= 5 && rule.bound(64) == 1);
+  }
+  assert(split_of_waves(384, active).bound(2064) == 1 && split_of_waves(768, active).bound(2064) == 2 && split_of_waves(640, active).bound(4096) == 4);
   DeviceNumber number;
   int asked = 0, holds = 16;
   auto most = [&](int device) { return number.get(device, [&] { return largest_cluster([&](int n) { ++asked; return n <= holds; }); }); };
