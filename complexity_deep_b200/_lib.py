@@ -107,6 +107,9 @@ SIGNATURES = {
     "cd_decode_step_attention": (c_int, [c_void_p] * 5 + [c_float, c_float, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
                                          c_longlong, c_longlong, c_longlong, c_int, c_void_p, c_void_p, c_void_p,
                                          c_void_p]),
+    "cd_decode_step_attention_ws": (c_int, [c_void_p] * 5 + [c_float, c_float, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
+                                            c_longlong, c_longlong, c_longlong, c_int, c_void_p, c_void_p, c_void_p,
+                                            c_void_p, c_size_t, c_void_p]),
     "cd_attention_prefill_supported": (c_int, [c_int, c_int, c_int, c_int, c_int]),
     "cd_attention_prefill": (c_int, [c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float,
                                      c_void_p]),

@@ -165,9 +165,10 @@ int cd_decode_rope_append(void* qkv, const void* q_w, const void* k_w, const flo
   return e == cudaSuccess ? CD_OK : cuda_fail(e, "decode rope/append launch");
 }
 
+// what the kernels take; other sizes need no workspace, since their calls are refused
 size_t cd_decode_attention_workspace_bytes(int B, int hq, int hkv, int L, int D) {
-  (void)B, (void)hq, (void)hkv, (void)L, (void)D;
-  return 0;
+  if (B < 1 || hq < 1 || hkv < 1 || L < 1 || hq % hkv || hq / hkv > 4 || (D != 64 && D != 128)) return 0;
+  return decode_attention_workspace_bytes(B, hq, hkv, L, D);
 }
 
 int cd_decode_attention(const void* q, long long q_stride_b, const void* k, const void* v,
@@ -178,14 +179,14 @@ int cd_decode_attention(const void* q, long long q_stride_b, const void* k, cons
   if (B < 1 || hq < 1 || hkv < 1 || L < 1 || hq % hkv) return CD_ERR_INVALID;
   if (D != 64 && D != 128) return CD_ERR_UNSUPPORTED;
   if (hq / hkv > 4) return CD_ERR_UNSUPPORTED;
-  (void)ws, (void)ws_bytes;
   if (!q || !k || !v || !out) return CD_ERR_INVALID;
+  if (ws && (!aligned16(ws) || ws_bytes < decode_attention_workspace_bytes(B, hq, hkv, L, D))) return CD_ERR_INVALID;
   if (!aligned16(q) || !aligned16(k) || !aligned16(v) || !aligned16(out)) return CD_ERR_INVALID;
   if ((q_stride_b & 7) || (kv_stride_b & 7) || (kv_stride_h & 7) || (kv_stride_t & 7))
     return CD_ERR_INVALID;
   cudaError_t e = launch_decode_attention(q, q_stride_b, k, v, kv_stride_b, kv_stride_h,
                                           kv_stride_t, mask, mask_stride_b, scale, B, hq, hkv, L,
-                                          D, out, as_stream(stream), kv_len_dev);
+                                          D, out, ws, as_stream(stream), kv_len_dev);
   return e == cudaSuccess ? CD_OK : cuda_fail(e, "decode attention launch");
 }
 
@@ -194,6 +195,15 @@ int cd_decode_step_attention(const void* qkv, const void* q_w, const void* k_w, 
                              void* k_cache, void* v_cache, long long kv_stride_b, long long kv_stride_h,
                              long long kv_stride_t, int capacity, const int32_t* pos_dev,
                              const int32_t* kv_len_dev, void* out, void* stream) {
+  return cd_decode_step_attention_ws(qkv, q_w, k_w, cos_t, sin_t, eps, scale, B, hq, hkv, D, k_cache, v_cache, kv_stride_b,
+                                     kv_stride_h, kv_stride_t, capacity, pos_dev, kv_len_dev, out, nullptr, 0, stream);
+}
+
+int cd_decode_step_attention_ws(const void* qkv, const void* q_w, const void* k_w, const float* cos_t,
+                                const float* sin_t, float eps, float scale, int B, int hq, int hkv, int D,
+                                void* k_cache, void* v_cache, long long kv_stride_b, long long kv_stride_h,
+                                long long kv_stride_t, int capacity, const int32_t* pos_dev,
+                                const int32_t* kv_len_dev, void* out, void* ws, size_t ws_bytes, void* stream) {
   if (B < 1 || hq < 1 || hkv < 1 || capacity < 1 || hq % hkv) return CD_ERR_INVALID;
   if (D != 64 && D != 128) return CD_ERR_UNSUPPORTED;
   if (hq / hkv > 4) return CD_ERR_UNSUPPORTED;
@@ -203,9 +213,10 @@ int cd_decode_step_attention(const void* qkv, const void* q_w, const void* k_w, 
       !aligned16(sin_t) || (q_w && (!aligned16(q_w) || !aligned16(k_w))))
     return CD_ERR_INVALID;
   if ((kv_stride_b & 7) || (kv_stride_h & 7) || (kv_stride_t & 7)) return CD_ERR_INVALID;
+  if (ws && (!aligned16(ws) || ws_bytes < decode_attention_workspace_bytes(B, hq, hkv, capacity, D))) return CD_ERR_INVALID;
   cudaError_t e = launch_decode_step_attention(qkv, q_w, k_w, cos_t, sin_t, eps, k_cache, v_cache, kv_stride_b,
                                                kv_stride_h, kv_stride_t, capacity, pos_dev, kv_len_dev, scale, B, hq,
-                                               hkv, D, out, as_stream(stream));
+                                               hkv, D, out, ws, as_stream(stream));
   return e == cudaSuccess ? CD_OK : cuda_fail(e, "decode step attention launch");
 }
 

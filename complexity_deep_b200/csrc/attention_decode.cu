@@ -13,7 +13,8 @@
 // per step; every lane group
 // keeps an online-softmax state (running max, sum, weighted V) per query head, merged across
 // the block through shared memory. The splits of a pair are one thread-block cluster and
-// merge through one another's shared memory, each block a share of the columns.
+// merge through one another's shared memory, each block a share of the columns; long caches of
+// few pairs take several clusters a pair and a kernel that adds what they leave in a workspace.
 //
 // A decode step (kStep) hands over the raw projections: every block normalises and rotates the query
 // heads of its group itself (8 lanes a head, as many as the rows need anyway), and the one
@@ -38,6 +39,7 @@ namespace {
 
 constexpr int kAttnThreads = 128;
 constexpr int kLanesPerRow = 8;
+constexpr int kMaxClusters = 4; // of a pair
 
 __device__ __forceinline__ float lo_f(uint32_t v) { return __uint_as_float(v << 16); }
 __device__ __forceinline__ float hi_f(uint32_t v) { return __uint_as_float(v & 0xffff0000u); }
@@ -63,7 +65,16 @@ constexpr short kActive[3][kMaxSplits] = {{296, 148, 93, 71, 56, 45, 37, 33, 30,
 //   More pairs: split_of_waves. us, cold L2, 2 x 128, one block / two / three / four a pair: 384 pairs of 300 rows 21 / 29 / 33 / 34,
 //   of 2 064 86 / 109 / 105 / 96; 640 of 300 39 / 41 / 47 / 54, of 1 024 100 / 90 / 87 / 94, of 4 096 310 / 262 / 252 / 244; 768 of
 //   300 41 / 45 / 55 / 64, of 2 064 188 / 161 / 171 / 171; 2 048 of 300 83 / 103 / 128 / 153, of 4 096 671 / 663 / 687 / 695.
-inline DecodeSplit choose_split(int B, int hkv, int per_sm) {
+//   Long caches of few pairs: as many clusters of eight as fit, up to four a pair, with a kernel behind them (some 2 us). A block
+//   is one chain of row steps, 0.43 us per 16 rows with an SM to itself whatever it has in flight (8 and 16 steps staged for four:
+//   no difference; two and four steps side by side 0.29 to 0.38, eight warps a block 0.26 and no gain beyond one block an SM).
+//   us of a step, cold L2, one cluster / several (three launches with up to 32 blocks a pair, before that): 4 pairs of 3 x 64,
+//   8 192 rows 22.5 / 18.3 (18.5), 32 768 65.7 / 41.1 (41.1); 8 pairs of 2 x 128, 4 096 14.5 / 16.1 (15.9), 8 192 21.1 / 19.5
+//   (20.4), 32 768 63.7 / 42.2 (43.3); 8 of 4 x 128, 8 192 34.9 / 27.0 (27.7), 32 768 109 / 64 (67.5); 16 of 2 x 128, 8 192
+//   26.5 / 25.8 (26.9), 32 768 80 / 66 (67); 16 of 3 x 64, 4 096 16.8 / 16.5 (18.5), 32 768 86 / 51 (53); 32 of 2 x 128,
+//   16 384 68.2 / 66.2 (66.8), 32 768 125 / 113 (112).
+inline DecodeSplit choose_split(int B, int hkv, int G, int D) {
+  const int per_sm = blocks_per_sm(G, D);
   const long long pairs = static_cast<long long>(B) * hkv;
   const short(&active)[kMaxSplits] = kActive[per_sm - 2];
   if (pairs <= active[1]) {
@@ -72,6 +83,9 @@ inline DecodeSplit choose_split(int B, int hkv, int per_sm) {
     DecodeSplit r;
     r.most = pairs <= 8 && fit == kMaxSplits ? kMaxSplits : pairs <= 24 && fit >= 13 ? 13 : fit > kPortable ? kPortable : fit;
     r.large_from = r.most * (pairs > 16 ? 64 : 48);
+    const long long clusters = active[kPortable - 1] / pairs;
+    r.many = kPortable * static_cast<int>(clusters < kMaxClusters ? clusters : kMaxClusters);
+    if (r.many > r.most) r.many_from = r.most == kMaxSplits ? 4096 : (r.most > kPortable ? 64 : 128) * D;
     return r;
   }
   return split_of_waves(pairs, active);
@@ -104,6 +118,25 @@ __device__ __forceinline__ float peer_load(const float* p, int rank) {
   asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
   return v;
 }
+
+// Sums of some rows for one column: the largest score, the weights relative to it, the weighted values.
+struct Sums {
+  float m = -FLT_MAX, l = 0.f, a = 0.f;
+};
+template <int N>
+__device__ __forceinline__ Sums add_sums(const Sums (&in)[N]) {
+  Sums r;
+#pragma unroll
+  for (int s = 0; s < N; ++s) r.m = fmaxf(r.m, in[s].m);
+#pragma unroll
+  for (int s = 0; s < N; ++s) {
+    const float w = in[s].m > -FLT_MAX ? __expf(in[s].m - r.m) : 0.f;
+    r.l += in[s].l * w;
+    r.a += in[s].a * w;
+  }
+  return r;
+}
+__device__ __forceinline__ __nv_bfloat16 quotient(const Sums& s) { return __float2bfloat16_rn(s.l > 0.f ? s.a / s.l : 0.f); }
 
 // What a decode step brings besides the query: norm weights (or none), rotation tables, where the new row goes.
 struct StepArgs {
@@ -199,6 +232,9 @@ constexpr int kStages = 4;   // row steps staged in shared memory per thread (3 
 // private slot of shared memory with cp.async (bytes in flight without holding registers:
 // 4 blocks per SM keep ~100 KB on the way) and reads them back with 16-byte loads, so no
 // block-level synchronisation is needed inside the loop.
+//
+// The blocks of a pair are clusters of `cl`. Several of them (part != NULL) leave their sums there for combine_kernel, which
+// adds them as one cluster adds its blocks: eight at a time, so the bits are the same.
 template <int DPL, int G, bool kStep>
 __global__ void __launch_bounds__(kAttnThreads, blocks_per_sm(G, DPL * kLanesPerRow))
 decode_attn_kernel(const __nv_bfloat16* __restrict__ q, long long q_stride_b,
@@ -206,7 +242,7 @@ decode_attn_kernel(const __nv_bfloat16* __restrict__ q, long long q_stride_b,
                    long long kv_stride_b, long long kv_stride_h, long long kv_stride_t,
                    const __nv_bfloat16* __restrict__ mask, long long mask_stride_b,
                    float scale, int L, DecodeSplit rule, __nv_bfloat16* __restrict__ out,
-                   const int* __restrict__ len_dev, StepArgs st) {
+                   const int* __restrict__ len_dev, StepArgs st, int cl, float* part) {
   constexpr int D = DPL * kLanesPerRow;
   constexpr int kV = DPL / 8;                               // 16-byte pieces of K (and of V) per lane
   constexpr int kStepBytes = kAttnThreads * 2 * kV * 16;    // one row step of the block
@@ -235,7 +271,7 @@ decode_attn_kernel(const __nv_bfloat16* __restrict__ q, long long q_stride_b,
     if (st.q_w) qw = load_halves<D>(st.q_w, sub);
   }
   if (len_dev) L = max(0, min(L, __ldg(len_dev)));
-  const int splits = rule.blocks(L);
+  const int splits = rule.bound(L);                          // the last of them may have no rows
   const int chunk = rule.chunk(L);
   const int t_begin = min(L, split * chunk);
   const int t_end = min(L, t_begin + chunk);
@@ -442,41 +478,67 @@ decode_attn_kernel(const __nv_bfloat16* __restrict__ q, long long q_stride_b,
     }
   }
 
-  // the splits of the pair: out = sum_s w_s acc_s / sum_s w_s l_s, w_s = exp(m_s - max m), every block a share of the columns
-  if (gridDim.x > 1) {
+  // the splits of the pair, every block a share of the columns
+  if (cl > 1) {
     __syncwarp();
     cluster_arrive();
     cluster_wait();
   } else {
     __syncthreads();
   }
-  for (int idx = split * kAttnThreads + threadIdx.x; idx < G * D; idx += gridDim.x * kAttnThreads) {
+  const int group = part ? split / kPortable : 0, rank = split - group * kPortable;
+  const int live = min(cl, splits - group * kPortable);      // blocks of this cluster that may have rows
+  // up to eight blocks: a thread a column; more: two, the first eight and the rest by themselves as several clusters do it
+  const int two = live > kPortable ? 1 : 0, from = two & threadIdx.x ? kPortable : 0, per = kAttnThreads >> two;
+  for (int idx = rank * per + (threadIdx.x >> two); idx < G * D; idx += cl * per) {
     const int g = idx / D;
-    float ms[kMaxSplits], ls[kMaxSplits], as[kMaxSplits], m = -FLT_MAX;
+    Sums in[kPortable];
 #pragma unroll
-    for (int s = 0; s < kMaxSplits; ++s) {
-      ms[s] = -FLT_MAX;
-      ls[s] = as[s] = 0.f;
-      if (s < splits) {
-        ms[s] = peer_load(&s_part[G * D + g], s);
-        ls[s] = peer_load(&s_part[G * D + G + g], s);
-        as[s] = peer_load(&s_part[idx], s);
+    for (int x = 0; x < kPortable; ++x) {
+      const int s = from + x;
+      if (s < live) in[x] = {peer_load(&s_part[G * D + g], s), peer_load(&s_part[G * D + G + g], s), peer_load(&s_part[idx], s)};
+    }
+    Sums total = add_sums(in);
+    if (two) {
+      const Sums both[2] = {total, {__shfl_down_sync(0xffffffffu, total.m, 1), __shfl_down_sync(0xffffffffu, total.l, 1),
+                                    __shfl_down_sync(0xffffffffu, total.a, 1)}};
+      total = add_sums(both);
+    }
+    if (from > 0) continue;
+    const long long pair = static_cast<long long>(b) * hkv + kvh;
+    if (part) {
+      float* dst = part + (pair * (gridDim.x / kPortable) + group) * (G * D + 2 * G);
+      dst[idx] = total.a;
+      if (idx == g * D) {
+        dst[G * D + g] = total.m;
+        dst[G * D + G + g] = total.l;
       }
-      m = fmaxf(m, ms[s]);
+    } else {
+      out[pair * G * D + idx] = quotient(total);
     }
-    float l = 0.f, a = 0.f;
-#pragma unroll
-    for (int s = 0; s < kMaxSplits; ++s) {
-      const float w = ms[s] > -FLT_MAX ? __expf(ms[s] - m) : 0.f;
-      l += ls[s] * w;
-      a += as[s] * w;
-    }
-    out[(static_cast<long long>(b) * hkv + kvh) * G * D + idx] = __float2bfloat16_rn(l > 0.f ? a / l : 0.f);
   }
-  if (gridDim.x > 1) {                 // nobody leaves while its sums are being read
+  if (cl > 1) {                        // nobody leaves while its sums are being read
     __syncwarp();
     cluster_arrive();
     cluster_wait();
+  }
+}
+
+// What the clusters of a pair left behind: grid (pairs), a column per thread.
+__global__ void __launch_bounds__(kAttnThreads)
+combine_kernel(const float* part, int groups, int G, int D, __nv_bfloat16* out) {
+  griddep_wait();
+  griddep_launch_dependents();
+  const float* src = part + static_cast<long long>(blockIdx.x) * groups * (G * D + 2 * G);
+  for (int idx = threadIdx.x; idx < G * D; idx += kAttnThreads) {
+    const int g = idx / D;
+    Sums in[kMaxClusters];
+#pragma unroll
+    for (int x = 0; x < kMaxClusters; ++x) {
+      const float* from = src + x * (G * D + 2 * G);
+      if (x < groups) in[x] = {from[G * D + g], from[G * D + G + g], from[idx]};
+    }
+    out[static_cast<long long>(blockIdx.x) * G * D + idx] = quotient(add_sums(in));
   }
 }
 
@@ -513,38 +575,45 @@ template <int DPL, int G, bool kStep>
 cudaError_t launch_one(int B, int hkv, cudaStream_t stream, const __nv_bfloat16* q, long long qsb, const __nv_bfloat16* k,
                        const __nv_bfloat16* v, long long sb, long long sh, long long stt, const __nv_bfloat16* mask,
                        long long msb, float scale, int L, DecodeSplit rule, __nv_bfloat16* out, const int* len_dev,
-                       const StepArgs& step) {
+                       const StepArgs& step, float* ws) {
   constexpr auto kKernel = decode_attn_kernel<DPL, G, kStep>;
   if (rule.most > kPortable) {
     const cudaError_t e = allow_clusters<kKernel>(rule);
     if (e != cudaSuccess) return e;
   }
+  const bool many = L >= rule.many_from;
+  const int cl = many ? kPortable : len_dev ? rule.bound(L) : rule.blocks(L);
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(len_dev ? rule.bound(L) : rule.blocks(L), hkv, B);
+  cfg.gridDim = dim3(many ? rule.many : cl, hkv, B);
   cfg.blockDim = dim3(kAttnThreads);
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
   attr[1].id = cudaLaunchAttributeClusterDimension;
-  attr[1].val.clusterDim.x = cfg.gridDim.x;
+  attr[1].val.clusterDim.x = cl;
   attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = cfg.gridDim.x > 1 ? 2 : 1;
-  return cudaLaunchKernelEx(&cfg, kKernel, q, qsb, k, v, sb, sh, stt, mask, msb, scale, L, rule, out, len_dev, step);
+  cfg.numAttrs = cl > 1 ? 2 : 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kKernel, q, qsb, k, v, sb, sh, stt, mask, msb, scale, L, rule, out, len_dev, step, cl,
+                                           many ? ws : static_cast<float*>(nullptr));
+  if (e != cudaSuccess || !many) return e;
+  return launch_kernel(combine_kernel, dim3(B * hkv), dim3(kAttnThreads), 0, stream, static_cast<const float*>(ws), rule.many / kPortable, G,
+                       DPL * kLanesPerRow, out);
 }
 
 template <bool kStep>
 cudaError_t launch_any(const void* q, long long qsb, const void* k, const void* v, long long sb, long long sh, long long stt,
                        const void* mask, long long msb, float scale, int B, int hq, int hkv, int L, int D, void* out,
-                       cudaStream_t stream, const int* len_dev, const StepArgs& step) {
+                       cudaStream_t stream, const int* len_dev, const StepArgs& step, void* ws) {
   const int G = hq / hkv;
-  const DecodeSplit rule = choose_split(B, hkv, blocks_per_sm(G, D));
+  DecodeSplit rule = choose_split(B, hkv, G, D);
+  if (!ws) rule.many_from = 1 << 30;
   auto b16 = [](const void* p) { return static_cast<const __nv_bfloat16*>(p); };
 #define CDEEP_ATTN_CASE(DPL, GG)                                                                                           \
   if (D == 8 * DPL && G == GG)                                                                                             \
     return launch_one<DPL, GG, kStep>(B, hkv, stream, b16(q), qsb, b16(k), b16(v), sb, sh, stt, b16(mask), msb, scale, L,  \
-                                      rule, static_cast<__nv_bfloat16*>(out), len_dev, step);
+                                      rule, static_cast<__nv_bfloat16*>(out), len_dev, step, static_cast<float*>(ws));
   CDEEP_ATTN_CASE(8, 1) CDEEP_ATTN_CASE(8, 2) CDEEP_ATTN_CASE(8, 3) CDEEP_ATTN_CASE(8, 4)
   CDEEP_ATTN_CASE(16, 1) CDEEP_ATTN_CASE(16, 2) CDEEP_ATTN_CASE(16, 3) CDEEP_ATTN_CASE(16, 4)
 #undef CDEEP_ATTN_CASE
@@ -553,18 +622,24 @@ cudaError_t launch_any(const void* q, long long qsb, const void* k, const void* 
 
 }  // namespace
 
+size_t decode_attention_workspace_bytes(int B, int hq, int hkv, int L, int D) {
+  const int G = hq / hkv;
+  const DecodeSplit rule = choose_split(B, hkv, G, D);
+  return L < rule.many_from ? 0 : sizeof(float) * B * hkv * (rule.many / kPortable) * (G * D + 2 * G);
+}
+
 cudaError_t launch_decode_attention(const void* q, long long q_stride_b, const void* k, const void* v, long long kv_stride_b,
                                     long long kv_stride_h, long long kv_stride_t, const void* mask, long long mask_stride_b,
-                                    float scale, int B, int hq, int hkv, int L, int D, void* out, cudaStream_t stream,
+                                    float scale, int B, int hq, int hkv, int L, int D, void* out, void* ws, cudaStream_t stream,
                                     const int* kv_len_dev) {
   return launch_any<false>(q, q_stride_b, k, v, kv_stride_b, kv_stride_h, kv_stride_t, mask, mask_stride_b, scale, B, hq, hkv,
-                           L, D, out, stream, kv_len_dev, StepArgs{});
+                           L, D, out, stream, kv_len_dev, StepArgs{}, ws);
 }
 
 cudaError_t launch_decode_step_attention(const void* qkv, const void* q_w, const void* k_w, const float* cos_t, const float* sin_t,
                                          float eps, void* k_cache, void* v_cache, long long kv_stride_b, long long kv_stride_h,
                                          long long kv_stride_t, int capacity, const int* pos_dev, const int* kv_len_dev,
-                                         float scale, int B, int hq, int hkv, int D, void* out, cudaStream_t stream) {
+                                         float scale, int B, int hq, int hkv, int D, void* out, void* ws, cudaStream_t stream) {
   StepArgs st;
   st.q_w = static_cast<const __nv_bfloat16*>(q_w);
   st.k_w = static_cast<const __nv_bfloat16*>(k_w);
@@ -576,7 +651,7 @@ cudaError_t launch_decode_step_attention(const void* qkv, const void* q_w, const
   st.pos_dev = pos_dev;
   st.capacity = capacity;
   return launch_any<true>(qkv, static_cast<long long>(hq + 2 * hkv) * D, k_cache, v_cache, kv_stride_b, kv_stride_h, kv_stride_t,
-                          nullptr, 0, scale, B, hq, hkv, capacity, D, out, stream, kv_len_dev, st);
+                          nullptr, 0, scale, B, hq, hkv, capacity, D, out, stream, kv_len_dev, st, ws);
 }
 
 }  // namespace cdeep

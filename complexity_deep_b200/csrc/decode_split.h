@@ -16,11 +16,13 @@ constexpr int kPortable = 8;    // the largest that every device takes
 
 struct DecodeSplit {
   int most = 1, large_from = 0;             // blocks at most, and from how many rows on more than eight of them
+  int many = 0, many_from = 1 << 30;        // from that many rows on: `many` blocks, in clusters of eight
   int waves = 0, more_from[4] = {};         // more pairs than two blocks of each fit: one block, and one more from each of these rows on
   // Blocks asked for: one for every 48 rows, up to eight; `most` beyond that. Never falls as L grows (large_from is at least eight
   // times 48), so a launch sized for L has the blocks for every shorter cache.
   CDEEP_HD int bound(int L) const {
     if (waves) return 1 + (L >= more_from[0]) + (L >= more_from[1]) + (L >= more_from[2]) + (L >= more_from[3]);
+    if (L >= many_from) return many;
     if (most > kPortable && L >= large_from) return most;
     const int n = (L + 47) / 48, cap = most < kPortable ? most : kPortable;
     return n < 1 ? 1 : n < cap ? n : cap;

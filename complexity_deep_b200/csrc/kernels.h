@@ -104,16 +104,17 @@ cudaError_t launch_pack_gate_up(const void* gate, const void* up, void* packed, 
                                 int block_n, int feature_major, cudaStream_t stream);
 cudaError_t launch_transpose(const void* in, void* out, int G, int R, int C, cudaStream_t stream);
 
+size_t decode_attention_workspace_bytes(int B, int hq, int hkv, int L, int D);
 cudaError_t launch_decode_attention(const void* q, long long q_stride_b, const void* k,
                                     const void* v, long long kv_stride_b, long long kv_stride_h,
                                     long long kv_stride_t, const void* mask,
                                     long long mask_stride_b, float scale, int B, int hq, int hkv,
-                                    int L, int D, void* out, cudaStream_t stream,
+                                    int L, int D, void* out, void* ws, cudaStream_t stream,
                                     const int* kv_len_dev = nullptr);
 cudaError_t launch_decode_step_attention(const void* qkv, const void* q_w, const void* k_w, const float* cos_t, const float* sin_t,
                                          float eps, void* k_cache, void* v_cache, long long kv_stride_b, long long kv_stride_h,
                                          long long kv_stride_t, int capacity, const int* pos_dev, const int* kv_len_dev,
-                                         float scale, int B, int hq, int hkv, int D, void* out, cudaStream_t stream);
+                                         float scale, int B, int hq, int hkv, int D, void* out, void* ws, cudaStream_t stream);
 
 // fp32 residual stream (stream_f32.cu)
 cudaError_t launch_embed_rows(const long long* ids, const void* table, float* x, int T, int V, int W, int ldw,

@@ -282,6 +282,12 @@ def decode_rope_append(qkv: torch.Tensor, q_w: Optional[torch.Tensor],
     return qkv
 
 
+def _decode_workspace(lib, B: int, hq: int, hkv: int, L: int, D: int, device):
+    """(buffer or None, bytes) for decode attention over L rows: long caches of few sequences only."""
+    n = lib.cd_decode_attention_workspace_bytes(B, hq, hkv, L, D)
+    return (torch.empty(n, dtype=torch.uint8, device=device) if n else None), n
+
+
 def decode_attention(qkv: torch.Tensor, k: torch.Tensor, v: torch.Tensor,
                      mask: Optional[torch.Tensor], hq: int, hkv: int, head_dim: int,
                      kv_len_dev: Optional[torch.Tensor] = None) -> torch.Tensor:
@@ -309,11 +315,12 @@ def decode_attention(qkv: torch.Tensor, k: torch.Tensor, v: torch.Tensor,
                                    or kv_len_dev.numel() != 1):
         raise RuntimeError("kv_len_dev: expected one int32 on the device")
     out = torch.empty(B, hq * D, dtype=BF16, device=qkv.device)
-    with _Span("decode_attention"):
+    ws, ws_bytes = _decode_workspace(lib, B, hq, hkv, L, D, qkv.device)
+    with _Span("decode_attention", 2 if ws_bytes else 1):
         _lib.check(lib.cd_decode_attention(
             qkv.data_ptr(), qkv.stride(0), k.data_ptr(), v.data_ptr(), k.stride(0), k.stride(1),
             k.stride(2), mptr, mstride, float(head_dim) ** -0.5, B, hq, hkv, L, _ptr(kv_len_dev),
-            D, out.data_ptr(), None, 0, _stream()), "cd_decode_attention")
+            D, out.data_ptr(), _ptr(ws), ws_bytes, _stream()), "cd_decode_attention")
     return out
 
 
@@ -332,11 +339,12 @@ def decode_step_attention(qkv: torch.Tensor, q_w: Optional[torch.Tensor], k_w: O
         rotated = decode_rope_append(qkv.clone(), q_w, k_w, cos, sin, eps, hq, hkv, D, k_cache, v_cache, pos_dev)
         return decode_attention(rotated, k_cache, v_cache, None, hq, hkv, D, kv_len_dev=kv_len_dev)
     out = torch.empty(B, hq * D, dtype=BF16, device=qkv.device)
-    with _Span("decode_attention"):
-        _lib.check(lib.cd_decode_step_attention(
+    ws, ws_bytes = _decode_workspace(lib, B, hq, hkv, k_cache.shape[2], D, qkv.device)
+    with _Span("decode_attention", 2 if ws_bytes else 1):
+        _lib.check(lib.cd_decode_step_attention_ws(
             qkv.data_ptr(), _ptr(q_w), _ptr(k_w), cos.data_ptr(), sin.data_ptr(), float(eps), float(D) ** -0.5, B, hq, hkv,
             D, k_cache.data_ptr(), v_cache.data_ptr(), k_cache.stride(0), k_cache.stride(1), k_cache.stride(2),
-            k_cache.shape[2], pos_dev.data_ptr(), kv_len_dev.data_ptr(), out.data_ptr(), _stream()),
+            k_cache.shape[2], pos_dev.data_ptr(), kv_len_dev.data_ptr(), out.data_ptr(), _ptr(ws), ws_bytes, _stream()),
             "cd_decode_step_attention")
     return out
 

@@ -188,8 +188,9 @@ int cd_decode_rope_append(void* qkv, const void* q_w, const void* k_w, const flo
  * projection buffer).  k, v: element strides (batch, kv head, token), D contiguous — the
  * cache is read in place, whatever buffer it lives in.  mask: bf16 additive [B, L] with row
  * stride mask_stride_b (0 = one row for all), or NULL.  out: [B, hq * D] bf16.
- * ws: not used any more (NULL will do; cd_decode_attention_workspace_bytes is 0): the blocks of a
- * pair meet in one another's shared memory.  D is 64 or 128, G <= 4; all strides
+ * ws: cd_decode_attention_workspace_bytes(...) bytes, or NULL: a few pairs with a long cache (from
+ * 4 096 to 16 384 rows on, by their number; elsewhere the size is 0) are then shared by fewer blocks.
+ * D is 64 or 128, G <= 4; all strides
  * multiples of 8 elements.  kv_len_dev (may be NULL): a device scalar; when given, only the
  * first min(L, *kv_len_dev) cached tokens are attended (L then is the capacity the launch is
  * sized for), with the same split of the rows over blocks, hence the same bits, as a call
@@ -209,6 +210,12 @@ int cd_decode_step_attention(const void* qkv, const void* q_w, const void* k_w, 
                              void* k_cache, void* v_cache, long long kv_stride_b, long long kv_stride_h,
                              long long kv_stride_t, int capacity, const int32_t* pos_dev,
                              const int32_t* kv_len_dev, void* out, void* stream);
+/* The same with the workspace of cd_decode_attention for L = capacity (NULL: as above). */
+int cd_decode_step_attention_ws(const void* qkv, const void* q_w, const void* k_w, const float* cos_t,
+                                const float* sin_t, float eps, float scale, int B, int hq, int hkv, int D,
+                                void* k_cache, void* v_cache, long long kv_stride_b, long long kv_stride_h,
+                                long long kv_stride_t, int capacity, const int32_t* pos_dev,
+                                const int32_t* kv_len_dev, void* out, void* ws, size_t ws_bytes, void* stream);
 
 /* ---- causal self-attention over a prompt (prefill) --------------------------------------------
  * Replaces, for a prompt without cached keys and without an additive mask,

@@ -33,6 +33,9 @@ int main() {
     rule.large_from = 48 * most;
     check(rule, most, 6000);
     for (int L = 1; L <= 6000; ++L) assert(rule.bound(L) <= kPortable || (rule.bound(L) == most && L > 48 * (most - 1)));
+    rule.many = 40;
+    rule.many_from = 3000;
+    check(rule, 40, 6000);
   }
   const short active[] = {592, 296, 187, 142, 112};
   for (int pairs = 297; pairs <= 3000; ++pairs) {

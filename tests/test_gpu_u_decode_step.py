@@ -76,6 +76,19 @@ def test_position_outside_the_rows_attended(pos, length):
     _check(2, 2, 2, 64, 200, pos, length)
 
 
+@pytest.mark.parametrize("B,hkv,G,D,cap", [(1, 8, 2, 128, 9000), (2, 8, 1, 64, 4200), (1, 2, 4, 128, 5000), (4, 8, 2, 64, 8300), (1, 30, 1, 64, 8200)])
+def test_a_length_below_the_capacity_gives_the_bits_of_a_launch_of_that_length(B, hkv, G, D, cap):
+    """One cluster a pair, and several whose sums are added by a kernel behind them."""
+    from complexity_deep_b200 import _lib, ops
+    assert _lib.load().cd_decode_attention_workspace_bytes(B, hkv * G, hkv, cap, D) > 0
+    qkv, k, v, *_ = _inputs(B, hkv, G, D, cap, False, cap)
+    for length in (1, 300, 1500, 4095, 4096, cap - 1, cap):
+        state = torch.tensor([length], dtype=torch.int32, device="cuda")
+        got = ops.decode_attention(qkv, k, v, None, hkv * G, hkv, D, kv_len_dev=state)
+        want = ops.decode_attention(qkv, k[:, :, :length], v[:, :, :length], None, hkv * G, hkv, D)
+        assert torch.equal(got, want), length
+
+
 @pytest.mark.parametrize("what", ["cos", "weight"])
 def test_off_a_16_byte_boundary(what):
     from complexity_deep_b200 import ops
