@@ -136,7 +136,7 @@ __device__ __forceinline__ Sums add_sums(const Sums (&in)[N]) {
   }
   return r;
 }
-__device__ __forceinline__ __nv_bfloat16 quotient(const Sums& s) { return __float2bfloat16_rn(s.l > 0.f ? s.a / s.l : 0.f); }
+__device__ __forceinline__ __nv_bfloat16 quotient(const Sums& s) { return __float2bfloat16_rn(s.l == 0.f ? 0.f : s.a / s.l); }   // no visible row: 0; a NaN score stays one
 
 // What a decode step brings besides the query: norm weights (or none), rotation tables, where the new row goes.
 struct StepArgs {

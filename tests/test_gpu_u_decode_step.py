@@ -107,3 +107,25 @@ def test_off_a_16_byte_boundary(what):
     assert torch.equal(k, k1) and torch.equal(v, v1) and torch.equal(qkv, before)
     # what a rounding of q to bf16 moves a score by (2^-8 of at most ~6), as above
     assert bool(((got.float() - want.float()).abs() <= want.float().abs() * 2.0 ** -7 + 2.0 ** -7).all())
+
+
+@pytest.mark.parametrize("B,hkv,G,D,cap", [(1, 2, 2, 64, 300), (2, 8, 2, 128, 1100), (64, 8, 1, 64, 700)])
+def test_nan_and_infinities(B, hkv, G, D, cap):
+    """A NaN score makes its head NaN and no other one; an infinite value its column; a row that sees nothing is zero."""
+    from complexity_deep_b200 import ops
+    hq, (qkv, k, v, cos, sin, (qw, kw)) = hkv * G, _inputs(B, hkv, G, D, cap, True, 11)
+    run = lambda k, v, m=None: ops.decode_attention(qkv, k, v, m, hq, hkv, D).view(B, hkv, G, D)
+    clean = run(k, v)
+    assert bool(clean.isfinite().all())
+    bad, worse = k.clone(), v.clone()
+    bad[0, 1, cap - 2, 3] = float("nan")
+    worse[0, 0, 5, 7] = float("inf")
+    hit = torch.zeros_like(clean, dtype=torch.bool)
+    hit[0, 1] = hit[0, 0, :, 7] = True
+    got = run(bad, worse)
+    assert bool(got[0, 1].isnan().all()) and not bool(got[hit].isfinite().any()) and torch.equal(got[~hit], clean[~hit])
+    state = torch.tensor([cap - 1, cap], dtype=torch.int32, device="cuda")
+    step = ops.decode_step_attention(qkv, qw, kw, cos, sin, 1e-6, hq, hkv, D, bad, worse, state[:1], state[1:]).view(B, hkv, G, D)
+    assert bool(step[0, 1].isnan().all()) and not bool(step[hit].isfinite().any()) and bool(step[~hit].isfinite().all())
+    mask = torch.full((1, 1, 1, cap), float("-inf"), dtype=torch.bfloat16, device="cuda")
+    assert not bool(run(k, v, mask).any())
