@@ -233,16 +233,19 @@ constexpr int kStages = 4;   // row steps staged in shared memory per thread (3 
 // 4 blocks per SM keep ~100 KB on the way) and reads them back with 16-byte loads, so no
 // block-level synchronisation is needed inside the loop.
 //
+// The kernel ahead may still run when this one starts, and it writes the query: nothing is read on the read-only path, whose
+// loads the compiler may move to before the wait.
+//
 // The blocks of a pair are clusters of `cl`. Several of them (part != NULL) leave their sums there for combine_kernel, which
 // adds them as one cluster adds its blocks: eight at a time, so the bits are the same.
 template <int DPL, int G, bool kStep>
 __global__ void __launch_bounds__(kAttnThreads, blocks_per_sm(G, DPL * kLanesPerRow))
-decode_attn_kernel(const __nv_bfloat16* __restrict__ q, long long q_stride_b,
+decode_attn_kernel(const __nv_bfloat16* q, long long q_stride_b,
                    const __nv_bfloat16* k, const __nv_bfloat16* v,
                    long long kv_stride_b, long long kv_stride_h, long long kv_stride_t,
-                   const __nv_bfloat16* __restrict__ mask, long long mask_stride_b,
-                   float scale, int L, DecodeSplit rule, __nv_bfloat16* __restrict__ out,
-                   const int* __restrict__ len_dev, StepArgs st, int cl, float* part) {
+                   const __nv_bfloat16* mask, long long mask_stride_b,
+                   float scale, int L, DecodeSplit rule, __nv_bfloat16* out,
+                   const int* len_dev, StepArgs st, int cl, float* part) {
   constexpr int D = DPL * kLanesPerRow;
   constexpr int kV = DPL / 8;                               // 16-byte pieces of K (and of V) per lane
   constexpr int kStepBytes = kAttnThreads * 2 * kV * 16;    // one row step of the block
@@ -265,12 +268,12 @@ decode_attn_kernel(const __nv_bfloat16* __restrict__ q, long long q_stride_b,
   Angles ang;
   int pos = -1;                      // the row that this step brings
   if constexpr (kStep) {
-    pos = __ldg(st.pos_dev);
+    pos = *st.pos_dev;
 #pragma unroll
     for (int g = 0; g < G; ++g) qx[g] = load_halves<D>(row + static_cast<long long>(kvh * G + g) * D, sub);
     if (st.q_w) qw = load_halves<D>(st.q_w, sub);
   }
-  if (len_dev) L = max(0, min(L, __ldg(len_dev)));
+  if (len_dev) L = max(0, min(L, *len_dev));
   const int splits = rule.bound(L);                          // the last of them may have no rows
   const int chunk = rule.chunk(L);
   const int t_begin = min(L, split * chunk);
