@@ -16,8 +16,8 @@
 // merge through one another's shared memory, each block a share of the columns; long caches of
 // few pairs take several clusters a pair and a kernel that adds what they leave in a workspace.
 //
-// A decode step (kStep) hands over the raw projections: every block normalises and rotates the query
-// heads of its group itself (8 lanes a head, as many as the rows need anyway), and the one
+// A decode step (kStep) hands over the raw projections: the first warp of every block normalises and
+// rotates the query heads of its group (8 lanes a head), and the block
 // whose rows include the new token does so for its key, writes key and value into the cache
 // and takes the row behind all others, from shared memory.
 //
@@ -255,6 +255,7 @@ decode_attn_kernel(const __nv_bfloat16* q, long long q_stride_b,
   __shared__ float s_m[16][G], s_l[16][G];
   __shared__ float s_part[G * D + 2 * G];                   // this block's sums, then its maxima and sums of weights
   __shared__ uint4 s_new[2 * kV][kStep ? kLanesPerRow : 1];
+  __shared__ uint4 s_q[G][kStep ? D / 8 : 1];               // the rotated query heads
 
   griddep_wait();
   griddep_launch_dependents();
@@ -264,14 +265,15 @@ decode_attn_kernel(const __nv_bfloat16* q, long long q_stride_b,
   const int rgrp = lane >> 3;        // which of the warp's 4 concurrent rows
   // all that a step needs besides the cache is asked for before the first rows, whose copies end the reach of a load
   const __nv_bfloat16* row = q + b * q_stride_b;
-  Halves qx[G], qw = {};
+  Halves qx, qw = {};
   Angles ang;
   int pos = -1;                      // the row that this step brings
   if constexpr (kStep) {
     pos = *st.pos_dev;
-#pragma unroll
-    for (int g = 0; g < G; ++g) qx[g] = load_halves<D>(row + static_cast<long long>(kvh * G + g) * D, sub);
-    if (st.q_w) qw = load_halves<D>(st.q_w, sub);
+    if (warp == 0) {                 // a head per lane group
+      qx = load_halves<D>(row + static_cast<long long>(kvh * G + min(rgrp, G - 1)) * D, sub);
+      if (st.q_w) qw = load_halves<D>(st.q_w, sub);
+    }
   }
   if (len_dev) L = max(0, min(L, *len_dev));
   const int splits = rule.bound(L);                          // the last of them may have no rows
@@ -282,7 +284,8 @@ decode_attn_kernel(const __nv_bfloat16* q, long long q_stride_b,
   if constexpr (kStep) {
     if (pos < 0 || pos >= st.capacity) pos = -1;
     owner = pos >= 0 && (pos < L ? pos >= t_begin && pos < t_end && warp == (((pos - t_begin) >> 2) & 3) : split + warp == 0);
-    load_angles<D>(ang, st.cos_t + static_cast<long long>(max(pos, 0)) * D, st.sin_t + static_cast<long long>(max(pos, 0)) * D, sub);
+    if (warp == 0 || owner)
+      load_angles<D>(ang, st.cos_t + static_cast<long long>(max(pos, 0)) * D, st.sin_t + static_cast<long long>(max(pos, 0)) * D, sub);
   }
 
   float m_run[G], l_run[G], acc[G][DPL];
@@ -319,28 +322,15 @@ decode_attn_kernel(const __nv_bfloat16* q, long long q_stride_b,
 #pragma unroll
   for (int s0 = 0; s0 < kStages - 1; ++s0) issue(s0);
 
-  // query fragments of the G heads, pre-scaled
-  float qf[G][DPL];
+  if constexpr (kStep) {
+    if (warp == 0) {
+      uint4 w[kV];
+      norm_rope<D>(qx, qw, st.q_w != nullptr, ang, st.eps, pos >= 0, sub, w);
+      if (rgrp < G) {
 #pragma unroll
-  for (int g = 0; g < G; ++g) {
-    uint4 w[kV];
-    if constexpr (kStep) {
-      norm_rope<D>(qx[g], qw, st.q_w != nullptr, ang, st.eps, pos >= 0, sub, w);
-    } else {
-#pragma unroll
-      for (int i = 0; i < kV; ++i) w[i] = *reinterpret_cast<const uint4*>(row + static_cast<long long>(kvh * G + g) * D + i * 64 + sub * 8);
-    }
-#pragma unroll
-    for (int i = 0; i < kV; ++i) {
-      const uint32_t ww[4] = {w[i].x, w[i].y, w[i].z, w[i].w};
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        qf[g][i * 8 + 2 * e] = lo_f(ww[e]) * scale;
-        qf[g][i * 8 + 2 * e + 1] = hi_f(ww[e]) * scale;
+        for (int i = 0; i < kV; ++i) s_q[rgrp][i * 8 + sub] = w[i];
       }
     }
-  }
-  if constexpr (kStep) {
     if (owner) {                       // the new row into the cache; its own step comes behind all others'
       uint4 w[kV];
       Halves kw = {};
@@ -358,6 +348,26 @@ decode_attn_kernel(const __nv_bfloat16* q, long long q_stride_b,
           *reinterpret_cast<uint4*>(st.k_cache + at) = w[i];
           *reinterpret_cast<uint4*>(st.v_cache + at) = x;
         }
+      }
+    }
+    __syncthreads();
+  }
+
+  // query fragments of the G heads, pre-scaled
+  float qf[G][DPL];
+#pragma unroll
+  for (int g = 0; g < G; ++g) {
+    uint4 w[kV];
+#pragma unroll
+    for (int i = 0; i < kV; ++i)
+      w[i] = kStep ? s_q[g][i * 8 + sub] : *reinterpret_cast<const uint4*>(row + static_cast<long long>(kvh * G + g) * D + i * 64 + sub * 8);
+#pragma unroll
+    for (int i = 0; i < kV; ++i) {
+      const uint32_t ww[4] = {w[i].x, w[i].y, w[i].z, w[i].w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        qf[g][i * 8 + 2 * e] = lo_f(ww[e]) * scale;
+        qf[g][i * 8 + 2 * e + 1] = hi_f(ww[e]) * scale;
       }
     }
   }
