@@ -818,11 +818,14 @@ def all_plain(wanted) -> bool:
 
 
 def complexity_block(tensors, x_lo: Optional[torch.Tensor], mu: torch.Tensor, routing: Routing, cos: torch.Tensor,
-                     sin: torch.Tensor, sizes, constants):
+                     sin: torch.Tensor, sizes, constants, want_qkv: bool):
     """One block of a prompt (cd_complexity_block).  `tensors`, checked by the caller (`all_plain`): hidden states, ln1, ln2,
     w_qkv, w_mu, w_o, packed gate/up of the routed and of the shared experts, their down weights, mu_proj, mu and, with Q/K
     norm, its two weights.  `sizes`: B, S, H, hq, hkv, D, E, I, I_s, block_n of the two packed layouts; `constants`: the three
-    eps, mu_min, mu_max and the clamp's bounds.  Returns (out, out_lo, mu, qkv), rows of tokens."""
+    eps, mu_min, mu_max and the clamp's bounds.  Returns (out, out_lo, mu, qkv or None), rows of tokens.
+
+    Intermediate results that are not alive at the same time share their memory, as they do where a caller makes the launches
+    one by one and gives each back."""
     lib = _lib.load()
     B, S, H, hq, hkv, D, E, I, I_s, bn, bn_s = sizes
     T, N = B * S, (hq + 2 * hkv) * D
@@ -842,22 +845,24 @@ def complexity_block(tensors, x_lo: Optional[torch.Tensor], mu: torch.Tensor, ro
         raise RuntimeError("cos/sin tables too short for the requested positions")
     _split_k_auto(x.view(T, H))
     new = functools.partial(torch.empty, dtype=BF16, device=x.device)
-    out, out_lo, mu_out, qkv = new(T, H), new(T, H), new(T, H), new(T, N)
-    # intermediate results, each on a boundary of its own
-    widths = (H, hq * D, H, H, H, I, I_s)
-    at, places = 0, []
-    for w in widths:
-        places.append(at)
-        at += -(-T * w // 128) * 128
-    scratch = new(at)
+    out, out_lo, mu_out = new(T, H), new(T, H), new(T, H)
+    qkv = new(T, N) if want_qkv else None
+    pad = lambda w: -(-T * w // 128) * 128                # elements of a [T, w] result, the next one on a boundary of its own
+    front = 0 if want_qkv else pad(N)                     # q, k, v; behind them the normalised rows, then what attention gives
+    attn = max(front, 2 * pad(H))                         # the stream behind attention lies in front of it, in their place
+    x_sorted = 2 * pad(H)                                 # behind that the rows of the experts
+    h_r = x_sorted + pad(H)
+    h_s = h_r + pad(I)
+    scratch = new(max(front + pad(H), attn + pad(hq * D), h_s + pad(I_s)))
     base = scratch.data_ptr()
-    normed, attn, h1, h1_lo, x_sorted, h_r, h_s = (base + 2 * a for a in places)
+    normed, attn, h1, h1_lo, x_sorted, h_r, h_s = (base + 2 * a for a in (front, attn, 0, pad(H), x_sorted, h_r, h_s))
+    qkv_at = qkv.data_ptr() if want_qkv else base
     p = [t.data_ptr() for t in tensors]
     q_norm, k_norm = (p[12], p[13]) if len(p) > 12 else (None, None)
     eps1, eps2, eps_qk, mu_min, mu_max, clamp_lo, clamp_hi = constants
     block = _lib.Block(p[0], _ptr(x_lo), mu.data_ptr(), p[1], p[2], p[3], p[4], q_norm, k_norm, p[5], p[6], p[7], p[8], p[9],
                        p[10], p[11], cos.data_ptr(), sin.data_ptr(), routing.offsets.data_ptr(), routing.perm.data_ptr(),
-                       routing.inv_perm.data_ptr(), normed, qkv.data_ptr(), attn, h1, h1_lo, x_sorted, h_r, h_s,
+                       routing.inv_perm.data_ptr(), normed, qkv_at, attn, h1, h1_lo, x_sorted, h_r, h_s,
                        out.data_ptr(), out_lo.data_ptr(), mu_out.data_ptr(), eps1, eps2, eps_qk, float(D) ** -0.5, mu_min,
                        mu_max, clamp_lo, clamp_hi, B, S, H, hq, hkv, D, E, I, I_s, bn, bn_s)
     _lib.check(lib.cd_complexity_block(ctypes.byref(block), _stream()), "cd_complexity_block")

@@ -69,3 +69,24 @@ def test_general_route_for_all_else(monkeypatch):
     model.layers[1].self_attn.o_proj.weight = torch.nn.Parameter(torch.zeros(256, 128, dtype=torch.bfloat16, device="cuda"))
     with torch.no_grad(), pytest.raises(RuntimeError):
         model(ids)
+
+
+@pytest.mark.parametrize("cached", [False, True])
+@pytest.mark.parametrize("hidden,inner,heads,kv,experts,T", [(1024, 2816, 8, 4, 2, 3000), (512, 2048, 8, 8, 1, 4001)])
+def test_no_more_memory_than_launch_by_launch(hidden, inner, heads, kv, experts, T, cached, monkeypatch):
+    """What a block holds at its fullest: intermediate results that do not live at the same time share their memory."""
+    from complexity_deep_b200.core.layer import TransformerBlock
+    model = _model(hidden, inner, heads, kv, experts)
+    ids = torch.randint(0, 1000, (1, T), device="cuda")
+    native, peaks = TransformerBlock._forward_native, []
+    for run in (native, lambda self, *a: None):
+        monkeypatch.setattr(TransformerBlock, "_forward_native", run)
+        with torch.no_grad():
+            model(ids, use_cache=cached)                   # weights are packed, tables made
+            torch.cuda.synchronize()
+            torch.cuda.reset_peak_memory_stats()
+            base = torch.cuda.memory_allocated()
+            out = model(ids, use_cache=cached)
+            peaks.append(torch.cuda.max_memory_allocated() - base)
+            del out
+    assert peaks[0] <= peaks[1] + 16 * 512                 # an allocation is rounded up to 512 bytes
