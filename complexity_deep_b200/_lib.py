@@ -169,6 +169,7 @@ SIGNATURES = {
     "cd_window_attention_rows": _WINDOW_FN,
     "cd_window_attention_decode_workspace_bytes": (c_size_t, [ctypes.POINTER(WindowAttn)]),
     "cd_window_attention_decode": (c_int, [ctypes.POINTER(WindowAttn), c_void_p, c_size_t, c_int, c_void_p]),
+    "cd_window_attention_decode_launches": (c_int, [ctypes.POINTER(WindowAttn), c_int]),
     "cd_window_attention_prefill_supported": (c_int, [ctypes.POINTER(WindowAttn)]),
     "cd_window_attention_prefill": (c_int, [ctypes.POINTER(WindowAttn), c_void_p]),
     "cd_window_attention_prefill_workspace_bytes": (c_size_t, [ctypes.POINTER(WindowAttn)]),

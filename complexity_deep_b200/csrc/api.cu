@@ -762,6 +762,10 @@ size_t cd_window_attention_decode_workspace_bytes(const cd_window_attn* a) {
   return window_args_ok(a) == CD_OK && window_decode_supported(*a) ? window_decode_workspace_bytes(*a) : 0;
 }
 
+int cd_window_attention_decode_launches(const cd_window_attn* a, int fp32) {
+  return window_args_ok(a) == CD_OK && window_decode_supported(*a) ? window_decode_launches(*a, fp32) : 0;
+}
+
 int cd_window_attention_decode(const cd_window_attn* a, void* ws, size_t ws_bytes, int fp32, void* stream) {
   if (window_args_ok(a) != CD_OK || !a->r1 || !a->r2 || !a->talk || !a->ring_k || !a->ring_v || !a->out ||
       a->normed || a->S != 1)

@@ -450,6 +450,27 @@ cudaError_t launch_values(const DecodeParams& p, dim3 grid, cudaStream_t st) {
   return cudaLaunchKernelEx(&cfg, kern, p);
 }
 
+// Blocks of one wave may make the mixed weights of their heads and keys themselves: each head group's blocks again, H exponentials a
+// key and block, but a launch and the weights' way through memory less. Both sides in us, as fitted to 277 calls on one B200 (6 to
+// 128 heads of 64 and 128, one to eight query heads a key head, 1 to 32 sequences, 516 to 4 100 keys): the kernel between the two
+// takes 4 + 0.024 H^2 (its blocks see all heads of 64 keys), mixing in the blocks `head_us` a head and 256 keys (at least one round
+// of the threads; another round of kMixKeys waits for the values in between). bf16, with the kernel / without: 16 heads on 8, 4
+// sequences of 1 028 keys 24.0 / 19.3, one of 4 100 24.1 / 28.1; 32 heads of their own keys, one of 516 35 / 15.5. fp32: 8 on 4,
+// 32 of 516 32.0 / 27.9; 16 of their own, 8 of 516 28.0 / 24.6, one of 4 100 28.3 / 34.1; 128 of their own, 2 of 2 052 346 / 495.
+// Fewer than 24 heads of their own keys in fp32 and clusters of eight on every SM are an exception: two such blocks fill an SM,
+// and the clusters wait for room (8 heads, 4 sequences of 516 keys 17.6 / 20.3). Over the 277 calls the rule is 0.05 us from the
+// better side on average and 2.8 (of 37) at most. Steps of Pimezen, us, with / without: 1024 wide, 32 sequences 484 / 477, one
+// 319 / 308; 2048 wide, 16 sequences of 300 keys 641 / 587.
+bool mix_beside_values(const WindowAttnParams& a, int splits, int size) {
+  const int rep = rep_block(a), keys = (a.keep + a.window + splits - 1) / splits;
+  const long long blocks = static_cast<long long>(splits) * a.G * ((a.H / a.G + rep - 1) / rep) * a.B, sms = current_sm_count();
+  if (blocks > values_per_sm(size, rep) * sms) return false;
+  if (size == 4 && rep == 1 && a.H < 24 && splits == kMostSplits && blocks > sms) return false;
+  const double head_us = size == 2 ? (rep == 1 ? 0.05 : 0.35) : rep == 1 ? 0.3 * static_cast<double>((blocks + sms - 1) / sms) : 0.1;
+  const double rounds = (keys > 256 ? keys / 256.0 : 1.0) + (keys > kMixKeys ? 0.5 : 0.0);
+  return rounds * a.H * head_us <= 4.0 + 0.024 * a.H * a.H;
+}
+
 template <typename T, int REP>
 cudaError_t launch_both(const DecodeParams& p, cudaStream_t st) {
   const int rep = p.a.H / p.a.G;
@@ -458,12 +479,10 @@ cudaError_t launch_both(const DecodeParams& p, cudaStream_t st) {
                   : p.a.dp <= 128 ? launch_scores<T, REP, 2>(p, grid, st)
                                   : launch_scores<T, REP, 4>(p, grid, st);
   if (e != cudaSuccess) return e;
-  // Blocks of one wave make the mixed weights of their heads and keys themselves: each key head's blocks again, H exponentials a
-  // key, but a launch and the weights' way through memory less. Steps of Pimezen, us, with the mixing kernel / without: 1024
-  // wide, 32 sequences 484 / 477, 1 319 / 308; 2048 wide, 16 sequences of 300 keys 641 / 587, 64 of 1 028 (two waves) 1 666 / 1 760.
   const long long blocks = static_cast<long long>(grid.x) * grid.y * grid.z, sms = current_sm_count();
   constexpr int kAhead = REP <= 2 && sizeof(T) == 2 ? 6 : 4;
-  if (blocks <= values_per_sm(sizeof(T), REP) * sms) return launch_values<T, REP, kAhead, values_per_sm(sizeof(T), REP), true>(p, grid, st);
+  if (mix_beside_values(p.a, p.splits, sizeof(T)))
+    return launch_values<T, REP, kAhead, values_per_sm(sizeof(T), REP), true>(p, grid, st);
   const int mix_bytes = p.a.H * (2 + kMixBlock) * static_cast<int>(sizeof(float));
   e = cudaFuncSetAttribute(window_decode_mix_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, mix_bytes);
   if (e != cudaSuccess) return e;
@@ -497,6 +516,11 @@ bool window_decode_supported(const WindowAttnParams& a) {
 
 size_t window_decode_workspace_bytes(const WindowAttnParams& a) {
   return static_cast<size_t>(a.B) * a.H * (a.keep + a.window + 2 * kMostSplits) * sizeof(float);    // of either storage type
+}
+
+int window_decode_launches(const WindowAttnParams& a, int fp32) {
+  const int size = fp32 ? 4 : 2;
+  return a.B == 0 ? 0 : mix_beside_values(a, choose_splits(a, size), size) ? 2 : 3;
 }
 
 cudaError_t launch_window_decode(const WindowAttnParams& a, void* ws, int fp32, cudaStream_t st) {

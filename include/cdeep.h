@@ -509,6 +509,8 @@ int cd_window_attention_norm(const cd_window_attn* h_args, int fp32, void* strea
 size_t cd_window_attention_decode_workspace_bytes(const cd_window_attn* h_args);
 int cd_window_attention_decode(const cd_window_attn* h_args, void* workspace, size_t bytes, int fp32,
                                void* stream);
+/* How many kernels that call launches. */
+int cd_window_attention_decode_launches(const cd_window_attn* h_args, int fp32);
 /* One query per thread-block cluster (normed = 1, any S): keys of the call from k / v, earlier ones
  * from the ring.  cd_window_attention_supported: the scores of a query fit in a cluster. */
 int cd_window_attention_supported(const cd_window_attn* h_args);
