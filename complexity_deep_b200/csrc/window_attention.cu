@@ -1,6 +1,6 @@
 // Sliding-window attention with kept first tokens, distance bias and head mixing: the per-head
-// norm, the ring append, and the kernel that handles one query per thread-block cluster.  The
-// latter serves prompts in 32-bit storage and head layouts that the kernels of
+// norm, the ring append, and the kernels that handle one query, or four behind one another, per
+// thread-block cluster.  These serve prompts in 32-bit storage and head layouts that the kernels of
 // window_attention_prefill.cu (prompts in bf16) and window_attention_decode.cu do not take.
 #include <cfloat>
 #include <type_traits>
@@ -553,7 +553,12 @@ cudaError_t launch_tile_hm(const WindowAttnParams& p, int cl, int cap, size_t by
 }
 
 // Tiles of kTileQ queries, where what single queries would read is worth the longer chain of a tile (keys in pairs, values one
-// by one, for four queries) and two blocks fit an SM. us, fp32, one query per cluster / tiles: 8 heads of 128 on 4, window 512:
+// by one, for four queries) and two blocks fit an SM. What the lines stand for:
+//   all        what one query per cluster reads through L2. Up to 160 MB, some 20 us, a call's time is that of its blocks' chains.
+//   per_query  up to 240 MB the reads only win where a query has 400 KB of them: with fewer or narrower key heads fewer threads
+//              have value columns of their own, and a tile's chain over the keys is the longer for it.
+//   seen       keys of a query in the middle of the prompt. With less than 128 a tile's 256 threads, two keys each, stand idle.
+// us, fp32, one query per cluster / tiles: 8 heads of 128 on 4, window 512:
 // 145 tokens (72 keys on average, 43 MB) 33 / 61, 300 (184 MB) 84 / 54, 800 265 / 119, 2 x 1 000 635 / 282; 145 tokens behind
 // 700 107 / 87; 16 heads on 8, window 1 024: 4 x 150 (75 keys, 368 MB) 184 / 269, 300 190 / 162, 2 x 1 000 2 657 / 1 276; 6
 // heads of 48 and 64 on 2, window 300: 4 x 150 behind 700 (161 MB, 270 KB a query) 74 / 77, 800 (200 MB) 64 / 66, 2 x 1 000 (250 MB)
@@ -567,7 +572,7 @@ bool launch_tiles(const WindowAttnParams& p, cudaStream_t st, cudaError_t& e) {
   const long long per_query = seen * p.G * (p.dp + p.vp) * static_cast<long long>(sizeof(T)), all = per_query * p.S * p.B;
   if (p.H > 32 || seen < 128 || all < 160000000ll || (all < 240000000ll && per_query < 400000ll)) return false;
   int cl = 1;
-  while (cl < 8 && (tiles * cl < 2 * 148 || bytes(cl) > kMaxDynSmem / 2)) cl *= 2;
+  while (cl < 8 && (tiles * cl < 2LL * current_sm_count() || bytes(cl) > kMaxDynSmem / 2)) cl *= 2;
   if (bytes(cl) > kMaxDynSmem / 2) return false;
   const int cap = (n_max + cl - 1) / cl;
   e = p.H <= 8 ? launch_tile_hm<T, 8>(p, cl, cap, bytes(cl), st)
