@@ -504,7 +504,7 @@ window_prefill_kernel(const WindowAttnParams p, const float* lse, int* status) {
     __syncthreads();                        // queries (when staged), talk, r1, r2, sStat are written
   } else {
     float m_run[kUnits][2], l_run[kUnits][2];
-  #pragma unroll
+#pragma unroll
     for (int u = 0; u < kUnits; ++u) {
       m_run[u][0] = m_run[u][1] = kMasked;
       l_run[u][0] = l_run[u][1] = 0.f;
@@ -517,19 +517,19 @@ window_prefill_kernel(const WindowAttnParams p, const float* lse, int* status) {
       __syncthreads();                        // tile t is there; everybody is done with tile t - 1
       const bf16* kbuf = (t & 1) ? sV : sK;
       load_tile(t + 1, (t & 1) ? sK : sV, ldk, new_k, ring_k, G * dp, &bars[(t + 1) & 1]);
-  #pragma unroll
+#pragma unroll
       for (int k0 = 0; k0 < KT; k0 += 16) {
         float s[kUnits][2][4];
         scores(t, k0, kbuf, s);
-  #pragma unroll
+#pragma unroll
         for (int u = 0; u < kUnits; ++u) {
           if (!kExact && (warp * kUnits + u) / MB >= H) break;
-  #pragma unroll
+#pragma unroll
           for (int r = 0; r < 2; ++r) {
             const float m = fmaxf(fmaxf(m_run[u][r], fmaxf(s[u][0][2 * r], s[u][0][2 * r + 1])),
                                   fmaxf(s[u][1][2 * r], s[u][1][2 * r + 1]));
             float l = l_run[u][r] * exp2_approx(m_run[u][r] - m);
-  #pragma unroll
+#pragma unroll
             for (int nt = 0; nt < 2; ++nt) l += exp2_approx(s[u][nt][2 * r] - m) + exp2_approx(s[u][nt][2 * r + 1] - m);
             m_run[u][r] = m;
             l_run[u][r] = l;
@@ -538,14 +538,14 @@ window_prefill_kernel(const WindowAttnParams p, const float* lse, int* status) {
       }
     }
     // merge the four lanes of a row (a lane that saw only masked keys drops out: exp2 of a huge negative)
-  #pragma unroll
+#pragma unroll
     for (int u = 0; u < kUnits; ++u) {
       const int unit = warp * kUnits + u, h = unit / MB, mb = unit - h * MB;
       if (!kExact && h >= H) break;
-  #pragma unroll
+#pragma unroll
       for (int r = 0; r < 2; ++r) {
         float m = m_run[u][r], l = l_run[u][r];
-  #pragma unroll
+#pragma unroll
         for (int x = 1; x < 4; x <<= 1) {
           const float mo = __shfl_xor_sync(0xffffffffu, m, x), lo = __shfl_xor_sync(0xffffffffu, l, x);
           const float mn = fmaxf(m, mo);
