@@ -1,7 +1,7 @@
 """Window attention in tiles of four queries (cd_window_attention_rows where what they read is worth it) against 64 bits: rows that
-are no multiple of four, one to eight blocks a tile, head counts on both sides of what a thread mixes (8, 16, 32), two query
-heads and more (and an odd number) a key head, kept tokens, earlier keys from the ring (the last
-case is small: one query at a time).
+are no multiple of four, one to eight blocks a tile (eight: 145 tokens behind 700), head counts on both sides of what a thread mixes
+(8, 16, 32), two query heads and more (and an odd number) a key head, kept tokens, earlier keys from the ring. Three cases go one
+query at a time: few bytes (145 tokens, 60 tokens), or more shared memory than two blocks on an SM have (32 heads of 128).
 
 fp32 storage: sums of at most `dim` and `window` fp32 products and CUDA's expf and log1pf, 2e-6 of the row's largest value; bf16
 storage adds its rounding of the result, 2^-8 of the value."""
@@ -63,7 +63,7 @@ def _run(proj, q, k, v, ring_k, ring_v, r1, r2, talk, window, keep, pos0):
 @pytest.mark.parametrize("B,S,H,G,dim,vdim,window,keep,pos0", [
     (16, 301, 6, 2, 48, 48, 300, 5, 0), (4, 1201, 12, 4, 32, 32, 130, 3, 0), (80, 5, 32, 8, 128, 128, 150, 2, 160),
     (2, 150, 16, 16, 128, 128, 200, 7, 230), (16, 130, 5, 5, 64, 32, 150, 1, 90), (2, 509, 8, 4, 128, 128, 512, 4, 0),
-    (2, 160, 32, 2, 128, 128, 700, 0, 650), (80, 151, 20, 2, 16, 16, 90, 130, 128),
+    (2, 160, 32, 2, 128, 128, 700, 0, 650), (1, 145, 8, 4, 128, 128, 512, 4, 700), (1, 145, 8, 4, 128, 128, 512, 4, 0), (80, 151, 20, 2, 16, 16, 90, 130, 128),
     (3, 60, 8, 4, 48, 64, 2, 4, 9)])
 def test_tiles(B, S, H, G, dim, vdim, window, keep, pos0, dtype):
     proj, *x = _inputs(B, S, H, G, dim, vdim, window, keep, dtype, S + H)
