@@ -34,23 +34,23 @@ struct DecodeSplit {
 };
 
 // More pairs than two blocks of each fit the device at once: c blocks a pair (a cluster; active[c - 1] of which fit) take as many waves
-// as their number asks for, each as long as a block's rows and some 170 more (its start, the query, the merge); the last wave is
-// shorter only down to 60 % of the others, below which its blocks have bandwidth to spare and are chains of their own.
+// as their number asks for, each as long as a block's rows and some 100 more (its start, the query, the merge); the last wave is
+// shorter only down to 65 % of the others, below which its blocks have bandwidth to spare and are chains of their own.
 inline DecodeSplit split_of_waves(long long pairs, const short* active) {
   DecodeSplit r;
   double waves[5];
   for (int c = 1; c <= 5; ++c) {
     const double full = static_cast<double>(pairs / active[c - 1]), last = static_cast<double>(pairs % active[c - 1]) / active[c - 1];
-    waves[c - 1] = full + (last > 0 && last < 0.6 ? 0.6 : last);
+    waves[c - 1] = full + (last > 0 && last < 0.65 ? 0.65 : last);
   }
   r.waves = r.most = 1;
   for (int& from : r.more_from) from = 1 << 30;
-  // time of L rows with c blocks: waves (L / c + 170); the next c is the first to undercut the one before
+  // time of L rows with c blocks: waves (L / c + 100); the next c is the first to undercut the one before
   for (int cur = 1; cur < 5;) {
     int next = 0;
     double at = 1e9;
     for (int c = cur + 1; c <= 5; ++c) {
-      const double gain = waves[cur - 1] / cur - waves[c - 1] / c, cost = 170 * (waves[c - 1] - waves[cur - 1]);
+      const double gain = waves[cur - 1] / cur - waves[c - 1] / c, cost = 100 * (waves[c - 1] - waves[cur - 1]);
       if (gain > 0 && cost / gain < at) next = c, at = cost / gain;
     }
     if (!next || at > 60000) break;
