@@ -50,7 +50,6 @@ __host__ __device__ constexpr int blocks_per_sm(int G, int D) { return G * D > 3
 // Clusters of 1 .. 16 blocks that a B200 holds at a time (cudaOccupancyMaxActiveClusters: a cluster lies within one GPC,
 // so the SMs that are left over in each go unused), by blocks per SM. Other devices take other sizes better; which of more than
 // eight blocks they take at all they are asked (allow_clusters).
-constexpr int kSms = 148;
 constexpr short kActive[3][kMaxSplits] = {{296, 148, 93, 71, 56, 45, 37, 33, 30, 26, 21, 21, 17, 14, 14, 14},
                                           {444, 222, 142, 104, 82, 71, 56, 48, 45, 41, 31, 31, 28, 24, 24, 21},
                                           {592, 296, 187, 142, 112, 93, 78, 71, 60, 56, 45, 42, 38, 35, 31, 31}};
@@ -85,7 +84,7 @@ inline DecodeSplit choose_split(int B, int hkv, int G, int D) {
     r.large_from = r.most * (pairs > 16 ? 64 : 48);
     const long long clusters = active[kPortable - 1] / pairs;
     r.many = kPortable * static_cast<int>(clusters < kMaxClusters ? clusters : kMaxClusters);
-    if (r.many > r.most) r.many_from = r.most == kMaxSplits ? 4096 : (r.most > kPortable ? 64 : 128) * D;
+    if (r.many > r.most) r.many_from = r.most == kMaxSplits ? 2048 + 32 * D : (r.most > kPortable ? 64 : 128) * D;
     return r;
   }
   return split_of_waves(pairs, active);
@@ -136,7 +135,8 @@ __device__ __forceinline__ Sums add_sums(const Sums (&in)[N]) {
   }
   return r;
 }
-__device__ __forceinline__ __nv_bfloat16 quotient(const Sums& s) { return __float2bfloat16_rn(s.l == 0.f ? 0.f : s.a / s.l); }   // no visible row: 0; a NaN score stays one
+// no visible row: 0; a NaN score stays one
+__device__ __forceinline__ __nv_bfloat16 quotient(const Sums& s) { return __float2bfloat16_rn(s.l == 0.f ? 0.f : s.a / s.l); }
 
 // What a decode step brings besides the query: norm weights (or none), rotation tables, where the new row goes.
 struct StepArgs {

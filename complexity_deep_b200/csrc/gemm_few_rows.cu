@@ -442,7 +442,8 @@ cudaError_t launch_warps(const FewParams& p, cudaStream_t stream) {
     if (p.g.M > 32 && p.g.num_groups > 1) return launch_few<EPI, MT, 4, WK, kGroups>(p, stream);
     if (p.g.M > 48) return launch_few<EPI, MT, 8, 8, kWhole, 2>(p, stream);
     if (p.g.M > 32) return launch_few<EPI, MT, 6, WK>(p, stream);
-    return p.g.M <= 8 ? launch_few<EPI, MT, 1, WK>(p, stream) : p.g.M <= 16 ? launch_few<EPI, MT, 2, WK>(p, stream) : launch_few<EPI, MT, 4, WK>(p, stream);
+    if (p.g.M > 16) return launch_few<EPI, MT, 4, WK>(p, stream);
+    return p.g.M <= 8 ? launch_few<EPI, MT, 1, WK>(p, stream) : launch_few<EPI, MT, 2, WK>(p, stream);
   } else {
     if (p.g.M <= 8) return launch_few<EPI, MT, 1, WK>(p, stream);
     if (p.g.num_groups > 1 || p.tiles2 > 0) {
@@ -450,7 +451,8 @@ cudaError_t launch_warps(const FewParams& p, cudaStream_t stream) {
       if (MT == 2 && blocks > p.sms * 16LL / WK) return launch_few<EPI, MT, 4, WK, kManyGroups>(p, stream);
       return launch_few<EPI, MT, 4, WK, kGroups>(p, stream);
     }
-    return p.g.M <= 16 ? launch_few<EPI, MT, 2, WK>(p, stream) : p.g.M <= 32 ? launch_few<EPI, MT, 4, WK>(p, stream) : launch_few<EPI, MT, 8, WK>(p, stream);
+    if (p.g.M > 32) return launch_few<EPI, MT, 8, WK>(p, stream);
+    return p.g.M <= 16 ? launch_few<EPI, MT, 2, WK>(p, stream) : launch_few<EPI, MT, 4, WK>(p, stream);
   }
 }
 // More blocks than the two of eight warps that an SM holds: four warps each and four on an SM, since a block is then
