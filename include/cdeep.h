@@ -511,7 +511,7 @@ int cd_window_attention_decode(const cd_window_attn* h_args, void* workspace, si
                                void* stream);
 /* How many kernels that call launches. */
 int cd_window_attention_decode_launches(const cd_window_attn* h_args, int fp32);
-/* One query per thread-block cluster (normed = 1, any S): keys of the call from k / v, earlier ones
+/* One query, or four behind one another, per thread-block cluster (normed = 1, any S): keys of the call from k / v, earlier ones
  * from the ring.  cd_window_attention_supported: the scores of a query fit in a cluster. */
 int cd_window_attention_supported(const cd_window_attn* h_args);
 int cd_window_attention_rows(const cd_window_attn* h_args, int fp32, void* stream);
